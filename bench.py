@@ -207,7 +207,7 @@ def hx_roofline(torch, device, w2, launches=10):
         prec = _lib.C128 if name == 'c128' else _lib.C64
         tile = H.get_tile(prec)
         label = ('direct' if tile == _lib.TILE_DIRECT else
-                 f'TMA tile {tile}' if tile >= _lib.TILE_TMA0 else f'staged tile {tile}')
+                 f'tile {tile}')
         out[name] = {'ms': t * 1e3, 'GBps': byts / t / 1e9, 'bytes': byts, 'launches': launches,
                      'kernel': label,
                      'tuner_GBps': {str(k): byts / v / 1e9 for k, v in secs.items()}}

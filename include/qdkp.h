@@ -152,17 +152,15 @@ int qdkp_apply_folded_noalloc(const qdkp_operator* op, const void* X, int64_t ld
 
 /*
  * H.X kernel selection (no counterpart in the reference, which multiplies an assembled CSR).
- * Eight-band operators are applied by a staged kernel: a CTA owns a (y, z) tile of sites and a
- * few columns, walks along x and keeps a ring of x planes in shared memory. Tiles 0..3 fill the
- * ring with cp.async (both precisions); tiles 4..11 (complex64 only) fill it with bulk tensor
- * copies (TMA) and give every thread two columns of a site; tiles 12..16 (complex64 only) do the
- * same with a producer warp and per-slot full/empty barriers, the record read from global
- * memory by the threads of its site. A block the tensor maps cannot
- * describe (odd leading dimension, a base not 16-byte aligned, fewer columns than a tile or a
- * grid smaller than a tile) falls back to a cp.async tile. The tile is chosen by a heuristic
- * unless set here or by qdkp_operator_tune; QDKP_TILE_DIRECT selects the unstaged
- * one-thread-per-(site, column) kernel (always used for 6- and 4-band slices). The choice is per
- * operator and precision.
+ * Eight- and six-band operators are applied by a marching kernel: a CTA owns a (y, z) tile of sites
+ * and a few columns and walks along x, one plane of the tile resident per shared-memory stage.
+ * Tiles 0..3 exist in both precisions, the further ones for complex64 only (a number past the
+ * built shapes takes shape 0). Planes are brought in by bulk tensor copies (TMA); a block the
+ * tensor maps cannot describe (odd complex64 leading dimension, a base not 16-byte aligned, fewer
+ * columns than a tile or a grid smaller than a tile) takes one shape fed by cp.async instead. The
+ * tile is chosen by a cost model unless set here or by qdkp_operator_tune; QDKP_TILE_DIRECT selects
+ * the unstaged one-thread-per-(site, column) kernel (always used for 4-band slices). The choice is
+ * per operator and precision.
  */
 enum { QDKP_TILE_AUTO = -1, QDKP_TILE_DIRECT = -2, QDKP_TILE_COUNT = 17 };
 int qdkp_operator_set_tile(qdkp_operator* op, int precision, int tile);
@@ -170,8 +168,8 @@ int qdkp_operator_get_tile(const qdkp_operator* op, int precision, int* tile);
 /* Autotuner: times every tile shape and the direct kernel on the caller's device blocks X, Y
  * (n x m, `precision`) with `reps` launches each, keeps the fastest for this operator and
  * precision, and writes the per-candidate seconds per launch to seconds[QDKP_TILE_COUNT + 1]
- * (may be NULL; index QDKP_TILE_COUNT is the direct kernel; -1 marks a candidate that does not
- * apply to this block or precision). Y is overwritten. Synchronous. */
+ * (may be NULL; index QDKP_TILE_COUNT is the direct kernel; -1 marks a tile that is not built for
+ * this precision or band count). Y is overwritten. Synchronous. */
 int qdkp_operator_tune(qdkp_operator* op, const void* X, int64_t ldx, void* Y, int64_t ldy,
                        int m, int precision, int reps, double* seconds, void* stream);
 

@@ -106,15 +106,11 @@ int qdkp_operator_create(int nx, int ny, int nz, double h, int n_bands, int flag
   op->n_sites = (int64_t)nx * ny * nz;
   op->h = h; op->n_bands = n_bands; op->flags = flags; op->device = device;
   const size_t bytes64 = (size_t)F_COUNT * op->n_sites * sizeof(double);
-  op->nzp = (nz + 3) / 4 * 4;
-  const size_t rec_doubles = record_doubles(nx, ny, op->nzp);
+  const size_t rec_values = record_values(op->n_sites);
   cudaError_t e = cudaMalloc(&op->fields64, bytes64);
-  if (e == cudaSuccess) e = cudaMalloc(&op->rec64, rec_doubles * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&op->rec32, rec_doubles * sizeof(float));
+  if (e == cudaSuccess) e = cudaMalloc(&op->rec64, rec_values * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&op->rec32, rec_values * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&op->nbmask, (size_t)op->n_sites * sizeof(unsigned));
-  // the z padding of the record stays zero
-  if (e == cudaSuccess) e = cudaMemset(op->rec64, 0, rec_doubles * sizeof(double));
-  if (e == cudaSuccess) e = cudaMemset(op->rec32, 0, rec_doubles * sizeof(float));
   if (e != cudaSuccess) {
     set_error(std::string("cudaMalloc of operator fields: ") + cudaGetErrorString(e));
     qdkp_operator_destroy(op);

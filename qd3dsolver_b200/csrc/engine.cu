@@ -698,7 +698,6 @@ int build_group(qdkp_engine* e, int g, const std::vector<int>& ids, int base, cu
       x.rec = pi ? (const void*)op->rec32 : (const void*)op->rec64;
       x.msk = op->nbmask; x.N = (int)op->n_sites;
       x.sx = op->ny * op->nz; x.sy = op->nz;
-      x.nzp = op->nzp; x.NP = op->nx * op->ny * op->nzp;
       x.tile0 = tile0[pi]; x.cb = apply_cb_weight(op);
       x.sigma = h.prm.sigma;
       x.shifted = h.prm.folded ? 1 : 0;

@@ -9,84 +9,97 @@
 //     (kp_pryor.py:430-454, central differences kp_confined.py:58-85),
 //   * twelve in-plane edge couplings: the symmetrised cross terms cross(g3, a, b)
 //     (kp_confined.py:146-183) feeding the imaginary part of R and all of S.
-// The block layout of those pieces is Pryor's table (kp_pryor.py:244-301) with the lower
-// triangle the adjoint of the upper (kp_pryor.py:216-241).
 //
-// Two kernels:
+// The uncoupled basis. Pryor's table (kp_pryor.py:244-301) is written in |J, m_J> states, in which
+// every k.p term mixes up to six bands with square-root factors. One constant unitary per site
+// takes them to |S>, |X>, |Y>, |Z> times spin (i |S>, so that the first-order terms are real):
+//   X+ = (x4 + t) / sqrt2, Y+ = -i (x4 - t) / sqrt2, t = (x2 + sqrt2 x7) / sqrt3,
+//   Z+ = -(sqrt2 x5 + x6) / sqrt3, S+ = i x0,
+//   X- = (q + p) / sqrt2,  Y- = -i (q - p) / sqrt2,  q = (sqrt2 x6 - x5) / sqrt3, p = -x3,
+//   Z- = (x7 - sqrt2 x2) / sqrt3, S- = i x1.
+// There every difference operator is the same real 4x4 matrix for both spins: a face along axis a
+// couples |a> with the weight -kp - 4 k2 and the other two with -kp + 2 k2, S with X, Y, Z by three
+// first-order weights, and an in-plane edge couples just the two states of its plane. Only the
+// spin-orbit term, local to the site, mixes the spins. A site and column takes 400 real
+// multiply-adds instead of 1046.
+//
+// Kernels:
 //   kp_record_kernel  once per operator (and per band-edge update): folds the 15 raw per-site
-//                     fields into a per-site record of stencil weights (local block, the three
-//                     "+" faces, the twelve edge weights) and a neighbour mask. The record is
-//                     kept in FP64 and FP32; the sign of the hole convention / negation is
-//                     folded in, so the apply kernel never branches on it.
-//   kp_apply_kernel   one thread per (site, column): loads the eight band components of the
-//                     site, its six faces and twelve edges (valence bands only) for that
-//                     column, and accumulates all eight output bands in registers. A "-" face
-//                     reads its weights from the neighbour's "+" face (the face weights are
-//                     symmetric; the first-order ones change sign). The edge terms of a plane
-//                     are summed with their scalar weights first and the constant band-mixing
-//                     matrix of that plane is applied once.
+//                     fields into a per-site record of stencil weights in that basis and a
+//                     neighbour mask; FP64 and FP32, the sign of the hole convention / negation
+//                     folded in.
+//   kp_march_kernel   a CTA owns a tile of (y, z) sites and a few columns and marches along x.
+//   kp_apply_kernel   one thread per (site, column), neighbours through L1/L2: small blocks,
+//                     four-band slices, and the batched engine.
 #include <cuda.h>   // CUtensorMap and its enums (the encoder is fetched from the runtime)
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "qdkp_common.cuh"
 
 namespace qdkp {
 
-// Record layout: entry k of site (ix, iy, iz) at rec[k * NP + (ix * ny + iy) * nzp + iz], with z
-// padded to nzp = a multiple of 4 (zeros in the padding) so that a z-run of a tile row starts on
-// a 16-byte boundary for the staged kernel's copies; NP = nx ny nzp.
+// Record layout, site-major: entry k of site s at rec[s * rec_stride<T>() + k]. A site's record is a
+// whole number of 16-byte words, and its pitch spreads the records of eight neighbouring sites over
+// all shared-memory banks.
 enum RecEntry {
-  K_A = 0,      // sign (Ec + 6 G / h^2): conduction diagonal
-  K_A2,         // sign (-P + Q): LH/HH diagonals of rows 2, 5
-  K_A3,         // sign (-P - Q): rows 3, 4
-  K_A6,         // sign (-P - Delta): split-off rows 6, 7
-  K_Q2,         // sign sqrt2 Q
-  K_RRE, K_RIM, K_SRE, K_SIM,
-  K_FACE = 9,   // per face f (x+, x-, y+, y-, z+, z-): K_FACE + 5f + {0 kp, 1 k2, 2 su, 3 svr, 4 svi}
-  K_EDGE = 39,  // per plane pl (xy, zx, zy) and edge e: K_EDGE + 4 pl + e
-  K_COUNT = 51
+  K_A = 0,        // sign (Ec + 6 G / h^2): S diagonal
+  K_DX, K_DY, K_DZ,   // X, Y, Z diagonals
+  K_XY, K_XZ, K_YZ,   // strain couplings of X, Y, Z
+  K_SO,           // sign Delta / 3: spin-orbit couplings
+  K_FYZ = 8,      // faces y+, y-, z+, z-: {along, across, cx, cy, cz} each
+  K_EZY = 28,     // zy edges e: sz = e & 1 ? -1 : 1, sy = e & 2 ? -1 : 1
+  // xy edges, stored with the plane they read: weight of x(ix, iy + s, iz) in the output of
+  // (ix - 1, iy, iz) [s = +, -], then of (ix + 1, iy, iz) [s = +, -]
+  K_PXY = 32,
+  K_PZX = 36,     // zx edges: x(ix, iy, iz + s) in the same way
+  K_FX = 40,      // faces x+, x-
+  K_COUNT = 50
 };
+template <typename T> __host__ __device__ constexpr int rec_stride() { return sizeof(T) == 8 ? 54 : 52; }
 
 // ---------------------------------------------------------------------------------------------
 // Record construction (FP64, once per operator)
 // ---------------------------------------------------------------------------------------------
+// first-order couplings of S with X, Y, Z of the derivative along each axis (P0 (1 - strain))
 __device__ __forceinline__ void first_order_coefs(const double* __restrict__ F, long long N,
-                                                  long long q, bool inter, double cu[3],
-                                                  double2 cv[3]) {
-  const double r3 = 0.57735026918962576451, r6 = 0.40824829046386301637;
+                                                  long long q, bool inter, double (&c)[3][3]) {
   const double P0 = F[F_P0 * N + q];
+  double e[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
   if (inter) {
-    const double exx = F[F_EXX * N + q], eyy = F[F_EYY * N + q], ezz = F[F_EZZ * N + q];
-    const double exy = F[F_EXY * N + q], eyz = F[F_EYZ * N + q], ezx = F[F_EZX * N + q];
-    cu[0] = -P0 * ezx * r3;
-    cu[1] = -P0 * eyz * r3;
-    cu[2] = P0 * (1.0 - ezz) * r3;
-    cv[0] = make_double2(P0 * (1.0 - exx) * r6, P0 * exy * r6);
-    cv[1] = make_double2(-P0 * exy * r6, P0 * (eyy - 1.0) * r6);
-    cv[2] = make_double2(-P0 * ezx * r6, P0 * eyz * r6);
-  } else {
-    cu[0] = 0.0; cu[1] = 0.0; cu[2] = P0 * r3;
-    cv[0] = make_double2(P0 * r6, 0.0);
-    cv[1] = make_double2(0.0, -P0 * r6);
-    cv[2] = make_double2(0.0, 0.0);
+    e[0][0] = F[F_EXX * N + q]; e[1][1] = F[F_EYY * N + q]; e[2][2] = F[F_EZZ * N + q];
+    e[0][1] = e[1][0] = F[F_EXY * N + q];
+    e[1][2] = e[2][1] = F[F_EYZ * N + q];
+    e[0][2] = e[2][0] = F[F_EZX * N + q];
   }
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) c[a][j] = P0 * ((a == j ? 1.0 : 0.0) - e[a][j]);
 }
 
-__global__ void kp_record_kernel(const double* __restrict__ F, long long N, int nx, int ny,
-                                 int nz, int nzp, double h, int flags, int nb, double sign,
+// A thread per site; the records of a CTA's sites are put together in shared memory and written out
+// as one contiguous run.
+constexpr int kRecThreads = 64;
+__global__ void __launch_bounds__(kRecThreads)
+kp_record_kernel(const double* __restrict__ F, long long N, int nx, int ny,
+                                 int nz, double h, int flags, int nb, double sign,
                                  double* __restrict__ rec64, float* __restrict__ rec32,
                                  unsigned* __restrict__ nbmask) {
   const double G = kG;
   const double ih2 = 1.0 / (h * h);
   const double i4h = 1.0 / (4.0 * h);
-  const double i8h2 = 1.0 / (8.0 * h * h);
-  const double sq2 = 1.41421356237309504880, sq3 = 1.73205080756887729353;
+  // an edge's weight in the plane's X/Y/Z pair: -sqrt3 x 2 sqrt3 G x -(sa sb) / (8 h^2)
+  const double ek = 6.0 * G / (8.0 * h * h);
+  const double sq3 = 1.73205080756887729353;
   const bool strain = (flags & QDKP_STRAIN) != 0;
   const bool inter = nb == 8 && strain && (flags & QDKP_INTERBAND_STRAIN);
-  for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < N;
-       s += (long long)gridDim.x * blockDim.x) {
+  __shared__ double sr[kRecThreads][rec_stride<double>() + 1];
+  for (long long s0 = blockIdx.x * (long long)kRecThreads; s0 < N; s0 += (long long)gridDim.x * kRecThreads) {
+    const int sites = (int)min((long long)kRecThreads, N - s0);
+    const long long s = s0 + min((int)threadIdx.x, sites - 1);     // spare threads repeat the last site
     const int iz = (int)(s % nz);
     const long long t = s / nz;
     const int iy = (int)(t % ny);
@@ -94,47 +107,46 @@ __global__ void kp_record_kernel(const double* __restrict__ F, long long N, int 
     const int coord[3] = {ix, iy, iz};
     const int ext[3] = {nx, ny, nz};
     const long long str[3] = {(long long)ny * nz, (long long)nz, 1LL};
-    double r[K_COUNT];
+    double* r = sr[threadIdx.x];
+    for (int k = 0; k < rec_stride<double>(); ++k) r[k] = 0.0;
     // neighbour mask: bit f (0..5) face x+, x-, y+, y-, z+, z-; bit 6 + 4 pl + e the in-plane
     // edge e of plane pl (xy, zx, zy) with signs sa = e & 1 ? -1 : 1, sb = e & 2 ? -1 : 1
     unsigned msk = 0;
+#pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
       if (coord[ax] + 1 < ext[ax]) msk |= 1u << (2 * ax);
       if (coord[ax] > 0) msk |= 1u << (2 * ax + 1);
     }
     const double g1 = F[F_G1 * N + s], g2 = F[F_G2 * N + s];
-    double cu_p[3]; double2 cv_p[3];
-    if (nb == 8) first_order_coefs(F, N, s, inter, cu_p, cv_p);
+    double c_p[3][3];
+    if (nb == 8) first_order_coefs(F, N, s, inter, c_p);
     double dk1 = 0.0, dk2[3];
+#pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
       double d1 = 0.0, d2 = 0.0;
+#pragma unroll
       for (int dir = 0; dir < 2; ++dir) {
         const bool in = dir == 0 ? (coord[ax] + 1 < ext[ax]) : (coord[ax] > 0);
-        double kp = 0.0, k2 = 0.0, su = 0.0, svr = 0.0, svi = 0.0;
+        const int kf = ax == 0 ? K_FX + 5 * dir : K_FYZ + 5 * (2 * (ax - 1) + dir);
         if (in) {
           const long long q = dir == 0 ? s + str[ax] : s - str[ax];
           const double t1 = (g1 + F[F_G1 * N + q]) * 0.5 * ih2;
           const double t2 = (g2 + F[F_G2 * N + q]) * 0.5 * ih2;
           d1 += t1; d2 += t2;
-          kp = -G * t1; k2 = -G * t2;
+          // P carries -G t1, the gamma2 stencil -G t2
+          r[kf + 0] = sign * G * (t1 + 4.0 * t2);
+          r[kf + 1] = sign * G * (t1 - 2.0 * t2);
           if (nb == 8) {
-            // symmetrised first derivative: (cu_p + cu_q) / 4h, signed by the face direction
-            double cu_q[3]; double2 cv_q[3];
-            first_order_coefs(F, N, q, inter, cu_q, cv_q);
+            // symmetrised first derivative: (c_p + c_q) / 4h, signed by the face direction
+            double c_q[3][3];
+            first_order_coefs(F, N, q, inter, c_q);
             const double sg = dir == 0 ? i4h : -i4h;
-            su = (cu_p[ax] + cu_q[ax]) * sg;
-            svr = (cv_p[ax].x + cv_q[ax].x) * sg;
-            svi = (cv_p[ax].y + cv_q[ax].y) * sg;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) r[kf + 2 + j] = sign * (c_p[ax][j] + c_q[ax][j]) * sg;
           }
         } else {  // hard wall: ghost term alpha_p / h^2 (kp_confined.py:133-137)
           d1 += g1 * ih2; d2 += g2 * ih2;
         }
-        const int kf = K_FACE + 5 * (2 * ax + dir);
-        r[kf + 0] = sign * kp;
-        r[kf + 1] = sign * k2;
-        r[kf + 2] = sign * su;
-        r[kf + 3] = sign * svr;
-        r[kf + 4] = sign * svi;
       }
       dk1 += d1; dk2[ax] = d2;
     }
@@ -150,197 +162,61 @@ __global__ void kp_record_kernel(const double* __restrict__ F, long long N, int 
       Sre = -d * ezx;
       Sim = d * eyz;
     }
-    const double A = F[F_EC * N + s] + 6.0 * G * ih2;
     const double P = -F[F_EV * N + s] + G * dk1;
-    const double Dl = F[F_DSO * N + s];
-    r[K_A] = sign * A;
-    r[K_A2] = sign * (-P + Q);
-    r[K_A3] = sign * (-P - Q);
-    r[K_A6] = sign * (-P - Dl);
-    r[K_Q2] = sign * sq2 * Q;
-    r[K_RRE] = sign * Rre; r[K_RIM] = sign * Rim;
-    r[K_SRE] = sign * Sre; r[K_SIM] = sign * Sim;
-    // cross(g3, a, b): coefficient of x(p + sa e_a + sb e_b) in the R / S slots is
-    // 2 sqrt3 G * (-(sa sb) / (8 h^2)) (g3(p + sa e_a) + g3(p + sb e_b))
-    for (int pl = 0; pl < 3; ++pl) {
-      const int ea = pl == 0 ? 0 : 2, eb = pl == 0 ? 1 : (pl == 1 ? 0 : 1);
-      for (int e = 0; e < 4; ++e) {
-        const int sa = (e & 1) ? -1 : 1, sb = (e & 2) ? -1 : 1;
-        const int ca = coord[ea] + sa, cb = coord[eb] + sb;
-        double c = 0.0;
-        if (ca >= 0 && ca < ext[ea] && cb >= 0 && cb < ext[eb]) {
-          msk |= 1u << (6 + 4 * pl + e);
-          const double ga = F[F_G3 * N + s + sa * str[ea]];
-          const double gb = F[F_G3 * N + s + sb * str[eb]];
-          c = 2.0 * sq3 * G * (-(double)(sa * sb) * i8h2) * (ga + gb);
-        }
-        r[K_EDGE + 4 * pl + e] = sign * c;
-      }
-    }
-    const long long NP = (long long)nx * ny * nzp;
-    const long long sp = t * nzp + iz;
-    for (int k = 0; k < K_COUNT; ++k) {
-      rec64[k * NP + sp] = r[k];
-      rec32[k * NP + sp] = (float)r[k];
-    }
-    nbmask[s] = msk;
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// The stencil arithmetic, shared by the kernels below. `L` supplies the neighbour values of one
-// column (centre, face f = x+, x-, y+, y-, z+, z-, edge (pl, e)); `Rc` the site's record
-// entries (own(k); face(ax, dir, k): entry k of face (ax, dir)).
-// ---------------------------------------------------------------------------------------------
-template <int NB> __device__ __forceinline__ constexpr bool has_band(int b) {
-  return NB == 8 ? true : (NB == 6 ? b >= 2 : (b >= 2 && b <= 5));
-}
-template <int NB> __device__ __forceinline__ constexpr int band_off() { return NB == 8 ? 0 : 2; }
-
-template <typename T, int NB, class L, class Rc>
-__device__ __forceinline__ void hx_math(const L& ld, const Rc& rc, unsigned msk, T shift, T cb,
-                                        cplx<T> (&y)[8]) {
-  const T sq2 = T(1.41421356237309504880), sq3 = T(1.73205080756887729353);
-  const T sq32 = T(1.22474487139158904910), isq2 = T(0.70710678118654752440);
-  const T wQ[3] = {T(1), T(1), T(-2)};
-  const T wR[3] = {-sq3, sq3, T(0)};
-  cplx<T> x[8];
-
-  // ---- local block (with the shift -sigma) -------------------------------------------
-  ld.centre(x);
-#pragma unroll
-  for (int b = 0; b < 8; ++b) y[b] = cscale(shift, x[b]);
-  {
-    const T a2 = rc.own(K_A2), a3 = rc.own(K_A3), a6 = rc.own(K_A6), q2 = rc.own(K_Q2);
-    const cplx<T> Rr = mk<T>(rc.own(K_RRE), rc.own(K_RIM));
-    const cplx<T> Sx = mk<T>(rc.own(K_SRE), rc.own(K_SIM));
-    if (NB == 8) {
-      const T A = rc.own(K_A);
-      caxpy(y[0], A, x[0]); caxpy(y[1], A, x[1]);
-    }
-    const cplx<T> R2 = cscale(sq2, Rr), S32 = cscale(sq32, Sx), Si2 = cscale(isq2, Sx);
-    caxpy(y[2], a2, x[2]); cfmac(y[2], Sx, cscale(T(-1), x[3])); cfma(y[2], Rr, x[4]);
-    cfma(y[2], S32, x[6]); caxpy(y[2], -q2, x[7]);
-    cfma(y[3], Sx, cscale(T(-1), x[2])); caxpy(y[3], a3, x[3]); cfma(y[3], Rr, x[5]);
-    cfma(y[3], R2, cscale(T(-1), x[6])); cfma(y[3], Si2, x[7]);
-    cfmac(y[4], Rr, x[2]); caxpy(y[4], a3, x[4]); cfmac(y[4], Sx, x[5]);
-    cfmac(y[4], Si2, x[6]); cfmac(y[4], R2, x[7]);
-    cfmac(y[5], Rr, x[3]); cfma(y[5], Sx, x[4]); caxpy(y[5], a2, x[5]);
-    caxpy(y[5], q2, x[6]); cfmac(y[5], S32, x[7]);
-    cfmac(y[6], S32, x[2]); cfmac(y[6], R2, cscale(T(-1), x[3]));
-    cfma(y[6], Si2, x[4]); caxpy(y[6], q2, x[5]); caxpy(y[6], a6, x[6]);
-    caxpy(y[7], -q2, x[2]); cfmac(y[7], Si2, x[3]); cfma(y[7], R2, x[4]);
-    cfma(y[7], S32, x[5]); caxpy(y[7], a6, x[7]);
-  }
-
-  // ---- six face neighbours ------------------------------------------------------------
-#pragma unroll
-  for (int f = 0; f < 6; ++f) {
-    const int ax = f >> 1, dir = f & 1;
-    if (!(msk & (1u << f))) continue;
-    ld.face(f, x);
-    const T kp = rc.face(ax, dir, 0), k2 = rc.face(ax, dir, 1);
-    const T kq = wQ[ax] * k2;
-    if (NB == 8) { caxpy(y[0], cb, x[0]); caxpy(y[1], cb, x[1]); }
-    caxpy(y[2], -kp + kq, x[2]); caxpy(y[2], -sq2 * kq, x[7]);
-    caxpy(y[3], -kp - kq, x[3]);
-    caxpy(y[4], -kp - kq, x[4]);
-    caxpy(y[5], -kp + kq, x[5]); caxpy(y[5], sq2 * kq, x[6]);
-    caxpy(y[6], -kp, x[6]); caxpy(y[6], sq2 * kq, x[5]);
-    caxpy(y[7], -kp, x[7]); caxpy(y[7], -sq2 * kq, x[2]);
-    if (ax < 2) {
-      const T kr = wR[ax] * k2;
-      caxpy(y[2], kr, x[4]);
-      caxpy(y[3], kr, x[5]); caxpy(y[3], -sq2 * kr, x[6]);
-      caxpy(y[4], kr, x[2]); caxpy(y[4], sq2 * kr, x[7]);
-      caxpy(y[5], kr, x[3]);
-      caxpy(y[6], -sq2 * kr, x[3]);
-      caxpy(y[7], sq2 * kr, x[4]);
-    }
-    if (NB == 8) {
-      // first-order weights of this face; U w = -i su w, V w = -i sv w, V^H w = -i conj(sv) w
-      // for the neighbour value w.
-      const T su = rc.face(ax, dir, 2);
-      const cplx<T> sv = mk<T>(rc.face(ax, dir, 3), rc.face(ax, dir, 4));
-      // conduction rows from valence inputs
-      cplx<T> m1 = x[2]; caxpy(m1, sq2, x[7]);                   // V^H (x2 + sqrt2 x7)
-      const cplx<T> m2 = cscale(sq3, x[4]);                      // V (sqrt3 x4)
-      cplx<T> m3 = cscale(-sq2, x[5]); m3 = csub(m3, x[6]);      // U (-sqrt2 x5 - x6)
-      cplx<T> acc = czero<T>();
-      cfmac(acc, sv, m1); cfma(acc, sv, m2); caxpy(acc, su, m3);
-      caxpy_i(y[0], T(-1), acc);
-      cplx<T> n1 = cscale(-sq2, x[2]); n1 = cadd(n1, x[7]);      // U (-sqrt2 x2 + x7)
-      const cplx<T> n2 = cscale(-sq3, x[3]);                     // V^H (-sqrt3 x3)
-      cplx<T> n3 = cscale(sq2, x[6]); n3 = csub(n3, x[5]);       // V (-x5 + sqrt2 x6)
-      acc = czero<T>();
-      caxpy(acc, su, n1); cfmac(acc, sv, n2); cfma(acc, sv, n3);
-      caxpy_i(y[1], T(-1), acc);
-      // valence rows from conduction inputs
-      cplx<T> Vw0 = czero<T>(), VHw0 = czero<T>(), Vw1 = czero<T>(), VHw1 = czero<T>();
-      cfma(Vw0, sv, x[0]); cfmac(VHw0, sv, x[0]); cfma(Vw1, sv, x[1]); cfmac(VHw1, sv, x[1]);
-      const cplx<T> Uw0 = cscale(su, x[0]), Uw1 = cscale(su, x[1]);
-      // every term carries the common factor -i
-      cplx<T> t2 = Vw0; caxpy(t2, -sq2, Uw1); caxpy_i(y[2], T(-1), t2);
-      caxpy_i(y[3], sq3, Vw1);
-      caxpy_i(y[4], -sq3, VHw0);
-      cplx<T> t5 = cscale(-sq2, Uw0); t5 = csub(t5, VHw1); caxpy_i(y[5], T(-1), t5);
-      cplx<T> t6 = cscale(sq2, VHw1); t6 = csub(t6, Uw0); caxpy_i(y[6], T(-1), t6);
-      cplx<T> t7 = cscale(sq2, Vw0); t7 = cadd(t7, Uw1); caxpy_i(y[7], T(-1), t7);
-    }
-  }
-
-  // ---- twelve edge neighbours: cross(g3, a, b) ---------------------------------------
-  // z = sum_e c_e x(p + sa e_a + sb e_b) over the plane's edges, then the plane's constant
-  // band mixing: xy -> R (+i z) / R^H (-i z); zx -> S, S^H (z); zy -> S (-i z), S^H (+i z).
-#pragma unroll
-  for (int pl = 0; pl < 3; ++pl) {
-    if (!(msk & (0xFu << (6 + 4 * pl)))) continue;
-    cplx<T> z[8];
-#pragma unroll
-    for (int b = 0; b < 8; ++b) z[b] = czero<T>();
+    // a four-band slice has no split-off states: its vectors are zero there, Delta does not enter
+    const double D3 = nb == 4 ? 0.0 : F[F_DSO * N + s] / 3.0;
+    r[K_A] = sign * (F[F_EC * N + s] + 6.0 * G * ih2);
+    r[K_DX] = sign * (-P - Q + sq3 * Rre - D3);
+    r[K_DY] = sign * (-P - Q - sq3 * Rre - D3);
+    r[K_DZ] = sign * (-P + 2.0 * Q - D3);
+    r[K_XY] = sign * -sq3 * Rim;
+    r[K_XZ] = sign * -sq3 * Sre;
+    r[K_YZ] = sign * sq3 * Sim;
+    r[K_SO] = sign * D3;
+    // cross(g3, a, b): x(p + sa e_a + sb e_b) enters with the g3 of the two sites between
+    auto g3 = [&](int dx, int dy, int dz) {
+      return F[F_G3 * N + s + dx * str[0] + dy * str[1] + dz * str[2]];
+    };
+    const bool xp = ix + 1 < nx, xm = ix > 0, yp = iy + 1 < ny, ym = iy > 0, zp = iz + 1 < nz,
+               zm = iz > 0;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      if (!(msk & (1u << (6 + 4 * pl + e)))) continue;
-      ld.edge(pl, e, x);
-      const T c = rc.own(K_EDGE + 4 * pl + e);
+      const int sa = (e & 1) ? -1 : 1, sb = (e & 2) ? -1 : 1;
+      const double w = sign * ek * (double)(sa * sb);
+      const bool xa = sa > 0 ? xp : xm, yb = sb > 0 ? yp : ym, za = sa > 0 ? zp : zm,
+                 xb = sb > 0 ? xp : xm;
+      if (xa && yb) msk |= 1u << (6 + e);
+      if (za && xb) msk |= 1u << (10 + e);
+      if (za && yb) { msk |= 1u << (14 + e); r[K_EZY + e] = w * (g3(0, 0, sa) + g3(0, sb, 0)); }
+    }
+    // the xy and zx edges of the outputs one plane down and up that read this plane
 #pragma unroll
-      for (int b = 2; b < 8; ++b) caxpy(z[b], c, x[b]);
+    for (int e = 0; e < 4; ++e) {
+      const int sx = (e & 2) ? 1 : -1, sb = (e & 1) ? -1 : 1;    // output at ix + sx
+      const bool xo = sx > 0 ? xp : xm;
+      const double w = sign * ek * (double)(-sx * sb);           // this plane lies at -sx of it
+      if (xo && (sb > 0 ? yp : ym)) r[K_PXY + e] = w * (g3(0, 0, 0) + g3(sx, sb, 0));
+      if (xo && (sb > 0 ? zp : zm)) r[K_PZX + e] = w * (g3(0, 0, 0) + g3(sx, 0, sb));
     }
-    if (pl == 0) {
-      caxpy_i(y[2], T(1), z[4]);
-      caxpy_i(y[4], T(-1), z[2]);
-      caxpy_i(y[3], T(1), z[5]);
-      caxpy_i(y[5], T(-1), z[3]);
-      caxpy_i(y[3], -sq2, z[6]);
-      caxpy_i(y[6], sq2, z[3]);
-      caxpy_i(y[4], -sq2, z[7]);
-      caxpy_i(y[7], sq2, z[4]);
-    } else if (pl == 1) {
-      caxpy(y[3], T(-1), z[2]); caxpy(y[2], sq32, z[6]); caxpy(y[3], isq2, z[7]);
-      caxpy(y[5], T(1), z[4]); caxpy(y[6], isq2, z[4]); caxpy(y[7], sq32, z[5]);
-      caxpy(y[2], T(-1), z[3]); caxpy(y[6], sq32, z[2]); caxpy(y[7], isq2, z[3]);
-      caxpy(y[4], T(1), z[5]); caxpy(y[4], isq2, z[6]); caxpy(y[5], sq32, z[7]);
-    } else {
-      caxpy_i(y[3], T(1), z[2]); caxpy_i(y[2], -sq32, z[6]); caxpy_i(y[3], -isq2, z[7]);
-      caxpy_i(y[5], T(-1), z[4]); caxpy_i(y[6], -isq2, z[4]); caxpy_i(y[7], -sq32, z[5]);
-      caxpy_i(y[2], T(-1), z[3]); caxpy_i(y[6], sq32, z[2]); caxpy_i(y[7], isq2, z[3]);
-      caxpy_i(y[4], T(1), z[5]); caxpy_i(y[4], isq2, z[6]); caxpy_i(y[5], sq32, z[7]);
-    }
+    nbmask[s] = msk;
+    __syncthreads();
+    for (int e = threadIdx.x; e < sites * rec_stride<double>(); e += kRecThreads)
+      rec64[s0 * rec_stride<double>() + e] = sr[e / rec_stride<double>()][e % rec_stride<double>()];
+    for (int e = threadIdx.x; e < sites * rec_stride<float>(); e += kRecThreads)
+      rec32[s0 * rec_stride<float>() + e] = (float)sr[e / rec_stride<float>()][e % rec_stride<float>()];
+    __syncthreads();
   }
 }
 
 // ---------------------------------------------------------------------------------------------
-// complex64 form of the same arithmetic on packed f32x2 registers (sm_100 `fma.rn.f32x2`):
-// a complex value is one 64-bit register pair, and every term is a real scalar (broadcast to
-// both halves) times a neighbour value. Products that carry a factor i go to a second
-// accumulator yi, so the result is Y = y + i yi and complex coefficients c = cr + i ci split
-// into cr -> y and ci -> yi. Half the issue slots of the scalar form for the same arithmetic.
+// Values and weights. A value is one complex128 number, or C adjacent complex64 columns on packed
+// f32x2 registers (sm_100 `fma.rn.f32x2`: a complex value is one 64-bit register pair and a real
+// weight is broadcast to both halves); every stencil term is a real weight times a value.
 // ---------------------------------------------------------------------------------------------
 typedef unsigned long long f2;
 __device__ __forceinline__ f2 f2pk(float a, float b) {
   f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r;
 }
-__device__ __forceinline__ f2 f2bc(float s) { return f2pk(s, s); }
 __device__ __forceinline__ float2 f2up(f2 v) {
   float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r;
 }
@@ -350,186 +226,200 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
 __device__ __forceinline__ f2 mul2(f2 a, f2 b) {
   f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d;
 }
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-  f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d;
+
+struct VD {                         // one complex128 value
+  typedef double T;
+  typedef double W;
+  static constexpr int C = 1;
+  double2 v;
+};
+template <int C_>
+struct VF {                         // C complex64 columns
+  typedef float T;
+  typedef f2 W;
+  static constexpr int C = C_;
+  f2 c[C_];
+};
+__device__ __forceinline__ double wt(double w, VD*) { return w; }
+template <int C> __device__ __forceinline__ f2 wt(float w, VF<C>*) { return f2pk(w, w); }
+template <class V> __device__ __forceinline__ typename V::W W_(typename V::T w) { return wt(w, (V*)nullptr); }
+
+__device__ __forceinline__ void vzero(VD& a) { a.v = make_double2(0.0, 0.0); }
+template <int C> __device__ __forceinline__ void vzero(VF<C>& a) {
+#pragma unroll
+  for (int i = 0; i < C; ++i) a.c[i] = 0ull;
 }
-__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
-  f2 d; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d;
+// a += w x
+__device__ __forceinline__ void vfma(VD& a, double w, const VD& x) {
+  a.v.x = fma(w, x.v.x, a.v.x); a.v.y = fma(w, x.v.y, a.v.y);
+}
+template <int C> __device__ __forceinline__ void vfma(VF<C>& a, f2 w, const VF<C>& x) {
+#pragma unroll
+  for (int i = 0; i < C; ++i) a.c[i] = fma2(w, x.c[i], a.c[i]);
+}
+// w x
+__device__ __forceinline__ VD vmul(double w, const VD& x) {
+  VD r; r.v = make_double2(w * x.v.x, w * x.v.y); return r;
+}
+template <int C> __device__ __forceinline__ VF<C> vmul(f2 w, const VF<C>& x) {
+  VF<C> r;
+#pragma unroll
+  for (int i = 0; i < C; ++i) r.c[i] = mul2(w, x.c[i]);
+  return r;
+}
+// i x
+__device__ __forceinline__ VD vi(const VD& x) { VD r; r.v = make_double2(-x.v.y, x.v.x); return r; }
+template <int C> __device__ __forceinline__ VF<C> vi(const VF<C>& x) {
+  VF<C> r;
+#pragma unroll
+  for (int i = 0; i < C; ++i) { const float2 u = f2up(x.c[i]); r.c[i] = f2pk(-u.y, u.x); }
+  return r;
+}
+// -i x
+__device__ __forceinline__ VD vmi(const VD& x) { VD r; r.v = make_double2(x.v.y, -x.v.x); return r; }
+template <int C> __device__ __forceinline__ VF<C> vmi(const VF<C>& x) {
+  VF<C> r;
+#pragma unroll
+  for (int i = 0; i < C; ++i) { const float2 u = f2up(x.c[i]); r.c[i] = f2pk(u.y, -u.x); }
+  return r;
+}
+__device__ __forceinline__ VD vload(const double2* p, VD*) { VD r; r.v = *p; return r; }
+__device__ __forceinline__ VF<1> vload(const float2* p, VF<1>*) {
+  VF<1> r; r.c[0] = *reinterpret_cast<const f2*>(p); return r;
+}
+__device__ __forceinline__ VF<2> vload(const float2* p, VF<2>*) {
+  VF<2> r; const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  r.c[0] = v.x; r.c[1] = v.y; return r;
+}
+__device__ __forceinline__ VD vldg(const double2* p, VD*) { VD r; r.v = __ldg(p); return r; }
+__device__ __forceinline__ VF<1> vldg(const float2* p, VF<1>*) {
+  VF<1> r; r.c[0] = __ldg(reinterpret_cast<const f2*>(p)); return r;
+}
+__device__ __forceinline__ VF<2> vldg(const float2* p, VF<2>*) {
+  VF<2> r; const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(p));
+  r.c[0] = v.x; r.c[1] = v.y; return r;
+}
+__device__ __forceinline__ void vstore(double2* p, const VD& a) { *p = a.v; }
+__device__ __forceinline__ void vstore(float2* p, const VF<1>& a) { *reinterpret_cast<f2*>(p) = a.c[0]; }
+__device__ __forceinline__ void vstore(float2* p, const VF<2>& a) {
+  *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(a.c[0], a.c[1]);
 }
 
-template <class L, class Rc>
-__device__ __forceinline__ void hx_math_packed(const L& ld, const Rc& rc, unsigned msk,
-                                               float shift, float cb, float2 (&Y)[8]) {
-  const float sq2 = 1.41421356237309504880f, sq3 = 1.73205080756887729353f;
-  const float sq32 = 1.22474487139158904910f, isq2 = 0.70710678118654752440f;
-  const f2 C2 = f2bc(sq2), CN2 = f2bc(-sq2), C3 = f2bc(sq3), C32 = f2bc(sq32);
-  const f2 CN32 = f2bc(-sq32), Ci2 = f2bc(isq2), CNi2 = f2bc(-isq2), CN1 = f2bc(-1.f);
-  const f2 CB = f2bc(cb);
-  f2 y[8], yi[8], x[8];
+// Order of the eight values of a site in the uncoupled basis
+enum { US = 0, UX, UY, UZ, DS, DX, DY, DZ };
 
-  // ---- local block, the shift -sigma folded into the diagonal ---------------------------
-  ld.centre2(x);
-  {
-    const float Rr = rc.own(K_RRE), Ri = rc.own(K_RIM), Sr = rc.own(K_SRE), Si = rc.own(K_SIM);
-    const float q2 = rc.own(K_Q2);
-    const f2 PA = f2bc(rc.own(K_A) + shift), P2 = f2bc(rc.own(K_A2) + shift);
-    const f2 P3 = f2bc(rc.own(K_A3) + shift), P6 = f2bc(rc.own(K_A6) + shift);
-    const f2 Q2 = f2bc(q2), NQ2 = f2bc(-q2);
-    const f2 SR = f2bc(Sr), NSR = f2bc(-Sr), SI = f2bc(Si), NSI = f2bc(-Si);
-    const f2 RR = f2bc(Rr), RI = f2bc(Ri), NRI = f2bc(-Ri);
-    const f2 S32R = f2bc(sq32 * Sr), S32I = f2bc(sq32 * Si), NS32I = f2bc(-sq32 * Si);
-    const f2 R2R = f2bc(sq2 * Rr), NR2R = f2bc(-sq2 * Rr), R2I = f2bc(sq2 * Ri);
-    const f2 NR2I = f2bc(-sq2 * Ri);
-    const f2 SI2R = f2bc(isq2 * Sr), SI2I = f2bc(isq2 * Si), NSI2I = f2bc(-isq2 * Si);
-    y[0] = mul2(PA, x[0]); y[1] = mul2(PA, x[1]);
-    yi[0] = 0ull; yi[1] = 0ull;
-    y[2] = fma2(NSR, x[3], mul2(P2, x[2]));   yi[2] = mul2(SI, x[3]);
-    y[2] = fma2(RR, x[4], y[2]);              yi[2] = fma2(RI, x[4], yi[2]);
-    y[2] = fma2(S32R, x[6], y[2]);            yi[2] = fma2(S32I, x[6], yi[2]);
-    y[2] = fma2(NQ2, x[7], y[2]);
-    y[3] = fma2(NSR, x[2], mul2(P3, x[3]));   yi[3] = mul2(NSI, x[2]);
-    y[3] = fma2(RR, x[5], y[3]);              yi[3] = fma2(RI, x[5], yi[3]);
-    y[3] = fma2(NR2R, x[6], y[3]);            yi[3] = fma2(NR2I, x[6], yi[3]);
-    y[3] = fma2(SI2R, x[7], y[3]);            yi[3] = fma2(SI2I, x[7], yi[3]);
-    y[4] = fma2(RR, x[2], mul2(P3, x[4]));    yi[4] = mul2(NRI, x[2]);
-    y[4] = fma2(SR, x[5], y[4]);              yi[4] = fma2(NSI, x[5], yi[4]);
-    y[4] = fma2(SI2R, x[6], y[4]);            yi[4] = fma2(NSI2I, x[6], yi[4]);
-    y[4] = fma2(R2R, x[7], y[4]);             yi[4] = fma2(NR2I, x[7], yi[4]);
-    y[5] = fma2(RR, x[3], mul2(P2, x[5]));    yi[5] = mul2(NRI, x[3]);
-    y[5] = fma2(SR, x[4], y[5]);              yi[5] = fma2(SI, x[4], yi[5]);
-    y[5] = fma2(Q2, x[6], y[5]);
-    y[5] = fma2(S32R, x[7], y[5]);            yi[5] = fma2(NS32I, x[7], yi[5]);
-    y[6] = fma2(S32R, x[2], mul2(P6, x[6]));  yi[6] = mul2(NS32I, x[2]);
-    y[6] = fma2(NR2R, x[3], y[6]);            yi[6] = fma2(R2I, x[3], yi[6]);
-    y[6] = fma2(SI2R, x[4], y[6]);            yi[6] = fma2(SI2I, x[4], yi[6]);
-    y[6] = fma2(Q2, x[5], y[6]);
-    y[7] = fma2(NQ2, x[2], mul2(P6, x[7]));
-    y[7] = fma2(SI2R, x[3], y[7]);            yi[7] = mul2(NSI2I, x[3]);
-    y[7] = fma2(R2R, x[4], y[7]);             yi[7] = fma2(R2I, x[4], yi[7]);
-    y[7] = fma2(S32R, x[5], y[7]);            yi[7] = fma2(S32I, x[5], yi[7]);
+// |J, m_J> values x (Pryor's band order) to the uncoupled basis u; six-band values leave S alone
+template <class V, int NB>
+__device__ __forceinline__ void to_uncoupled(const V (&x)[8], V (&u)[8]) {
+  const auto c = [](double w) { return W_<V>((typename V::T)w); };
+  const double i3 = 0.57735026918962576451, s23 = 0.81649658092772603273;   // 1/sqrt3, sqrt(2/3)
+  const double i2 = 0.70710678118654752440, i6 = 0.40824829046386301637;    // 1/sqrt2, 1/sqrt6
+  const auto one = c(1.0), none = c(-1.0);
+  V t = vmul(c(i6), x[2]); vfma(t, c(i3), x[7]);                // t / sqrt2
+  V a = vmul(c(i2), x[4]);
+  u[UX] = a; vfma(u[UX], one, t);
+  vfma(a, none, t);
+  u[UY] = vmi(a);
+  u[UZ] = vmul(c(-s23), x[5]); vfma(u[UZ], c(-i3), x[6]);
+  V q = vmul(c(i3), x[6]); vfma(q, c(-i6), x[5]);               // q / sqrt2
+  const V p = vmul(c(i2), x[3]);                                // -p / sqrt2
+  u[DX] = q; vfma(u[DX], none, p);
+  vfma(q, one, p);
+  u[DY] = vmi(q);
+  u[DZ] = vmul(c(i3), x[7]); vfma(u[DZ], c(-s23), x[2]);
+  if (NB == 8) { u[US] = vi(x[0]); u[DS] = vi(x[1]); }
+}
+
+// the adjoint: uncoupled values u to |J, m_J>
+template <class V, int NB>
+__device__ __forceinline__ void from_uncoupled(const V (&u)[8], V (&x)[8]) {
+  const auto c = [](double w) { return W_<V>((typename V::T)w); };
+  const double i3 = 0.57735026918962576451, s23 = 0.81649658092772603273;
+  const double i2 = 0.70710678118654752440, i6 = 0.40824829046386301637;
+  const V iyu = vi(u[UY]), iyd = vi(u[DY]);
+  x[4] = vmul(c(i2), u[UX]); vfma(x[4], c(i2), iyu);
+  V t = u[UX]; vfma(t, c(-1.0), iyu);                           // sqrt2 t
+  x[2] = vmul(c(i6), t); vfma(x[2], c(-s23), u[DZ]);
+  x[7] = vmul(c(i3), t); vfma(x[7], c(i3), u[DZ]);
+  V q = u[DX]; vfma(q, c(1.0), iyd);                            // sqrt2 q
+  x[3] = vmul(c(-i2), u[DX]); vfma(x[3], c(i2), iyd);           // -p
+  x[5] = vmul(c(-s23), u[UZ]); vfma(x[5], c(-i6), q);
+  x[6] = vmul(c(-i3), u[UZ]); vfma(x[6], c(i3), q);
+  if (NB == 8) { x[0] = vmi(u[US]); x[1] = vmi(u[DS]); }
+}
+
+// ---- stencil terms in the uncoupled basis ----------------------------------------------------
+// the local block: y += (diagonal + shift) x, strain couplings, spin-orbit
+template <class V, int NB>
+__device__ __forceinline__ void local_term(V (&y)[8], const V (&x)[8], const typename V::T (&w)[8],
+                                           typename V::T shift) {
+  const auto dx = W_<V>(w[K_DX] + shift), dy = W_<V>(w[K_DY] + shift), dz = W_<V>(w[K_DZ] + shift);
+  const auto xy = W_<V>(w[K_XY]), xz = W_<V>(w[K_XZ]), yz = W_<V>(w[K_YZ]);
+  if (NB == 8) {
+    const auto a = W_<V>(w[K_A] + shift);
+    vfma(y[US], a, x[US]); vfma(y[DS], a, x[DS]);
   }
-
-  // ---- six face neighbours ------------------------------------------------------------
 #pragma unroll
-  for (int f = 0; f < 6; ++f) {
-    const int ax = f >> 1, dir = f & 1;
-    if (!(msk & (1u << f))) continue;
-    ld.face2(f, x);
-    const float kp = rc.face(ax, dir, 0), k2 = rc.face(ax, dir, 1);
-    const float kq = (ax == 2 ? -2.f : 1.f) * k2;
-    y[0] = fma2(CB, x[0], y[0]); y[1] = fma2(CB, x[1], y[1]);
-    const f2 KPQ = f2bc(kq - kp), NKPQ = f2bc(-kp - kq), NKP = f2bc(-kp);
-    const f2 K2Q = f2bc(sq2 * kq), NK2Q = f2bc(-sq2 * kq);
-    y[2] = fma2(KPQ, x[2], y[2]); y[2] = fma2(NK2Q, x[7], y[2]);
-    y[3] = fma2(NKPQ, x[3], y[3]);
-    y[4] = fma2(NKPQ, x[4], y[4]);
-    y[5] = fma2(KPQ, x[5], y[5]); y[5] = fma2(K2Q, x[6], y[5]);
-    y[6] = fma2(NKP, x[6], y[6]); y[6] = fma2(K2Q, x[5], y[6]);
-    y[7] = fma2(NKP, x[7], y[7]); y[7] = fma2(NK2Q, x[2], y[7]);
-    if (ax < 2) {
-      const float kr = (ax == 0 ? -sq3 : sq3) * k2;
-      const f2 KR = f2bc(kr), K2R = f2bc(sq2 * kr), NK2R = f2bc(-sq2 * kr);
-      y[2] = fma2(KR, x[4], y[2]);
-      y[3] = fma2(KR, x[5], y[3]); y[3] = fma2(NK2R, x[6], y[3]);
-      y[4] = fma2(KR, x[2], y[4]); y[4] = fma2(K2R, x[7], y[4]);
-      y[5] = fma2(KR, x[3], y[5]);
-      y[6] = fma2(NK2R, x[3], y[6]);
-      y[7] = fma2(K2R, x[4], y[7]);
-    }
-    // first-order (U, V) couplings with the face weights su (real), sv = svr + i svi:
-    //   y0 += -i [conj(sv)(x2 + sqrt2 x7) + sv sqrt3 x4 + su (-sqrt2 x5 - x6)]
-    //   y1 += -i [su (-sqrt2 x2 + x7) - conj(sv) sqrt3 x3 + sv (-x5 + sqrt2 x6)]
-    //   y2..y7 from x0, x1 (the adjoint blocks)
-    const float su = rc.face(ax, dir, 2), svr = rc.face(ax, dir, 3), svi = rc.face(ax, dir, 4);
-    const f2 SVI = f2bc(svi), SVR = f2bc(svr), SU = f2bc(su), NSVR = f2bc(-svr), NSU = f2bc(-su);
-    const f2 S2SU = f2bc(sq2 * su), N3SVI = f2bc(-sq3 * svi), S3SVR = f2bc(sq3 * svr);
-    const f2 N3SVR = f2bc(-sq3 * svr), N2SVI = f2bc(-sq2 * svi), N2SVR = f2bc(-sq2 * svr);
-    const f2 S2SVI = f2bc(sq2 * svi);
-    {
-      const f2 t = fma2(C2, x[7], x[2]);        // x2 + sqrt2 x7
-      const f2 u = mul2(C3, x[4]);              // sqrt3 x4
-      y[0] = fma2(SVI, sub2(u, t), y[0]);
-      yi[0] = fma2(NSVR, add2(u, t), yi[0]);
-      yi[0] = fma2(SU, fma2(C2, x[5], x[6]), yi[0]);
-      const f2 v = mul2(C3, x[3]);              // sqrt3 x3
-      const f2 w = fma2(CN2, x[6], x[5]);       // x5 - sqrt2 x6
-      y[1] = fma2(SVI, sub2(v, w), y[1]);
-      yi[1] = fma2(SVR, add2(v, w), yi[1]);
-      yi[1] = fma2(SU, fma2(C2, x[2], mul2(CN1, x[7])), yi[1]);
-    }
-    y[2] = fma2(SVI, x[0], y[2]);   yi[2] = fma2(NSVR, x[0], yi[2]); yi[2] = fma2(S2SU, x[1], yi[2]);
-    y[3] = fma2(N3SVI, x[1], y[3]); yi[3] = fma2(S3SVR, x[1], yi[3]);
-    y[4] = fma2(N3SVI, x[0], y[4]); yi[4] = fma2(N3SVR, x[0], yi[4]);
-    y[5] = fma2(SVI, x[1], y[5]);   yi[5] = fma2(S2SU, x[0], yi[5]); yi[5] = fma2(SVR, x[1], yi[5]);
-    y[6] = fma2(N2SVI, x[1], y[6]); yi[6] = fma2(N2SVR, x[1], yi[6]); yi[6] = fma2(SU, x[0], yi[6]);
-    y[7] = fma2(S2SVI, x[0], y[7]); yi[7] = fma2(N2SVR, x[0], yi[7]); yi[7] = fma2(NSU, x[1], yi[7]);
+  for (int s = 0; s < 8; s += 4) {
+    vfma(y[s + 1], dx, x[s + 1]); vfma(y[s + 2], dy, x[s + 2]); vfma(y[s + 3], dz, x[s + 3]);
+    vfma(y[s + 1], xy, x[s + 2]); vfma(y[s + 2], xy, x[s + 1]); vfma(y[s + 3], xz, x[s + 1]);
+    vfma(y[s + 1], xz, x[s + 3]); vfma(y[s + 2], yz, x[s + 3]); vfma(y[s + 3], yz, x[s + 2]);
   }
+  const auto d = W_<V>(w[K_SO]), nd = W_<V>(-w[K_SO]);
+  const V iyu = vi(x[UY]), iyd = vi(x[DY]), ixu = vi(x[UX]), ixd = vi(x[DX]);
+  const V izu = vi(x[UZ]), izd = vi(x[DZ]);
+  vfma(y[UX], d, iyu);  vfma(y[UX], nd, x[DZ]);
+  vfma(y[UY], nd, ixu); vfma(y[UY], nd, izd);
+  vfma(y[UZ], d, x[DX]); vfma(y[UZ], d, iyd);
+  vfma(y[DX], nd, iyd); vfma(y[DX], d, x[UZ]);
+  vfma(y[DY], d, ixd);  vfma(y[DY], nd, izu);
+  vfma(y[DZ], nd, x[UX]); vfma(y[DZ], d, iyu);
+}
 
-  // ---- twelve edge neighbours: z = sum_e c_e x_e, then the plane's band mixing ---------
+// a face neighbour x along AX: w = {along, across, cx, cy, cz}; NEG: the first-order weights enter
+// with the other sign (the same face seen from its other side); INIT: y is set, not added to
+template <class V, int NB, int AX, bool NEG, bool INIT = false>
+__device__ __forceinline__ void face_term(V (&y)[8], const V (&x)[8], const typename V::T* w,
+                                          typename V::W cb) {
+  const auto wl = W_<V>(w[0]), wm = W_<V>(w[1]);
+  const auto add = [](V& a, typename V::W c, const V& v) {
+    if (INIT) a = vmul(c, v);
+    else vfma(a, c, v);
+  };
 #pragma unroll
-  for (int pl = 0; pl < 3; ++pl) {
-    if (!(msk & (0xFu << (6 + 4 * pl)))) continue;
-    f2 z[8];
-#pragma unroll
-    for (int b = 2; b < 8; ++b) z[b] = 0ull;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (!(msk & (1u << (6 + 4 * pl + e)))) continue;
-      ld.edge2(pl, e, x);
-      const f2 C = f2bc(rc.own(K_EDGE + 4 * pl + e));
-#pragma unroll
-      for (int b = 2; b < 8; ++b) z[b] = fma2(C, x[b], z[b]);
-    }
-    if (pl == 0) {            // R: +i z, R^H: -i z
-      yi[2] = add2(yi[2], z[4]); yi[4] = sub2(yi[4], z[2]);
-      yi[3] = add2(yi[3], z[5]); yi[5] = sub2(yi[5], z[3]);
-      yi[3] = fma2(CN2, z[6], yi[3]); yi[6] = fma2(C2, z[3], yi[6]);
-      yi[4] = fma2(CN2, z[7], yi[4]); yi[7] = fma2(C2, z[4], yi[7]);
-    } else if (pl == 1) {     // S, S^H: z
-      y[3] = sub2(y[3], z[2]); y[2] = fma2(C32, z[6], y[2]); y[3] = fma2(Ci2, z[7], y[3]);
-      y[5] = add2(y[5], z[4]); y[6] = fma2(Ci2, z[4], y[6]); y[7] = fma2(C32, z[5], y[7]);
-      y[2] = sub2(y[2], z[3]); y[6] = fma2(C32, z[2], y[6]); y[7] = fma2(Ci2, z[3], y[7]);
-      y[4] = add2(y[4], z[5]); y[4] = fma2(Ci2, z[6], y[4]); y[5] = fma2(C32, z[7], y[5]);
-    } else {                  // S: -i z, S^H: +i z
-      yi[3] = add2(yi[3], z[2]); yi[2] = fma2(CN32, z[6], yi[2]); yi[3] = fma2(CNi2, z[7], yi[3]);
-      yi[5] = sub2(yi[5], z[4]); yi[6] = fma2(CNi2, z[4], yi[6]); yi[7] = fma2(CN32, z[5], yi[7]);
-      yi[2] = sub2(yi[2], z[3]); yi[6] = fma2(C32, z[2], yi[6]); yi[7] = fma2(Ci2, z[3], yi[7]);
-      yi[4] = add2(yi[4], z[5]); yi[4] = fma2(Ci2, z[6], yi[4]); yi[5] = fma2(C32, z[7], yi[5]);
-    }
+  for (int s = 0; s < 8; s += 4) {
+    add(y[s + 1], AX == 0 ? wl : wm, x[s + 1]);
+    add(y[s + 2], AX == 1 ? wl : wm, x[s + 2]);
+    add(y[s + 3], AX == 2 ? wl : wm, x[s + 3]);
   }
-
-  // ---- Y = y + i yi -------------------------------------------------------------------
+  if (NB == 8) {
+    add(y[US], cb, x[US]); add(y[DS], cb, x[DS]);
 #pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    const float2 a = f2up(y[b]), c = f2up(yi[b]);
-    Y[b] = make_float2(a.x - c.y, a.y + c.x);
+    for (int j = 0; j < 3; ++j) {
+      const auto c = W_<V>(NEG ? -w[2 + j] : w[2 + j]), nc = W_<V>(NEG ? w[2 + j] : -w[2 + j]);
+      vfma(y[US], c, x[UX + j]); vfma(y[DS], c, x[DX + j]);
+      vfma(y[UX + j], nc, x[US]); vfma(y[DX + j], nc, x[DS]);
+    }
   }
 }
 
-// complex64 eight-band blocks take the packed form, everything else the scalar one
-template <typename T, int NB, class L, class Rc>
-__device__ __forceinline__ void hx_compute(const L& ld, const Rc& rc, unsigned msk, T shift,
-                                           T cb, cplx<T> (&y)[8]) {
-  if constexpr (std::is_same<T, float>::value && NB == 8) hx_math_packed(ld, rc, msk, shift, cb, y);
-  else hx_math<T, NB>(ld, rc, msk, shift, cb, y);
+// an edge neighbour in the plane of the states A and B (1 X, 2 Y, 3 Z)
+template <class V, int A, int B>
+__device__ __forceinline__ void edge_term(V (&y)[8], const V (&x)[8], typename V::T w) {
+  const auto c = W_<V>(w);
+#pragma unroll
+  for (int s = 0; s < 8; s += 4) { vfma(y[s + A], c, x[s + B]); vfma(y[s + B], c, x[s + A]); }
 }
 
-// neighbour mask of site (ix, iy, iz): bit f (0..5) face x+, x-, y+, y-, z+, z-; bit
-// 6 + 4 pl + e the in-plane edge e of plane pl (xy, zx, zy), sa = e & 1 ? -1 : 1,
-// sb = e & 2 ? -1 : 1 (a = x, z, z; b = y, x, y). An edge exists when both of its faces do.
-__device__ __forceinline__ unsigned site_mask(int ix, int iy, int iz, int nx, int ny, int nz) {
-  const unsigned xp = ix + 1 < nx, xm = ix > 0, yp = iy + 1 < ny, ym = iy > 0;
-  const unsigned zp = iz + 1 < nz, zm = iz > 0;
-  unsigned m = xp | (xm << 1) | (yp << 2) | (ym << 3) | (zp << 4) | (zm << 5);
-  m |= (xp & yp) << 6 | (xm & yp) << 7 | (xp & ym) << 8 | (xm & ym) << 9;      // xy
-  m |= (zp & xp) << 10 | (zm & xp) << 11 | (zp & xm) << 12 | (zm & xm) << 13;  // zx
-  m |= (zp & yp) << 14 | (zm & yp) << 15 | (zp & ym) << 16 | (zm & ym) << 17;  // zy
-  return m;
+template <int NB> __device__ __forceinline__ constexpr bool has_band(int b) {
+  return NB == 8 ? true : (NB == 6 ? b >= 2 : (b >= 2 && b <= 5));
 }
+template <int NB> __device__ __forceinline__ constexpr int band_off() { return NB == 8 ? 0 : 2; }
 
 // ---------------------------------------------------------------------------------------------
-// Direct kernel: one thread per (site, column), neighbours read through L1/L2. Serves the six-
-// and four-band slices, blocks the staged kernel cannot take, and the batched engine.
+// Direct kernel: one thread per (site, column), neighbours read through L1/L2. Bound by load latency
+// and L1 wavefronts (128 16-byte loads per value). 48x48x36 x 12: complex128 119 us (185 in Pryor's
+// basis with branches at the walls), complex64 59 us (116).
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 struct HXArgs {
@@ -538,81 +428,139 @@ struct HXArgs {
   const cplx<T>* __restrict__ X;
   cplx<T>* __restrict__ Y;
   int N, ldx, ldy, m, sx, sy;   // sites, leading dimensions, columns, site strides of x and y
-  int nz, nzp, NP;              // z extent, its padded record extent, record entry stride
   T shift;                      // -sigma for a shifted apply, else 0
   T cb;                         // conduction-band face weight sign (-G / h^2)
 };
 
-// x[b] = X[band b, site s + offset, column j] with xs = &X[0, s, j], bs = N ldx (elements);
-// every offset fits 32 bits for the grids this library accepts (n ldx < 2^31).
-template <typename T, int NB>
-struct GlobalLoader {
-  const cplx<T>* __restrict__ xs;
-  int bs, xstr[3];
-  __device__ __forceinline__ void at(int off, bool vb_only, cplx<T> (&x)[8]) const {
+// Values of one column (or column pair) of the block in Pryor's band order at site offset `off`
+// (in elements), xs = &X[0, s, j], bs = N ldx. Every offset fits 32 bits for the blocks this
+// library accepts (n ldx < 2^31).
+template <class V, int NB>
+__device__ __forceinline__ void load_bands(const cplx<typename V::T>* __restrict__ xs, int bs,
+                                           int off, bool vb_only, V (&x)[8]) {
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      if (!has_band<NB>(b) || (vb_only && b < 2)) { x[b] = czero<T>(); continue; }
-      x[b] = __ldg(xs + ((b - band_off<NB>()) * bs + off));
+  for (int b = 0; b < 8; ++b) {
+    if (!has_band<NB>(b) || (vb_only && b < 2)) { vzero(x[b]); continue; }
+    x[b] = vldg(xs + ((b - band_off<NB>()) * bs + off), (V*)nullptr);
+  }
+}
+
+// K entries of a record, in global (LDG) or shared memory
+template <bool LDG, typename T, int K>
+__device__ __forceinline__ void load_rec(const T* r, T (&w)[K]) {
+  constexpr int E = 16 / (int)sizeof(T);
+  static_assert(K % E == 0, "records are read in 16-byte words");
+#pragma unroll
+  for (int k = 0; k < K; k += E) {
+    if constexpr (sizeof(T) == 8) {
+      const double2* p = reinterpret_cast<const double2*>(r + k);
+      const double2 v = LDG ? __ldg(p) : *p;
+      w[k] = v.x; w[k + 1] = v.y;
+    } else {
+      const float4* p = reinterpret_cast<const float4*>(r + k);
+      const float4 v = LDG ? __ldg(p) : *p;
+      w[k] = v.x; w[k + 1] = v.y; w[k + 2] = v.z; w[k + 3] = v.w;
     }
   }
-  __device__ __forceinline__ void centre(cplx<T> (&x)[8]) const { at(0, false, x); }
-  __device__ __forceinline__ void face(int f, cplx<T> (&x)[8]) const {
-    at((f & 1) ? -xstr[f >> 1] : xstr[f >> 1], false, x);
-  }
-  __device__ __forceinline__ void edge(int pl, int e, cplx<T> (&x)[8]) const {
-    const int ea = pl == 0 ? 0 : 2, eb = pl == 0 ? 1 : (pl == 1 ? 0 : 1);
-    const int sa = (e & 1) ? -1 : 1, sb = (e & 2) ? -1 : 1;
-    at(sa * xstr[ea] + sb * xstr[eb], true, x);
-  }
-  // packed complex64 loads (eight bands only)
-  __device__ __forceinline__ void at2(int off, int b0, f2 (&x)[8]) const {
-    const unsigned long long* p = reinterpret_cast<const unsigned long long*>(xs);
+}
+
+// Faces are taken to the uncoupled basis one by one; the four edge neighbours of a plane share
+// one weight per band, so their weighted sum is formed first and taken there once. Nothing
+// branches on the walls: a missing neighbour reads the site itself under a zero weight, so the
+// loads of several neighbours can be in flight together.
+// wall_self: the conduction bands' face weight, the one that is not zero at a wall, stays on there
+// and multiplies the site itself. That is the operator complex64 engine slots of even width iterate
+// on; it differs from the hard-wall operator only in rows next to a wall, and the complex128 finish
+// of a mixed solve does not use it.
+template <class V, int NB>
+__device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, int j,
+                                        bool wall_self = false) {
+  typedef typename V::T T;
+  const cplx<T>* xs = a.X + ((long long)s * a.ldx + j);
+  const int bs = a.N * a.ldx;
+  const int sx = a.sx * a.ldx, sy = a.sy * a.ldx, sz = a.ldx;
+  const T* rp = a.rec + (long long)s * rec_stride<T>();
+  const long long rx = (long long)a.sx * rec_stride<T>();          // the x neighbours' records
+  const unsigned msk = __ldg(a.msk + s);
+  V y[8], x[8], u[8];
 #pragma unroll
-    for (int b = b0; b < 8; ++b) x[b] = __ldg(p + (b * bs + off));
+  for (int b = 0; b < 8; ++b) vzero(y[b]);
+  {
+    T w[8];
+    load_rec<true>(rp, w);
+    load_bands<V, NB>(xs, bs, 0, false, x);
+    to_uncoupled<V, NB>(x, u);
+    local_term<V, NB>(y, u, w, a.shift);
   }
-  __device__ __forceinline__ void centre2(f2 (&x)[8]) const { at2(0, 0, x); }
-  __device__ __forceinline__ void face2(int f, f2 (&x)[8]) const {
-    at2((f & 1) ? -xstr[f >> 1] : xstr[f >> 1], 0, x);
+  const auto cbf = [&](int f) { return W_<V>(wall_self || (msk >> f & 1u) ? a.cb : T(0)); };
+  const auto face_off = [&](int f, int d) { return (msk >> f & 1u) ? d : 0; };
+  {
+    T w[20];
+    load_rec<true>(rp + K_FYZ, w);
+#pragma unroll
+    for (int f = 2; f < 6; ++f) {
+      const int d = f < 4 ? sy : sz;
+      load_bands<V, NB>(xs, bs, face_off(f, (f & 1) ? -d : d), false, x);
+      to_uncoupled<V, NB>(x, u);
+      if (f < 4) face_term<V, NB, 1, false>(y, u, w + 5 * (f - 2), cbf(f));
+      else face_term<V, NB, 2, false>(y, u, w + 5 * (f - 2), cbf(f));
+    }
   }
-  __device__ __forceinline__ void edge2(int pl, int e, f2 (&x)[8]) const {
-    const int ea = pl == 0 ? 0 : 2, eb = pl == 0 ? 1 : (pl == 1 ? 0 : 1);
-    const int sa = (e & 1) ? -1 : 1, sb = (e & 2) ? -1 : 1;
-    at2(sa * xstr[ea] + sb * xstr[eb], 2, x);
+  {
+    T w[12];
+    load_rec<true>(rp + K_FX, w);
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      load_bands<V, NB>(xs, bs, face_off(f, f ? -sx : sx), false, x);
+      to_uncoupled<V, NB>(x, u);
+      face_term<V, NB, 0, false>(y, u, w + 5 * f, cbf(f));
+    }
   }
-};
-
-template <typename T>
-struct GlobalRecord {
-  const T* __restrict__ R;   // record base + padded site index
-  int NP;
-  __device__ __forceinline__ T own(int k) const { return __ldg(R + k * NP); }
-  __device__ __forceinline__ T face(int ax, int dir, int k) const {
-    return own(K_FACE + 5 * (2 * ax + dir) + k);
+#pragma unroll
+  for (int pl = 0; pl < 3; ++pl) {
+    const int sa = pl == 0 ? sx : sz, sb = pl == 1 ? sx : sy;
+    // weights by e: an xy or zx edge's stands in the record of the x neighbour on its side
+    T w[4];
+    if (pl == 2) {
+      load_rec<true>(rp + K_EZY, w);
+    } else {
+      T p[4];
+      const int k = pl == 0 ? K_PXY : K_PZX;
+      const bool up = msk & 1u, dn = msk & 2u;
+      load_rec<true>(rp + (up ? rx : 0) + k, p);
+      w[0] = up ? p[0] : T(0); w[pl == 0 ? 2 : 1] = up ? p[1] : T(0);
+      load_rec<true>(rp - (dn ? rx : 0) + k, p);
+      w[pl == 0 ? 1 : 2] = dn ? p[2] : T(0); w[3] = dn ? p[3] : T(0);
+    }
+    V z[8];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) vzero(z[b]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int off = ((e & 1) ? -sa : sa) + ((e & 2) ? -sb : sb);
+      load_bands<V, NB>(xs, bs, (msk >> (6 + 4 * pl + e) & 1u) ? off : 0, true, x);
+      const auto c = W_<V>(w[e]);
+#pragma unroll
+      for (int b = 2; b < 8; ++b) if (has_band<NB>(b)) vfma(z[b], c, x[b]);
+    }
+    to_uncoupled<V, 6>(z, u);
+    if (pl == 0) edge_term<V, 1, 2>(y, u, T(1));
+    else if (pl == 1) edge_term<V, 1, 3>(y, u, T(1));
+    else edge_term<V, 2, 3>(y, u, T(1));
   }
-};
-
-template <typename T, int NB>
-__device__ __forceinline__ void hx_item(const HXArgs<T>& a, int s, int j) {
-  GlobalLoader<T, NB> ld;
-  ld.xs = a.X + ((long long)s * a.ldx + j);
-  ld.bs = a.N * a.ldx;
-  ld.xstr[0] = a.sx * a.ldx; ld.xstr[1] = a.sy * a.ldx; ld.xstr[2] = a.ldx;
-  GlobalRecord<T> rc;
-  rc.R = a.rec + (s + (s / a.nz) * (a.nzp - a.nz));
-  rc.NP = a.NP;
-  cplx<T> y[8];
-  hx_compute<T, NB>(ld, rc, __ldg(a.msk + s), a.shift, a.cb, y);
+  from_uncoupled<V, NB>(y, x);
   cplx<T>* __restrict__ ys = a.Y + ((long long)s * a.ldy + j);
   const int ybs = a.N * a.ldy;
 #pragma unroll
   for (int b = 0; b < 8; ++b) {
     if (!has_band<NB>(b)) continue;
-    ys[(b - band_off<NB>()) * ybs] = y[b];
+    vstore(ys + (b - band_off<NB>()) * ybs, x[b]);
   }
 }
 
 constexpr int kApplyThreads = 256;
+template <typename T> struct Column { typedef VF<1> V; };     // one column's value type
+template <> struct Column<double> { typedef VD V; };
 template <typename T> struct ApplyOcc;
 template <> struct ApplyOcc<double> { static constexpr int kMinBlocks = 2; };
 template <> struct ApplyOcc<float> { static constexpr int kMinBlocks = 3; };
@@ -620,428 +568,16 @@ template <> struct ApplyOcc<float> { static constexpr int kMinBlocks = 3; };
 template <typename T, int NB>
 __global__ void __launch_bounds__(kApplyThreads, ApplyOcc<T>::kMinBlocks)
 kp_apply_kernel(const HXArgs<T> a) {
-  const int it = blockIdx.x * kApplyThreads + threadIdx.x;
+  const int it = blockIdx.x * blockDim.x + threadIdx.x;
   if (it >= a.N * a.m) return;
   const int s = it / a.m;
-  hx_item<T, NB>(a, s, it - s * a.m);
-}
-
-// ---------------------------------------------------------------------------------------------
-// Staged kernel (eight bands): a CTA owns a TY x TZ tile of (y, z) sites and MC consecutive
-// columns and walks a run of x planes. A ring of four shared-memory plane buffers holds planes
-// x-1, x, x+1 of the tile with a one-site halo in y and z while plane x+2 streams in with
-// cp.async, so every X value crosses L2 about once (plus the halo) and the 19-point stencil reads
-// come from shared memory. Smem layout of a plane: [band][y + 1][z + 1][column].
-// ---------------------------------------------------------------------------------------------
-template <typename T, int MC_, int TY_, int TZ_>
-struct Staged {
-  static constexpr int MC = MC_, TY = TY_, TZ = TZ_;
-  static constexpr int PY = TY + 2, PZ = TZ + 2;
-  static constexpr int BAND = PY * PZ * MC;        // complex elements per band of a plane
-  static constexpr int PLANE = 8 * BAND;
-  static constexpr int NSLOT = 4;
-  static constexpr int RPLANE = K_COUNT * TY * TZ;   // record values of one tile plane
-  static constexpr int THREADS = TY * TZ * MC;
-  static constexpr size_t VEC_BYTES = (size_t)NSLOT * PLANE * sizeof(cplx<T>);
-  static constexpr size_t SMEM = VEC_BYTES + (size_t)2 * RPLANE * sizeof(T);
-  static_assert(TZ % 4 == 0, "record rows are copied in 16-byte z runs");
-  static_assert(SMEM <= 231424, "over the opt-in shared memory of one CTA");
-};
-
-template <typename T>
-struct StagedArgs {
-  const T* __restrict__ rec;
-  const cplx<T>* __restrict__ X;
-  cplx<T>* __restrict__ Y;
-  int N, nx, ny, nz, ldx, ldy, m;
-  int nzp, NP;
-  int tiles_z, chunks, xsplit, xlen;
-  T shift, cb;
-};
-
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void* smem_dst, const void* gmem_src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  if (BYTES == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(d), "l"(gmem_src) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" :: "r"(d), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-template <typename T, class G>
-struct SmemLoader {
-  const cplx<T>* p[3];   // planes x-1, x, x+1 at this thread's (y, z, column)
-  __device__ __forceinline__ void at(const cplx<T>* q, int off, bool vb_only, cplx<T> (&x)[8]) const {
-#pragma unroll
-    for (int b = 0; b < 8; ++b) x[b] = (vb_only && b < 2) ? czero<T>() : q[b * G::BAND + off];
-  }
-  __device__ __forceinline__ void centre(cplx<T> (&x)[8]) const { at(p[1], 0, false, x); }
-  __device__ __forceinline__ void face(int f, cplx<T> (&x)[8]) const {
-    const int ax = f >> 1, sg = (f & 1) ? -1 : 1;
-    if (ax == 0) at(p[1 + sg], 0, false, x);
-    else if (ax == 1) at(p[1], sg * G::PZ * G::MC, false, x);
-    else at(p[1], sg * G::MC, false, x);
-  }
-  __device__ __forceinline__ void edge(int pl, int e, cplx<T> (&x)[8]) const {
-    const int sa = (e & 1) ? -1 : 1, sb = (e & 2) ? -1 : 1;
-    if (pl == 0) at(p[1 + sa], sb * G::PZ * G::MC, true, x);                 // a = x, b = y
-    else if (pl == 1) at(p[1 + sb], sa * G::MC, true, x);                    // a = z, b = x
-    else at(p[1], sa * G::MC + sb * G::PZ * G::MC, true, x);                 // a = z, b = y
-  }
-  // packed complex64 loads
-  __device__ __forceinline__ void at2(const cplx<T>* q, int off, int b0, f2 (&x)[8]) const {
-#pragma unroll
-    for (int b = b0; b < 8; ++b) x[b] = *reinterpret_cast<const f2*>(q + b * G::BAND + off);
-  }
-  __device__ __forceinline__ void centre2(f2 (&x)[8]) const { at2(p[1], 0, 0, x); }
-  __device__ __forceinline__ void face2(int f, f2 (&x)[8]) const {
-    const int ax = f >> 1, sg = (f & 1) ? -1 : 1;
-    if (ax == 0) at2(p[1 + sg], 0, 0, x);
-    else if (ax == 1) at2(p[1], sg * G::PZ * G::MC, 0, x);
-    else at2(p[1], sg * G::MC, 0, x);
-  }
-  __device__ __forceinline__ void edge2(int pl, int e, f2 (&x)[8]) const {
-    const int sa = (e & 1) ? -1 : 1, sb = (e & 2) ? -1 : 1;
-    if (pl == 0) at2(p[1 + sa], sb * G::PZ * G::MC, 2, x);
-    else if (pl == 1) at2(p[1 + sb], sa * G::MC, 2, x);
-    else at2(p[1], sa * G::MC + sb * G::PZ * G::MC, 2, x);
-  }
-};
-
-template <typename T, class G, bool V16>
-__device__ __forceinline__ void copy_plane(const StagedArgs<T>& a, cplx<T>* slot, int xp,
-                                           int y0, int z0, int c0) {
-  constexpr int EPU = V16 ? (int)(16 / sizeof(cplx<T>)) : 1;   // complex elements per copy
-  constexpr int UPC = G::MC / EPU;                              // copies per (band, y, z) cell
-  constexpr int UNITS = 8 * G::PY * G::PZ * UPC;
-  for (int u = threadIdx.x; u < UNITS; u += G::THREADS) {
-    const int cu = u % UPC;
-    int r = u / UPC;
-    const int zz = r % G::PZ; r /= G::PZ;
-    const int yy = r % G::PY;
-    const int bb = r / G::PY;
-    const int gy = y0 - 1 + yy, gz = z0 - 1 + zz, gc = c0 + cu * EPU;
-    if (gy < 0 || gy >= a.ny || gz < 0 || gz >= a.nz || gc >= a.m) continue;
-    const int site = (xp * a.ny + gy) * a.nz + gz;
-    const cplx<T>* src = a.X + ((long long)(bb * a.N + site) * a.ldx + gc);
-    cplx<T>* dst = slot + ((bb * G::PY + yy) * G::PZ + zz) * G::MC + cu * EPU;
-    cp_async<V16 ? 16 : (int)sizeof(cplx<T>)>(dst, src);
-  }
-}
-
-// The tile's records of plane xp: rows (entry k, y) of TZ values, in 16-byte runs (z0 and TZ are
-// multiples of 4, nzp too, so a run never straddles the padded row end).
-template <typename T, class G>
-__device__ __forceinline__ void copy_record(const StagedArgs<T>& a, T* slot, int xp, int y0,
-                                            int z0) {
-  constexpr int EPU = (int)(16 / sizeof(T));
-  constexpr int RUNS = G::TZ / EPU;
-  constexpr int UNITS = K_COUNT * G::TY * RUNS;
-  for (int u = threadIdx.x; u < UNITS; u += G::THREADS) {
-    const int ru = u % RUNS;
-    const int r = u / RUNS;
-    const int ty = r % G::TY;
-    const int k = r / G::TY;
-    const int gy = y0 + ty, gz = z0 + ru * EPU;
-    if (gy >= a.ny || gz >= a.nzp) continue;
-    const T* src = a.rec + ((long long)k * a.NP + ((long long)xp * a.ny + gy) * a.nzp + gz);
-    cp_async<16>(slot + (k * G::TY + ty) * G::TZ + ru * EPU, src);
-  }
-}
-
-template <typename T, class G>
-struct SmemRecord {
-  const T* r;     // record slot + ty * TZ + tz
-  __device__ __forceinline__ T own(int k) const { return r[k * G::TY * G::TZ]; }
-  __device__ __forceinline__ T face(int ax, int dir, int k) const {
-    return own(K_FACE + 5 * (2 * ax + dir) + k);
-  }
-};
-
-template <typename T, class G, bool V16>
-__global__ void __launch_bounds__(G::THREADS, 1) kp_apply_staged_kernel(const StagedArgs<T> a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* ring = reinterpret_cast<cplx<T>*>(smem_raw);
-  T* rring = reinterpret_cast<T*>(smem_raw + G::VEC_BYTES);
-  int bid = blockIdx.x;
-  const int xs = bid % a.xsplit; bid /= a.xsplit;
-  const int ch = bid % a.chunks; bid /= a.chunks;
-  const int tzi = bid % a.tiles_z;
-  const int tyi = bid / a.tiles_z;
-  const int c0 = ch * G::MC, y0 = tyi * G::TY, z0 = tzi * G::TZ;
-  const int xa = xs * a.xlen, xb = min(a.nx, xa + a.xlen);
-  if (c0 >= a.m || xa >= xb) return;          // uniform over the CTA
-  const int t = threadIdx.x;
-  const int c = t % G::MC, tz = (t / G::MC) % G::TZ, ty = t / (G::MC * G::TZ);
-  const int iy = y0 + ty, iz = z0 + tz, col = c0 + c;
-  const bool active = iy < a.ny && iz < a.nz && col < a.m;
-  const int cell = ((ty + 1) * G::PZ + (tz + 1)) * G::MC + c;
-
-  if (xa > 0) copy_plane<T, G, V16>(a, ring + ((xa - 1) & 3) * G::PLANE, xa - 1, y0, z0, c0);
-  cp_async_commit();
-  copy_plane<T, G, V16>(a, ring + (xa & 3) * G::PLANE, xa, y0, z0, c0);
-  copy_record<T, G>(a, rring + (xa & 1) * G::RPLANE, xa, y0, z0);
-  cp_async_commit();
-  if (xa + 1 < a.nx) copy_plane<T, G, V16>(a, ring + ((xa + 1) & 3) * G::PLANE, xa + 1, y0, z0, c0);
-  cp_async_commit();
-  for (int x = xa; x < xb; ++x) {
-    cp_async_wait_all();
-    __syncthreads();                          // planes x-1..x+1 landed; slot (x+2) & 3 is free
-    if (x + 2 <= xb && x + 2 < a.nx)
-      copy_plane<T, G, V16>(a, ring + ((x + 2) & 3) * G::PLANE, x + 2, y0, z0, c0);
-    if (x + 1 < xb) copy_record<T, G>(a, rring + ((x + 1) & 1) * G::RPLANE, x + 1, y0, z0);
-    cp_async_commit();
-    if (!active) continue;
-    SmemLoader<T, G> ld;
-    ld.p[0] = ring + ((x + 3) & 3) * G::PLANE + cell;
-    ld.p[1] = ring + (x & 3) * G::PLANE + cell;
-    ld.p[2] = ring + ((x + 1) & 3) * G::PLANE + cell;
-    const int s = (x * a.ny + iy) * a.nz + iz;
-    SmemRecord<T, G> rc;
-    rc.r = rring + (x & 1) * G::RPLANE + ty * G::TZ + tz;
-    cplx<T> y[8];
-    hx_compute<T, 8>(ld, rc, site_mask(x, iy, iz, a.nx, a.ny, a.nz), a.shift, a.cb, y);
-    cplx<T>* __restrict__ ys = a.Y + ((long long)s * a.ldy + col);
-    const int ybs = a.N * a.ldy;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) ys[b * ybs] = y[b];
-  }
-  cp_async_wait_all();
-}
-
-// ---------------------------------------------------------------------------------------------
-// TMA kernel (eight bands, complex64). The same x walk as the staged kernel, with three changes:
-//   * the planes and the record rows are brought in by the tensor-memory accelerator
-//     (cp.async.bulk.tensor, one elected thread, completion on an mbarrier per ring slot) from
-//     tensor maps over this GPU's X and record; coordinates outside the grid (the halo at a wall,
-//     planes -1 and nx) read as zeros, so no thread computes an address or a neighbour mask:
-//     every weight a missing neighbour would need is zero in the record anyway;
-//   * every thread owns one site and two adjacent columns: each coefficient broadcast and record
-//     read serves both, and a band of both columns is one 16-byte shared load;
-//   * a ring of NSLOT planes keeps NSLOT - 3 planes in flight ahead of the compute.
-// Smem of a plane as the TMA box lands it: [band][y + 1][z + 1][column] (MC columns).
-// ---------------------------------------------------------------------------------------------
-template <int C, class L, class Rc>
-__device__ __forceinline__ void hx_packed_cols(const L& ld, const Rc& rc, float shift, float cb,
-                                               float2 (&Y)[C][8]) {
-  const float sq2 = 1.41421356237309504880f, sq3 = 1.73205080756887729353f;
-  const float sq32 = 1.22474487139158904910f, isq2 = 0.70710678118654752440f;
-  const f2 C2 = f2bc(sq2), CN2 = f2bc(-sq2), C3 = f2bc(sq3), C32 = f2bc(sq32);
-  const f2 CN32 = f2bc(-sq32), Ci2 = f2bc(isq2), CNi2 = f2bc(-isq2), CN1 = f2bc(-1.f);
-  const f2 CB = f2bc(cb);
-  f2 y[C][8], yi[C][8], x[C][8];
-
-  // ---- local block, the shift -sigma folded into the diagonal ---------------------------
-  ld.centre(x);
-  {
-    const float Rr = rc.own(K_RRE), Ri = rc.own(K_RIM), Sr = rc.own(K_SRE), Si = rc.own(K_SIM);
-    const float q2 = rc.own(K_Q2);
-    const f2 PA = f2bc(rc.own(K_A) + shift), P2 = f2bc(rc.own(K_A2) + shift);
-    const f2 P3 = f2bc(rc.own(K_A3) + shift), P6 = f2bc(rc.own(K_A6) + shift);
-    const f2 Q2 = f2bc(q2), NQ2 = f2bc(-q2);
-    const f2 SR = f2bc(Sr), NSR = f2bc(-Sr), SI = f2bc(Si), NSI = f2bc(-Si);
-    const f2 RR = f2bc(Rr), RI = f2bc(Ri), NRI = f2bc(-Ri);
-    const f2 S32R = f2bc(sq32 * Sr), S32I = f2bc(sq32 * Si), NS32I = f2bc(-sq32 * Si);
-    const f2 R2R = f2bc(sq2 * Rr), NR2R = f2bc(-sq2 * Rr), R2I = f2bc(sq2 * Ri);
-    const f2 NR2I = f2bc(-sq2 * Ri);
-    const f2 SI2R = f2bc(isq2 * Sr), SI2I = f2bc(isq2 * Si), NSI2I = f2bc(-isq2 * Si);
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      const f2* xc = x[c];
-      f2* yc = y[c];
-      f2* ic = yi[c];
-      yc[0] = mul2(PA, xc[0]); yc[1] = mul2(PA, xc[1]);
-      ic[0] = 0ull; ic[1] = 0ull;
-      yc[2] = fma2(NSR, xc[3], mul2(P2, xc[2]));   ic[2] = mul2(SI, xc[3]);
-      yc[2] = fma2(RR, xc[4], yc[2]);              ic[2] = fma2(RI, xc[4], ic[2]);
-      yc[2] = fma2(S32R, xc[6], yc[2]);            ic[2] = fma2(S32I, xc[6], ic[2]);
-      yc[2] = fma2(NQ2, xc[7], yc[2]);
-      yc[3] = fma2(NSR, xc[2], mul2(P3, xc[3]));   ic[3] = mul2(NSI, xc[2]);
-      yc[3] = fma2(RR, xc[5], yc[3]);              ic[3] = fma2(RI, xc[5], ic[3]);
-      yc[3] = fma2(NR2R, xc[6], yc[3]);            ic[3] = fma2(NR2I, xc[6], ic[3]);
-      yc[3] = fma2(SI2R, xc[7], yc[3]);            ic[3] = fma2(SI2I, xc[7], ic[3]);
-      yc[4] = fma2(RR, xc[2], mul2(P3, xc[4]));    ic[4] = mul2(NRI, xc[2]);
-      yc[4] = fma2(SR, xc[5], yc[4]);              ic[4] = fma2(NSI, xc[5], ic[4]);
-      yc[4] = fma2(SI2R, xc[6], yc[4]);            ic[4] = fma2(NSI2I, xc[6], ic[4]);
-      yc[4] = fma2(R2R, xc[7], yc[4]);             ic[4] = fma2(NR2I, xc[7], ic[4]);
-      yc[5] = fma2(RR, xc[3], mul2(P2, xc[5]));    ic[5] = mul2(NRI, xc[3]);
-      yc[5] = fma2(SR, xc[4], yc[5]);              ic[5] = fma2(SI, xc[4], ic[5]);
-      yc[5] = fma2(Q2, xc[6], yc[5]);
-      yc[5] = fma2(S32R, xc[7], yc[5]);            ic[5] = fma2(NS32I, xc[7], ic[5]);
-      yc[6] = fma2(S32R, xc[2], mul2(P6, xc[6]));  ic[6] = mul2(NS32I, xc[2]);
-      yc[6] = fma2(NR2R, xc[3], yc[6]);            ic[6] = fma2(R2I, xc[3], ic[6]);
-      yc[6] = fma2(SI2R, xc[4], yc[6]);            ic[6] = fma2(SI2I, xc[4], ic[6]);
-      yc[6] = fma2(Q2, xc[5], yc[6]);
-      yc[7] = fma2(NQ2, xc[2], mul2(P6, xc[7]));
-      yc[7] = fma2(SI2R, xc[3], yc[7]);            ic[7] = mul2(NSI2I, xc[3]);
-      yc[7] = fma2(R2R, xc[4], yc[7]);             ic[7] = fma2(R2I, xc[4], ic[7]);
-      yc[7] = fma2(S32R, xc[5], yc[7]);            ic[7] = fma2(S32I, xc[5], ic[7]);
-    }
-  }
-
-  // ---- six face neighbours (a missing neighbour reads as zero, its weights are zero) ----
-#pragma unroll
-  for (int f = 0; f < 6; ++f) {
-    const int ax = f >> 1, dir = f & 1;
-    ld.face(f, x);
-    const float kp = rc.face(ax, dir, 0), k2 = rc.face(ax, dir, 1);
-    const float kq = (ax == 2 ? -2.f : 1.f) * k2;
-    const f2 KPQ = f2bc(kq - kp), NKPQ = f2bc(-kp - kq), NKP = f2bc(-kp);
-    const f2 K2Q = f2bc(sq2 * kq), NK2Q = f2bc(-sq2 * kq);
-    const float kr = (ax == 0 ? -sq3 : sq3) * k2;
-    const f2 KR = f2bc(kr), K2R = f2bc(sq2 * kr), NK2R = f2bc(-sq2 * kr);
-    const float su = rc.face(ax, dir, 2), svr = rc.face(ax, dir, 3), svi = rc.face(ax, dir, 4);
-    const f2 SVI = f2bc(svi), SVR = f2bc(svr), SU = f2bc(su), NSVR = f2bc(-svr), NSU = f2bc(-su);
-    const f2 S2SU = f2bc(sq2 * su), N3SVI = f2bc(-sq3 * svi), S3SVR = f2bc(sq3 * svr);
-    const f2 N3SVR = f2bc(-sq3 * svr), N2SVI = f2bc(-sq2 * svi), N2SVR = f2bc(-sq2 * svr);
-    const f2 S2SVI = f2bc(sq2 * svi);
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      const f2* xc = x[c];
-      f2* yc = y[c];
-      f2* ic = yi[c];
-      yc[0] = fma2(CB, xc[0], yc[0]); yc[1] = fma2(CB, xc[1], yc[1]);
-      yc[2] = fma2(KPQ, xc[2], yc[2]); yc[2] = fma2(NK2Q, xc[7], yc[2]);
-      yc[3] = fma2(NKPQ, xc[3], yc[3]);
-      yc[4] = fma2(NKPQ, xc[4], yc[4]);
-      yc[5] = fma2(KPQ, xc[5], yc[5]); yc[5] = fma2(K2Q, xc[6], yc[5]);
-      yc[6] = fma2(NKP, xc[6], yc[6]); yc[6] = fma2(K2Q, xc[5], yc[6]);
-      yc[7] = fma2(NKP, xc[7], yc[7]); yc[7] = fma2(NK2Q, xc[2], yc[7]);
-      if (ax < 2) {
-        yc[2] = fma2(KR, xc[4], yc[2]);
-        yc[3] = fma2(KR, xc[5], yc[3]); yc[3] = fma2(NK2R, xc[6], yc[3]);
-        yc[4] = fma2(KR, xc[2], yc[4]); yc[4] = fma2(K2R, xc[7], yc[4]);
-        yc[5] = fma2(KR, xc[3], yc[5]);
-        yc[6] = fma2(NK2R, xc[3], yc[6]);
-        yc[7] = fma2(K2R, xc[4], yc[7]);
-      }
-      {
-        const f2 t = fma2(C2, xc[7], xc[2]);        // x2 + sqrt2 x7
-        const f2 u = mul2(C3, xc[4]);               // sqrt3 x4
-        yc[0] = fma2(SVI, sub2(u, t), yc[0]);
-        ic[0] = fma2(NSVR, add2(u, t), ic[0]);
-        ic[0] = fma2(SU, fma2(C2, xc[5], xc[6]), ic[0]);
-        const f2 v = mul2(C3, xc[3]);               // sqrt3 x3
-        const f2 w = fma2(CN2, xc[6], xc[5]);       // x5 - sqrt2 x6
-        yc[1] = fma2(SVI, sub2(v, w), yc[1]);
-        ic[1] = fma2(SVR, add2(v, w), ic[1]);
-        ic[1] = fma2(SU, fma2(C2, xc[2], mul2(CN1, xc[7])), ic[1]);
-      }
-      yc[2] = fma2(SVI, xc[0], yc[2]);   ic[2] = fma2(NSVR, xc[0], ic[2]); ic[2] = fma2(S2SU, xc[1], ic[2]);
-      yc[3] = fma2(N3SVI, xc[1], yc[3]); ic[3] = fma2(S3SVR, xc[1], ic[3]);
-      yc[4] = fma2(N3SVI, xc[0], yc[4]); ic[4] = fma2(N3SVR, xc[0], ic[4]);
-      yc[5] = fma2(SVI, xc[1], yc[5]);   ic[5] = fma2(S2SU, xc[0], ic[5]); ic[5] = fma2(SVR, xc[1], ic[5]);
-      yc[6] = fma2(N2SVI, xc[1], yc[6]); ic[6] = fma2(N2SVR, xc[1], ic[6]); ic[6] = fma2(SU, xc[0], ic[6]);
-      yc[7] = fma2(S2SVI, xc[0], yc[7]); ic[7] = fma2(N2SVR, xc[0], ic[7]); ic[7] = fma2(NSU, xc[1], ic[7]);
-    }
-  }
-
-  // ---- twelve edge neighbours: z = sum_e c_e x_e, then the plane's band mixing ---------
-#pragma unroll
-  for (int pl = 0; pl < 3; ++pl) {
-    f2 z[C][8];
-#pragma unroll
-    for (int c = 0; c < C; ++c)
-#pragma unroll
-      for (int b = 2; b < 8; ++b) z[c][b] = 0ull;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      ld.edge(pl, e, x);
-      const f2 W = f2bc(rc.own(K_EDGE + 4 * pl + e));
-#pragma unroll
-      for (int c = 0; c < C; ++c)
-#pragma unroll
-        for (int b = 2; b < 8; ++b) z[c][b] = fma2(W, x[c][b], z[c][b]);
-    }
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      const f2* zc = z[c];
-      f2* yc = y[c];
-      f2* ic = yi[c];
-      if (pl == 0) {            // R: +i z, R^H: -i z
-        ic[2] = add2(ic[2], zc[4]); ic[4] = sub2(ic[4], zc[2]);
-        ic[3] = add2(ic[3], zc[5]); ic[5] = sub2(ic[5], zc[3]);
-        ic[3] = fma2(CN2, zc[6], ic[3]); ic[6] = fma2(C2, zc[3], ic[6]);
-        ic[4] = fma2(CN2, zc[7], ic[4]); ic[7] = fma2(C2, zc[4], ic[7]);
-      } else if (pl == 1) {     // S, S^H: z
-        yc[3] = sub2(yc[3], zc[2]); yc[2] = fma2(C32, zc[6], yc[2]); yc[3] = fma2(Ci2, zc[7], yc[3]);
-        yc[5] = add2(yc[5], zc[4]); yc[6] = fma2(Ci2, zc[4], yc[6]); yc[7] = fma2(C32, zc[5], yc[7]);
-        yc[2] = sub2(yc[2], zc[3]); yc[6] = fma2(C32, zc[2], yc[6]); yc[7] = fma2(Ci2, zc[3], yc[7]);
-        yc[4] = add2(yc[4], zc[5]); yc[4] = fma2(Ci2, zc[6], yc[4]); yc[5] = fma2(C32, zc[7], yc[5]);
-      } else {                  // S: -i z, S^H: +i z
-        ic[3] = add2(ic[3], zc[2]); ic[2] = fma2(CN32, zc[6], ic[2]); ic[3] = fma2(CNi2, zc[7], ic[3]);
-        ic[5] = sub2(ic[5], zc[4]); ic[6] = fma2(CNi2, zc[4], ic[6]); ic[7] = fma2(CN32, zc[5], ic[7]);
-        ic[2] = sub2(ic[2], zc[3]); ic[6] = fma2(C32, zc[2], ic[6]); ic[7] = fma2(Ci2, zc[3], ic[7]);
-        ic[4] = add2(ic[4], zc[5]); ic[4] = fma2(Ci2, zc[6], ic[4]); ic[5] = fma2(C32, zc[7], ic[5]);
-      }
-    }
-  }
-
-  // ---- Y = y + i yi -------------------------------------------------------------------
-#pragma unroll
-  for (int c = 0; c < C; ++c)
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const float2 a = f2up(y[c][b]), d = f2up(yi[c][b]);
-      Y[c][b] = make_float2(a.x - d.y, a.y + d.x);
-    }
-}
-
-// Two adjacent complex64 columns of one site from global memory, eight bands, for
-// hx_packed_cols: a band of both columns is one 16-byte load. A neighbour outside the grid reads
-// the site itself instead: its weight in the record is zero, so it adds nothing.
-struct GlobalPairLoader {
-  const unsigned long long* __restrict__ xs;   // &X[0, s, j], j even
-  long long bs;                                // band stride N ldx (complex values)
-  int xstr[3];                                 // site strides of x, y, z (complex values)
-  unsigned msk;                                // neighbour mask of the site (site_mask)
-  __device__ __forceinline__ void at(int off, int b0, f2 (&x)[2][8]) const {
-#pragma unroll
-    for (int b = b0; b < 8; ++b) {
-      const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(xs + (b * bs + off)));
-      x[0][b] = v.x;
-      x[1][b] = v.y;
-    }
-  }
-  __device__ __forceinline__ void centre(f2 (&x)[2][8]) const { at(0, 0, x); }
-  __device__ __forceinline__ void face(int f, f2 (&x)[2][8]) const {
-    const int off = (f & 1) ? -xstr[f >> 1] : xstr[f >> 1];
-    at(((msk >> f) & 1u) ? off : 0, 0, x);
-  }
-  __device__ __forceinline__ void edge(int pl, int e, f2 (&x)[2][8]) const {
-    const int ea = pl == 0 ? 0 : 2, eb = pl == 0 ? 1 : (pl == 1 ? 0 : 1);
-    const int sa = (e & 1) ? -1 : 1, sb = (e & 2) ? -1 : 1;
-    const int off = sa * xstr[ea] + sb * xstr[eb];
-    at(((msk >> (6 + 4 * pl + e)) & 1u) ? off : 0, 2, x);
-  }
-};
-
-// complex64, eight bands: columns j, j + 1 of site s (m, ldx and ldy even, X and Y 16-byte
-// aligned)
-__device__ __forceinline__ void hx_item_pair(const HXArgs<float>& a, int s, int j) {
-  GlobalPairLoader ld;
-  ld.xs = reinterpret_cast<const unsigned long long*>(a.X + ((long long)s * a.ldx + j));
-  ld.bs = (long long)a.N * a.ldx;
-  ld.xstr[0] = a.sx * a.ldx; ld.xstr[1] = a.sy * a.ldx; ld.xstr[2] = a.ldx;
-  ld.msk = __ldg(a.msk + s);
-  GlobalRecord<float> rc;
-  rc.R = a.rec + (s + (s / a.nz) * (a.nzp - a.nz));
-  rc.NP = a.NP;
-  float2 y[2][8];
-  hx_packed_cols<2>(ld, rc, a.shift, a.cb, y);
-  float2* __restrict__ ys = a.Y + ((long long)s * a.ldy + j);
-  const long long ybs = (long long)a.N * a.ldy;
-#pragma unroll
-  for (int b = 0; b < 8; ++b)
-    *reinterpret_cast<float4*>(ys + b * ybs) = make_float4(y[0][b].x, y[0][b].y, y[1][b].x, y[1][b].y);
+  hx_item<typename Column<T>::V, NB>(a, s, it - s * a.m);
 }
 
 // Many operators and blocks in one launch (the batched engine): CTA b serves slot k with
 // tile0[k] <= b < tile0[k+1]; the column count is read on the device (the slot's active width).
 template <typename T>
-__global__ void __launch_bounds__(kApplyThreads, 2)
+__global__ void __launch_bounds__(kApplyThreads, ApplyOcc<T>::kMinBlocks)
 kp_apply_multi_kernel(const HXSlot* __restrict__ slots, int nslots) {
   int k = 0;
   while (k + 1 < nslots && (int)blockIdx.x >= slots[k + 1].tile0) ++k;
@@ -1057,55 +593,325 @@ kp_apply_multi_kernel(const HXSlot* __restrict__ slots, int nslots) {
   a.Y = static_cast<cplx<T>*>(d.Y);
   a.N = d.N; a.ldx = d.ld_same ? m : d.ldx; a.ldy = d.ld_same ? m : d.ldy;
   a.m = m; a.sx = d.sx; a.sy = d.sy;
-  a.nz = d.sy; a.nzp = d.nzp; a.NP = d.NP;
   a.shift = d.shifted ? (T)(-d.sigma) : T(0);
   a.cb = (T)d.cb;
-  if constexpr (std::is_same<T, float>::value) {
-    // complex64: two columns per thread where the widths and pointers allow 16-byte words (the
-    // slot's CTAs past the pairs' count exit)
-    if (((m | a.ldx | a.ldy) & 1) == 0 &&
-        ((reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.Y)) & 15) == 0) {
-      const int mp = m >> 1;
-      if (it >= d.N * mp) return;
-      const int s = it / mp;
-      hx_item_pair(a, s, 2 * (it - s * mp));
-      return;
+  const bool wall_self = std::is_same<T, float>::value && ((m | a.ldx | a.ldy) & 1) == 0 &&
+                         ((reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.Y)) & 15) == 0;
+  const int s = it / m;
+  hx_item<typename Column<T>::V, 8>(a, s, it - s * m, wall_self);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Marching kernel: a CTA owns a TY x TZ tile of (y, z) sites and MC columns and marches along x.
+// Plane x + 1 of the tile (a one-site halo in y and z, zero beyond the walls) and its records
+// stream into shared memory with cp.async while plane x is worked on. The thread that copied a
+// cell takes it to the uncoupled basis in place, so every value is converted once; then each
+// thread reads the nine in-plane points of its site once and adds their contributions to the
+// outputs of planes x - 1, x and x + 1, kept in registers: 56 shared loads per value where
+// gathering the nineteen points takes 104, and one plane (not three) resident per stage. Bound by
+// shared-memory wavefronts (complex128, 68% of the pipe) and, with eight warps of 200 registers on
+// an SM, by fixed latencies; 128x128x96 x 24 columns: complex128 2.43 ms (7.36 before, direct),
+// complex64 1.29 ms (2.19 before, three resident planes in Pryor's basis), 3.8 - 4.0 TB/s.
+// Smem of a stage: [band][y + 1][z + 1][column], then the records [site][kPitch].
+// ---------------------------------------------------------------------------------------------
+template <typename T_, int TY_, int TZ_, int MC_, int MINB_>
+struct March {
+  typedef T_ T;
+  typedef typename std::conditional<std::is_same<T_, double>::value, VD, VF<2>>::type V;
+  static constexpr int TY = TY_, TZ = TZ_, MC = MC_, MINB = MINB_;
+  static constexpr int G = MC / V::C;                  // 16-byte column groups per cell
+  static constexpr int PY = TY + 2, PZ = TZ + 2;
+  static constexpr int BAND = PY * PZ * G;             // 16-byte words per band of a plane
+  static constexpr int THREADS = TY * TZ * G;
+  static constexpr int UNITS = PY * PZ * G;            // cell columns a plane copy is made of
+  static constexpr int ROUNDS = (UNITS + THREADS - 1) / THREADS;
+  static constexpr int kPitch = rec_stride<T>();
+  static constexpr int RUNITS = kPitch * (int)sizeof(T) / 16;           // 16-byte words per site
+  static_assert(MC % V::C == 0, "whole 16-byte groups");
+  template <int NB> static constexpr size_t stage_bytes() {
+    return (size_t)NB * BAND * 16 + (size_t)TY * TZ * kPitch * sizeof(T);
+  }
+  template <int NB> static constexpr size_t smem() { return 2 * stage_bytes<NB>(); }
+};
+
+template <typename T>
+struct MarchArgs {
+  const T* __restrict__ rec;
+  const cplx<T>* __restrict__ X;
+  cplx<T>* __restrict__ Y;
+  long long bsx, bsy;           // band strides N ldx, N ldy
+  int nx, ny, nz, ldx, ldy, m;
+  int tiles_z, chunks, xsplit, xlen;
+  int v16;                      // complex64: 16-byte column pairs in X
+  int v16y;                     // ... and in Y
+  T shift, cb;
+};
+
+// cp.async of 16 (or 8) bytes of which the first `src_bytes` are read, the rest zero
+__device__ __forceinline__ void cp16z(unsigned dst, const void* src, int src_bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" :: "r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void cp8z(unsigned dst, const void* src, int src_bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" :: "r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+// Band order of the values in shared memory: Pryor's as copied (band b at word b - band_off),
+// the uncoupled order after conversion: S+, X+, Y+, Z+, S-, X-, Y-, Z- (six bands: no S; RAW: the
+// S values stay in words 0 and 1, the others follow).
+template <int NB, bool RAW> __device__ __forceinline__ constexpr int uslot(int b) {
+  return NB != 8 ? (b < 4 ? b - 1 : b - 2) : (RAW ? (b < 4 ? b + 1 : b) : b);
+}
+
+// raw_s: a converted cell keeps its two S values as copied (x0, x1 in slots 0 and 1) and the
+// reader takes i times them, which complex128 folds into its multiply-adds; in complex64 the
+// conversion does it.
+template <class V> __device__ __forceinline__ constexpr bool raw_s() { return V::C == 1; }
+
+template <class V, int NB, int BAND, bool RAW>
+__device__ __forceinline__ void smem_cell(const cplx<typename V::T>* q, V (&x)[8]) {
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    if (NB != 8 && (b & 3) == 0) continue;
+    if (RAW && (b & 3) == 0) { x[b] = vi(vload(q + (size_t)(b >> 2) * BAND * V::C, (V*)nullptr)); continue; }
+    x[b] = vload(q + (size_t)uslot<NB, RAW>(b) * BAND * V::C, (V*)nullptr);
+  }
+}
+
+// one cell column in shared memory from Pryor's basis to the uncoupled one, in place
+template <class G, int NB>
+__device__ __forceinline__ void convert_cell(cplx<typename G::T>* q) {
+  typedef typename G::V V;
+  constexpr bool RAW = raw_s<V>() && NB == 8;
+  V x[8], u[8];
+#pragma unroll
+  for (int b = RAW ? 2 : 0; b < 8; ++b)
+    if (has_band<NB>(b)) x[b] = vload(q + (size_t)(b - band_off<NB>()) * G::BAND * V::C, (V*)nullptr);
+  to_uncoupled<V, RAW ? 6 : NB>(x, u);
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    if ((NB != 8 || RAW) && (b & 3) == 0) continue;
+    vstore(q + (size_t)uslot<NB, RAW>(b) * G::BAND * V::C, u[b]);
+  }
+}
+
+// the nine points of one plane added to the outputs of the plane below (lo) and its own (me), and
+// the first part of the plane above's (up, set); a part that is not wanted is left out
+template <class G, int NB, bool RAW, bool LO, bool ME, bool UP>
+__device__ __forceinline__ void march_plane(const cplx<typename G::T>* cell,
+                                            const typename G::T* r, typename G::T shift,
+                                            typename G::V::W cb, typename G::V (&lo)[8],
+                                            typename G::V (&me)[8], typename G::V (&up)[8]) {
+  typedef typename G::V V;
+  typedef typename G::T T;
+  constexpr int DY_ = G::PZ * G::G * V::C, DZ_ = G::G * V::C;    // y and z strides (elements)
+  V x[8];
+  smem_cell<V, NB, G::BAND, RAW>(cell, x);
+  if (ME) {
+    T w[8];
+    load_rec<false>(r, w);
+    local_term<V, NB>(me, x, w, shift);
+  }
+  if (LO || UP) {
+    T w[sizeof(T) == 8 ? 10 : 12];
+    load_rec<false>(r + K_FX, w);
+    // the face between this plane and the one above as the plane above sees it: same second-order
+    // weights, opposite first-order ones
+    if (UP) face_term<V, NB, 0, true, true>(up, x, w, cb);
+    if (LO) face_term<V, NB, 0, true>(lo, x, w + 5, cb);
+  }
+  T wxy[4], wzx[4], wf[20];
+  if (LO || UP) { load_rec<false>(r + K_PXY, wxy); load_rec<false>(r + K_PZX, wzx); }
+  if (ME) load_rec<false>(r + K_FYZ, wf);
+  smem_cell<V, NB, G::BAND, RAW>(cell + DY_, x);
+  if (ME) face_term<V, NB, 1, false>(me, x, wf, cb);
+  if (LO) edge_term<V, 1, 2>(lo, x, wxy[0]);
+  if (UP) edge_term<V, 1, 2>(up, x, wxy[2]);
+  smem_cell<V, NB, G::BAND, RAW>(cell - DY_, x);
+  if (ME) face_term<V, NB, 1, false>(me, x, wf + 5, cb);
+  if (LO) edge_term<V, 1, 2>(lo, x, wxy[1]);
+  if (UP) edge_term<V, 1, 2>(up, x, wxy[3]);
+  smem_cell<V, NB, G::BAND, RAW>(cell + DZ_, x);
+  if (ME) face_term<V, NB, 2, false>(me, x, wf + 10, cb);
+  if (LO) edge_term<V, 1, 3>(lo, x, wzx[0]);
+  if (UP) edge_term<V, 1, 3>(up, x, wzx[2]);
+  smem_cell<V, NB, G::BAND, RAW>(cell - DZ_, x);
+  if (ME) face_term<V, NB, 2, false>(me, x, wf + 15, cb);
+  if (LO) edge_term<V, 1, 3>(lo, x, wzx[1]);
+  if (UP) edge_term<V, 1, 3>(up, x, wzx[3]);
+  if (ME) {
+    T w[4];
+    load_rec<false>(r + K_EZY, w);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const cplx<T>* q = cell + ((e & 1) ? -DZ_ : DZ_) + ((e & 2) ? -DY_ : DY_);
+#pragma unroll
+      for (int b = 0; b < 8; ++b)
+        if ((b & 3) >= 2) x[b] = vload(q + (size_t)uslot<NB, RAW>(b) * G::BAND * V::C, (V*)nullptr);
+      edge_term<V, 2, 3>(me, x, w[e]);
     }
   }
-  const int s = it / m;
-  hx_item<T, 8>(a, s, it - s * m);
 }
 
-
-// mbarrier and bulk-tensor copy primitives (PTX ISA: mbarrier, cp.async.bulk.tensor)
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
+template <class G, int NB>
+__global__ void __launch_bounds__(G::THREADS, G::MINB)
+kp_march_kernel(const MarchArgs<typename G::T> a) {
+  typedef typename G::V V;
+  typedef typename G::T T;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool RAW = raw_s<V>() && NB == 8;
+  constexpr int STAGE = (int)G::template stage_bytes<NB>();
+  int bid = blockIdx.x;
+  const int xs = bid % a.xsplit; bid /= a.xsplit;
+  const int ch = bid % a.chunks; bid /= a.chunks;
+  const int tzi = bid % a.tiles_z;
+  const int tyi = bid / a.tiles_z;
+  const int c0 = ch * G::MC, y0 = tyi * G::TY, z0 = tzi * G::TZ;
+  const int xa = xs * a.xlen, xb = min(a.nx, xa + a.xlen);
+  if (c0 >= a.m || xa >= xb) return;          // uniform over the CTA
+  const int t = threadIdx.x;
+  const int g = t % G::G, tz = (t / G::G) % G::TZ, ty = t / (G::G * G::TZ);
+  const int iy = y0 + ty, iz = z0 + tz, col = c0 + g * V::C;
+  const bool active = iy < a.ny && iz < a.nz && col < a.m;
+  const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem_raw);
+  // the cell columns this thread copies and converts: source of band 0 in plane 0, valid bytes
+  const cplx<T>* src[G::ROUNDS];
+  int bytes[G::ROUNDS];
+#pragma unroll
+  for (int k = 0; k < G::ROUNDS; ++k) {
+    const int u = t + k * G::THREADS;
+    const int cu = u % G::G, zz = (u / G::G) % G::PZ, yy = u / (G::G * G::PZ);
+    const int gy = y0 - 1 + yy, gz = z0 - 1 + zz, gc = c0 + cu * V::C;
+    const bool in = u < G::UNITS && gy >= 0 && gy < a.ny && gz >= 0 && gz < a.nz && gc < a.m;
+    bytes[k] = in ? min(V::C, a.m - gc) * (int)sizeof(cplx<T>) : 0;
+    src[k] = a.X + (in ? ((long long)gy * a.nz + gz) * a.ldx + gc : 0);
+  }
+  const long long xstr = (long long)a.ny * a.nz * a.ldx;
+  auto copy_plane = [&](int p) {
+    const unsigned st = sbase + (p & 1) * STAGE;
+#pragma unroll
+    for (int k = 0; k < G::ROUNDS; ++k) {
+      const int u = t + k * G::THREADS;
+      if (u < G::UNITS) {
+        const unsigned dst = st + u * 16;
+        const cplx<T>* s = src[k] + (bytes[k] ? p * xstr : 0);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          const cplx<T>* sb = s + (bytes[k] ? b * a.bsx : 0);
+          if (sizeof(T) == 8 || a.v16) {
+            cp16z(dst + b * G::BAND * 16, sb, bytes[k]);
+          } else {
+            cp8z(dst + b * G::BAND * 16, sb, min(bytes[k], 8));
+            cp8z(dst + b * G::BAND * 16 + 8, sb + (bytes[k] > 8 ? 1 : 0), max(bytes[k] - 8, 0));
+          }
+        }
+      }
+    }
+    // records of the tile's sites
+    const unsigned rt = st + NB * G::BAND * 16;
+    for (int u = t; u < G::TY * G::TZ * G::RUNITS; u += G::THREADS) {
+      const int w = u % G::RUNITS, site = u / G::RUNITS;
+      const int gy = y0 + site / G::TZ, gz = z0 + site % G::TZ;
+      if (gy < a.ny && gz < a.nz)
+        cp16z(rt + site * (G::kPitch * (int)sizeof(T)) + w * 16,
+              a.rec + (((long long)p * a.ny + gy) * a.nz + gz) * G::kPitch + w * (16 / (int)sizeof(T)), 16);
+    }
+    cp_async_commit();
+  };
+  auto convert_plane = [&](int p) {
+    cplx<T>* st = reinterpret_cast<cplx<T>*>(smem_raw + (p & 1) * STAGE);
+#pragma unroll
+    for (int k = 0; k < G::ROUNDS; ++k) {
+      if (bytes[k] == 0) continue;
+      cplx<T>* q = st + (size_t)(t + k * G::THREADS) * V::C;
+      convert_cell<G, NB>(q);
+    }
+  };
+  V lo[8], me[8], up[8];
+#pragma unroll
+  for (int b = 0; b < 8; ++b) { vzero(lo[b]); vzero(me[b]); vzero(up[b]); }
+  const int p0 = max(xa - 1, 0), p1 = min(xb, a.nx - 1);     // planes read
+  const auto cb = W_<V>(a.cb);
+  const int cell = ((ty + 1) * G::PZ + (tz + 1)) * G::G + g;
+  cplx<T>* __restrict__ yout = a.Y + ((long long)iy * a.nz + iz) * a.ldy + col;
+  const long long ystr = (long long)a.ny * a.nz * a.ldy;
+  copy_plane(p0);
+  for (int p = p0; p <= p1; ++p) {
+    cp_async_wait_all();
+    convert_plane(p);
+    __syncthreads();          // plane p is complete; every thread is done with plane p - 1
+    if (p < p1) copy_plane(p + 1);
+    if (active) {
+      const cplx<T>* c = reinterpret_cast<const cplx<T>*>(smem_raw + (p & 1) * STAGE) + (size_t)cell * V::C;
+      const T* r = reinterpret_cast<const T*>(smem_raw + (p & 1) * STAGE + NB * G::BAND * 16) +
+                   (ty * G::TZ + tz) * G::kPitch;
+      if (p < xa) march_plane<G, NB, RAW, false, false, true>(c, r, a.shift, cb, lo, me, up);
+      else if (p == xb) march_plane<G, NB, RAW, true, false, false>(c, r, a.shift, cb, lo, me, up);
+      else march_plane<G, NB, RAW, true, true, true>(c, r, a.shift, cb, lo, me, up);
+    }
+    // output of plane q = p - 1 is complete; the last one also when no plane follows
+#pragma unroll 1
+    for (int q = p - 1; q <= p; ++q) {
+      const bool write = q == p - 1 ? q >= xa : (p == p1 && p < xb);
+      if (q == p && !write) break;
+      if (write && active) {
+        V x[8];
+        from_uncoupled<V, NB>(lo, x);
+        cplx<T>* ys = yout + q * ystr;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          if (!has_band<NB>(b)) continue;
+          cplx<T>* yb = ys + (b - band_off<NB>()) * a.bsy;
+          if constexpr (V::C == 1) {
+            vstore(yb, x[b]);
+          } else if (a.v16y && col + 1 < a.m) {
+            vstore(yb, x[b]);
+          } else {
+            const float2 e0 = f2up(x[b].c[0]), e1 = f2up(x[b].c[1]);
+            yb[0] = e0;
+            if (col + 1 < a.m) yb[1] = e1;
+          }
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < 8; ++b) { lo[b] = me[b]; me[b] = up[b]; }
+    }
+  }
 }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+
+// ---------------------------------------------------------------------------------------------
+// The same march fed by the tensor-memory accelerator: one elected thread brings in a plane with
+// one bulk tensor copy (coordinates beyond the walls read as zeros) and the tile's records with
+// one bulk copy per tile row, completion on an mbarrier per stage, so no thread computes a copy
+// address. NS stages of planes are in flight; a plane is converted (CONV) after the previous
+// one's arithmetic, before the barrier that the two share. The launcher takes it where a tensor
+// map can describe the block (tma_fits).
+// ---------------------------------------------------------------------------------------------
+__device__ int g_apply_fault;      // set when a wait on a copy gave up (qdkp_device_fault)
+
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_fence_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes)
                : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
+__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
+  unsigned ok;
   asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
                " selp.b32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
 // Bounded wait: gives up after about a second of SM clocks (a copy that never lands).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   while (!mbar_try_wait(bar, parity))
     if (clock64() - t0 > 2000000000LL) return false;
   return true;
 }
-__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
+__device__ __forceinline__ void tma_load_5d(unsigned dst, const CUtensorMap* map, unsigned bar,
                                             int c0, int c1, int c2, int c3, int c4) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
@@ -1113,98 +919,25 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
       :: "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2),
          "r"(c3), "r"(c4) : "memory");
 }
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
-                                            int c0, int c1, int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      :: "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2),
-         "r"(c3) : "memory");
+__device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
-struct RegRecord {                 // a site's record row in registers
-  float v[K_COUNT];
-  __device__ __forceinline__ float own(int k) const { return v[k]; }
-  __device__ __forceinline__ float face(int ax, int dir, int k) const {
-    return v[K_FACE + 5 * (2 * ax + dir) + k];
-  }
-};
-
-// Set by a TMA kernel whose wait on a copy gave up (qdkp_device_fault reads and clears it).
-__device__ int g_apply_fault;
-
-// RREG: the record row of each site is prefetched by its threads into registers one plane ahead
-// (no record slots in shared memory, which leaves room for larger tiles)
-template <int TY_, int TZ_, int G_, int NSLOT_, int MINB_ = 1, bool RREG_ = false>
-struct Tma {
-  static constexpr int TY = TY_, TZ = TZ_, G = G_, NSLOT = NSLOT_, MINB = MINB_;
-  static constexpr bool RREG = RREG_;
-  static constexpr int CPT = 2;                          // columns per thread
-  static constexpr int MC = CPT * G;                     // columns per CTA
-  static constexpr int PY = TY + 2, PZ = TZ + 2;
-  static constexpr int BAND = PY * PZ * MC;              // complex64 elements per band of a plane
-  static constexpr int PLANE_BYTES = 8 * BAND * 8;
-  static constexpr int RPLANE_BYTES = K_COUNT * TY * TZ * 4;
-  static constexpr int RSTRIDE = (RPLANE_BYTES + 127) / 128 * 128;
-  static constexpr int THREADS = TY * TZ * G;
-  static constexpr int BARS = NSLOT + (RREG ? 0 : 2);
-  static constexpr size_t SMEM = 1024 + (size_t)NSLOT * PLANE_BYTES + (RREG ? 0 : 2 * RSTRIDE) +
-                                 8 * BARS;
-  static_assert(TZ % 4 == 0, "record rows are copied in 16-byte z runs");
-  static_assert(PLANE_BYTES % 128 == 0, "ring slots stay 128-byte aligned");
-  static_assert(NSLOT >= 4, "planes x-1, x, x+1 and at least one in flight");
-  static_assert(SMEM * MINB <= 232448, "over the shared memory of one SM");
-};
-
-struct TmaArgs {
-  float2* __restrict__ Y;
-  const float* __restrict__ rec;   // the FP32 record (read directly by RREG shapes)
-  int nzp, NP;
-  int N, nx, ny, nz, ldy, m;
-  int tiles_z, chunks, xsplit, xlen;
-  int vec_store;          // Y is 16-byte aligned with an even leading dimension
-  float shift, cb;
-};
-
-template <class G>
-struct TmaLoader {
-  const unsigned long long* p[3];   // planes x-1, x, x+1 at this thread's (y, z, column pair)
-  __device__ __forceinline__ void at(const unsigned long long* q, int off, int b0,
-                                     f2 (&x)[2][8]) const {
-#pragma unroll
-    for (int b = b0; b < 8; ++b) {
-      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(q + b * G::BAND + off);
-      x[0][b] = v.x;
-      x[1][b] = v.y;
-    }
-  }
-  __device__ __forceinline__ void centre(f2 (&x)[2][8]) const { at(p[1], 0, 0, x); }
-  __device__ __forceinline__ void face(int f, f2 (&x)[2][8]) const {
-    const int ax = f >> 1, sg = (f & 1) ? -1 : 1;
-    if (ax == 0) at(p[1 + sg], 0, 0, x);
-    else if (ax == 1) at(p[1], sg * G::PZ * G::MC, 0, x);
-    else at(p[1], sg * G::MC, 0, x);
-  }
-  __device__ __forceinline__ void edge(int pl, int e, f2 (&x)[2][8]) const {
-    const int sa = (e & 1) ? -1 : 1, sb = (e & 2) ? -1 : 1;
-    if (pl == 0) at(p[1 + sa], sb * G::PZ * G::MC, 2, x);                 // a = x, b = y
-    else if (pl == 1) at(p[1 + sb], sa * G::MC, 2, x);                    // a = z, b = x
-    else at(p[1], sa * G::MC + sb * G::PZ * G::MC, 2, x);                 // a = z, b = y
-  }
-};
-
-template <class G>
+template <class G, int NB, int NS, bool CONV>
 __global__ void __launch_bounds__(G::THREADS, G::MINB)
-kp_apply_tma_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmr,
-                    const TmaArgs a) {
+kp_march_tma_kernel(const __grid_constant__ CUtensorMap tmx, const MarchArgs<typename G::T> a) {
+  typedef typename G::V V;
+  typedef typename G::T T;
   extern __shared__ unsigned char smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t pad = ((raw + 1023u) & ~1023u) - raw;
-  unsigned char* sb = smem_raw + pad;
-  const uint32_t ring = raw + pad;
-  const uint32_t rring = ring + G::NSLOT * G::PLANE_BYTES;
-  // NSLOT plane barriers, then 2 record ones (staged records only)
-  const uint32_t bars = rring + (G::RREG ? 0 : 2 * G::RSTRIDE);
+  constexpr bool RAW = CONV && raw_s<V>() && NB == 8;
+  constexpr int STAGE = (int)G::template stage_bytes<NB>();
+  constexpr int XBYTES = NB * G::BAND * 16;
+  static_assert(STAGE % 128 == 0 && XBYTES % 128 == 0, "stages stay 128-byte aligned");
+  const unsigned raw = (unsigned)__cvta_generic_to_shared(smem_raw);
+  const unsigned pad = ((raw + 127u) & ~127u) - raw;
+  unsigned char* sm = smem_raw + pad;
+  const unsigned sbase = raw + pad, bars = sbase + NS * STAGE;
   int bid = blockIdx.x;
   const int xs = bid % a.xsplit; bid /= a.xsplit;
   const int ch = bid % a.chunks; bid /= a.chunks;
@@ -1215,269 +948,170 @@ kp_apply_tma_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_consta
   if (c0 >= a.m || xa >= xb) return;          // uniform over the CTA
   const int t = threadIdx.x;
   const int g = t % G::G, tz = (t / G::G) % G::TZ, ty = t / (G::G * G::TZ);
-  const int iy = y0 + ty, iz = z0 + tz, col = c0 + g * G::CPT;
+  const int iy = y0 + ty, iz = z0 + tz, col = c0 + g * V::C;
   const bool active = iy < a.ny && iz < a.nz && col < a.m;
-  const int cell = ((ty + 1) * G::PZ + (tz + 1)) * G::MC + g * G::CPT;
-
-  // plane with sequence number q (plane index xa - 1 + q) lives in slot q % NSLOT, and its
-  // barrier completes phase q / NSLOT; the record of plane xa + r in slot r & 1, phase r >> 1
-  auto plane_bar = [&](int q) { return bars + 8u * (uint32_t)(q % G::NSLOT); };
-  auto rec_bar = [&](int r) { return bars + 8u * (uint32_t)(G::NSLOT + (r & 1)); };
-  auto issue_plane = [&](int q) {
-    const uint32_t bar = plane_bar(q);
-    mbar_expect_tx(bar, G::PLANE_BYTES);
-    tma_load_5d(ring + (uint32_t)(q % G::NSLOT) * G::PLANE_BYTES, &tmx, bar, c0, z0 - 1, y0 - 1,
-                xa - 1 + q, 0);
+  const int p0 = max(xa - 1, 0), p1 = min(xb, a.nx - 1);     // planes read
+  const int rrows = min(G::TY, a.ny - y0), rsites = min(G::TZ, a.nz - z0);
+  // plane p lives in stage (p - p0) % NS, whose barrier completes phase (p - p0) / NS
+  auto issue = [&](int p) {
+    const int q = (p - p0) % NS;
+    const unsigned bar = bars + 8u * q, st = sbase + q * STAGE;
+    const unsigned rb = (unsigned)(rsites * G::kPitch * (int)sizeof(T));
+    mbar_expect_tx(bar, XBYTES + rrows * rb);
+    tma_load_5d(st, &tmx, bar, c0 * (int)(sizeof(cplx<T>) / 8), z0 - 1, y0 - 1, p, 0);
+    for (int r = 0; r < rrows; ++r)
+      bulk_load(st + XBYTES + r * (G::TZ * G::kPitch * (int)sizeof(T)),
+                a.rec + (((long long)p * a.ny + y0 + r) * a.nz + z0) * G::kPitch, rb, bar);
   };
-  auto issue_record = [&](int r) {
-    const uint32_t bar = rec_bar(r);
-    mbar_expect_tx(bar, G::RPLANE_BYTES);
-    tma_load_4d(rring + (uint32_t)(r & 1) * G::RSTRIDE, &tmr, bar, z0, y0, xa + r, 0);
-  };
-
   if (t == 0) {
-    for (int i = 0; i < G::BARS; ++i) mbar_init(bars + 8u * i, 1);
-    mbar_fence_init();
+    for (int i = 0; i < NS; ++i) mbar_init(bars + 8u * i, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int p = p0; p < p0 + NS && p <= p1; ++p) issue(p);
   }
   __syncthreads();
-  const int nplanes = xb - xa + 2;            // planes xa - 1 .. xb
-  int q_issued = 0, r_issued = 0;
-  if (t == 0) {
-    for (; q_issued < G::NSLOT - 1 && q_issued < nplanes; ++q_issued) issue_plane(q_issued);
-    if (!G::RREG) issue_record(r_issued++);
-  }
-  // RREG: this thread's record row of plane x, and the one of plane x + 1 in flight
-  RegRecord rcur, rnxt;
-  const long long rsite = (long long)iy * a.nzp + iz;
-  if (G::RREG && active) {
-    const float* rp = a.rec + (long long)xa * a.ny * a.nzp + rsite;
+  // the cells this thread converts (those of the halo beyond a wall hold zeros)
+  auto convert = [&](unsigned char* st) {
 #pragma unroll
-    for (int k = 0; k < K_COUNT; ++k) rcur.v[k] = __ldg(rp + (long long)k * a.NP);
-  }
-  bool ok = true;
-  for (int x = xa; x < xb; ++x) {
-    const int qx = x - xa + 1;
-    ok = ok && mbar_wait(plane_bar(qx - 1), ((qx - 1) / G::NSLOT) & 1) &&
-         mbar_wait(plane_bar(qx), (qx / G::NSLOT) & 1) &&
-         mbar_wait(plane_bar(qx + 1), ((qx + 1) / G::NSLOT) & 1);
-    // every thread is past plane x - 1: its ring slot and record slot may be refilled
-    const bool all_ok = __syncthreads_and(ok) != 0;
-    if (t == 0 && all_ok) {
-      if (q_issued < nplanes) issue_plane(q_issued++);
-      if (!G::RREG && x + 1 < xb) issue_record(r_issued++);
+    for (int k = 0; k < G::ROUNDS; ++k) {
+      const int u = t + k * G::THREADS;
+      if (u >= G::UNITS) break;
+      cplx<T>* q = reinterpret_cast<cplx<T>*>(st) + (size_t)u * V::C;
+      convert_cell<G, NB>(q);
     }
-    const int r = x - xa;
-    if (G::RREG) ok = all_ok;
-    else ok = all_ok && mbar_wait(rec_bar(r), (r >> 1) & 1);
-    if (!ok || !active) continue;
-    if (G::RREG && x + 1 < xb) {                // prefetch plane x + 1's record row
-      const float* rp = a.rec + (long long)(x + 1) * a.ny * a.nzp + rsite;
+    // these stores are ordered before the copy that refills the stage
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  };
+  V lo[8], me[8], up[8];
 #pragma unroll
-      for (int k = 0; k < K_COUNT; ++k) rnxt.v[k] = __ldg(rp + (long long)k * a.NP);
-    }
-    TmaLoader<G> ld;
-    const unsigned long long* pl = reinterpret_cast<const unsigned long long*>(sb);
-    ld.p[0] = pl + (size_t)((qx - 1) % G::NSLOT) * (G::PLANE_BYTES / 8) + cell;
-    ld.p[1] = pl + (size_t)(qx % G::NSLOT) * (G::PLANE_BYTES / 8) + cell;
-    ld.p[2] = pl + (size_t)((qx + 1) % G::NSLOT) * (G::PLANE_BYTES / 8) + cell;
-    float2 yv[2][8];
-    if constexpr (G::RREG) {
-      hx_packed_cols<2>(ld, rcur, a.shift, a.cb, yv);
-#pragma unroll
-      for (int k = 0; k < K_COUNT; ++k) rcur.v[k] = rnxt.v[k];
-    } else {
-      SmemRecord<float, G> rc;                  // record slot layout [k][ty][tz]
-      rc.r = reinterpret_cast<const float*>(sb + G::NSLOT * G::PLANE_BYTES + (r & 1) * G::RSTRIDE) +
-             ty * G::TZ + tz;
-      hx_packed_cols<2>(ld, rc, a.shift, a.cb, yv);
-    }
-    const int s = (x * a.ny + iy) * a.nz + iz;
-    float2* __restrict__ ys = a.Y + ((long long)s * a.ldy + col);
-    const long long ybs = (long long)a.N * a.ldy;
-    if (a.vec_store && col + 1 < a.m) {
-#pragma unroll
-      for (int b = 0; b < 8; ++b)
-        *reinterpret_cast<float4*>(ys + b * ybs) = make_float4(yv[0][b].x, yv[0][b].y,
-                                                               yv[1][b].x, yv[1][b].y);
-    } else {
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        ys[b * ybs] = yv[0][b];
-        if (col + 1 < a.m) ys[b * ybs + 1] = yv[1][b];
-      }
-    }
+  for (int b = 0; b < 8; ++b) { vzero(lo[b]); vzero(me[b]); vzero(up[b]); }
+  const auto cb = W_<V>(a.cb);
+  const int cell = ((ty + 1) * G::PZ + (tz + 1)) * G::G + g;
+  cplx<T>* __restrict__ yout = a.Y + ((long long)iy * a.nz + iz) * a.ldy + col;
+  const long long ystr = (long long)a.ny * a.nz * a.ldy;
+  bool ok = mbar_wait(bars, 0);
+  if (CONV) {
+    if (ok) convert(sm);
+    ok = __syncthreads_and(ok) != 0;
   }
-  if (__syncthreads_or(!ok) && t == 0) {
-    // a copy never landed: flag it, then give the copies still in flight a bounded chance to
-    // finish before the CTA's shared memory is released (thread 0 keeps the CTA resident)
-    atomicExch(&g_apply_fault, 1);
-    for (int q = max(0, q_issued - G::NSLOT); q < q_issued; ++q)
-      mbar_wait(plane_bar(q), (q / G::NSLOT) & 1);
-    for (int r = max(0, r_issued - 2); r < r_issued; ++r) mbar_wait(rec_bar(r), (r >> 1) & 1);
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// TMA kernel with a producer warp (eight bands, complex64). The ring of NSLOT planes is filled
-// by one producer warp; every ring slot has a "full" barrier (the copy landed) and an "empty"
-// barrier (every compute warp is done with the plane), so compute warps never meet at a CTA-wide
-// barrier: a warp moves on to plane x + 1 as soon as that plane has landed, and releases plane
-// x - 1 when it finishes x. Each site's record row is read by its own threads straight from
-// global memory (a record entry is used by the two threads of its site only), which leaves the
-// shared memory to the plane ring: larger tiles, or two CTAs per SM.
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
-}
-
-template <int TY_, int TZ_, int G_, int NSLOT_, int MINB_>
-struct Tma2 {
-  static constexpr int TY = TY_, TZ = TZ_, G = G_, NSLOT = NSLOT_, MINB = MINB_;
-  static constexpr int CPT = 2;
-  static constexpr int MC = CPT * G;
-  static constexpr int PY = TY + 2, PZ = TZ + 2;
-  static constexpr int BAND = PY * PZ * MC;
-  static constexpr int PLANE_BYTES = 8 * BAND * 8;
-  static constexpr int CTHREADS = TY * TZ * G;            // compute threads
-  static constexpr int CWARPS = CTHREADS / 32;
-  static constexpr int THREADS = CTHREADS + 32;           // + the producer warp
-  static constexpr size_t SMEM = 1024 + (size_t)NSLOT * PLANE_BYTES + 16 * NSLOT;
-  static_assert(CTHREADS % 32 == 0, "compute threads fill whole warps");
-  static_assert(PLANE_BYTES % 128 == 0, "ring slots stay 128-byte aligned");
-  static_assert(NSLOT >= 4, "planes x-1, x, x+1 and at least one in flight");
-  static_assert(SMEM * MINB <= 232448, "over the shared memory of one SM");
-};
-
-
-struct Tma2Args {
-  float2* __restrict__ Y;
-  const float* __restrict__ rec;
-  int N, nx, ny, nz, nzp, NP, ldy, m;
-  int tiles_z, chunks, xsplit, xlen;
-  int vec_store;
-  float shift, cb;
-};
-
-template <class G>
-__global__ void __launch_bounds__(G::THREADS, G::MINB)
-kp_apply_tma2_kernel(const __grid_constant__ CUtensorMap tmx, const Tma2Args a) {
-  extern __shared__ unsigned char smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t pad = ((raw + 1023u) & ~1023u) - raw;
-  unsigned char* sb = smem_raw + pad;
-  const uint32_t ring = raw + pad;
-  const uint32_t full = ring + G::NSLOT * G::PLANE_BYTES;        // NSLOT barriers
-  const uint32_t empty = full + 8 * G::NSLOT;                     // NSLOT barriers
-  int bid = blockIdx.x;
-  const int xs = bid % a.xsplit; bid /= a.xsplit;
-  const int ch = bid % a.chunks; bid /= a.chunks;
-  const int tzi = bid % a.tiles_z;
-  const int tyi = bid / a.tiles_z;
-  const int c0 = ch * G::MC, y0 = tyi * G::TY, z0 = tzi * G::TZ;
-  const int xa = xs * a.xlen, xb = min(a.nx, xa + a.xlen);
-  if (c0 >= a.m || xa >= xb) return;          // uniform over the CTA
-  const int t = threadIdx.x;
-  if (t == 0) {
-    for (int i = 0; i < G::NSLOT; ++i) {
-      mbar_init(full + 8u * i, 1);
-      mbar_init(empty + 8u * i, G::CWARPS);
+  int slot = 0;
+  unsigned phase = 0;
+  for (int p = p0; p <= p1; ++p) {
+    unsigned char* st = sm + slot * STAGE;
+    if (active && ok) {
+      const cplx<T>* c = reinterpret_cast<const cplx<T>*>(st) + (size_t)cell * V::C;
+      const T* r = reinterpret_cast<const T*>(st + XBYTES) + (ty * G::TZ + tz) * G::kPitch;
+      if (p < xa) march_plane<G, NB, RAW, false, false, true>(c, r, a.shift, cb, lo, me, up);
+      else if (p == xb) march_plane<G, NB, RAW, true, false, false>(c, r, a.shift, cb, lo, me, up);
+      else march_plane<G, NB, RAW, true, true, true>(c, r, a.shift, cb, lo, me, up);
     }
-    mbar_fence_init();
-  }
-  __syncthreads();
-  const int nplanes = xb - xa + 2;            // planes xa - 1 .. xb, sequence q = plane - xa + 1
-  // plane sequence q lives in slot q % NSLOT; its full barrier completes phase q / NSLOT, and
-  // the empty barrier of that slot completes phase q / NSLOT once every compute warp is done
-  if (t >= G::CTHREADS) {
-    // ---- producer warp -----------------------------------------------------------------
-    if (t == G::CTHREADS) {
-      bool ok = true;
-      int q = 0;
-      for (; q < nplanes && ok; ++q) {
-        const int s = q % G::NSLOT;
-        if (q >= G::NSLOT) ok = mbar_wait(empty + 8u * s, ((q / G::NSLOT) - 1) & 1);
-        if (!ok) break;
-        mbar_expect_tx(full + 8u * s, G::PLANE_BYTES);
-        tma_load_5d(ring + (uint32_t)s * G::PLANE_BYTES, &tmx, full + 8u * s, c0, z0 - 1, y0 - 1,
-                    xa - 1 + q, 0);
-      }
-      // keep the CTA resident until the last copies issued have landed (or given up)
-      for (int r = max(0, q - G::NSLOT); r < q; ++r)
-        ok = mbar_wait(full + 8u * (r % G::NSLOT), (r / G::NSLOT) & 1) && ok;
-      if (!ok) atomicExch(&g_apply_fault, 1);
-    }
-    return;
-  }
-  // ---- compute warps -----------------------------------------------------------------------
-  const int lane = t & 31;
-  const int g = t % G::G, tz = (t / G::G) % G::TZ, ty = t / (G::G * G::TZ);
-  const int iy = y0 + ty, iz = z0 + tz, col = c0 + g * G::CPT;
-  const bool active = iy < a.ny && iz < a.nz && col < a.m;
-  const int cell = ((ty + 1) * G::PZ + (tz + 1)) * G::MC + g * G::CPT;
-  const unsigned long long* pl = reinterpret_cast<const unsigned long long*>(sb);
-  bool ok = true;
-  for (int x = xa; x < xb; ++x) {
-    const int qx = x - xa + 1;
-    ok = ok && mbar_wait(full + 8u * ((qx - 1) % G::NSLOT), ((qx - 1) / G::NSLOT) & 1) &&
-         mbar_wait(full + 8u * (qx % G::NSLOT), (qx / G::NSLOT) & 1) &&
-         mbar_wait(full + 8u * ((qx + 1) % G::NSLOT), ((qx + 1) / G::NSLOT) & 1);
-    if (ok && active) {
-      RegRecord rc;
-      const float* rp = a.rec + ((long long)x * a.ny + iy) * a.nzp + iz;
+    // output of plane q = p - 1 is complete; the last one also when no plane follows
+#pragma unroll 1
+    for (int q = p - 1; q <= p; ++q) {
+      const bool write = q == p - 1 ? q >= xa : (p == p1 && p < xb);
+      if (q == p && !write) break;
+      if (write && active && ok) {
+        V x[8];
+        if (CONV) {
+          from_uncoupled<V, NB>(lo, x);
+        } else {
 #pragma unroll
-      for (int k = 0; k < K_COUNT; ++k) rc.v[k] = __ldg(rp + (long long)k * a.NP);
-      TmaLoader<G> ld;
-      ld.p[0] = pl + (size_t)((qx - 1) % G::NSLOT) * (G::PLANE_BYTES / 8) + cell;
-      ld.p[1] = pl + (size_t)(qx % G::NSLOT) * (G::PLANE_BYTES / 8) + cell;
-      ld.p[2] = pl + (size_t)((qx + 1) % G::NSLOT) * (G::PLANE_BYTES / 8) + cell;
-      float2 yv[2][8];
-      hx_packed_cols<2>(ld, rc, a.shift, a.cb, yv);
-      const int s = (x * a.ny + iy) * a.nz + iz;
-      float2* __restrict__ ys = a.Y + ((long long)s * a.ldy + col);
-      const long long ybs = (long long)a.N * a.ldy;
-      if (a.vec_store && col + 1 < a.m) {
-#pragma unroll
-        for (int b = 0; b < 8; ++b)
-          *reinterpret_cast<float4*>(ys + b * ybs) = make_float4(yv[0][b].x, yv[0][b].y,
-                                                                 yv[1][b].x, yv[1][b].y);
-      } else {
+          for (int b = 0; b < 8; ++b) x[b] = lo[b];
+        }
+        cplx<T>* ys = yout + q * ystr;
 #pragma unroll
         for (int b = 0; b < 8; ++b) {
-          ys[b * ybs] = yv[0][b];
-          if (col + 1 < a.m) ys[b * ybs + 1] = yv[1][b];
+          if (CONV ? !has_band<NB>(b) : (NB != 8 && (b & 3) == 0)) continue;
+          cplx<T>* yb = ys + (CONV ? b - band_off<NB>() : uslot<NB, false>(b)) * a.bsy;
+          if constexpr (V::C == 1) {
+            vstore(yb, x[b]);
+          } else if (a.v16y && col + 1 < a.m) {
+            vstore(yb, x[b]);
+          } else {
+            const float2 e0 = f2up(x[b].c[0]), e1 = f2up(x[b].c[1]);
+            yb[0] = e0;
+            if (col + 1 < a.m) yb[1] = e1;
+          }
         }
       }
+#pragma unroll
+      for (int b = 0; b < 8; ++b) { lo[b] = me[b]; me[b] = up[b]; }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty + 8u * ((qx - 1) % G::NSLOT));   // plane x - 1 is done
+    if (p == p1) break;
+    const int next = slot + 1 == NS ? 0 : slot + 1;
+    const unsigned nphase = next == 0 ? phase ^ 1u : phase;
+    ok = ok && mbar_wait(bars + 8u * next, nphase);
+    if (CONV && ok) convert(sm + next * STAGE);
+    ok = __syncthreads_and(ok) != 0;       // plane p + 1 is complete, stage `slot` may be refilled
+    if (!ok) break;
+    if (t == 0 && p + NS <= p1) issue(p + NS);
+    slot = next;
+    phase = nphase;
   }
-  if (!ok && lane == 0) atomicExch(&g_apply_fault, 1);
+  if (!ok && t == 0) {
+    // a copy never landed: flag it, then give the copies still in flight a bounded chance to
+    // finish before the CTA's shared memory is released
+    atomicExch(&g_apply_fault, 1);
+    for (int i = 0; i < NS; ++i) { mbar_wait(bars + 8u * i, 0); mbar_wait(bars + 8u * i, 1); }
+  }
 }
 
-// Tile shapes the staged kernel is built for: {precision, MC, TY, TZ}.
-template <typename T> struct StagedCfgs;
-template <> struct StagedCfgs<float> {
-  using C0 = Staged<float, 4, 8, 12>;
-  using C1 = Staged<float, 4, 6, 16>;
-  using C2 = Staged<float, 4, 4, 20>;
-  using C3 = Staged<float, 2, 8, 24>;
+// ---------------------------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------------------------
+// Tile shapes {TY, TZ, columns, CTAs per SM} of the TMA march, the shape of its cp.async form, and
+// per shape the time of one plane of a CTA (us, measured at 128x128x96 with 24 columns: launch time
+// over waves x planes), which pick_tile compares shapes by. Tile numbers 0..3 exist in both
+// precisions, the others in complex64 only; a number past the built ones takes shape 0.
+template <typename T> struct MarchCfgs;
+template <> struct MarchCfgs<double> {
+  using C0 = March<double, 8, 8, 4, 1>;
+  using C1 = March<double, 4, 8, 4, 2>;
+  using C2 = March<double, 8, 12, 4, 1>;
+  using C3 = March<double, 8, 8, 2, 2>;
+  using C4 = C0;
+  using C5 = C0;
+  using Any = C3;
+  static constexpr int kShapes = 4;
 };
-template <> struct StagedCfgs<double> {
-  using C0 = Staged<double, 2, 8, 12>;
-  using C1 = Staged<double, 2, 6, 16>;
-  using C2 = Staged<double, 2, 4, 20>;
-  using C3 = Staged<double, 1, 8, 16>;
+template <> struct MarchCfgs<float> {
+  using C0 = March<float, 8, 8, 8, 1>;
+  using C1 = March<float, 4, 8, 8, 2>;
+  using C2 = March<float, 8, 12, 8, 1>;
+  using C3 = March<float, 8, 8, 4, 2>;
+  using C4 = March<float, 4, 12, 8, 2>;
+  using C5 = March<float, 4, 8, 4, 4>;
+  using Any = C3;
+  static constexpr int kShapes = 6;
 };
-constexpr int kStagedCfgs = 4;
-constexpr int kDirect = -2;      // staged_cfg value selecting the direct kernel
-constexpr int kDefaultTma = 3;   // TMA shape taken when no tile was tuned or set
+constexpr int kBothCfgs = 4;               // tiles built for both precisions
+constexpr int kDirect = QDKP_TILE_DIRECT;  // staged_cfg value selecting the direct kernel
 
-struct StagedGeom { int tiles_y, tiles_z, chunks, xsplit, xlen, ctas; };
+// f(shape tag, plane time) over the shapes of a precision; f returns true to stop
+template <class S> struct ShapeTag { using G = S; };
+template <typename T, class F>
+static void each_shape(F f) {
+  using C = MarchCfgs<T>;
+  if constexpr (std::is_same<T, double>::value) {
+    if (f(0, ShapeTag<typename C::C0>(), 2.34)) return;
+    if (f(1, ShapeTag<typename C::C1>(), 2.49)) return;
+    if (f(2, ShapeTag<typename C::C2>(), 3.41)) return;
+    f(3, ShapeTag<typename C::C3>(), 2.72);
+  } else {
+    if (f(0, ShapeTag<typename C::C0>(), 2.58)) return;
+    if (f(1, ShapeTag<typename C::C1>(), 2.48)) return;
+    if (f(2, ShapeTag<typename C::C2>(), 3.41)) return;
+    if (f(3, ShapeTag<typename C::C3>(), 2.67)) return;
+    if (f(4, ShapeTag<typename C::C4>(), 3.27)) return;
+    f(5, ShapeTag<typename C::C5>(), 2.57);
+  }
+}
 
-// CTA decomposition for a grid: x is split so that the CTA count fills whole waves of one CTA
-// per SM, trading the two halo planes each extra x run costs.
-static StagedGeom staged_geom(int nx, int ny, int nz, int m, int MC, int TY, int TZ, int sms) {
-  StagedGeom g;
+struct MarchGeom { int tiles_y, tiles_z, chunks, xsplit, xlen, ctas; double steps; };   // steps: waves x planes
+
+// CTA decomposition for a grid: x is split so that the CTA count fills whole waves, trading the
+// two extra planes that each x run reads.
+static MarchGeom march_geom(int nx, int ny, int nz, int m, int MC, int TY, int TZ, int slots) {
+  MarchGeom g;
   g.tiles_y = (ny + TY - 1) / TY;
   g.tiles_z = (nz + TZ - 1) / TZ;
   g.chunks = (m + MC - 1) / MC;
@@ -1488,63 +1122,52 @@ static StagedGeom staged_geom(int nx, int ny, int nz, int m, int MC, int TY, int
     const int xlen = (nx + xs - 1) / xs;
     if ((long long)(xs - 1) * xlen >= nx) continue;
     const long long ctas = base * xs;
-    const double cost = (double)((ctas + sms - 1) / sms) * (xlen + 2);
+    const double cost = (double)((ctas + slots - 1) / slots) * (xlen + 2);
     if (cost < best - 1e-9) { best = cost; g.xsplit = xs; }
   }
   g.xlen = (nx + g.xsplit - 1) / g.xsplit;
   g.ctas = (int)(base * g.xsplit);
+  g.steps = best;
   return g;
 }
 
-template <typename T, class G, bool V16>
-static int launch_staged_g(const qdkp_operator* op, const T* rec, const void* X, int ldx,
-                           void* Y, int ldy, int m, T shift, T cb, int sms, cudaStream_t st) {
-  static bool attr_done = false;     // per instantiation; the attribute is per device function
-  if (!attr_done) {
-    QDKP_CUDA_TRY(cudaFuncSetAttribute(kp_apply_staged_kernel<T, G, V16>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM));
-    attr_done = true;
-  }
-  const StagedGeom g = staged_geom(op->nx, op->ny, op->nz, m, G::MC, G::TY, G::TZ, sms);
-  StagedArgs<T> a;
+// A kernel's shared-memory limit, raised once per device.
+template <class K>
+static cudaError_t raise_smem(K kernel, size_t bytes, int device, std::atomic<unsigned long long>& done) {
+  const unsigned long long bit = 1ull << (device & 63);
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess && device < 64) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
+
+template <class G, int NB>
+static int launch_march_g(const qdkp_operator* op, const typename G::T* rec, const void* X, int ldx,
+                          void* Y, int ldy, int m, typename G::T shift, typename G::T cb, int sms,
+                          cudaStream_t st) {
+  typedef typename G::T T;
+  constexpr size_t smem = G::template smem<NB>();
+  static_assert((smem + 1024) * G::MINB <= 233472, "over the shared memory of one SM");
+  static std::atomic<unsigned long long> raised{0};
+  QDKP_CUDA_TRY(raise_smem(kp_march_kernel<G, NB>, smem, op->device, raised));
+  const MarchGeom g = march_geom(op->nx, op->ny, op->nz, m, G::MC, G::TY, G::TZ, sms * G::MINB);
+  MarchArgs<T> a;
   a.rec = rec;
   a.X = static_cast<const cplx<T>*>(X);
   a.Y = static_cast<cplx<T>*>(Y);
-  a.N = (int)op->n_sites; a.nx = op->nx; a.ny = op->ny; a.nz = op->nz;
+  a.bsx = (long long)op->n_sites * ldx; a.bsy = (long long)op->n_sites * ldy;
+  a.nx = op->nx; a.ny = op->ny; a.nz = op->nz;
   a.ldx = ldx; a.ldy = ldy; a.m = m;
-  a.nzp = op->nzp; a.NP = op->nx * op->ny * op->nzp;
   a.tiles_z = g.tiles_z; a.chunks = g.chunks; a.xsplit = g.xsplit; a.xlen = g.xlen;
+  a.v16 = ((uintptr_t)X & 15) == 0 && ldx % 2 == 0;
+  a.v16y = ((uintptr_t)Y & 15) == 0 && ldy % 2 == 0;
   a.shift = shift; a.cb = cb;
-  kp_apply_staged_kernel<T, G, V16><<<g.ctas, G::THREADS, G::SMEM, st>>>(a);
+  kp_march_kernel<G, NB><<<g.ctas, G::THREADS, smem, st>>>(a);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;
 }
 
-template <typename T, class G>
-static int launch_staged_v(const qdkp_operator* op, const T* rec, const void* X, int ldx,
-                           void* Y, int ldy, int m, T shift, T cb, int sms, cudaStream_t st) {
-  // 16-byte copies need 16-byte aligned sources: always true for complex128 (with an aligned
-  // base); for complex64 the leading dimension, the column count and the chunk must be even.
-  const bool aligned = ((uintptr_t)X & 15) == 0;
-  const bool v16 = aligned && (sizeof(T) == 8 || (ldx % 2 == 0 && m % 2 == 0 && G::MC % 2 == 0));
-  if (v16) return launch_staged_g<T, G, true>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
-  return launch_staged_g<T, G, false>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
-}
-
-template <typename T>
-static int launch_staged(int cfg, const qdkp_operator* op, const T* rec, const void* X, int ldx,
-                         void* Y, int ldy, int m, T shift, T cb, int sms, cudaStream_t st) {
-  using C = StagedCfgs<T>;
-  switch (cfg) {
-    case 0: return launch_staged_v<T, typename C::C0>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 1: return launch_staged_v<T, typename C::C1>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 2: return launch_staged_v<T, typename C::C2>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    default: return launch_staged_v<T, typename C::C3>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
-  }
-}
-
-// ---- TMA kernel launch ------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -1552,204 +1175,80 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda)
 static EncodeTiledFn tensor_map_encoder() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  static const EncodeTiledFn fn = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) ==
-            cudaSuccess && q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
+    const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) ==
+                        cudaSuccess && q == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<EncodeTiledFn>(p) : nullptr;
+  }();
   return fn;
 }
 
-// TMA tile shapes {TY, TZ, column pairs per CTA, ring slots}; staged_cfg kTmaBase + i selects
-// shape i (complex64 only).
-struct TmaCfgs {
-  using C0 = Tma<6, 16, 2, 4>;
-  using C1 = Tma<6, 16, 2, 5>;
-  using C2 = Tma<8, 12, 2, 5>;
-  using C3 = Tma<4, 24, 2, 4>;
-  using C4 = Tma<4, 12, 2, 4, 2>;      // two CTAs per SM: one CTA's plane barrier overlaps
-  using C5 = Tma<6, 8, 2, 4, 2>;       // the other's compute
-  using C6 = Tma<8, 16, 2, 4, 1, true>;   // records in registers: 256 and 288 threads
-  using C7 = Tma<6, 24, 2, 4, 1, true>;
-};
-constexpr int kTmaBase = 4;
-constexpr int kTmaCfgs = 8;
-
+// tensor-map rules: 16-byte aligned base and strides; every box no larger than its tensor
 template <class G>
 static bool tma_fits(const qdkp_operator* op, const void* X, int64_t ldx, int m) {
-  // tensor-map rules: 16-byte aligned base and strides; every box no larger than its tensor
-  return op->n_bands == 8 && ((uintptr_t)X & 15) == 0 && ldx % 2 == 0 && m >= G::MC &&
-         op->ny >= G::PY && op->nz >= G::PZ && op->nzp >= G::TZ && tensor_map_encoder() != nullptr;
-}
-
-static bool tma_fits_cfg(int i, const qdkp_operator* op, const void* X, int64_t ldx, int m) {
-  switch (i) {
-    case 0: return tma_fits<TmaCfgs::C0>(op, X, ldx, m);
-    case 1: return tma_fits<TmaCfgs::C1>(op, X, ldx, m);
-    case 2: return tma_fits<TmaCfgs::C2>(op, X, ldx, m);
-    case 3: return tma_fits<TmaCfgs::C3>(op, X, ldx, m);
-    case 4: return tma_fits<TmaCfgs::C4>(op, X, ldx, m);
-    case 5: return tma_fits<TmaCfgs::C5>(op, X, ldx, m);
-    case 6: return tma_fits<TmaCfgs::C6>(op, X, ldx, m);
-    default: return tma_fits<TmaCfgs::C7>(op, X, ldx, m);
-  }
-}
-
-template <class G>
-static int launch_tma_g(const qdkp_operator* op, const void* X, int ldx, void* Y, int ldy, int m,
-                        float shift, float cb, int sms, cudaStream_t st) {
-  const EncodeTiledFn enc = tensor_map_encoder();
-  static bool attr_done = false;     // per instantiation; the attribute is per device function
-  if (!attr_done) {
-    QDKP_CUDA_TRY(cudaFuncSetAttribute(kp_apply_tma_kernel<G>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM));
-    attr_done = true;
-  }
-  const cuuint64_t N = (cuuint64_t)op->n_sites, ld = (cuuint64_t)ldx;
-  CUtensorMap tmx, tmr;
-  // X as [band][x][y][z][column] with the column innermost (8-byte elements)
-  const cuuint64_t xdim[5] = {(cuuint64_t)m, (cuuint64_t)op->nz, (cuuint64_t)op->ny,
-                              (cuuint64_t)op->nx, 8};
-  const cuuint64_t xstr[4] = {ld * 8, (cuuint64_t)op->nz * ld * 8,
-                              (cuuint64_t)op->ny * op->nz * ld * 8, N * ld * 8};
-  const cuuint32_t xbox[5] = {(cuuint32_t)G::MC, (cuuint32_t)G::PZ, (cuuint32_t)G::PY, 1, 8};
-  const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
-  CUresult r = enc(&tmx, CU_TENSOR_MAP_DATA_TYPE_INT64, 5, const_cast<void*>(X), xdim, xstr,
-                   xbox, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_error("cuTensorMapEncodeTiled failed for the X block (code " + std::to_string((int)r) + ")");
-    return QDKP_ERR_CUDA;
-  }
-  // the FP32 record as [entry][x][y][z_padded]
-  const cuuint64_t NP = (cuuint64_t)op->nx * op->ny * op->nzp;
-  const cuuint64_t rdim[4] = {(cuuint64_t)op->nzp, (cuuint64_t)op->ny, (cuuint64_t)op->nx,
-                              (cuuint64_t)K_COUNT};
-  const cuuint64_t rstr[3] = {(cuuint64_t)op->nzp * 4, (cuuint64_t)op->ny * op->nzp * 4, NP * 4};
-  const cuuint32_t rbox[4] = {(cuuint32_t)G::TZ, (cuuint32_t)G::TY, 1, (cuuint32_t)K_COUNT};
-  r = enc(&tmr, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, op->rec32, rdim, rstr, rbox, ones,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_error("cuTensorMapEncodeTiled failed for the record (code " + std::to_string((int)r) + ")");
-    return QDKP_ERR_CUDA;
-  }
-  const StagedGeom g = staged_geom(op->nx, op->ny, op->nz, m, G::MC, G::TY, G::TZ,
-                                   sms * G::MINB);
-  TmaArgs a;
-  a.Y = static_cast<float2*>(Y);
-  a.rec = op->rec32;
-  a.nzp = op->nzp; a.NP = op->nx * op->ny * op->nzp;
-  a.N = (int)op->n_sites; a.nx = op->nx; a.ny = op->ny; a.nz = op->nz;
-  a.ldy = ldy; a.m = m;
-  a.tiles_z = g.tiles_z; a.chunks = g.chunks; a.xsplit = g.xsplit; a.xlen = g.xlen;
-  a.vec_store = ((uintptr_t)Y & 15) == 0 && ldy % 2 == 0;
-  a.shift = shift; a.cb = cb;
-  kp_apply_tma_kernel<G><<<g.ctas, G::THREADS, G::SMEM, st>>>(tmx, tmr, a);
-  count_launch();
-  QDKP_CUDA_TRY(cudaGetLastError());
-  return QDKP_OK;
-}
-
-static int launch_tma(int i, const qdkp_operator* op, const void* X, int ldx, void* Y, int ldy,
-                      int m, float shift, float cb, int sms, cudaStream_t st) {
-  switch (i) {
-    case 0: return launch_tma_g<TmaCfgs::C0>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 1: return launch_tma_g<TmaCfgs::C1>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 2: return launch_tma_g<TmaCfgs::C2>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 3: return launch_tma_g<TmaCfgs::C3>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 4: return launch_tma_g<TmaCfgs::C4>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 5: return launch_tma_g<TmaCfgs::C5>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 6: return launch_tma_g<TmaCfgs::C6>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    default: return launch_tma_g<TmaCfgs::C7>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-  }
-}
-
-// Producer-warp TMA shapes {TY, TZ, column pairs per CTA, ring slots, CTAs per SM};
-// staged_cfg kTma2Base + i selects shape i (complex64 only).
-struct Tma2Cfgs {
-  using D0 = Tma2<6, 16, 2, 4, 1>;
-  using D1 = Tma2<8, 16, 2, 4, 1>;
-  using D2 = Tma2<8, 16, 1, 4, 2>;
-  using D3 = Tma2<6, 16, 2, 5, 1>;
-  using D4 = Tma2<4, 24, 2, 4, 1>;
-};
-constexpr int kTma2Base = kTmaBase + kTmaCfgs;
-constexpr int kTma2Cfgs = 5;
-
-template <class G>
-static bool tma2_fits(const qdkp_operator* op, const void* X, int64_t ldx, int m) {
-  return op->n_bands == 8 && ((uintptr_t)X & 15) == 0 && ldx % 2 == 0 && m >= G::MC &&
+  return ((uintptr_t)X & 15) == 0 && (sizeof(typename G::T) == 8 || ldx % 2 == 0) && m >= G::MC &&
          op->ny >= G::PY && op->nz >= G::PZ && tensor_map_encoder() != nullptr;
 }
 
-static bool tma2_fits_cfg(int i, const qdkp_operator* op, const void* X, int64_t ldx, int m) {
-  switch (i) {
-    case 0: return tma2_fits<Tma2Cfgs::D0>(op, X, ldx, m);
-    case 1: return tma2_fits<Tma2Cfgs::D1>(op, X, ldx, m);
-    case 2: return tma2_fits<Tma2Cfgs::D2>(op, X, ldx, m);
-    case 3: return tma2_fits<Tma2Cfgs::D3>(op, X, ldx, m);
-    default: return tma2_fits<Tma2Cfgs::D4>(op, X, ldx, m);
-  }
-}
-
-template <class G>
-static int launch_tma2_g(const qdkp_operator* op, const void* X, int ldx, void* Y, int ldy, int m,
-                         float shift, float cb, int sms, cudaStream_t st) {
-  const EncodeTiledFn enc = tensor_map_encoder();
-  static bool attr_done = false;
-  if (!attr_done) {
-    QDKP_CUDA_TRY(cudaFuncSetAttribute(kp_apply_tma2_kernel<G>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM));
-    attr_done = true;
-  }
-  const cuuint64_t N = (cuuint64_t)op->n_sites, ld = (cuuint64_t)ldx;
-  CUtensorMap tmx;
-  const cuuint64_t xdim[5] = {(cuuint64_t)m, (cuuint64_t)op->nz, (cuuint64_t)op->ny,
-                              (cuuint64_t)op->nx, 8};
-  const cuuint64_t xstr[4] = {ld * 8, (cuuint64_t)op->nz * ld * 8,
-                              (cuuint64_t)op->ny * op->nz * ld * 8, N * ld * 8};
-  const cuuint32_t xbox[5] = {(cuuint32_t)G::MC, (cuuint32_t)G::PZ, (cuuint32_t)G::PY, 1, 8};
+template <class G, int NB, int NS, bool CONV>
+static int launch_march_tma(const qdkp_operator* op, const typename G::T* rec, const void* X, int ldx,
+                            void* Y, int ldy, int m, typename G::T shift, typename G::T cb, int sms,
+                            cudaStream_t st) {
+  typedef typename G::T T;
+  constexpr size_t smem = 128 + NS * G::template stage_bytes<NB>() + 8 * NS;
+  static_assert((smem + 1024) * G::MINB <= 233472, "over the shared memory of one SM");
+  static std::atomic<unsigned long long> raised{0};
+  QDKP_CUDA_TRY(raise_smem(kp_march_tma_kernel<G, NB, NS, CONV>, smem, op->device, raised));
+  // X as [band][x][y][z][column], in 8-byte elements with the column innermost
+  constexpr int E = (int)sizeof(cplx<T>) / 8;
+  const cuuint64_t ld = (cuuint64_t)ldx * sizeof(cplx<T>);
+  const cuuint64_t dim[5] = {(cuuint64_t)m * E, (cuuint64_t)op->nz, (cuuint64_t)op->ny,
+                             (cuuint64_t)op->nx, (cuuint64_t)NB};
+  const cuuint64_t str[4] = {ld, (cuuint64_t)op->nz * ld, (cuuint64_t)op->ny * op->nz * ld,
+                             (cuuint64_t)op->n_sites * ld};
+  const cuuint32_t box[5] = {(cuuint32_t)(G::MC * E), (cuuint32_t)G::PZ, (cuuint32_t)G::PY, 1, (cuuint32_t)NB};
   const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
-  CUresult r = enc(&tmx, CU_TENSOR_MAP_DATA_TYPE_INT64, 5, const_cast<void*>(X), xdim, xstr,
-                   xbox, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUtensorMap tmx;
+  const CUresult r = tensor_map_encoder()(
+      &tmx, CU_TENSOR_MAP_DATA_TYPE_INT64, 5, const_cast<void*>(X), dim, str, box, ones,
+      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed for the X block (code " + std::to_string((int)r) + ")");
     return QDKP_ERR_CUDA;
   }
-  // one wave holds MINB CTAs per SM
-  const StagedGeom g = staged_geom(op->nx, op->ny, op->nz, m, G::MC, G::TY, G::TZ,
-                                   sms * G::MINB);
-  Tma2Args a;
-  a.Y = static_cast<float2*>(Y);
-  a.rec = op->rec32;
-  a.N = (int)op->n_sites; a.nx = op->nx; a.ny = op->ny; a.nz = op->nz;
-  a.nzp = op->nzp; a.NP = op->nx * op->ny * op->nzp;
-  a.ldy = ldy; a.m = m;
+  const MarchGeom g = march_geom(op->nx, op->ny, op->nz, m, G::MC, G::TY, G::TZ, sms * G::MINB);
+  MarchArgs<T> a{};
+  a.rec = rec;
+  a.Y = static_cast<cplx<T>*>(Y);
+  a.bsy = (long long)op->n_sites * ldy;
+  a.nx = op->nx; a.ny = op->ny; a.nz = op->nz;
+  a.ldx = ldx; a.ldy = ldy; a.m = m;
   a.tiles_z = g.tiles_z; a.chunks = g.chunks; a.xsplit = g.xsplit; a.xlen = g.xlen;
-  a.vec_store = ((uintptr_t)Y & 15) == 0 && ldy % 2 == 0;
+  a.v16y = ((uintptr_t)Y & 15) == 0 && ldy % 2 == 0;
   a.shift = shift; a.cb = cb;
-  kp_apply_tma2_kernel<G><<<g.ctas, G::THREADS, G::SMEM, st>>>(tmx, a);
+  kp_march_tma_kernel<G, NB, NS, CONV><<<g.ctas, G::THREADS, smem, st>>>(tmx, a);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;
 }
 
-static int launch_tma2(int i, const qdkp_operator* op, const void* X, int ldx, void* Y, int ldy,
-                       int m, float shift, float cb, int sms, cudaStream_t st) {
-  switch (i) {
-    case 0: return launch_tma2_g<Tma2Cfgs::D0>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 1: return launch_tma2_g<Tma2Cfgs::D1>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 2: return launch_tma2_g<Tma2Cfgs::D2>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    case 3: return launch_tma2_g<Tma2Cfgs::D3>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-    default: return launch_tma2_g<Tma2Cfgs::D4>(op, X, ldx, Y, ldy, m, shift, cb, sms, st);
-  }
+template <typename T, int NB>
+static int launch_march(int cfg, const qdkp_operator* op, const T* rec, const void* X, int ldx,
+                        void* Y, int ldy, int m, T shift, T cb, int sms, cudaStream_t st) {
+  int rc = QDKP_OK;
+  bool done = false;
+  each_shape<T>([&](int i, auto tag, double) {
+    using G = typename decltype(tag)::G;
+    if (i != (cfg < MarchCfgs<T>::kShapes ? cfg : 0) || !tma_fits<G>(op, X, ldx, m)) return false;
+    rc = launch_march_tma<G, NB, 2, true>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
+    return done = true;
+  });
+  if (done) return rc;
+  // a block no tensor map describes, or a grid or block smaller than the tile
+  return launch_march_g<typename MarchCfgs<T>::Any, NB>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
 }
 
 int launch_apply_multi(const HXSlot* slots_dev, int nslots, int total_tiles, int precision,
@@ -1779,17 +1278,16 @@ double apply_cb_weight(const qdkp_operator* op) { return op_sign(op) * (-kG / (o
 
 int build_records(qdkp_operator* op) {
   const long long N = op->n_sites;
-  const int blocks = (int)std::min<long long>((N + 127) / 128, 148 * 16);
-  kp_record_kernel<<<blocks, 128>>>(op->fields64, N, op->nx, op->ny, op->nz, op->nzp, op->h,
-                                     op->flags, op->n_bands, op_sign(op), op->rec64, op->rec32,
-                                     op->nbmask);
+  const int blocks = (int)std::min<long long>((N + kRecThreads - 1) / kRecThreads, 148 * 16);
+  kp_record_kernel<<<blocks, kRecThreads>>>(op->fields64, N, op->nx, op->ny, op->nz, op->h, op->flags,
+                                     op->n_bands, op_sign(op), op->rec64, op->rec32, op->nbmask);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   QDKP_CUDA_TRY(cudaDeviceSynchronize());
   return QDKP_OK;
 }
 
-size_t record_doubles(int nx, int ny, int nzp) { return (size_t)K_COUNT * nx * ny * nzp; }
+size_t record_values(int64_t n_sites) { return (size_t)rec_stride<double>() * n_sites; }
 
 static int num_sms(int device) {
   static int cached[64] = {0};
@@ -1803,27 +1301,38 @@ static int num_sms(int device) {
   return cached[device];
 }
 
-// Default kernel for a launch without a tuned choice, from measurements of both kernels over
-// grids of 23x23x20 to 128x128x96 and blocks of 12 and 24 columns on B200: complex128 is FP64-
-// issue bound and the direct kernel (more resident warps) is as fast or faster everywhere;
-// complex64 takes a shared-memory kernel on grids of 50k sites and more, where its reuse pays:
-// the TMA kernel where its tensor maps fit, else the cp.async staged kernel with the tile shape
-// that pads the (y, z) plane least. qdkp_operator_tune refines this per operator.
-static int pick_staged_cfg(const qdkp_operator* op, int precision, const void* X, int64_t ldx,
-                           int m) {
-  if (precision == QDKP_C128 || op->n_sites < 50000) return kDirect;
-  if (tma_fits_cfg(kDefaultTma, op, X, ldx, m)) return kTmaBase + kDefaultTma;
-  // the four-column shapes (0, 1) measured fastest on every grid; pick the one that pads less
-  static const int shape[2][2] = {{8, 12}, {6, 16}};   // TY, TZ
-  int best = 0;
-  double best_w = 1e30;
-  for (int c = 0; c < 2; ++c) {
-    const int TY = shape[c][0], TZ = shape[c][1];
-    const double w = (double)((op->ny + TY - 1) / TY * TY) * ((op->nz + TZ - 1) / TZ * TZ) *
-                     (1.0 + 2.0 / TY) * (1.0 + 2.0 / TZ);
-    if (w < best_w - 1e-9) { best_w = w; best = c; }
-  }
-  return best;
+// Default kernel of a launch: the shape with the smallest waves x planes x plane time, against the
+// direct kernel's time per (site, column). Measured (us, direct / march): complex128 23x23x20 x 12
+// 20 / 18, 48x48x36 x 12 119 / 82, 91x91x76 x 24 2111 / 1160; complex64 10 / 15, 59 / 51, 947 / 560.
+// qdkp_operator_tune refines this per operator.
+template <typename T>
+static int pick_tile(const qdkp_operator* op, const void* X, int64_t ldx, int m, int sms) {
+  if (op->n_bands == 4) return kDirect;
+  const double items = (double)op->n_sites * m;
+  double best = 3.0 + items * (sizeof(T) == 8 ? 1.18e-4 : 0.57e-4);
+  int tile = kDirect;
+  each_shape<T>([&](int i, auto tag, double plane) {
+    using G = typename decltype(tag)::G;
+    if (!tma_fits<G>(op, X, ldx, m)) return false;
+    const MarchGeom g = march_geom(op->nx, op->ny, op->nz, m, G::MC, G::TY, G::TZ, sms * G::MINB);
+    const double us = 3.0 + g.steps * plane;
+    if (us < best) { best = us; tile = i; }
+    return false;
+  });
+  return tile;
+}
+
+// The direct kernel; a block of few items is spread over the whole chip in small CTAs (23x23x20 x 1:
+// 42 CTAs of 256 threads would leave 106 SMs idle; 8.0 -> 5.1 us with 64).
+template <typename T, int NB>
+static int launch_direct(const qdkp_operator* op, const HXArgs<T>& a, int sms, cudaStream_t st) {
+  const int64_t items = op->n_sites * a.m;
+  int threads = kApplyThreads;
+  while (threads > 64 && items < (int64_t)threads * 2 * sms) threads /= 2;
+  kp_apply_kernel<T, NB><<<(unsigned)((items + threads - 1) / threads), threads, 0, st>>>(a);
+  count_launch();
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
 }
 
 template <typename T>
@@ -1837,21 +1346,13 @@ static int launch_apply_t(const qdkp_operator* op, const T* rec, const void* X, 
   const T shift = shifted ? (T)(-sigma) : T(0);
   const T cb = (T)apply_cb_weight(op);
   const int forced = op->staged_cfg[precision == QDKP_C64];
-  int cfg = forced == QDKP_TILE_AUTO ? pick_staged_cfg(op, precision, X, ldx, m) : forced;
-  if (cfg >= kTma2Base) {
-    if (std::is_same<T, float>::value && tma2_fits_cfg(cfg - kTma2Base, op, X, ldx, m))
-      return launch_tma2(cfg - kTma2Base, op, X, (int)ldx, Y, (int)ldy, m, (float)shift,
-                         (float)cb, num_sms(op->device), st);
-    cfg = 1;       // a block the tensor maps cannot describe: the cp.async staged kernel
-  } else if (cfg >= kTmaBase) {
-    if (std::is_same<T, float>::value && tma_fits_cfg(cfg - kTmaBase, op, X, ldx, m))
-      return launch_tma(cfg - kTmaBase, op, X, (int)ldx, Y, (int)ldy, m, (float)shift, (float)cb,
-                        num_sms(op->device), st);
-    cfg = 1;
+  const int sms = num_sms(op->device);
+  const int cfg = forced == QDKP_TILE_AUTO ? pick_tile<T>(op, X, ldx, m, sms) : forced;
+  if (cfg != kDirect && op->n_bands != 4 && ((uintptr_t)X % sizeof(cplx<T>)) == 0) {
+    if (op->n_bands == 8)
+      return launch_march<T, 8>(cfg, op, rec, X, (int)ldx, Y, (int)ldy, m, shift, cb, sms, st);
+    return launch_march<T, 6>(cfg, op, rec, X, (int)ldx, Y, (int)ldy, m, shift, cb, sms, st);
   }
-  if (op->n_bands == 8 && cfg >= 0 && ((uintptr_t)X % sizeof(cplx<T>)) == 0)
-    return launch_staged<T>(cfg, op, rec, X, (int)ldx, Y, (int)ldy, m, shift, cb,
-                            num_sms(op->device), st);
   HXArgs<T> a;
   a.rec = rec;
   a.msk = op->nbmask;
@@ -1859,19 +1360,14 @@ static int launch_apply_t(const qdkp_operator* op, const T* rec, const void* X, 
   a.Y = static_cast<cplx<T>*>(Y);
   a.N = (int)op->n_sites; a.ldx = (int)ldx; a.ldy = (int)ldy; a.m = m;
   a.sx = op->ny * op->nz; a.sy = op->nz;
-  a.nz = op->nz; a.nzp = op->nzp; a.NP = op->nx * op->ny * op->nzp;
   a.shift = shift;
   a.cb = cb;
-  const unsigned grid = (unsigned)apply_tiles(op->n_sites, m);
   switch (op->n_bands) {
-    case 8: kp_apply_kernel<T, 8><<<grid, kApplyThreads, 0, st>>>(a); break;
-    case 6: kp_apply_kernel<T, 6><<<grid, kApplyThreads, 0, st>>>(a); break;
-    case 4: kp_apply_kernel<T, 4><<<grid, kApplyThreads, 0, st>>>(a); break;
+    case 8: return launch_direct<T, 8>(op, a, sms, st);
+    case 6: return launch_direct<T, 6>(op, a, sms, st);
+    case 4: return launch_direct<T, 4>(op, a, sms, st);
     default: set_error("n_bands must be 8, 6 or 4"); return QDKP_ERR_ARG;
   }
-  count_launch();
-  QDKP_CUDA_TRY(cudaGetLastError());
-  return QDKP_OK;
 }
 
 // Y = sign*H X (- sigma X if shifted) for one block in the given precision.
@@ -1894,10 +1390,9 @@ extern "C" {
 int qdkp_operator_set_tile(qdkp_operator* op, int precision, int tile) {
   QDKP_CHECK_ARG(op != nullptr, "operator must not be NULL");
   QDKP_CHECK_ARG(precision == QDKP_C128 || precision == QDKP_C64, "bad precision");
-  QDKP_CHECK_ARG(tile >= QDKP_TILE_DIRECT && tile < kStagedCfgs + kTmaCfgs + kTma2Cfgs,
-                 "tile out of range");
-  QDKP_CHECK_ARG(precision == QDKP_C64 || tile < kStagedCfgs,
-                 "the TMA tile shapes are built for complex64 only");
+  QDKP_CHECK_ARG(tile >= QDKP_TILE_DIRECT && tile < QDKP_TILE_COUNT, "tile out of range");
+  QDKP_CHECK_ARG(precision == QDKP_C64 || tile < kBothCfgs,
+                 "the tile shapes from 4 on are built for complex64 only");
   op->staged_cfg[precision == QDKP_C64] = tile;
   return QDKP_OK;
 }
@@ -1924,18 +1419,13 @@ int qdkp_operator_tune(qdkp_operator* op, const void* X, int64_t ldx, void* Y, i
   int best = saved;
   float best_ms = 3.4e38f;
   int rc = QDKP_OK;
-  // candidates: the staged shapes, the TMA shapes (complex64), the direct kernel last; the
-  // seconds array has one entry per candidate, -1 for one that does not apply
-  const int nbuilt = kStagedCfgs + kTmaCfgs + kTma2Cfgs;
-  const int ncand = nbuilt + 1;
-  for (int c = 0; c < ncand && rc == QDKP_OK; ++c) {
-    const int tile = c < nbuilt ? c : kDirect;
+  // candidates: the built shapes, the direct kernel last; the seconds array has one entry per
+  // tile number, -1 for one that does not apply
+  for (int c = 0; c <= QDKP_TILE_COUNT && rc == QDKP_OK; ++c) {
+    const int tile = c < QDKP_TILE_COUNT ? c : kDirect;
     if (seconds) seconds[c] = -1.0;
-    if (op->n_bands != 8 && tile != kDirect) continue;                // 6/4-band: direct only
-    if (tile >= kTmaBase && precision != QDKP_C64) continue;
-    if (tile >= kTma2Base && !tma2_fits_cfg(tile - kTma2Base, op, X, ldx, m)) continue;
-    if (tile >= kTmaBase && tile < kTma2Base && !tma_fits_cfg(tile - kTmaBase, op, X, ldx, m))
-      continue;
+    if (op->n_bands == 4 && tile != kDirect) continue;                // four bands: direct only
+    if (tile != kDirect && tile >= (precision == QDKP_C64 ? MarchCfgs<float>::kShapes : MarchCfgs<double>::kShapes)) continue;
     op->staged_cfg[pi] = tile;
     rc = launch_apply(op, X, ldx, Y, ldy, m, 0.0, 0, precision, st);      // warm-up
     if (rc != QDKP_OK) break;

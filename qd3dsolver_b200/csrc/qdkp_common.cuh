@@ -94,7 +94,6 @@ struct HXSlot {
   const int* m_dev;       // device column count (active width), or NULL
   const int* skip;        // nonzero: slot idle this tick
   int ld_same;            // leading dimensions equal the column count
-  int nzp, NP;            // padded z extent of the record and its entry stride
   int shifted;
   double sigma;
   double cb;              // conduction-band face weight (apply_cb_weight)
@@ -107,7 +106,8 @@ int apply_tiles(int64_t n_sites, int m);
 double apply_cb_weight(const qdkp_operator* op);
 // (re)build the per-site stencil record and neighbour masks from fields64
 int build_records(qdkp_operator* op);
-size_t record_doubles(int nx, int ny, int nzp);
+// values of the record of n_sites sites
+size_t record_values(int64_t n_sites);
 
 }  // namespace qdkp
 
@@ -120,10 +120,9 @@ struct qdkp_operator {
   int flags;              // QDKP_* flags
   int device;
   double* fields64;       // device, F_COUNT * n_sites doubles (library-owned)
-  int nzp;                // nz rounded up to a multiple of 4 (record rows)
-  double* rec64;          // device, per-site stencil record (FP64), record_doubles(nx, ny, nzp)
+  double* rec64;          // device, per-site stencil record (FP64), record_values(n_sites)
   float* rec32;           // the same record in FP32
   unsigned* nbmask;       // device, per-site neighbour mask
-  int staged_cfg[2];      // staged H.X tile shape per precision (c128, c64); -1 = by heuristic
+  int staged_cfg[2];      // H.X tile shape per precision (c128, c64); -1 = by heuristic
   int64_t nnz_equiv;      // CSR nonzero count of the equivalent assembled matrix
 };

@@ -204,9 +204,8 @@ class KPOperator(spla.LinearOperator):
         return Y
 
     def set_tile(self, tile, precision=_lib.C128):
-        """Force the H.X kernel for this operator and precision: a staged tile shape
-        0..TILE_COUNT-1 (TILE_TMA0.. are the complex64 TMA shapes), TILE_DIRECT, or TILE_AUTO
-        (heuristic)."""
+        """Force the H.X kernel for this operator and precision: a tile shape 0..TILE_COUNT-1
+        (TILE_TMA0.. are complex64 only), TILE_DIRECT, or TILE_AUTO (cost model)."""
         check(lib().qdkp_operator_set_tile(self.handle, precision, int(tile)),
               'qdkp_operator_set_tile')
 
@@ -218,7 +217,7 @@ class KPOperator(spla.LinearOperator):
 
     def tune(self, m, dtype=None, reps=5):
         """Autotune the H.X kernel for (n, m) blocks of `dtype` (complex128 by default): time
-        every staged tile shape and the direct kernel on a random block, keep the fastest for
+        every built tile shape and the direct kernel on a random block, keep the fastest for
         this operator. Returns {tile: seconds per launch}."""
         torch = _torch()
         dtype = dtype or torch.complex128
