@@ -9,6 +9,7 @@
 #include <cstring>
 
 #include "dense_dev.cuh"
+#include "gram_dev.cuh"
 #include "umma_dev.cuh"
 
 namespace qdkp {
@@ -144,47 +145,66 @@ int launch_copy(const cplx<TS>* src, long long lds, int cols, long long n, cplx<
 }
 
 // ------------------------------------------------------------------------------------------------
-// Gram: out = A^H B over concatenated column lists, FP64 accumulation, deterministic.
+// Gram: out = A^H B over concatenated column lists, FP64 accumulation, deterministic (gram_dev.cuh).
 // ------------------------------------------------------------------------------------------------
-constexpr int kGramParts = 296;
-
-// The complex product A^H B is one real GEMM over the interleaved (re, im) view: with
-// A' (n x 2P) and B' (n x 2Q) the real views, C' = A'^T B' and
-//   Re G_ij = C'_{2i,2j} + C'_{2i+1,2j+1},   Im G_ij = C'_{2i,2j+1} - C'_{2i+1,2j}.
-// C' is accumulated on the FP64 tensor cores (mma.sync.m8n8k4.f64; the tcgen05 family has no
-// f64 kind). A CTA of 3 x 3 warps owns all 8x8 tiles of C' for its slice of rows; each warp
-// owns a rectangle of up to 6 x 6 tiles and keeps them in registers across the slice.
-
-constexpr int kGramSplit = 16;
-
-// A CTA per (row part, column panel): its partial of C', then the last CTAs reduce the
-// partials into `result` (gram_finish_last; `counters`: kGramSplit + 1 zeroed ints)
-template <int MR, int MC, typename T>
-__global__ void __launch_bounds__(512)
-gram_partial_kernel(const BlockList<T> A, const BlockList<T> B, long long n,
-                    long long rows_per_part, double* __restrict__ partial, int ptc,
-                    int* __restrict__ counters, double2* __restrict__ result) {
+template <typename T>
+__global__ void __launch_bounds__(32 * (kGramMaxWarps + 1), 1)
+gram_kernel(const GramTask<T> t, int parts, double* __restrict__ partial) {
   extern __shared__ __align__(16) unsigned char gsm_d[];
-  const int RP = (2 * A.total() + 7) / 8 * 8, RQ = (2 * B.total() + 7) / 8 * 8;
-  const long long r0 = blockIdx.x * rows_per_part;
-  double* out = partial + (long long)blockIdx.x * RP * RQ;
-  bool done = false;
-  if constexpr (std::is_same<T, float>::value) {
-    if (gridDim.y == 1 && gram_tf32_rects(A.total(), B.total()) <= (int)(blockDim.x >> 5)) {
-      gram_core_tf32(A, B, r0, min(n, r0 + rows_per_part), out, gsm_d);
-      done = true;
-    }
-  }
-  if (!done)
-    gram_core<MR, MC>(A, B, r0, min(n, r0 + rows_per_part), out, gsm_d, blockIdx.y * ptc, ptc);
-  gram_finish_last(partial, (int)gridDim.x, kGramSplit, counters, A.total(), B.total(),
-                   (int)blockIdx.x, result);
+  gram_core(t, (int)blockIdx.x, parts, (int)blockIdx.y, partial, gsm_d);
+}
+
+// out row-major with leading dimension Q (GK_FULL, GK_HERM: both triangles); the pencil kinds write
+// the layouts of gram_put
+template <typename T>
+__global__ void __launch_bounds__(kGramRedThreads)
+gram_reduce_kernel(const GramTask<T> t, int parts, const double* __restrict__ partial,
+                   double2* __restrict__ out, double2* __restrict__ outS) {
+  gram_reduce_core(t, parts, partial, (int)blockIdx.x, (int)gridDim.x,
+                   [&](int i, int j, double2 v) { gram_put(t, i, j, v, out, outS); });
 }
 
 size_t gram_partial_elems(int P, int Q) {
-  const size_t RP = (2 * P + 7) / 8 * 8, RQ = (2 * Q + 7) / 8 * 8;
-  // the partials, the group sums, then the kGramSplit + 1 counters
-  return (size_t)(kGramParts + kGramSplit) * RP * RQ / 2 + 1 + (kGramSplit + 1 + 3) / 4;
+  const size_t rects = (size_t)((P + kGramRect - 1) / kGramRect) * ((Q + kGramRect - 1) / kGramRect);
+  return rects * kGramMaxParts * kGramRectElems / 2;
+}
+
+template <typename T>
+static int launch_gram_task(const GramTask<T>& t, double2* partial, size_t partial_elems, double2* out,
+                            double2* outS, cudaStream_t st) {
+  const GramShape sh = gram_shape(t.kind, t.P, t.Q, t.m, t.ma, t.mp);
+  const int parts = gram_parts(t.n);
+  if (gram_partial_doubles(sh.rects, parts) > 2 * partial_elems) {
+    set_error("gram partial buffer too small");
+    return QDKP_ERR_WORKSPACE;
+  }
+  const size_t smem = gram_smem<T>(t.tc, sh.warps);
+  QDKP_CUDA_TRY(cudaFuncSetAttribute(gram_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramMaxSmem));
+  double* pd = reinterpret_cast<double*>(partial);
+  gram_kernel<T><<<dim3((unsigned)parts, (unsigned)sh.panels), 32 * (sh.warps + 1), smem, st>>>(t, parts, pd);
+  gram_reduce_kernel<T><<<(t.P * t.Q + 31) / 32, kGramRedThreads, 0, st>>>(t, parts, pd, out, outS);
+  count_launch(2);
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
+}
+
+int launch_gram_rz(const BlockList<double>& W, const BlockList<double>& AW, bool explicit_gram,
+                   long long n, double2* partial, size_t partial_elems, double2* gT, double2* gS,
+                   cudaStream_t st) {
+  GramTask<double> t{};
+  auto add = [&](const BlockList<double>& L, int b) {
+    t.p[t.nblk] = L.p[b]; t.ld[t.nblk] = (int)L.ld[b]; t.cols[t.nblk] = L.cols[b];
+    ++t.nblk;
+    t.tc += L.cols[b];
+  };
+  for (int b = 0; b < W.nblk; ++b) add(W, b);
+  for (int b = explicit_gram ? 0 : 1; b < AW.nblk; ++b) add(AW, b);
+  t.m = W.cols[0]; t.ma = W.cols[1]; t.mp = W.nblk > 2 ? W.cols[2] : 0;
+  t.P = t.m + t.ma + t.mp;
+  t.n = n;
+  if (explicit_gram) { t.kind = GK_EXPLICIT; t.b0 = 0; t.Q = 2 * t.P; }
+  else { t.kind = GK_PENCIL; t.b0 = t.m + t.ma; t.Q = 2 * t.mp + t.ma; }
+  return launch_gram_task(t, partial, partial_elems, gT, gS, st);
 }
 
 template <typename T>
@@ -195,39 +215,22 @@ int launch_gram(const BlockList<T>& A, const BlockList<T>& B, long long n,
     set_error("gram dimensions out of range");
     return QDKP_ERR_ARG;
   }
-  const int RP = (2 * P + 7) / 8 * 8, RQ = (2 * Q + 7) / 8 * 8;
-  long long parts = (n + 255) / 256;
-  if (parts > kGramParts) parts = kGramParts;
-  if (parts < 1) parts = 1;
-  long long rpp = (n + parts - 1) / parts;
-  rpp = (rpp + 3) / 4 * 4;
-  parts = (n + rpp - 1) / rpp;
-  const size_t counter_at = ((size_t)(parts + kGramSplit) * RP * RQ + 1) / 2 + 1;   // double2 units
-  if (counter_at + (kGramSplit + 1 + 3) / 4 > partial_elems) {
-    set_error("gram partial buffer too small");
-    return QDKP_ERR_WORKSPACE;
+  bool same = A.nblk == B.nblk;
+  for (int b = 0; b < A.nblk && same; ++b)
+    same = A.p[b] == B.p[b] && A.cols[b] == B.cols[b] && A.ld[b] == B.ld[b];
+  GramTask<T> t{};
+  for (int side = 0; side < (same ? 1 : 2); ++side) {
+    const BlockList<T>& L = side ? B : A;
+    for (int b = 0; b < L.nblk; ++b) {
+      t.p[t.nblk] = L.p[b]; t.ld[t.nblk] = (int)L.ld[b]; t.cols[t.nblk] = L.cols[b];
+      ++t.nblk;
+    }
   }
-  int* counters = reinterpret_cast<int*>(partial + counter_at);
-  QDKP_CUDA_TRY(cudaMemsetAsync(counters, 0, (kGramSplit + 1) * sizeof(int), st));
-  const size_t smem = gram_smem_bytes(P, Q, (int)sizeof(cplx<T>));
-  static bool attr = false;
-  if (!attr) {
-    const int big = 200 * 1024;
-    cudaFuncSetAttribute(gram_partial_kernel<3, 3, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-    attr = true;
-  }
-  const GramPlan gp = gram_plan(P, Q);
-  int threads = gp.threads;
-  if (std::is_same<T, float>::value && gp.panels == 1) {   // the TF32 core: a warp per rectangle
-    const int G = gram_tf32_rects(P, Q);
-    if (G > threads / 32 && G <= 16) threads = 512;
-  }
-  double* pd = reinterpret_cast<double*>(partial);
-  gram_partial_kernel<3, 3, T><<<dim3((unsigned)parts, gp.panels), threads, smem, st>>>(
-      A, B, n, rpp, pd, gp.ptc, counters, out);
-  count_launch();
-  QDKP_CUDA_TRY(cudaGetLastError());
-  return QDKP_OK;
+  t.tc = same ? P : P + Q;
+  t.a0 = 0; t.P = P; t.b0 = same ? 0 : P; t.Q = Q;
+  t.kind = same ? GK_HERM : GK_FULL;
+  t.n = n;
+  return launch_gram_task(t, partial, partial_elems, out, out, st);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -12,12 +12,6 @@ constexpr int kMaxBlock = 24;          // largest LOBPCG block width (columns) s
 constexpr int kMaxSmall = 3 * kMaxBlock;  // largest Rayleigh-Ritz dimension
 constexpr int kTallThreads = 256;
 constexpr int kSmallThreads = 512;
-// Gram kernels: 3 x 3 warps, each owning up to kGramMaxT x kGramMaxT 8x8 tiles of the real
-// product, rows staged kGramChunk at a time.
-constexpr int kGramWarpsR = 3, kGramWarpsC = 3;
-constexpr int kGramThreads = 32 * kGramWarpsR * kGramWarpsC;
-constexpr int kGramMaxT = 6;                        // tiles per warp per dimension
-constexpr int kGramChunk = 32;                      // rows staged per step
 
 // A group of up to three column blocks concatenated along the columns: [B0 | B1 | B2].
 template <typename T>
@@ -77,6 +71,12 @@ template <typename T>
 int launch_gram(const BlockList<T>& A, const BlockList<T>& B, long long n,
                 double2* partial, size_t partial_elems, double2* out, cudaStream_t st);
 size_t gram_partial_elems(int P, int Q);
+// The products of the Rayleigh-Ritz pencil in one pass over W = [X | R (| P)], AW = [AX | AR (| AP)]:
+// explicit: gS = W^H W and gT = W^H AW (tot x tot); otherwise gS = [X | R]^H P and gT = W^H [AR | AP].
+// Entries that the pencils do not read (lobpcg.py:826-909) are not formed.
+int launch_gram_rz(const BlockList<double>& W, const BlockList<double>& AW, bool explicit_gram,
+                   long long n, double2* partial, size_t partial_elems, double2* gT, double2* gS,
+                   cudaStream_t st);
 // Y = beta * Y + sum_k A_k C_k; C_k (cols_k x q, row-major, ld q) in device memory.
 template <typename T>
 int launch_update(const BlockList<T>& A, const double2* const* C, int q, long long n,

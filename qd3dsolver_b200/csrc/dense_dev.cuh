@@ -3,56 +3,9 @@
 // eigensolver routines.
 #pragma once
 #include "blockops.cuh"
+#include "gram_dev.cuh"
 
 namespace qdkp {
-
-static __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
-}
-
-
-constexpr int kStageBudget = 64 * 1024;    // shared memory for the row stages of one CTA
-
-// Stages in flight: as many (2..4) as fit the budget, so that a CTA keeps several chunk loads
-// outstanding while it works on one (the kernels are latency- or bandwidth-bound otherwise).
-__host__ __device__ __forceinline__ int stage_count(size_t stage_bytes) {
-  const int ns = (int)(kStageBudget / stage_bytes);
-  return ns < 2 ? 2 : (ns > 4 ? 4 : ns);
-}
-
-// Dynamic shared memory this launch was given (the %dynamic_smem_size special register). The
-// staged kernels fit their stage count and chunk size into it, so a product narrower than the
-// one the launch was sized for can never over-run its allocation.
-__device__ __forceinline__ unsigned dyn_smem_bytes() {
-  unsigned r;
-  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(r));
-  return r;
-}
-
-// Stages (2..4) of `stage_bytes` that fit both the budget and `avail` bytes.
-__device__ __forceinline__ int stage_count_fit(size_t stage_bytes, size_t avail) {
-  int ns = stage_count(stage_bytes);
-  while (ns > 2 && (size_t)ns * stage_bytes > avail) --ns;
-  return ns;
-}
-
-// cp.async.wait_group takes an immediate: wait until at most n (0..3) groups are pending
-__device__ __forceinline__ void cp_async_wait_pending(int n) {
-  if (n >= 3) asm volatile("cp.async.wait_group 3;\n" ::: "memory");
-  else if (n == 2) asm volatile("cp.async.wait_group 2;\n" ::: "memory");
-  else if (n == 1) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-  else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-}
-
-template <typename T>
-static __device__ __forceinline__ double2 list_elem(const BlockList<T>& L, long long r, int c) {
-  int b = 0;
-  while (b < L.nblk - 1 && c >= L.cols[b]) { c -= L.cols[b]; ++b; }
-  const cplx<T> v = L.p[b][r * L.ld[b] + c];
-  return make_double2((double)v.x, (double)v.y);
-}
-
 
 // In-place upper Cholesky of the Hermitian matrix in S (n x n, ld n): S = U^H U, U in the upper
 // triangle. Returns nonzero (block-uniform) if a pivot is not positive and finite.
@@ -291,61 +244,6 @@ static __device__ int block_tql(double2* S0, double2* S1, int n, double2* gtmp) 
   return fail;
 }
 
-
-// Partial Gram sums reduced by the CTAs that finish last, with no waiting. The partials
-// (RP x RQ real each, one per part, `parts` of them) form `split` groups of consecutive parts;
-// every CTA of the launch (all parts, all column panels on blockIdx.y) counts itself in its
-// group's counter once its partial is written; the last of a group sums the group's partials
-// in part order into the group's slot after the partials, and the last group to finish folds
-// the group sums, in group order, into the complex P x Q result. The CTA that completes a count
-// resets it to zero. Sums and their order are those of a two-pass reduction.
-static __device__ void gram_finish_last(double* __restrict__ partial, int parts, int split,
-                                        int* __restrict__ counters, int P, int Q, int part,
-                                        double2* __restrict__ out) {
-  __shared__ int s_last;
-  const int RP = (2 * P + 7) / 8 * 8, RQ = (2 * Q + 7) / 8 * 8;
-  const int elems = RP * RQ;
-  const int per = (parts + split - 1) / split;
-  const int ngroups = (parts + per - 1) / per;
-  const int grp = part / per;
-  const int b0 = grp * per, b1 = min(parts, b0 + per);
-  __threadfence();                                   // this CTA's partial, device-wide
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int members = (b1 - b0) * (int)gridDim.y;
-    s_last = atomicAdd(&counters[grp], 1) == members - 1;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  double* sums = partial + (long long)(parts + grp) * elems;
-  for (int e = threadIdx.x; e < elems; e += blockDim.x) {
-    double acc = 0.0;
-    for (int b = b0; b < b1; ++b) acc += __ldcg(partial + (long long)b * elems + e);
-    sums[e] = acc;
-  }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    counters[grp] = 0;
-    s_last = atomicAdd(&counters[split], 1) == ngroups - 1;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  for (int o = threadIdx.x; o < P * Q; o += blockDim.x) {
-    const int i = o / Q, j = o - i * Q;
-    const long long rr = (long long)(2 * i) * RQ + 2 * j;   // C'_{2i,2j}
-    double re = 0.0, im = 0.0;
-    for (int g = 0; g < ngroups; ++g) {
-      const double* c = partial + (long long)(parts + g) * elems;
-      re += __ldcg(c + rr) + __ldcg(c + rr + RQ + 1);
-      im += __ldcg(c + rr + 1) - __ldcg(c + rr + RQ);
-    }
-    out[o] = make_double2(re, im);
-  }
-  if (threadIdx.x == 0) counters[split] = 0;
-}
 
 // =============================================================================================
 // Rayleigh-Ritz eigensolve for the wanted eigenpairs only: LOBPCG keeps the m smallest of the
@@ -1213,213 +1111,6 @@ static __device__ void update_rows(const BlockList<double>& A, const double2* co
 }
 
 // ---------------------------------------------------------------------------------------------
-// Gram core: partial C' = A'^T B' (real views: row r, column 2c + {re, im}) of rows [r0, r1) on
-// the FP64 MMA units (mma.sync.m8n8k4.f64; the tcgen05 family has no f64 kind). Rows stream
-// through shared memory in chunks (gram_chunk_rows), 2-4 stages in flight with cp.async and one
-// CTA barrier per chunk: every block of
-// the two lists is copied as a flat run of chunk-rows x cols complex values (the engine's blocks
-// are compact, ld = cols; other leading dimensions are handled row by row). Each warp owns a
-// rectangle of MR x MC 8x8 tiles of C' and a slice of the chunk's 4-row k steps, reads its
-// m8n8k4 fragments from shared memory (lane (g, t4): row k0 + t4, real column 8 tile + g) and
-// keeps its tiles in registers. The row slices of a rectangle are summed in shared memory in a
-// fixed order at the end (deterministic), giving one RP x RQ partial per CTA. complex64 blocks
-// are staged as they are and widened to FP64 in the fragment loads.
-// ---------------------------------------------------------------------------------------------
-constexpr int kGramCtaThreads = 256;
-constexpr int kGramRows = 32;       // fewest rows per shared-memory chunk (a multiple of 8)
-constexpr int kGramStageTarget = 24 * 1024;   // bytes a chunk brings in per barrier
-
-// Rows per chunk: about kGramStageTarget bytes of the two lists, a multiple of 8 in
-// [kGramRows, 512], so that narrow products still move many rows per CTA barrier.
-__host__ __device__ __forceinline__ int gram_chunk_rows(int P, int Q, int elem_bytes) {
-  int r = kGramStageTarget / ((P + Q) * elem_bytes);
-  r = r / 8 * 8;
-  return r < kGramRows ? kGramRows : (r > 512 ? 512 : r);
-}
-
-__host__ __device__ __forceinline__ size_t gram_smem_bytes(int P, int Q, int elem_bytes) {
-  const size_t RP = (2 * P + 7) / 8 * 8, RQ = (2 * Q + 7) / 8 * 8;
-  const size_t stage = (size_t)gram_chunk_rows(P, Q, elem_bytes) * (P + Q) * elem_bytes;
-  const size_t red = RP * RQ * sizeof(double);
-  const size_t st = stage_count(stage) * stage;
-  return st > red ? st : red;
-}
-
-template <typename T>
-__device__ __forceinline__ void gram_copy_rows(const BlockList<T>& L, long long r, int nrows,
-                                               cplx<T>* dst, int crow) {
-  int off = 0;
-  for (int b = 0; b < L.nblk; ++b) {
-    const int cols = L.cols[b];
-    const int units = nrows * cols;
-    const cplx<T>* src = L.p[b] + r * L.ld[b];
-    cplx<T>* d = dst + (long long)off * crow;
-    if (L.ld[b] == cols) {
-      if (sizeof(cplx<T>) == 8 && (units & 1) == 0 && ((uintptr_t)src & 15) == 0 &&
-          ((uintptr_t)d & 15) == 0) {
-        // complex64 run that starts and ends on 16 bytes: two values per copy
-        for (int u = 2 * threadIdx.x; u < units; u += 2 * blockDim.x) {
-          const unsigned sa = (unsigned)__cvta_generic_to_shared(d + u);
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(sa), "l"(src + u) : "memory");
-        }
-      } else {
-        for (int u = threadIdx.x; u < units; u += blockDim.x) {
-          const unsigned sa = (unsigned)__cvta_generic_to_shared(d + u);
-          if (sizeof(cplx<T>) == 16)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(sa), "l"(src + u) : "memory");
-          else
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" :: "r"(sa), "l"(src + u) : "memory");
-        }
-      }
-    } else {
-      for (int u = threadIdx.x; u < units; u += blockDim.x) {
-        const int rr = u / cols, c = u - rr * cols;
-        const unsigned sa = (unsigned)__cvta_generic_to_shared(d + u);
-        const cplx<T>* g = src + (long long)rr * L.ld[b] + c;
-        if (sizeof(cplx<T>) == 16)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(sa), "l"(g) : "memory");
-        else
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" :: "r"(sa), "l"(g) : "memory");
-      }
-    }
-    off += cols;
-  }
-}
-
-// tile rectangles: tile rows split in groups of MR, tile columns in groups of MC. A CTA covers
-// the tile columns [tc_lo, tc_lo + tc_cnt) of C' (a column panel; a wide product is split into
-// panels over blockIdx.y so that every rectangle fits one warp's registers) and writes only
-// those columns of its partial.
-template <int MR, int MC, typename T>
-static __device__ void gram_core(const BlockList<T>& A, const BlockList<T>& B,
-                                 long long r0, long long r1, double* __restrict__ out,
-                                 unsigned char* smem, int tc_lo = 0, int tc_cnt = 1 << 30) {
-  const int P = A.total(), Q = B.total();
-  const int RP = (2 * P + 7) / 8 * 8, RQ = (2 * Q + 7) / 8 * 8;
-  const int TR = RP / 8;
-  const int tc_hi = min(RQ / 8, tc_lo + tc_cnt);
-  const int TC = tc_hi - tc_lo;                   // this panel's tile columns
-  if (TC <= 0) return;                            // an empty panel (uniform over the CTA)
-  const int GR = (TR + MR - 1) / MR, GC = (TC + MC - 1) / MC;
-  const int G = GR * GC;                          // tile rectangles (<= warps by construction)
-  const int nwarps = blockDim.x >> 5;
-  const int slices = nwarps / G;                  // warps per rectangle
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t4 = lane & 3;
-  const int rect = warp % G, slice = warp / G;
-  const bool active_warp = slice < slices;
-  const int tr0 = (rect / GC) * MR, tc0 = tc_lo + (rect % GC) * MC;
-  // stage layout: per list, per block, crow x cols complex values; A's blocks first
-  const unsigned avail = dyn_smem_bytes();
-  int crow = gram_chunk_rows(P, Q, (int)sizeof(cplx<T>));
-  {   // two stages must fit the launch's shared memory
-    const int fit = (int)(avail / (2 * (size_t)(P + Q) * sizeof(cplx<T>))) / 8 * 8;
-    if (crow > fit) crow = fit;
-  }
-  const size_t stage_elems = (size_t)crow * (P + Q);
-  const int NS = stage_count_fit(stage_elems * sizeof(cplx<T>), avail);
-  cplx<T>* stage0 = reinterpret_cast<cplx<T>*>(smem);
-  // per tile: the real offset of its column inside a staged row block (-1: outside P / Q)
-  // as (block start in complex columns * crow, block width, real column in the row)
-  int sa_off[MR], sa_w[MR], sa_c[MR], sb_off[MC], sb_w[MC], sb_c[MC];
-#pragma unroll
-  for (int i = 0; i < MR; ++i) {
-    const int col = (tr0 + i) * 8 + g;           // real column of A'
-    int c = col >> 1, blk = 0, start = 0;
-    while (blk < A.nblk - 1 && c >= A.cols[blk]) { c -= A.cols[blk]; start += A.cols[blk]; ++blk; }
-    const bool ok = active_warp && tr0 + i < TR && col < 2 * P;
-    sa_off[i] = ok ? start * crow : -1;
-    sa_w[i] = A.cols[blk];
-    sa_c[i] = 2 * c + (col & 1);
-  }
-#pragma unroll
-  for (int j = 0; j < MC; ++j) {
-    const int col = (tc0 + j) * 8 + g;
-    int c = col >> 1, blk = 0, start = 0;
-    while (blk < B.nblk - 1 && c >= B.cols[blk]) { c -= B.cols[blk]; start += B.cols[blk]; ++blk; }
-    const bool ok = active_warp && tc0 + j < tc_hi && col < 2 * Q;
-    sb_off[j] = ok ? (P + start) * crow : -1;
-    sb_w[j] = B.cols[blk];
-    sb_c[j] = 2 * c + (col & 1);
-  }
-  double acc[MR][MC][2];
-#pragma unroll
-  for (int i = 0; i < MR; ++i)
-#pragma unroll
-    for (int j = 0; j < MC; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-  const long long nrows = r1 - r0;
-  const int nchunks = (int)((nrows + crow - 1) / crow);
-  // chunk c lives in stage c % NS; NS - 1 chunks are in flight while one is consumed
-  auto issue = [&](int c) {
-    if (c < nchunks) {
-      const long long rn = r0 + (long long)c * crow;
-      const int nn = (int)min((long long)crow, r1 - rn);
-      cplx<T>* st = stage0 + (size_t)(c % NS) * stage_elems;
-      gram_copy_rows(A, rn, nn, st, crow);
-      gram_copy_rows(B, rn, nn, st + (size_t)P * crow, crow);
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
-  for (int c = 0; c < NS - 1; ++c) issue(c);
-  for (int ch = 0; ch < nchunks; ++ch) {
-    const long long rc = r0 + (long long)ch * crow;
-    const int rows = (int)min((long long)crow, r1 - rc);
-    // chunk ch has landed once at most NS - 2 groups are pending; the barrier also means every
-    // warp is done with chunk ch - 1, whose stage the next copy reuses
-    cp_async_wait_pending(NS - 2);
-    __syncthreads();
-    issue(ch + NS - 1);
-    const T* sr = reinterpret_cast<const T*>(stage0 + (size_t)(ch % NS) * stage_elems);
-    if (active_warp) {
-      for (int k0 = 4 * slice; k0 < rows; k0 += 4 * slices) {
-        const int row = k0 + t4;
-        const bool ok = row < rows;
-        double a[MR], b[MC];
-#pragma unroll
-        for (int i = 0; i < MR; ++i)
-          a[i] = (ok && sa_off[i] >= 0)
-                     ? (double)sr[2 * sa_off[i] + row * 2 * sa_w[i] + sa_c[i]] : 0.0;
-#pragma unroll
-        for (int j = 0; j < MC; ++j)
-          b[j] = (ok && sb_off[j] >= 0)
-                     ? (double)sr[2 * sb_off[j] + row * 2 * sb_w[j] + sb_c[j]] : 0.0;
-#pragma unroll
-        for (int i = 0; i < MR; ++i)
-#pragma unroll
-          for (int j = 0; j < MC; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-      }
-    }
-  }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  __syncthreads();
-  // fixed-order sum of the row slices of each rectangle
-  double* gsm = reinterpret_cast<double*>(smem);
-  for (int e = threadIdx.x; e < RP * RQ; e += blockDim.x) gsm[e] = 0.0;
-  __syncthreads();
-  for (int sl = 0; sl < slices; ++sl) {
-    if (active_warp && slice == sl) {
-#pragma unroll
-      for (int i = 0; i < MR; ++i)
-#pragma unroll
-        for (int j = 0; j < MC; ++j) {
-          const int ti = tr0 + i, tj = tc0 + j;
-          if (ti < TR && tj < tc_hi) {
-            const int rr = ti * 8 + g, cc = tj * 8 + 2 * t4;
-            gsm[rr * RQ + cc] += acc[i][j][0];
-            gsm[rr * RQ + cc + 1] += acc[i][j][1];
-          }
-        }
-    }
-    __syncthreads();
-  }
-  for (int e = threadIdx.x; e < RP * RQ; e += blockDim.x) {
-    const int cc = e % RQ;
-    if (cc >= 8 * tc_lo && cc < 8 * tc_hi) out[e] = gsm[e];
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
 // complex64 blocks: split-precision TF32 tensor-core products (mma.sync.m16n8k8 .tf32, FP32
 // accumulation). Every FP32 value x is split into x = hi + lo with hi, lo TF32 (10-bit
 // mantissas; cvt.rna), and a product is formed as lo*hi + hi*lo + hi*hi (the lo*lo term is below
@@ -1450,154 +1141,6 @@ __device__ __forceinline__ void mma_tf32x3(float (&d)[4], const unsigned (&ah)[4
   mma_tf32(d, al[0], al[1], al[2], al[3], bh[0], bh[1]);
   mma_tf32(d, ah[0], ah[1], ah[2], ah[3], bl[0], bl[1]);
   mma_tf32(d, ah[0], ah[1], ah[2], ah[3], bh[0], bh[1]);
-}
-
-// Gram partial C' = A'^T B' over rows [r0, r1) of complex64 lists (same staging and output as
-// gram_core). MMA tiles: 16 columns of A' (M) x 8 columns of B' (N) x 8 rows (K); a warp owns a
-// rectangle of kTfMR x kTfMC tiles and a slice of the chunk's 8-row k steps.
-// Fragments (m16n8k8 tf32; g = lane / 4, t = lane % 4): A_mma[m][k] = A'[k][m]:
-// a0 = (k t, m g), a1 = (k t, m g + 8), a2 = (k t + 4, m g), a3 = (k t + 4, m g + 8);
-// B_mma[k][n] = B'[k][n]: b0 = (k t, n g), b1 = (k t + 4, n g); D: (m g, n 2t), (m g, n 2t + 1),
-// (m g + 8, n 2t), (m g + 8, n 2t + 1).
-constexpr int kTfMR = 3, kTfMC = 3;
-
-__host__ __device__ __forceinline__ int gram_tf32_rects(int P, int Q) {
-  const int TR = (2 * P + 15) / 16, TC = (2 * Q + 7) / 8;
-  return ((TR + kTfMR - 1) / kTfMR) * ((TC + kTfMC - 1) / kTfMC);
-}
-
-static __device__ void gram_core_tf32(const BlockList<float>& A, const BlockList<float>& B,
-                                      long long r0, long long r1, double* __restrict__ out,
-                                      unsigned char* smem) {
-  const int P = A.total(), Q = B.total();
-  const int RP = (2 * P + 7) / 8 * 8, RQ = (2 * Q + 7) / 8 * 8;   // partial layout (as FP64 core)
-  const int TR = (2 * P + 15) / 16, TC = (2 * Q + 7) / 8;
-  const int GC = (TC + kTfMC - 1) / kTfMC;
-  const int G = gram_tf32_rects(P, Q);
-  const int nwarps = blockDim.x >> 5;
-  const int slices = nwarps / G;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int rect = warp % G, slice = warp / G;
-  const bool active_warp = slice < slices;
-  const int tr0 = (rect / GC) * kTfMR, tc0 = (rect % GC) * kTfMC;
-  const unsigned avail = dyn_smem_bytes();
-  int crow = gram_chunk_rows(P, Q, (int)sizeof(float2));
-  {
-    const int fit = (int)(avail / (2 * (size_t)(P + Q) * sizeof(float2))) / 8 * 8;
-    if (crow > fit) crow = fit;
-  }
-  const size_t stage_elems = (size_t)crow * (P + Q);
-  const int NS = stage_count_fit(stage_elems * sizeof(float2), avail);
-  float2* stage0 = reinterpret_cast<float2*>(smem);
-  // staged real offset of a real column of A' (two per M tile: m g, m g + 8) and of B' (n g)
-  int ao[kTfMR][2], aw[kTfMR][2], bo[kTfMC], bw[kTfMC];
-#pragma unroll
-  for (int i = 0; i < kTfMR; ++i)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int col = (tr0 + i) * 16 + g + 8 * h;
-      int c = col >> 1, blk = 0, start = 0;
-      while (blk < A.nblk - 1 && c >= A.cols[blk]) { c -= A.cols[blk]; start += A.cols[blk]; ++blk; }
-      const bool ok = active_warp && tr0 + i < TR && col < 2 * P;
-      ao[i][h] = ok ? 2 * start * crow + 2 * c + (col & 1) : -1;
-      aw[i][h] = 2 * A.cols[blk];
-    }
-#pragma unroll
-  for (int j = 0; j < kTfMC; ++j) {
-    const int col = (tc0 + j) * 8 + g;
-    int c = col >> 1, blk = 0, start = 0;
-    while (blk < B.nblk - 1 && c >= B.cols[blk]) { c -= B.cols[blk]; start += B.cols[blk]; ++blk; }
-    const bool ok = active_warp && tc0 + j < TC && col < 2 * Q;
-    bo[j] = ok ? 2 * (P + start) * crow + 2 * c + (col & 1) : -1;
-    bw[j] = 2 * B.cols[blk];
-  }
-  float acc[kTfMR][kTfMC][4];
-#pragma unroll
-  for (int i = 0; i < kTfMR; ++i)
-#pragma unroll
-    for (int j = 0; j < kTfMC; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
-
-  const long long nrows = r1 - r0;
-  const int nchunks = (int)((nrows + crow - 1) / crow);
-  auto issue = [&](int c) {
-    if (c < nchunks) {
-      const long long rn = r0 + (long long)c * crow;
-      const int nn = (int)min((long long)crow, r1 - rn);
-      float2* st = stage0 + (size_t)(c % NS) * stage_elems;
-      gram_copy_rows(A, rn, nn, st, crow);
-      gram_copy_rows(B, rn, nn, st + (size_t)P * crow, crow);
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
-  for (int c = 0; c < NS - 1; ++c) issue(c);
-  for (int ch = 0; ch < nchunks; ++ch) {
-    const long long rc = r0 + (long long)ch * crow;
-    const int rows = (int)min((long long)crow, r1 - rc);
-    // chunk ch has landed once at most NS - 2 groups are pending; the barrier also means every
-    // warp is done with chunk ch - 1, whose stage the next copy reuses
-    cp_async_wait_pending(NS - 2);
-    __syncthreads();
-    issue(ch + NS - 1);
-    const float* sr = reinterpret_cast<const float*>(stage0 + (size_t)(ch % NS) * stage_elems);
-    if (active_warp) {
-      for (int k0 = 8 * slice; k0 < rows; k0 += 8 * slices) {
-        const int ra = k0 + t, rb = k0 + t + 4;      // the two rows of this lane's fragments
-        const bool oka = ra < rows, okb = rb < rows;
-        unsigned bh[kTfMC][2], bl[kTfMC][2];
-#pragma unroll
-        for (int j = 0; j < kTfMC; ++j) {
-          const float x0 = (oka && bo[j] >= 0) ? sr[bo[j] + ra * bw[j]] : 0.f;
-          const float x1 = (okb && bo[j] >= 0) ? sr[bo[j] + rb * bw[j]] : 0.f;
-          tf32_split(x0, bh[j][0], bl[j][0]);
-          tf32_split(x1, bh[j][1], bl[j][1]);
-        }
-#pragma unroll
-        for (int i = 0; i < kTfMR; ++i) {
-          const float v0 = (oka && ao[i][0] >= 0) ? sr[ao[i][0] + ra * aw[i][0]] : 0.f;
-          const float v1 = (oka && ao[i][1] >= 0) ? sr[ao[i][1] + ra * aw[i][1]] : 0.f;
-          const float v2 = (okb && ao[i][0] >= 0) ? sr[ao[i][0] + rb * aw[i][0]] : 0.f;
-          const float v3 = (okb && ao[i][1] >= 0) ? sr[ao[i][1] + rb * aw[i][1]] : 0.f;
-          unsigned ah[4], al[4];
-          tf32_split(v0, ah[0], al[0]);
-          tf32_split(v1, ah[1], al[1]);
-          tf32_split(v2, ah[2], al[2]);
-          tf32_split(v3, ah[3], al[3]);
-#pragma unroll
-          for (int j = 0; j < kTfMC; ++j) mma_tf32x3(acc[i][j], ah, al, bh[j], bl[j]);
-        }
-      }
-    }
-  }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  __syncthreads();
-  double* gsm = reinterpret_cast<double*>(smem);
-  for (int e = threadIdx.x; e < RP * RQ; e += blockDim.x) gsm[e] = 0.0;
-  __syncthreads();
-  for (int sl = 0; sl < slices; ++sl) {
-    if (active_warp && slice == sl) {
-#pragma unroll
-      for (int i = 0; i < kTfMR; ++i)
-#pragma unroll
-        for (int j = 0; j < kTfMC; ++j) {
-          const int ti = tr0 + i, tj = tc0 + j;
-          if (ti < TR && tj < TC) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int rr = ti * 16 + g + 8 * h, cc = tj * 8 + 2 * t;
-              if (rr < RP && cc < RQ) {
-                gsm[rr * RQ + cc] += (double)acc[i][j][2 * h];
-                gsm[rr * RQ + cc + 1] += (double)acc[i][j][2 * h + 1];
-              }
-            }
-          }
-        }
-    }
-    __syncthreads();
-  }
-  for (int e = threadIdx.x; e < RP * RQ; e += blockDim.x) out[e] = gsm[e];
 }
 
 // Y' = A' C'' for rows [r0, r1) of complex64 blocks on TF32 tensor cores (split as above).
@@ -1792,23 +1335,6 @@ static __device__ void update_rows_tf32(const BlockList<float>& A, const double2
     default: break;
   }
 #undef QDKP_TF_CASE
-}
-
-// Launch plan of an FP64 Gram product of P x Q complex columns: 3 x 3-tile rectangles (the
-// register-resident size), 8 or 16 warps, and, for a product wider than 16 rectangles, column
-// panels of `ptc` tile columns on blockIdx.y. Depends only on P and Q.
-struct GramPlan { int threads, ptc, panels; };
-static inline GramPlan gram_plan(int P, int Q) {
-  const int TR = ((2 * P + 7) / 8 * 8) / 8, TC = ((2 * Q + 7) / 8 * 8) / 8;
-  const int GR = (TR + 2) / 3, GC = (TC + 2) / 3;
-  GramPlan g;
-  if (GR * GC <= 8) { g.threads = 256; g.ptc = TC; g.panels = 1; return g; }
-  if (GR * GC <= 16) { g.threads = 512; g.ptc = TC; g.panels = 1; return g; }
-  const int gcp = GR >= 16 ? 1 : 16 / GR;        // rectangle columns per panel
-  g.threads = 512;
-  g.ptc = 3 * gcp;
-  g.panels = (TC + g.ptc - 1) / g.ptc;
-  return g;
 }
 
 }  // namespace qdkp

@@ -21,11 +21,9 @@ int launch_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, i
 
 constexpr int kERowsPerCta = 512;    // rows per CTA of the row kernels
 constexpr int kENormRows = 2048;     // rows per CTA of the norm kernel
-// Gram CTAs per slot: ceil(n / 256) up to this many. The split depends only on the slot's own
-// size, so the order of every Gram sum -- and so the result -- is the same alone and in a mix.
-constexpr int kEGramMaxParts = 296;
 
-enum GramWhich { GR_XR = 0, GR_RR, GR_PP, GR_WW, GR_WAW, GR_BA, GR_BB };
+// GR_RZ: the products of the Rayleigh-Ritz pencil, in one pass (GK_PENCIL or GK_EXPLICIT)
+enum GramWhich { GR_XR = 0, GR_RR, GR_PP, GR_RZ };
 // UP_XPNEW: P = R Cr + P Cp and X = X Cx + R Cr + P Cp from one pass over [X | R | P]
 // (lobpcg.py:921-973); UP_AXPNEW: the same for AP and AX.
 enum UpdWhich { UP_RPROJ = 0, UP_RNORM, UP_PNORM, UP_APNORM, UP_XPNEW, UP_AXPNEW };
@@ -189,96 +187,95 @@ e_row_kernel(const ESlot* __restrict__ S, int ns, int which) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Gram products, multi-slot (same FP64 MMA scheme as gram_partial_kernel)
+// Gram products, multi-slot (gram_dev.cuh). complex64 slots form them in FP64 too: the Gram matrices
+// of the search stay exact to FP64 (a split TF32 form loses convergence in the explicit-Gram regime
+// of scipy's method).
 // ---------------------------------------------------------------------------------------------
 template <typename T>
-__device__ bool gram_lists(const ESlot& d, int which, BlockList<T>& A, BlockList<T>& B,
-                           double2*& out) {
+__device__ bool gram_task(const ESlot& d, int which, GramTask<T>& t, double2*& out, double2*& outS) {
   const EState* st = d.st;
-  if (st->idle) return false;
+  if (st->idle || (which == GR_PP && st->skip_p)) return false;
   const int m = d.m, ma = st->ma, mp = st->mp;
-  auto set1 = [](BlockList<T>& L, const cplx<T>* p, int c) {
-    L.nblk = 1; L.p[0] = p; L.ld[0] = c; L.cols[0] = c;
+  t.nblk = 0; t.tc = 0;
+  t.m = m; t.ma = ma; t.mp = mp; t.n = d.n;
+  t.a0 = 0; t.b0 = 0;
+  auto add = [&](double2* p, int ld, int cols) {
+    t.p[t.nblk] = blk<T>(p); t.ld[t.nblk] = ld; t.cols[t.nblk] = cols;
+    ++t.nblk;
+    t.tc += cols;
   };
-  const cplx<T>* X = blk<T>(d.X);
-  const cplx<T>* AX = blk<T>(d.AX);
-  const cplx<T>* Ra = blk<T>(d.Ra);
-  const cplx<T>* ARa = blk<T>(d.ARa);
-  const cplx<T>* Pa = blk<T>(d.Pa);
-  const cplx<T>* APa = blk<T>(d.APa);
+  outS = nullptr;
   switch (which) {
-    case GR_XR: set1(A, X, m); set1(B, Ra, ma); out = d.W; return true;
-    case GR_RR: set1(A, Ra, ma); set1(B, Ra, ma); out = d.G; return true;
-    case GR_PP:
-      if (st->skip_p) return false;
-      set1(A, Pa, ma); set1(B, Pa, ma); out = d.G; return true;
-    case GR_BA:      // non-explicit: [X | R | P]^H [AR | AP]
-      if (st->explicit_gram) return false;
-      A.nblk = mp ? 3 : 2;
-      A.p[0] = X; A.ld[0] = m; A.cols[0] = m;
-      A.p[1] = Ra; A.ld[1] = ma; A.cols[1] = ma;
-      A.p[2] = Pa; A.ld[2] = ma; A.cols[2] = mp;
-      B.nblk = mp ? 2 : 1;
-      B.p[0] = ARa; B.ld[0] = ma; B.cols[0] = ma;
-      B.p[1] = APa; B.ld[1] = ma; B.cols[1] = mp;
-      out = d.gT;
+    case GR_XR:
+      add(d.X, m, m); add(d.Ra, ma, ma);
+      t.P = m; t.b0 = m; t.Q = ma; t.kind = GK_FULL; out = d.W;
       return true;
-    case GR_BB:      // non-explicit: [X | R]^H P
-      if (st->explicit_gram || mp == 0) return false;
-      A.nblk = 2;
-      A.p[0] = X; A.ld[0] = m; A.cols[0] = m;
-      A.p[1] = Ra; A.ld[1] = ma; A.cols[1] = ma;
-      set1(B, Pa, mp);
-      B.ld[0] = ma;
-      out = d.gS;
+    case GR_RR: case GR_PP:
+      add(which == GR_RR ? d.Ra : d.Pa, ma, ma);
+      t.P = t.Q = ma; t.kind = GK_HERM; out = d.G;
       return true;
-    default: {       // explicit Gram mode: the full W^H W and W^H AW
-      if (!st->explicit_gram) return false;
-      A.nblk = mp ? 3 : 2;
-      A.p[0] = X; A.ld[0] = m; A.cols[0] = m;
-      A.p[1] = Ra; A.ld[1] = ma; A.cols[1] = ma;
-      A.p[2] = Pa; A.ld[2] = ma; A.cols[2] = mp;
-      if (which == GR_WW) { B = A; out = d.gS; return true; }
-      B.nblk = A.nblk;
-      B.p[0] = AX; B.ld[0] = m; B.cols[0] = m;
-      B.p[1] = ARa; B.ld[1] = ma; B.cols[1] = ma;
-      B.p[2] = APa; B.ld[2] = ma; B.cols[2] = mp;
-      out = d.gT;
+    default:
+      add(d.X, m, m); add(d.Ra, ma, ma); add(d.Pa, ma, mp);
+      t.P = m + ma + mp;
+      if (st->explicit_gram) {
+        add(d.AX, m, m); add(d.ARa, ma, ma); add(d.APa, ma, mp);
+        t.Q = 2 * t.P; t.kind = GK_EXPLICIT;
+      } else {
+        add(d.ARa, ma, ma); add(d.APa, ma, mp);
+        t.b0 = m + ma; t.Q = mp + ma + mp; t.kind = GK_PENCIL;
+      }
+      out = d.gT; outS = d.gS;
       return true;
-    }
   }
 }
 
-// Launched once per distinct block width m present: the tile shape (and so the order of every
-// sum) then depends only on the slot's own sizes, never on which other solves share the batch.
-template <int MR, int MC>
-__global__ void __launch_bounds__(512)
-e_gram_kernel(const ESlot* __restrict__ S, int ns, int which, int m_only, int ptc) {
+// Launched once per distinct block width m present: the warps of a CTA (and so the order of every
+// sum) then depend only on the slot's own sizes, never on which other solves share the batch.
+template <typename T>
+__device__ void e_gram_body(const ESlot& d, int which, int part, unsigned char* smem) {
+  __shared__ GramTask<T> t;
+  __shared__ int go;
+  if (threadIdx.x == 0) {
+    double2 *out, *outS;
+    go = gram_task<T>(d, which, t, out, outS);
+  }
+  __syncthreads();
+  if (go) gram_core(t, part, d.gparts, (int)blockIdx.y, d.gpart, smem);
+}
+
+__global__ void __launch_bounds__(32 * (kGramMaxWarps + 1), 1)
+e_gram_kernel(const ESlot* __restrict__ S, int ns, int which, int m_only) {
   extern __shared__ __align__(16) unsigned char gsm_e[];
   const int k = slot_of(S, ns, blockIdx.x, &ESlot::gram0);
   const ESlot& d = S[k];
   if (d.m != m_only) return;
   const int part = blockIdx.x - d.gram0;
-  const long long r0 = (long long)part * d.rows_per_gpart;
-  double2* out;
-  if (d.prec == QDKP_C64) {
-    BlockList<float> A, B;
-    if (!gram_lists<float>(d, which, A, B, out)) return;
-    const int RP = (2 * A.total() + 7) / 8 * 8, RQ = (2 * B.total() + 7) / 8 * 8;
-    // complex64 blocks, FP64 products: the Gram matrices of the search stay exact to FP64
-    // (the split TF32 form loses convergence in the explicit-Gram regime of scipy's method)
-    double* po = d.gpart + (long long)part * RP * RQ;
-    gram_core<MR, MC>(A, B, r0, min(d.n, r0 + d.rows_per_gpart), po, gsm_e, blockIdx.y * ptc,
-                      ptc);
-    gram_finish_last(d.gpart, d.gparts, kEGramSplit, d.st->gram_done, A.total(), B.total(), part, out);
-  } else {
-    BlockList<double> A, B;
-    if (!gram_lists<double>(d, which, A, B, out)) return;
-    const int RP = (2 * A.total() + 7) / 8 * 8, RQ = (2 * B.total() + 7) / 8 * 8;
-    gram_core<MR, MC>(A, B, r0, min(d.n, r0 + d.rows_per_gpart),
-                      d.gpart + (long long)part * RP * RQ, gsm_e, blockIdx.y * ptc, ptc);
-    gram_finish_last(d.gpart, d.gparts, kEGramSplit, d.st->gram_done, A.total(), B.total(), part, out);
+  if (d.prec == QDKP_C64) e_gram_body<float>(d, which, part, gsm_e);
+  else e_gram_body<double>(d, which, part, gsm_e);
+}
+
+// a row of CTAs (blockIdx.y) per slot
+template <typename T>
+__device__ void e_gram_reduce_body(const ESlot& d, int which) {
+  __shared__ GramTask<T> t;
+  __shared__ double2 *out, *outS;
+  __shared__ int go;
+  if (threadIdx.x == 0) {
+    double2 *o = nullptr, *oS = nullptr;
+    go = gram_task<T>(d, which, t, o, oS);
+    out = o; outS = oS;
   }
+  __syncthreads();
+  if (go)
+    gram_reduce_core(t, d.gparts, d.gpart, (int)blockIdx.x, (int)gridDim.x,
+                     [&](int i, int j, double2 v) { gram_put(t, i, j, v, out, outS); });
+}
+
+__global__ void __launch_bounds__(kGramRedThreads)
+e_gram_reduce_kernel(const ESlot* __restrict__ S, int which) {
+  const ESlot& d = S[blockIdx.y];
+  if (d.prec == QDKP_C64) e_gram_reduce_body<float>(d, which);
+  else e_gram_reduce_body<double>(d, which);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -536,7 +533,6 @@ size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 struct SlotLayout {
   size_t blk, small, npart, gpart, total;
   int nparts, gparts;
-  long long rows_per_gpart;
 };
 
 SlotLayout slot_layout(int64_t n, int m, int prec) {
@@ -545,15 +541,9 @@ SlotLayout slot_layout(int64_t n, int m, int prec) {
   L.small = align256((size_t)(3 * m) * (3 * m) * sizeof(double2));
   L.nparts = (int)((n + kENormRows - 1) / kENormRows);
   L.npart = align256((size_t)L.nparts * m * sizeof(double));
-  long long parts = (n + 255) / 256;
-  if (parts > kEGramMaxParts) parts = kEGramMaxParts;
-  if (parts < 1) parts = 1;
-  long long rpp = (n + parts - 1) / parts;
-  rpp = (rpp + 3) / 4 * 4;
-  L.gparts = (int)((n + rpp - 1) / rpp);
-  L.rows_per_gpart = rpp;
-  const size_t RP = (6 * m + 7) / 8 * 8;
-  L.gpart = align256((size_t)(L.gparts + kEGramSplit) * RP * RP * sizeof(double));
+  L.gparts = gram_parts(n);
+  // the widest task: 3 m x 6 m columns (explicit Gram matrices)
+  L.gpart = align256(gram_partial_elems(3 * m, 6 * m) * sizeof(double2));
   L.total = align256(sizeof(EState)) + 10 * L.blk + 14 * L.small +
             align256(3 * m * sizeof(double)) + L.npart + L.gpart;
   return L;
@@ -765,20 +755,23 @@ int rebuild(qdkp_engine* e, cudaStream_t st) {
 }
 
 int launch_gram_multi(const EGroup& G, int which, cudaStream_t st) {
+  int mmax = 0;
   for (int m : G.widths) {
-    int P = m, Q = m;
-    if (which == GR_BA) { P = 3 * m; Q = 2 * m; }
-    else if (which == GR_BB) { P = 2 * m; Q = m; }
-    else if (which == GR_WW || which == GR_WAW) { P = 3 * m; Q = 3 * m; }
-    const size_t smem = std::max(gram_smem_bytes(P, Q, (int)sizeof(double2)),
-                                 gram_smem_bytes(P, Q, (int)sizeof(float2)));
-    // the plan for the widest product this width can form; a narrower one on the device leaves
-    // its last panels empty
-    const GramPlan gp = gram_plan(P, Q);
-    e_gram_kernel<3, 3><<<dim3(G.gram_ctas, gp.panels), gp.threads, smem, st>>>(
-        G.d_slots, G.ns, which, m, gp.ptc);
+    // the warps for the product at full width; panels for the most rectangles any active width and
+    // either pencil can form (the CTAs of panels that stay empty return at once)
+    const int P = which == GR_RZ ? 3 * m : m, Q = P, tc = which == GR_RZ ? 6 * m : 2 * m;
+    const int kind = which == GR_XR ? GK_FULL : (which == GR_RZ ? GK_PENCIL : GK_HERM);
+    const GramShape sh = gram_shape(kind, P, Q, m, m, m);
+    const int most = (P + kGramRect - 1) / kGramRect * (((which == GR_RZ ? 6 * m : m) + kGramRect - 1) / kGramRect);
+    const size_t smem = std::max(gram_smem<double>(tc, sh.warps), gram_smem<float>(tc, sh.warps));
+    e_gram_kernel<<<dim3(G.gram_ctas, (most + sh.warps - 1) / sh.warps), 32 * (sh.warps + 1), smem, st>>>(
+        G.d_slots, G.ns, which, m);
     count_launch();
+    mmax = std::max(mmax, m);
   }
+  const int outs = (which == GR_RZ ? 3 * mmax * 6 * mmax : mmax * mmax);
+  e_gram_reduce_kernel<<<dim3((outs + 31) / 32, G.ns), kGramRedThreads, 0, st>>>(G.d_slots, which);
+  count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;
 }
@@ -848,10 +841,7 @@ int tick(const qdkp_engine* e, const EGroup& G, cudaStream_t st) {
   count_launch();
   ETRY(launch_update_multi(G, UP_PNORM, st));
   ETRY(launch_update_multi(G, UP_APNORM, st));
-  ETRY(launch_gram_multi(G, GR_BA, st));
-  ETRY(launch_gram_multi(G, GR_BB, st));
-  ETRY(launch_gram_multi(G, GR_WW, st));
-  ETRY(launch_gram_multi(G, GR_WAW, st));
+  ETRY(launch_gram_multi(G, GR_RZ, st));
   e_rr_kernel<<<ns, kSmallThreads, rr_smem, st>>>(G.d_slots);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
@@ -961,7 +951,7 @@ int qdkp_engine_create(int max_slots, int device, qdkp_engine** out) {
   }
   // dynamic shared memory limits of the engine kernels
   const int big = 200 * 1024;
-  cudaFuncSetAttribute(e_gram_kernel<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramMaxSmem);
   cudaFuncSetAttribute(e_update_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(e_update_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(e_update_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1044,7 +1034,7 @@ int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg
   d.maxiter = prm->maxiter;
   d.stall_iterations = prm->stall_iterations;
   d.restart_control = prm->restart_control > 0 ? prm->restart_control : 20;
-  d.nparts = L.nparts; d.gparts = L.gparts; d.rows_per_gpart = L.rows_per_gpart;
+  d.nparts = L.nparts; d.gparts = L.gparts;
   d.rows_per_cta = kERowsPerCta;
   int rc;
 #define ATRY(x) do { rc = (x); if (rc != QDKP_OK) return rc; } while (0)

@@ -8,8 +8,6 @@
 namespace qdkp {
 
 // Per-slot mutable state (device memory, written by the decision kernels).
-constexpr int kEGramSplit = 16;      // groups of Gram partials summed by their last CTA
-
 struct EState {
   int running;          // 1 while the slot iterates
   int status;           // QDKP_LOBPCG_* once it stopped
@@ -28,9 +26,6 @@ struct EState {
   int idx[kMaxBlock];
   double lam[kMaxBlock];
   double norms[kMaxBlock];
-  // CTAs of the current Gram product done, per partial group; the last slot counts the groups
-  // reduced. The CTA that completes a count resets it to 0.
-  int gram_done[kEGramSplit + 1];
 };
 
 // Per-slot constant descriptor (built on the host at admission, device resident).
@@ -51,10 +46,9 @@ struct ESlot {
   double2 *W, *G, *U, *gS, *gT, *gA, *gB, *E, *scr, *Cx, *Cr, *Cp, *Im;
   double* w;
   double* npart;        // [nparts][m] residual-norm partials
-  double* gpart;        // Gram partials (real), then the split sums
+  double* gpart;        // Gram partials (real)
   int nparts;           // CTAs of the norm kernel
-  int gparts;           // CTAs of the Gram kernel
-  long long rows_per_gpart;
+  int gparts;           // row parts (CTAs) of the Gram kernel
   int norm0, gram0, row0;   // first CTA of this slot in the norm / Gram / row-kernel launches
   int utile0;           // complex64 slots: first 128-row tile in the group's tcgen05 update space
   int rows_per_cta;     // rows per CTA in the row kernels (gather, update)

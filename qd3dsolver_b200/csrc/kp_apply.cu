@@ -31,13 +31,11 @@
 //   kp_march_kernel   a CTA owns a tile of (y, z) sites and a few columns and marches along x.
 //   kp_apply_kernel   one thread per (site, column), neighbours through L1/L2: small blocks,
 //                     four-band slices, and the batched engine.
-#include <cuda.h>   // CUtensorMap and its enums (the encoder is fetched from the runtime)
-
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
 
-#include "qdkp_common.cuh"
+#include "mbar_dev.cuh"     // CUtensorMap and its enums (the encoder is fetched from the runtime)
 
 namespace qdkp {
 
@@ -890,40 +888,6 @@ kp_march_kernel(const MarchArgs<typename G::T> a) {
 // ---------------------------------------------------------------------------------------------
 __device__ int g_apply_fault;      // set when a wait on a copy gave up (qdkp_device_fault)
 
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
-  unsigned ok;
-  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-               " selp.b32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  return ok != 0;
-}
-// Bounded wait: gives up after about a second of SM clocks (a copy that never lands).
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity))
-    if (clock64() - t0 > 2000000000LL) return false;
-  return true;
-}
-__device__ __forceinline__ void tma_load_5d(unsigned dst, const CUtensorMap* map, unsigned bar,
-                                            int c0, int c1, int c2, int c3, int c4) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-      :: "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2),
-         "r"(c3), "r"(c4) : "memory");
-}
-__device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-
 template <class G, int NB, int NS, bool CONV>
 __global__ void __launch_bounds__(G::THREADS, G::MINB)
 kp_march_tma_kernel(const __grid_constant__ CUtensorMap tmx, const MarchArgs<typename G::T> a) {
@@ -965,7 +929,7 @@ kp_march_tma_kernel(const __grid_constant__ CUtensorMap tmx, const MarchArgs<typ
   };
   if (t == 0) {
     for (int i = 0; i < NS; ++i) mbar_init(bars + 8u * i, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_init_fence();
     for (int p = p0; p < p0 + NS && p <= p1; ++p) issue(p);
   }
   __syncthreads();

@@ -42,7 +42,7 @@ struct Layout {
 Layout layout(int64_t n, int m, int folded) {
   Layout L;
   L.blk = ((size_t)n * m * sizeof(double2) + 255) / 256 * 256;
-  L.gpart_elems = gram_partial_elems(3 * m, 3 * m);
+  L.gpart_elems = gram_partial_elems(3 * m, 6 * m);
   const size_t small = (size_t)(3 * m) * (3 * m) * sizeof(double2);
   L.total = (size_t)(9 + (folded ? 1 : 0)) * L.blk          // X AX P AP best Ra ARa Pa APa [T]
             + L.gpart_elems * sizeof(double2)                 // gram partials
@@ -403,30 +403,22 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
     hS.assign((size_t)tot * tot, make_double2(0.0, 0.0));
     hT.assign((size_t)tot * tot, make_double2(0.0, 0.0));
     if (explicit_gram) {
-      TRY(s.gram(Wl, Wl, b.gS));
-      TRY(s.gram(Wl, AWl, b.gT));
+      TRY(launch_gram_rz(Wl, AWl, true, n, b.gpart, s.L.gpart_elems, b.gT, b.gS, st));
       TRY(s.sync_read(hS.data(), b.gS, hS.size() * sizeof(double2)));
       TRY(s.sync_read(hT.data(), b.gT, hT.size() * sizeof(double2)));
     } else {
-      // only the blocks the non-explicit pencils read (lobpcg.py:856-861): [X|R|P]^H [AR|AP]
-      // and [X|R]^H P, scattered into the full W^H AW / W^H W layouts
+      // only the blocks the non-explicit pencils read (lobpcg.py:856-861): [X|R|P]^H [AR|AP] and
+      // [X|R]^H P, scattered into the full W^H AW / W^H W layouts
       const int nAB = ma + mp;
-      BlockList<double> ABl = mp ? blist({{b.ARa, ma}, {b.APa, mp}}) : blist({{b.ARa, ma}});
-      ABl.ld[0] = ma; if (mp) ABl.ld[1] = ma;
-      TRY(s.gram(Wl, ABl, b.gT));
-      std::vector<double2> t2((size_t)tot * nAB);
-      TRY(s.sync_read(t2.data(), b.gT, t2.size() * sizeof(double2)));
+      TRY(launch_gram_rz(Wl, AWl, false, n, b.gpart, s.L.gpart_elems, b.gT, b.gS, st));
+      std::vector<double2> t2((size_t)tot * nAB), s2((size_t)(m + ma) * mp);
+      QDKP_CUDA_TRY(cudaMemcpyAsync(t2.data(), b.gT, t2.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
+      if (mp) QDKP_CUDA_TRY(cudaMemcpyAsync(s2.data(), b.gS, s2.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
+      QDKP_CUDA_TRY(cudaStreamSynchronize(st));
       for (int i = 0; i < tot; ++i)
         for (int c = 0; c < nAB; ++c) hT[(size_t)i * tot + m + c] = t2[(size_t)i * nAB + c];
-      if (mp) {
-        BlockList<double> XR = blist({{b.X, m}, {b.Ra, ma}});
-        XR.ld[0] = m; XR.ld[1] = ma;
-        TRY(s.gram(XR, blist({{b.Pa, mp}}, ma), b.gS));
-        std::vector<double2> s2((size_t)(m + ma) * mp);
-        TRY(s.sync_read(s2.data(), b.gS, s2.size() * sizeof(double2)));
-        for (int i = 0; i < m + ma; ++i)
-          for (int c = 0; c < mp; ++c) hS[(size_t)i * tot + m + ma + c] = s2[(size_t)i * mp + c];
-      }
+      for (int i = 0; i < m + ma; ++i)
+        for (int c = 0; c < mp; ++c) hS[(size_t)i * tot + m + ma + c] = s2[(size_t)i * mp + c];
     }
     int dim = 0;
     bool solved = false;
