@@ -59,14 +59,14 @@ colnorm2_partial(const cplx<T>* __restrict__ A, long long lda, const cplx<T>* __
   }
 }
 
-__global__ void reduce_partials(const double* __restrict__ partial, int nparts, int m,
-                                double* __restrict__ out) {
-  const int j = threadIdx.x;
-  if (j < m) {
-    double s = 0.0;
-    for (int b = 0; b < nparts; ++b) s += partial[(long long)b * m + j];
-    out[j] = s;
-  }
+// a warp per column (a thread per column took 20 us for 296 parts: one load after the other)
+__global__ void __launch_bounds__(32 * kMaxBlock)
+reduce_partials(const double* __restrict__ partial, int nparts, int m, double* __restrict__ out) {
+  const int j = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double s = 0.0;
+  for (int b = lane; b < nparts; b += 32) s += partial[(long long)b * m + j];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) out[j] = s;
 }
 
 template <typename T>
@@ -76,7 +76,7 @@ int launch_colnorm2(const cplx<T>* A, long long lda, const cplx<T>* B, long long
   if (m > kMaxBlock) { set_error("block wider than kMaxBlock"); return QDKP_ERR_ARG; }
   colnorm2_partial<T><<<nparts, kTallThreads, 0, st>>>(A, lda, B, ldb, lambda, m, n, partial);
   count_launch();
-  reduce_partials<<<1, 32, 0, st>>>(partial, nparts, m, out);
+  reduce_partials<<<1, 32 * m, 0, st>>>(partial, nparts, m, out);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;
@@ -246,7 +246,7 @@ update_kernel(const BlockList<T> A, const CoefList C, int q, long long n, cplx<T
               long long ldy, int accumulate) {
   extern __shared__ __align__(16) unsigned char usm[];
   const double2* Cf[3] = {C.c[0], C.c[1], C.c[2]};
-  constexpr int chunk = std::is_same<T, float>::value ? kTfUpdChunk : kUpdChunk;
+  constexpr int chunk = kUpdChunk;
   const long long per = ((n + gridDim.x - 1) / gridDim.x + chunk - 1) / chunk * chunk;
   const long long r0 = (long long)blockIdx.x * per;
   if (r0 >= n) return;

@@ -919,195 +919,337 @@ static __device__ int block_eigh(const double2* __restrict__ A, const double2* _
 
 
 
-// Y' = A' C'' for rows [r0, r1) of complex128 blocks on the FP64 MMA (mma.sync.m8n8k4.f64),
-// with A' (rows x 2P) the real view of [A_0 | A_1 | A_2] and C'' (2P x 2q) the real
-// representation of the stacked complex coefficients: C''_{2i,2j} = Re C_ij,
-// C''_{2i,2j+1} = Im C_ij, C''_{2i+1,2j} = -Im C_ij, C''_{2i+1,2j+1} = Re C_ij (negated when
-// neg). Nothing is staged: a warp owns 8-row M tiles (tiles warp, warp + warps, ... of the CTA's
-// rows) and loads its A fragments from global memory into registers, a ring of k-step pairs
-// ahead of the MMAs. The k order is permuted over pairs of k steps: a pair covers complex
-// columns c0 .. c0 + 3 of one block, MMA k = t of its first step is Re A[.][c0 + t] and of its
-// second step Im A[.][c0 + t] (g = lane / 4, t = lane % 4), so a lane's A values of the pair are
-// one 16-byte load, A[row g][c0 + t]. Those loads stream through a ring of kDmRing pairs in
-// shared memory private to the warp: each lane cp.async-copies exactly the 16 bytes it later
-// reads, so its own cp.async.wait_group orders them and no barrier is needed, and the ring holds
-// twice the bytes in flight that registers could. C'' is stored in the pair's k order as one
-// 16-byte word per (pair, 8-column N tile, lane): {C''[2 (c0 + t)][n g],
-// C''[2 (c0 + t) + 1][n g]}. A row is read (by the four lanes of its quad) before any of its
-// outputs is written and no other warp touches it, so Y may alias an input.
-constexpr int kUpdRows = 8;
+// ---------------------------------------------------------------------------------------------
+// Block updates of complex128 blocks on the FP64 MMA (mma.sync.m8n8k4.f64): Y' = A' C'' with A'
+// (rows x 2P) the real view of [A_0 | A_1 | A_2] and C'' (2P x 2q) the real representation of the
+// stacked complex coefficients: C''_{2i,2j} = Re C_ij, C''_{2i,2j+1} = Im C_ij, C''_{2i+1,2j} =
+// -Im C_ij, C''_{2i+1,2j+1} = Re C_ij. A warp owns MT 8-row M tiles at a time. The k order is permuted
+// over pairs of k steps: a pair covers complex columns c0 .. c0 + 3 of one block, MMA k = t of its
+// first step is Re A[.][c0 + t] and of its second step Im A[.][c0 + t] (g = lane / 4, t = lane % 4),
+// so a lane's A values of the pair are one 16-byte load, A[row g][c0 + t]. Those loads stream
+// through a ring of pairs in shared memory private to the warp: each lane cp.async-copies exactly
+// the 16 bytes it later reads, so its own cp.async.wait_group orders them and no barrier is needed.
+// C'' is stored in the pair's k order as one 16-byte word per (pair, 8-column N tile, lane):
+// {C''[2 (c0 + t)][n g], C''[2 (c0 + t) + 1][n g]}. A row is read (by the four lanes of its quad)
+// before any of its outputs is written and no other warp touches it, so outputs may alias inputs.
+// ---------------------------------------------------------------------------------------------
 constexpr int kUpdThreads = 256;
 constexpr int kUpdWarps = kUpdThreads / 32;
-constexpr int kUpdChunk = kUpdRows * kUpdWarps;     // row granularity of a CTA's span
-constexpr int kDmRing = 16;                         // k-step pairs in flight per warp (2^k)
+constexpr int kUpdChunk = 16 * kUpdWarps;           // row granularity of a CTA's span
+constexpr int kDmRing = 16;                         // 16-byte words in flight per lane
 constexpr size_t kDmRingBytes = (size_t)kUpdWarps * kDmRing * 32 * sizeof(double2);
 
 // k-step pairs of a list of at most three blocks with P columns in all (ceil(cols / 4) each)
 __host__ __device__ __forceinline__ int dmma_pairs_bound(int P) { return (P + 3) / 4 + 2; }
 // the warps' load rings, then the packed coefficients
-__host__ __device__ __forceinline__ size_t update_smem_bytes(int P, int q, int nout = 1) {
-  return kDmRingBytes + (size_t)nout * dmma_pairs_bound(P) * ((q + 3) / 4) * 32 * sizeof(double2);
+__host__ __device__ __forceinline__ size_t update_smem_bytes(int P, int q) {
+  return kDmRingBytes + (size_t)dmma_pairs_bound(P) * ((q + 3) / 4) * 32 * sizeof(double2);
 }
 
-// one k-step pair of an update's A list: columns c0 .. c0 + 3 of a block (p points at c0)
-struct DmKStep {
-  const double2* p;
+// one k-step pair of an update's A list: four columns of a block
+template <typename T>
+struct KStep {
+  const cplx<T>* p;
   int ld;
-  int rem;          // columns of the block from c0 on
+  int n;            // columns that exist (1..4)
+  int col[4];       // their places in a row
 };
 
-template <int NT, int NOUT, bool ACC>
-static __device__ __forceinline__ void update_dmma_core(const DmKStep* __restrict__ sK,
-                                                        const double2* __restrict__ sB,
-                                                        double2* __restrict__ ring, int KS,
-                                                        int q, long long r0, long long r1,
-                                                        double2* Y, double2* Y2, long long ldy) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int nw = blockDim.x >> 5;
-  const int ntiles = (int)((r1 - r0 + kUpdRows - 1) / kUpdRows);
-  const int mine = ntiles > warp ? (ntiles - warp + nw - 1) / nw : 0;
-  const int nitems = mine * KS;
-  if (nitems == 0) return;
-  // this lane's slots of the warp's ring: ring[slot * 32 + lane]; one commit group per item
-  ring += (size_t)warp * kDmRing * 32 + lane;
-  int l_tile = warp, l_s = 0;
-  auto fetch = [&](int slot) {
-    const DmKStep k = sK[l_s];
-    const long long ra = r0 + (long long)l_tile * kUpdRows + g;
-    double2* dst = ring + slot * 32;
-    if (t < k.rem && ra < r1) {
-      const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(sa), "l"(k.p + ra * k.ld + t) : "memory");
-    } else {
-      *dst = make_double2(0.0, 0.0);
+// Appends the k steps of block p (ld, cols columns; gather: column c at gather[c]); one thread.
+template <typename T>
+static __device__ __forceinline__ int add_ksteps(KStep<T>* k, int s, const cplx<T>* p, long long ld,
+                                                 int cols, const int* gather) {
+  for (int c0 = 0; c0 < cols; c0 += 4, ++s) {
+    k[s].p = p; k[s].ld = (int)ld; k[s].n = min(4, cols - c0);
+    for (int t = 0; t < 4; ++t)
+      k[s].col[t] = c0 + t < cols ? (gather ? gather[c0 + t] : c0 + t) : 0;
+  }
+  return s;
+}
+
+// Packs the cols x q row-major complex coefficients C of one block (k steps s0 .. of the list) for
+// the FP64 MMA; every thread of the CTA
+static __device__ __forceinline__ void pack_dmma(double2* __restrict__ sB, int s0, const double2* __restrict__ C,
+                                                 int cols, int q, double sg) {
+  const int NT = (q + 3) / 4, KS = (cols + 3) / 4;
+  for (int e = threadIdx.x; e < KS * NT * 32; e += blockDim.x) {
+    const int s = e / (NT * 32), r = e - s * NT * 32;
+    const int j = r >> 5, ln = r & 31, gg = ln >> 2, tt = ln & 3;
+    const int i = 4 * s + tt, jj = j * 4 + (gg >> 1);
+    double2 w = make_double2(0.0, 0.0);
+    if (i < cols && jj < q) {
+      const double2 c = C[(size_t)i * q + jj];
+      const double re = sg * c.x, im = sg * c.y;
+      w = (gg & 1) ? make_double2(im, re)          // C''[2i][2jj+1], C''[2i+1][2jj+1]
+                   : make_double2(re, -im);        // C''[2i][2jj],   C''[2i+1][2jj]
+    }
+    sB[(size_t)s0 * NT * 32 + e] = w;
+  }
+}
+
+// A warp's stream of A fragments: items are (tile group of MT 8-row tiles, k step), kDmRing / MT in
+// flight. take() gives item `it`'s fragments, done() refills its slot.
+template <int MT>
+struct DmStream {
+  static constexpr int DEPTH = kDmRing / MT;
+  const KStep<double>* k;
+  double2* ring;
+  int KS, nitems, nw, g, t, l_group, l_s;
+  long long r0, r1;
+  __device__ __forceinline__ DmStream(const KStep<double>* k_, double2* ring_, int KS_, long long r0_,
+                                      long long r1_)
+      : k(k_), KS(KS_), r0(r0_), r1(r1_) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    g = lane >> 2; t = lane & 3; nw = blockDim.x >> 5;
+    const int groups = (int)((r1 - r0 + 8 * MT - 1) / (8 * MT));
+    nitems = (groups > warp ? (groups - warp + nw - 1) / nw : 0) * KS;
+    ring = ring_ + (size_t)warp * kDmRing * 32 + lane;
+    l_group = warp; l_s = 0;
+    for (int d = 0; d < DEPTH; ++d) fetch(d, d < nitems);
+  }
+  __device__ __forceinline__ void fetch(int slot, bool any) {
+    if (any) {
+      const KStep<double> ks = k[l_s];
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const long long ra = r0 + (long long)l_group * (8 * MT) + 8 * i + g;
+        double2* dst = ring + (slot * MT + i) * 32;
+        if (t < ks.n && ra < r1) {
+          const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(sa), "l"(ks.p + ra * ks.ld + ks.col[t]) : "memory");
+        } else {
+          *dst = make_double2(0.0, 0.0);
+        }
+      }
+      if (++l_s == KS) { l_s = 0; l_group += nw; }
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-    if (++l_s == KS) { l_s = 0; l_tile += nw; }
-  };
-  for (int d = 0; d < kDmRing; ++d) {
-    if (d < nitems) fetch(d);
-    else asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
-  double acc[NOUT][NT][2];
-  double2 yo[ACC ? NT : 1];
+  __device__ __forceinline__ void take(int it, double2 (&a)[MT]) const {
+    // item it's group is complete once at most DEPTH - 1 younger groups are pending
+    asm volatile("cp.async.wait_group %0;\n" :: "n"(DEPTH - 1) : "memory");
 #pragma unroll
-  for (int o = 0; o < NOUT; ++o)
+    for (int i = 0; i < MT; ++i) a[i] = ring[((it & (DEPTH - 1)) * MT + i) * 32];
+  }
+  // after the MMAs on item it: their reads of its slot are done
+  __device__ __forceinline__ void done(int it) { fetch(it & (DEPTH - 1), it + DEPTH < nitems); }
+};
+
+template <int NT, int MT>
+static __device__ __forceinline__ void dm_step(const double2 (&a)[MT], const double2* __restrict__ bp,
+                                               double (&acc)[MT][NT][2]) {
 #pragma unroll
-    for (int j = 0; j < NT; ++j) acc[o][j][0] = acc[o][j][1] = 0.0;
-  int c_s = 0, c_tile = warp;
-  {
-    for (int it = 0; it < nitems; ++it) {
-      const int slot = it & (kDmRing - 1);
-      // item it's group is complete once at most kDmRing - 1 younger groups are pending
-      asm volatile("cp.async.wait_group %0;\n" :: "n"(kDmRing - 1) : "memory");
-      const double2 a = ring[slot * 32];
-      const long long ra = r0 + (long long)c_tile * kUpdRows + g;
-      if (ACC && c_s == 0) {
+  for (int j = 0; j < NT; ++j) {
+    const double2 b = bp[j * 32];
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+      dmma(acc[i][j][0], acc[i][j][1], a[i].x, b.x);
+      dmma(acc[i][j][0], acc[i][j][1], a[i].y, b.y);
+    }
+  }
+}
+
+template <int NT, bool ACC>
+static __device__ __forceinline__ void update_dmma_core(const KStep<double>* __restrict__ sK,
+                                                        const double2* __restrict__ sB,
+                                                        double2* __restrict__ ring, int KS, int q,
+                                                        long long r0, long long r1, double2* Y,
+                                                        long long ldy) {
+  constexpr int MT = NT <= 3 ? 2 : 1;               // wide outputs hold more accumulators
+  DmStream<MT> st(sK, ring, KS, r0, r1);
+  const int lane = threadIdx.x & 31;
+  double acc[MT][NT][2];
+  int group = threadIdx.x >> 5, c_s = 0;
+  for (int it = 0; it < st.nitems; ++it) {
+    double2 a[MT];
+    if (c_s == 0) {
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const long long ra = r0 + (long long)group * (8 * MT) + 8 * i + st.g;
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
-          const int col = j * 4 + t;
-          yo[j] = (col < q && ra < r1) ? Y[ra * ldy + col] : make_double2(0.0, 0.0);
+          const int col = j * 4 + st.t;
+          double2 y = make_double2(0.0, 0.0);
+          if (ACC && col < q && ra < r1) y = Y[ra * ldy + col];
+          acc[i][j][0] = y.x; acc[i][j][1] = y.y;
         }
       }
-      const double2* bp = sB + (size_t)c_s * NT * 32 + lane;
+    }
+    st.take(it, a);
+    dm_step<NT, MT>(a, sB + (size_t)c_s * NT * 32 + lane, acc);
+    st.done(it);
+    if (++c_s == KS) {
 #pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const double2 b = bp[j * 32];
-        dmma(acc[0][j][0], acc[0][j][1], a.x, b.x);
-        dmma(acc[0][j][0], acc[0][j][1], a.y, b.y);
-        if (NOUT == 2) {
-          const double2 b2 = bp[(size_t)KS * NT * 32 + j * 32];
-          dmma(acc[NOUT - 1][j][0], acc[NOUT - 1][j][1], a.x, b2.x);
-          dmma(acc[NOUT - 1][j][0], acc[NOUT - 1][j][1], a.y, b2.y);
-        }
-      }
-      // refill the slot only now: the MMAs above consumed `a`, so its shared-memory read is done
-      if (it + kDmRing < nitems) fetch(slot);
-      else asm volatile("cp.async.commit_group;\n" ::: "memory");
-      if (++c_s == KS) {
+      for (int i = 0; i < MT; ++i) {
+        const long long ra = r0 + (long long)group * (8 * MT) + 8 * i + st.g;
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
-          const int col = j * 4 + t;
-          if (col < q && ra < r1) {
-            double2 v = make_double2(acc[0][j][0], acc[0][j][1]);
-            if (ACC) { v.x += yo[j].x; v.y += yo[j].y; }
-            Y[ra * ldy + col] = v;
-            if (NOUT == 2) Y2[ra * ldy + col] = make_double2(acc[NOUT - 1][j][0], acc[NOUT - 1][j][1]);
-          }
-#pragma unroll
-          for (int o = 0; o < NOUT; ++o) acc[o][j][0] = acc[o][j][1] = 0.0;
+          const int col = j * 4 + st.t;
+          if (col < q && ra < r1) Y[ra * ldy + col] = make_double2(acc[i][j][0], acc[i][j][1]);
         }
-        c_s = 0;
-        c_tile += nw;
       }
+      c_s = 0;
+      group += st.nw;
     }
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
-// Y (+)= sg A C over rows [r0, r1) and, with C2/Y2, Y2 = sg A C2 (one pass over A; the fused
-// X / P Ritz update reads [X | R | P] once for both). C[b] is the cols_b x q row-major
-// coefficient block of A's block b (NULL: the block does not enter); q <= kMaxBlock. Called by
-// every thread of the CTA; smem holds update_smem_bytes. The two-output form that also
-// accumulates into Y takes two passes over A, so there Y must not alias an input.
+#define QDKP_NT_SWITCH(NT, CALL)                                                                  \
+  switch (NT) {                                                                                  \
+    case 1: { CALL(1) break; } case 2: { CALL(2) break; } case 3: { CALL(3) break; }              \
+    case 4: { CALL(4) break; } case 5: { CALL(5) break; } case 6: { CALL(6) break; }              \
+    default: break;                                                                              \
+  }
+
+// Y (+)= sg A C over rows [r0, r1). C[b] is the cols_b x q row-major coefficient block of A's block
+// b; gather: columns of block 0 (NULL: as they stand); q <= kMaxBlock. Called by every thread of
+// the CTA; smem holds update_smem_bytes.
 static __device__ void update_rows(const BlockList<double>& A, const double2* const* C, int q,
                                    long long r0, long long r1, double2* Y, long long ldy,
                                    int accumulate, int neg, unsigned char* smem,
-                                   const double2* const* C2 = nullptr, double2* Y2 = nullptr) {
-  __shared__ int2 sK[kMaxSmall / 4 + 3];
-  __shared__ DmKStep sKp[kMaxSmall / 4 + 3];
-  __shared__ int sKS;
-  const int nout = Y2 ? 2 : 1;
-  const int NT = (q + 3) / 4;
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int b = 0; b < A.nblk; ++b)
-      for (int c0 = 0; c0 < A.cols[b]; c0 += 4) {
-        sKp[s].p = A.p[b] + c0; sKp[s].ld = (int)A.ld[b]; sKp[s].rem = A.cols[b] - c0;
-        sK[s++] = make_int2(b, c0);
-      }
-    sKS = s;
-  }
-  __syncthreads();
-  const int KS = sKS;
+                                   const int* gather = nullptr) {
+  __shared__ KStep<double> sK[kMaxSmall / 4 + 3];
   double2* ring = reinterpret_cast<double2*>(smem);
   double2* sB = reinterpret_cast<double2*>(smem + kDmRingBytes);
-  const double sg = neg ? -1.0 : 1.0;
-  const int per_out = KS * NT * 32;
-  for (int e = threadIdx.x; e < nout * per_out; e += blockDim.x) {
-    const int o = e / per_out, r = e - o * per_out;
-    const int s = r / (NT * 32), r2 = r - s * NT * 32;
-    const int j = r2 >> 5, ln = r2 & 31;
-    const int gg = ln >> 2, tt = ln & 3;
-    const int2 k = sK[s];
-    const int cols = k.x == 0 ? A.cols[0] : k.x == 1 ? A.cols[1] : A.cols[2];
-    const double2* Cb = (o ? C2 : C)[k.x];
-    const int i = k.y + tt, jj = j * 4 + (gg >> 1);
-    double2 w = make_double2(0.0, 0.0);
-    if (Cb && i < cols && jj < q) {
-      const double2 c = Cb[(size_t)i * q + jj];
-      const double re = sg * c.x, im = sg * c.y;
-      if (gg & 1) w = make_double2(im, re);      // C''[2i][2jj+1], C''[2i+1][2jj+1]
-      else w = make_double2(re, -im);            // C''[2i][2jj],   C''[2i+1][2jj]
-    }
-    sB[e] = w;
+  int KS = 0;
+  for (int b = 0; b < A.nblk; ++b) {
+    if (threadIdx.x == 0) add_ksteps(sK, KS, A.p[b], A.ld[b], A.cols[b], b ? nullptr : gather);
+    pack_dmma(sB, KS, C[b], A.cols[b], q, neg ? -1.0 : 1.0);
+    KS += (A.cols[b] + 3) / 4;
   }
   __syncthreads();
-#define QDKP_DM_CASE(nt)                                                                          \
-  case nt:                                                                                        \
-    if (nout == 2 && accumulate) {                                                                \
-      update_dmma_core<nt, 1, true>(sKp, sB, ring, KS, q, r0, r1, Y, Y2, ldy);                          \
-      update_dmma_core<nt, 1, false>(sKp, sB + per_out, ring, KS, q, r0, r1, Y2, Y2, ldy);              \
-    } else if (nout == 2) update_dmma_core<nt, 2, false>(sKp, sB, ring, KS, q, r0, r1, Y, Y2, ldy);     \
-    else if (accumulate) update_dmma_core<nt, 1, true>(sKp, sB, ring, KS, q, r0, r1, Y, Y2, ldy);       \
-    else update_dmma_core<nt, 1, false>(sKp, sB, ring, KS, q, r0, r1, Y, Y2, ldy);                      \
-    break;
-  switch (NT) {
-    QDKP_DM_CASE(1) QDKP_DM_CASE(2) QDKP_DM_CASE(3) QDKP_DM_CASE(4) QDKP_DM_CASE(5) QDKP_DM_CASE(6)
-    default: break;
+#define QDKP_UPD(nt)                                                                              \
+  if (accumulate) update_dmma_core<nt, true>(sK, sB, ring, KS, q, r0, r1, Y, ldy);                \
+  else update_dmma_core<nt, false>(sK, sB, ring, KS, q, r0, r1, Y, ldy);
+  QDKP_NT_SWITCH((q + 3) / 4, QDKP_UPD)
+#undef QDKP_UPD
+}
+
+// ---------------------------------------------------------------------------------------------
+// The Ritz update of an iteration in one pass over [X | R | P] and [AX | AR | AP] (lobpcg.py:
+// 921-973): P = R Cr + P Cp, X = X Cx + P, the same for AP and AX, all in place, and with them the
+// residuals A X - X lambda of the new iterate: their squared norms per column, and, if Rout is not
+// NULL, the block itself. Six blocks are read and four (five) written, where two two-output updates,
+// the norm and the residual kernels read ten and write five. P's sum is carried on into X's, so
+// the six products are six block multiplications, not ten. Memory bounds it: 1.13 M rows of 12
+// columns, complex128 (seven slots), 408 us at 5.9 TB/s; the four kernels took 960 us. The FP64 MMAs
+// need 220 us of that; two M tiles a warp share the coefficient fragments while the accumulators and
+// the kept X rows fit the registers (12 columns).
+// ---------------------------------------------------------------------------------------------
+template <typename T>
+struct RitzArgs {
+  cplx<T> *X, *R, *P, *AX, *AR, *AP;   // X, P, AX, AP: n x m (outputs); R, AR: n x ma; P, AP in: Pin, APin
+  const cplx<T> *Pin, *APin;           // n x mp
+  cplx<T>* Rout;                       // n x m, may be R when ma == m
+  const double2 *Cx, *Cr, *Cp;
+  const double* lam;
+  double* npart;                       // m sums of this CTA
+  int m, ma, mp;
+};
+
+constexpr int kRitzMaxKs = 2 * (kMaxSmall / 4 + 3);
+
+// sum over the CTA's rows of nacc (lane: columns 4 j + t) into npart
+template <int NT>
+static __device__ __forceinline__ void ritz_norms(double (&nacc)[NT], int m, double* __restrict__ npart) {
+  __shared__ double red[kUpdWarps][4 * NT];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int j = 0; j < NT; ++j) {
+    double v = nacc[j];
+    for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane < 4) red[warp][4 * j + lane] = v;
   }
-#undef QDKP_DM_CASE
+  __syncthreads();
+  if ((int)threadIdx.x < m) {
+    double v = 0.0;
+    for (int w = 0; w < kUpdWarps; ++w) v += red[w][threadIdx.x];
+    npart[threadIdx.x] = v;
+  }
+}
+
+template <int NT>
+static __device__ __forceinline__ void ritz_dmma_core(const RitzArgs<double>& t, const KStep<double>* __restrict__ sK,
+                                                      const double2* __restrict__ sB, double2* __restrict__ ring,
+                                                      int KP, int KX, long long r0, long long r1) {
+  constexpr int MT = NT <= 3 ? 2 : 1;
+  const int KH = KP + KX;                           // k steps of one side
+  DmStream<MT> st(sK, ring, 2 * KH, r0, r1);
+  const int lane = threadIdx.x & 31, m = t.m;
+  double lam[NT], nacc[NT];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) {
+    nacc[j] = 0.0;
+    lam[j] = j * 4 + st.t < m ? t.lam[j * 4 + st.t] : 0.0;
+  }
+  double acc[MT][NT][2], xs[MT][NT][2];
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  int group = threadIdx.x >> 5, c_s = 0, k = 0;     // k step of the item, and within its side
+  for (int it = 0; it < st.nitems; ++it) {
+    double2 a[MT];
+    st.take(it, a);
+    dm_step<NT, MT>(a, sB + (size_t)k * NT * 32 + lane, acc);
+    st.done(it);
+    ++c_s;
+    ++k;
+    if (k == KP || k == KH) {
+      const bool ax = c_s > KH;
+      double2* out = k == KP ? (ax ? t.AP : t.P) : (ax ? t.AX : t.X);
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const long long ra = r0 + (long long)group * (8 * MT) + 8 * i + st.g;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          const int col = j * 4 + st.t;
+          const double2 v = make_double2(acc[i][j][0], acc[i][j][1]);
+          if (col < m && ra < r1) {
+            out[ra * m + col] = v;
+            if (c_s == 2 * KH) {
+              const double re = v.x - lam[j] * xs[i][j][0], im = v.y - lam[j] * xs[i][j][1];
+              nacc[j] = fma(re, re, fma(im, im, nacc[j]));
+              if (t.Rout) t.Rout[ra * m + col] = make_double2(re, im);
+            }
+          }
+          if (k == KH) {
+            xs[i][j][0] = v.x; xs[i][j][1] = v.y;
+            acc[i][j][0] = acc[i][j][1] = 0.0;
+          }
+        }
+      }
+      if (k == KH) k = 0;
+      if (c_s == 2 * KH) { c_s = 0; group += st.nw; }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  ritz_norms<NT>(nacc, m, t.npart);
+}
+
+__host__ __device__ __forceinline__ size_t ritz_smem_bytes(int m) { return update_smem_bytes(3 * m, m); }
+
+static __device__ void ritz_rows(const RitzArgs<double>& t, long long r0, long long r1, unsigned char* smem) {
+  __shared__ KStep<double> sK[kRitzMaxKs];
+  double2* ring = reinterpret_cast<double2*>(smem);
+  double2* sB = reinterpret_cast<double2*>(smem + kDmRingBytes);
+  const int kr = (t.ma + 3) / 4, kp = (t.mp + 3) / 4, KX = (t.m + 3) / 4, KP = kr + kp;
+  if (threadIdx.x == 0) {
+    int s = add_ksteps<double>(sK, 0, t.R, t.ma, t.ma, nullptr);
+    s = add_ksteps<double>(sK, s, t.Pin, t.mp, t.mp, nullptr);
+    s = add_ksteps<double>(sK, s, t.X, t.m, t.m, nullptr);
+    s = add_ksteps<double>(sK, s, t.AR, t.ma, t.ma, nullptr);
+    s = add_ksteps<double>(sK, s, t.APin, t.mp, t.mp, nullptr);
+    add_ksteps<double>(sK, s, t.AX, t.m, t.m, nullptr);
+  }
+  pack_dmma(sB, 0, t.Cr, t.ma, t.m, 1.0);
+  pack_dmma(sB, kr, t.Cp, t.mp, t.m, 1.0);
+  pack_dmma(sB, KP, t.Cx, t.m, t.m, 1.0);
+  __syncthreads();
+#define QDKP_RITZ(nt) ritz_dmma_core<nt>(t, sK, sB, ring, KP, KX, r0, r1);
+  QDKP_NT_SWITCH(KX, QDKP_RITZ)
+#undef QDKP_RITZ
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1155,162 +1297,26 @@ __device__ __forceinline__ void mma_tf32x3(float (&d)[4], const unsigned (&ah)[4
 // k order as one 16-byte word per (k step, 8-column N tile, lane): {hi b0, hi b1, lo b0, lo b1}
 // with b0 = C''[k t][n g], b1 = C''[k t + 4][n g]. A row is read (by the four lanes of its quad)
 // before any of its outputs is written and no other warp touches it, so Y may alias an input.
-constexpr int kTfUpdChunk = 128;   // row granularity of a CTA's span (a multiple of the M tile)
 constexpr int kTfRing = 8;         // k steps of A fragments in flight per warp (narrow outputs)
-constexpr int kTfMaxKs = kMaxSmall / 4 + 3;
 
 // k steps of a list of at most three blocks with P columns in all (ceil(cols / 4) per block)
 __host__ __device__ __forceinline__ int tf32_ksteps_bound(int P) { return (P + 3) / 4 + 2; }
 
-__host__ __device__ __forceinline__ size_t update_tf32_smem_bytes(int P, int q, int nout = 1) {
-  return (size_t)nout * tf32_ksteps_bound(P) * ((q + 3) / 4) * 32 * sizeof(uint4);
+__host__ __device__ __forceinline__ size_t update_tf32_smem_bytes(int P, int q) {
+  return (size_t)tf32_ksteps_bound(P) * ((q + 3) / 4) * 32 * sizeof(uint4);
 }
 
-// one k step of an update's A list: columns c0 .. c0 + 3 of a block (p points at column c0)
-struct TfKStep {
-  const float2* p;
-  int ld;
-  int rem;          // columns of the block from c0 on
-};
-
-template <int NT, int NOUT, bool ACC>
-static __device__ __forceinline__ void update_tf32_core(const TfKStep* __restrict__ sK,
-                                                        const uint4* __restrict__ sB, int KS,
-                                                        int q, long long r0, long long r1,
-                                                        float2* Y, float2* Y2, long long ldy) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int nw = blockDim.x >> 5;
-  const int ntiles = (int)((r1 - r0 + 15) / 16);
-  const int mine = ntiles > warp ? (ntiles - warp + nw - 1) / nw : 0;
-  const int nitems = mine * KS;
-  if (nitems == 0) return;
-  // wide outputs hold more accumulators: a shorter ring keeps the warp within 128 registers
-  constexpr int RING = NT * NOUT <= 6 ? kTfRing : kTfRing / 2;
-  float2 fa[RING], fb[RING];
-  int l_tile = warp, l_s = 0;
-  auto fetch = [&](float2& xa, float2& xb) {
-    const TfKStep k = sK[l_s];
-    const long long ra = r0 + (long long)l_tile * 16 + g, rb = ra + 8;
-    xa = (t < k.rem && ra < r1) ? __ldcs(k.p + ra * k.ld + t) : make_float2(0.f, 0.f);
-    xb = (t < k.rem && rb < r1) ? __ldcs(k.p + rb * k.ld + t) : make_float2(0.f, 0.f);
-    if (++l_s == KS) { l_s = 0; l_tile += nw; }
-  };
-#pragma unroll
-  for (int d = 0; d < RING; ++d)
-    if (d < nitems) fetch(fa[d], fb[d]);
-  float acc[NOUT][NT][4];
-  float2 yo[ACC ? NT : 1][2];
-#pragma unroll
-  for (int o = 0; o < NOUT; ++o)
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[o][j][e] = 0.f;
-  int c_s = 0, c_tile = warp;
-  for (int base = 0; base < nitems; base += RING) {
-#pragma unroll
-    for (int d = 0; d < RING; ++d) {
-      const int it = base + d;
-      if (it >= nitems) break;
-      unsigned ah[4], al[4];
-      tf32_split(fa[d].x, ah[0], al[0]);
-      tf32_split(fb[d].x, ah[1], al[1]);
-      tf32_split(fa[d].y, ah[2], al[2]);
-      tf32_split(fb[d].y, ah[3], al[3]);
-      if (it + RING < nitems) fetch(fa[d], fb[d]);
-      const long long ra = r0 + (long long)c_tile * 16 + g, rb = ra + 8;
-      if (ACC && c_s == 0) {
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          const int col = j * 4 + t;
-          yo[j][0] = (col < q && ra < r1) ? Y[ra * ldy + col] : make_float2(0.f, 0.f);
-          yo[j][1] = (col < q && rb < r1) ? Y[rb * ldy + col] : make_float2(0.f, 0.f);
-        }
-      }
-      const uint4* bp = sB + (size_t)c_s * NT * 32 + lane;
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const uint4 b = bp[j * 32];
-        const unsigned bh[2] = {b.x, b.y}, bl[2] = {b.z, b.w};
-        mma_tf32x3(acc[0][j], ah, al, bh, bl);
-        if (NOUT == 2) {
-          const uint4 b2 = bp[(size_t)KS * NT * 32 + j * 32];
-          const unsigned bh2[2] = {b2.x, b2.y}, bl2[2] = {b2.z, b2.w};
-          mma_tf32x3(acc[NOUT - 1][j], ah, al, bh2, bl2);
-        }
-      }
-      if (++c_s == KS) {
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          const int col = j * 4 + t;
-          if (col < q) {
-            float2 va = make_float2(acc[0][j][0], acc[0][j][1]);
-            float2 vb = make_float2(acc[0][j][2], acc[0][j][3]);
-            if (ACC) {
-              va.x += yo[j][0].x; va.y += yo[j][0].y;
-              vb.x += yo[j][1].x; vb.y += yo[j][1].y;
-            }
-            if (ra < r1) Y[ra * ldy + col] = va;
-            if (rb < r1) Y[rb * ldy + col] = vb;
-            if (NOUT == 2) {
-              if (ra < r1) Y2[ra * ldy + col] = make_float2(acc[NOUT - 1][j][0], acc[NOUT - 1][j][1]);
-              if (rb < r1) Y2[rb * ldy + col] = make_float2(acc[NOUT - 1][j][2], acc[NOUT - 1][j][3]);
-            }
-          }
-#pragma unroll
-          for (int o = 0; o < NOUT; ++o)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[o][j][e] = 0.f;
-        }
-        c_s = 0;
-        c_tile += nw;
-      }
-    }
-  }
-}
-
-// Y (+)= sg A C over rows [r0, r1) and, with C2/Y2, Y2 = sg A C2 (one pass over A). C[b] is the
-// cols_b x q row-major coefficient block of A's block b (NULL: the block does not enter);
-// q <= kMaxBlock. Called by every thread of the CTA; smem holds update_tf32_smem_bytes. The
-// two-output form that also accumulates into Y takes two passes over A, so there Y must not
-// alias an input.
-static __device__ void update_rows_tf32(const BlockList<float>& A, const double2* const* C, int q,
-                                        long long r0, long long r1, float2* Y, long long ldy,
-                                        int accumulate, int neg, unsigned char* smem,
-                                        const double2* const* C2 = nullptr,
-                                        float2* Y2 = nullptr) {
-  __shared__ int2 sK[kTfMaxKs];
-  __shared__ TfKStep sKp[kTfMaxKs];
-  __shared__ int sKS;
-  const int nout = Y2 ? 2 : 1;
-  const int NT = (q + 3) / 4;
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int b = 0; b < A.nblk; ++b)
-      for (int c0 = 0; c0 < A.cols[b]; c0 += 4) {
-        sKp[s].p = A.p[b] + c0; sKp[s].ld = (int)A.ld[b]; sKp[s].rem = A.cols[b] - c0;
-        sK[s++] = make_int2(b, c0);
-      }
-    sKS = s;
-  }
-  __syncthreads();
-  const int KS = sKS;
-  uint4* sB = reinterpret_cast<uint4*>(smem);
-  const float sg = neg ? -1.f : 1.f;
-  const int per_out = KS * NT * 32;
-  for (int e = threadIdx.x; e < nout * per_out; e += blockDim.x) {
-    const int o = e / per_out, r = e - o * per_out;
-    const int s = r / (NT * 32), r2 = r - s * NT * 32;
-    const int j = r2 >> 5, ln = r2 & 31;
-    const int gg = ln >> 2, tt = ln & 3;
-    const int2 k = sK[s];
-    const int cols = k.x == 0 ? A.cols[0] : k.x == 1 ? A.cols[1] : A.cols[2];
-    const double2* Cb = (o ? C2 : C)[k.x];
-    const int i = k.y + tt, jj = j * 4 + (gg >> 1);
+// Packs one block's coefficients for the TF32 MMA (k steps s0 .. of the list); every thread
+static __device__ __forceinline__ void pack_tf32(uint4* __restrict__ sB, int s0, const double2* __restrict__ C,
+                                                 int cols, int q, float sg) {
+  const int NT = (q + 3) / 4, KS = (cols + 3) / 4;
+  for (int e = threadIdx.x; e < KS * NT * 32; e += blockDim.x) {
+    const int s = e / (NT * 32), r = e - s * NT * 32;
+    const int j = r >> 5, ln = r & 31, gg = ln >> 2, tt = ln & 3;
+    const int i = 4 * s + tt, jj = j * 4 + (gg >> 1);
     float v0 = 0.f, v1 = 0.f;
-    if (Cb && i < cols && jj < q) {
-      const double2 c = Cb[(size_t)i * q + jj];
+    if (i < cols && jj < q) {
+      const double2 c = C[(size_t)i * q + jj];
       const float re = sg * (float)c.x, im = sg * (float)c.y;
       if (gg & 1) { v0 = im; v1 = re; }          // C''[2i][2jj+1], C''[2i+1][2jj+1]
       else { v0 = re; v1 = -im; }                // C''[2i][2jj],   C''[2i+1][2jj]
@@ -1318,23 +1324,216 @@ static __device__ void update_rows_tf32(const BlockList<float>& A, const double2
     uint4 w;
     tf32_split(v0, w.x, w.z);
     tf32_split(v1, w.y, w.w);
-    sB[e] = w;
+    sB[(size_t)s0 * NT * 32 + e] = w;
+  }
+}
+
+// A warp's stream of A fragments over (16-row tile, k step) items, RING in flight in registers
+template <int RING>
+struct TfStream {
+  const KStep<float>* k;
+  int KS, nitems, nw, g, t, l_tile, l_s;
+  long long r0, r1;
+  float2 fa[RING], fb[RING];
+  __device__ __forceinline__ TfStream(const KStep<float>* k_, int KS_, long long r0_, long long r1_)
+      : k(k_), KS(KS_), r0(r0_), r1(r1_) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    g = lane >> 2; t = lane & 3; nw = blockDim.x >> 5;
+    const int ntiles = (int)((r1 - r0 + 15) / 16);
+    nitems = (ntiles > warp ? (ntiles - warp + nw - 1) / nw : 0) * KS;
+    l_tile = warp; l_s = 0;
+#pragma unroll
+    for (int d = 0; d < RING; ++d)
+      if (d < nitems) fetch(d);
+  }
+  __device__ __forceinline__ void fetch(int d) {
+    const KStep<float> ks = k[l_s];
+    const long long ra = r0 + (long long)l_tile * 16 + g, rb = ra + 8;
+    fa[d] = (t < ks.n && ra < r1) ? __ldcs(ks.p + ra * ks.ld + ks.col[t]) : make_float2(0.f, 0.f);
+    fb[d] = (t < ks.n && rb < r1) ? __ldcs(ks.p + rb * ks.ld + ks.col[t]) : make_float2(0.f, 0.f);
+    if (++l_s == KS) { l_s = 0; l_tile += nw; }
+  }
+  // item `it` in slot d: its split fragments; the slot is refilled
+  __device__ __forceinline__ void take(int it, int d, unsigned (&ah)[4], unsigned (&al)[4]) {
+    tf32_split(fa[d].x, ah[0], al[0]);
+    tf32_split(fb[d].x, ah[1], al[1]);
+    tf32_split(fa[d].y, ah[2], al[2]);
+    tf32_split(fb[d].y, ah[3], al[3]);
+    if (it + RING < nitems) fetch(d);
+  }
+};
+
+template <int NT>
+static __device__ __forceinline__ void tf_step(const unsigned (&ah)[4], const unsigned (&al)[4],
+                                               const uint4* __restrict__ bp, float (&acc)[NT][4]) {
+#pragma unroll
+  for (int j = 0; j < NT; ++j) {
+    const uint4 b = bp[j * 32];
+    const unsigned bh[2] = {b.x, b.y}, bl[2] = {b.z, b.w};
+    mma_tf32x3(acc[j], ah, al, bh, bl);
+  }
+}
+
+template <int NT, bool ACC>
+static __device__ __forceinline__ void update_tf32_core(const KStep<float>* __restrict__ sK,
+                                                        const uint4* __restrict__ sB, int KS,
+                                                        int q, long long r0, long long r1,
+                                                        float2* Y, long long ldy) {
+  constexpr int RING = kTfRing;
+  TfStream<RING> st(sK, KS, r0, r1);
+  const int lane = threadIdx.x & 31;
+  float acc[NT][4];
+  float2 yo[ACC ? NT : 1][2];
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+  int c_s = 0, tile = threadIdx.x >> 5;
+  for (int base = 0; base < st.nitems; base += RING) {
+#pragma unroll
+    for (int d = 0; d < RING; ++d) {
+      const int it = base + d;
+      if (it >= st.nitems) break;
+      unsigned ah[4], al[4];
+      st.take(it, d, ah, al);
+      const long long ra = r0 + (long long)tile * 16 + st.g, rb = ra + 8;
+      if (ACC && c_s == 0) {
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          const int col = j * 4 + st.t;
+          yo[j][0] = (col < q && ra < r1) ? Y[ra * ldy + col] : make_float2(0.f, 0.f);
+          yo[j][1] = (col < q && rb < r1) ? Y[rb * ldy + col] : make_float2(0.f, 0.f);
+        }
+      }
+      tf_step<NT>(ah, al, sB + (size_t)c_s * NT * 32 + lane, acc);
+      if (++c_s == KS) {
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          const int col = j * 4 + st.t;
+          if (col < q) {
+            float2 va = make_float2(acc[j][0], acc[j][1]), vb = make_float2(acc[j][2], acc[j][3]);
+            if (ACC) {
+              va.x += yo[j][0].x; va.y += yo[j][0].y;
+              vb.x += yo[j][1].x; vb.y += yo[j][1].y;
+            }
+            if (ra < r1) Y[ra * ldy + col] = va;
+            if (rb < r1) Y[rb * ldy + col] = vb;
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+        }
+        c_s = 0;
+        tile += st.nw;
+      }
+    }
+  }
+}
+
+// Y (+)= sg A C over rows [r0, r1) of complex64 blocks; arguments as update_rows. smem holds
+// update_tf32_smem_bytes.
+static __device__ void update_rows_tf32(const BlockList<float>& A, const double2* const* C, int q,
+                                        long long r0, long long r1, float2* Y, long long ldy,
+                                        int accumulate, int neg, unsigned char* smem,
+                                        const int* gather = nullptr) {
+  __shared__ KStep<float> sK[kMaxSmall / 4 + 3];
+  uint4* sB = reinterpret_cast<uint4*>(smem);
+  int KS = 0;
+  for (int b = 0; b < A.nblk; ++b) {
+    if (threadIdx.x == 0) add_ksteps(sK, KS, A.p[b], A.ld[b], A.cols[b], b ? nullptr : gather);
+    pack_tf32(sB, KS, C[b], A.cols[b], q, neg ? -1.f : 1.f);
+    KS += (A.cols[b] + 3) / 4;
   }
   __syncthreads();
-#define QDKP_TF_CASE(nt)                                                                          \
-  case nt:                                                                                        \
-    if (nout == 2 && accumulate) {                                                                \
-      update_tf32_core<nt, 1, true>(sKp, sB, KS, q, r0, r1, Y, Y2, ldy);                          \
-      update_tf32_core<nt, 1, false>(sKp, sB + per_out, KS, q, r0, r1, Y2, Y2, ldy);              \
-    } else if (nout == 2) update_tf32_core<nt, 2, false>(sKp, sB, KS, q, r0, r1, Y, Y2, ldy);     \
-    else if (accumulate) update_tf32_core<nt, 1, true>(sKp, sB, KS, q, r0, r1, Y, Y2, ldy);       \
-    else update_tf32_core<nt, 1, false>(sKp, sB, KS, q, r0, r1, Y, Y2, ldy);                      \
-    break;
-  switch (NT) {
-    QDKP_TF_CASE(1) QDKP_TF_CASE(2) QDKP_TF_CASE(3) QDKP_TF_CASE(4) QDKP_TF_CASE(5) QDKP_TF_CASE(6)
-    default: break;
+#define QDKP_UPD(nt)                                                                              \
+  if (accumulate) update_tf32_core<nt, true>(sK, sB, KS, q, r0, r1, Y, ldy);                      \
+  else update_tf32_core<nt, false>(sK, sB, KS, q, r0, r1, Y, ldy);
+  QDKP_NT_SWITCH((q + 3) / 4, QDKP_UPD)
+#undef QDKP_UPD
+}
+
+// the Ritz update (ritz_rows) of complex64 blocks; the residual in FP64 from the rounded X and A X
+template <int NT>
+static __device__ __forceinline__ void ritz_tf32_core(const RitzArgs<float>& t, const KStep<float>* __restrict__ sK,
+                                                      const uint4* __restrict__ sB, int KP, int KX,
+                                                      long long r0, long long r1) {
+  constexpr int RING = NT <= 3 ? kTfRing : kTfRing / 2;
+  const int KH = KP + KX;
+  TfStream<RING> st(sK, 2 * KH, r0, r1);
+  const int lane = threadIdx.x & 31, m = t.m;
+  double nacc[NT];
+  float acc[NT][4], xs[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) {
+    nacc[j] = 0.0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
   }
-#undef QDKP_TF_CASE
+  int c_s = 0, k = 0, tile = threadIdx.x >> 5;
+  for (int base = 0; base < st.nitems; base += RING) {
+#pragma unroll
+    for (int d = 0; d < RING; ++d) {
+      const int it = base + d;
+      if (it >= st.nitems) break;
+      unsigned ah[4], al[4];
+      st.take(it, d, ah, al);
+      tf_step<NT>(ah, al, sB + (size_t)k * NT * 32 + lane, acc);
+      ++c_s;
+      ++k;
+      if (k == KP || k == KH) {
+        const bool ax = c_s > KH;
+        float2* out = k == KP ? (ax ? t.AP : t.P) : (ax ? t.AX : t.X);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const long long ra = r0 + (long long)tile * 16 + st.g + 8 * h;
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            const int col = j * 4 + st.t;
+            const float2 v = make_float2(acc[j][2 * h], acc[j][2 * h + 1]);
+            if (col < m && ra < r1) {
+              out[ra * m + col] = v;
+              if (c_s == 2 * KH) {
+                const double l = t.lam[col];
+                const double re = (double)v.x - l * (double)xs[j][2 * h];
+                const double im = (double)v.y - l * (double)xs[j][2 * h + 1];
+                nacc[j] = fma(re, re, fma(im, im, nacc[j]));
+                if (t.Rout) t.Rout[ra * m + col] = make_float2((float)re, (float)im);
+              }
+            }
+            if (k == KH) {
+              xs[j][2 * h] = v.x; xs[j][2 * h + 1] = v.y;
+              acc[j][2 * h] = acc[j][2 * h + 1] = 0.f;
+            }
+          }
+        }
+        if (k == KH) k = 0;
+        if (c_s == 2 * KH) { c_s = 0; tile += st.nw; }
+      }
+    }
+  }
+  ritz_norms<NT>(nacc, m, t.npart);
+}
+
+__host__ __device__ __forceinline__ size_t ritz_tf32_smem_bytes(int m) { return update_tf32_smem_bytes(3 * m, m); }
+
+static __device__ void ritz_rows_tf32(const RitzArgs<float>& t, long long r0, long long r1, unsigned char* smem) {
+  __shared__ KStep<float> sK[kRitzMaxKs];
+  uint4* sB = reinterpret_cast<uint4*>(smem);
+  const int kr = (t.ma + 3) / 4, kp = (t.mp + 3) / 4, KX = (t.m + 3) / 4, KP = kr + kp;
+  if (threadIdx.x == 0) {
+    int s = add_ksteps<float>(sK, 0, t.R, t.ma, t.ma, nullptr);
+    s = add_ksteps<float>(sK, s, t.Pin, t.mp, t.mp, nullptr);
+    s = add_ksteps<float>(sK, s, t.X, t.m, t.m, nullptr);
+    s = add_ksteps<float>(sK, s, t.AR, t.ma, t.ma, nullptr);
+    s = add_ksteps<float>(sK, s, t.APin, t.mp, t.mp, nullptr);
+    add_ksteps<float>(sK, s, t.AX, t.m, t.m, nullptr);
+  }
+  pack_tf32(sB, 0, t.Cr, t.ma, t.m, 1.f);
+  pack_tf32(sB, kr, t.Cp, t.mp, t.m, 1.f);
+  pack_tf32(sB, KP, t.Cx, t.m, t.m, 1.f);
+  __syncthreads();
+#define QDKP_RITZ(nt) ritz_tf32_core<nt>(t, sK, sB, KP, KX, r0, r1);
+  QDKP_NT_SWITCH(KX, QDKP_RITZ)
+#undef QDKP_RITZ
 }
 
 }  // namespace qdkp

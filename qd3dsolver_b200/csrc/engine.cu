@@ -20,26 +20,29 @@ int launch_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, i
                  int m, double sigma, int shifted, int precision, cudaStream_t st);
 
 constexpr int kERowsPerCta = 512;    // rows per CTA of the row kernels
-constexpr int kENormRows = 2048;     // rows per CTA of the norm kernel
 
 // GR_RZ: the products of the Rayleigh-Ritz pencil, in one pass (GK_PENCIL or GK_EXPLICIT)
 enum GramWhich { GR_XR = 0, GR_RR, GR_PP, GR_RZ };
-// UP_XPNEW: P = R Cr + P Cp and X = X Cx + R Cr + P Cp from one pass over [X | R | P]
-// (lobpcg.py:921-973); UP_AXPNEW: the same for AP and AX.
+// UP_XPNEW, UP_AXPNEW: the Ritz update of complex64 slots on the tcgen05 tensor cores, P and X (AP and
+// AX) from one pass over [X | R | P] ([AX | AR | AP]); otherwise e_ritz_kernel forms all four.
 enum UpdWhich { UP_RPROJ = 0, UP_RNORM, UP_PNORM, UP_APNORM, UP_XPNEW, UP_AXPNEW };
 enum RowWhich { RW_COPYBEST = 0, RW_RESID, RW_GATHERP };
 
 // ---------------------------------------------------------------------------------------------
-// residual norms of A X - X lambda: partials per CTA, reduced in the decision kernel
+// residual norms of A X - X lambda: partials per CTA, reduced in the decision kernel. Only where the
+// Ritz update does not leave them (complex64 slots updated by the tcgen05 kernels).
 // ---------------------------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ void e_norm_body(const ESlot& d, int part) {
+__global__ void __launch_bounds__(kTallThreads)
+e_norm_kernel(const ESlot* __restrict__ S, int ns) {
+  const ESlot& d = S[slot_of(S, ns, blockIdx.x, &ESlot::row0)];
   const EState* st = d.st;
-  const cplx<T>* AX = blk<T>(d.AX);
-  const cplx<T>* X = blk<T>(d.X);
+  if (d.prec != QDKP_C64 || !st->running) return;
+  const int part = blockIdx.x - d.row0;
+  const float2* AX = blk<float>(d.AX);
+  const float2* X = blk<float>(d.X);
   const int m = d.m;
-  const long long r0 = (long long)part * kENormRows;
-  const long long r1 = min(d.n, r0 + kENormRows);
+  const long long r0 = (long long)part * d.rows_per_cta;
+  const long long r1 = min(d.n, r0 + d.rows_per_cta);
   double acc[kMaxBlock];
 #pragma unroll
   for (int j = 0; j < kMaxBlock; ++j) acc[j] = 0.0;
@@ -47,7 +50,7 @@ __device__ __forceinline__ void e_norm_body(const ESlot& d, int part) {
 #pragma unroll
     for (int j = 0; j < kMaxBlock; ++j) {
       if (j < m) {
-        const cplx<T> a = AX[r * m + j], x = X[r * m + j];
+        const float2 a = AX[r * m + j], x = X[r * m + j];
         const double l = st->lam[j];
         const double re = (double)a.x - l * (double)x.x, im = (double)a.y - l * (double)x.y;
         acc[j] = fma(re, re, fma(im, im, acc[j]));
@@ -72,27 +75,24 @@ __device__ __forceinline__ void e_norm_body(const ESlot& d, int part) {
   }
 }
 
-__global__ void __launch_bounds__(kTallThreads)
-e_norm_kernel(const ESlot* __restrict__ S, int ns) {
-  const int k = slot_of(S, ns, blockIdx.x, &ESlot::norm0);
-  const ESlot& d = S[k];
-  if (!d.st->running) return;
-  if (d.prec == QDKP_C64) e_norm_body<float>(d, blockIdx.x - d.norm0);
-  else e_norm_body<double>(d, blockIdx.x - d.norm0);
-}
-
 // ---------------------------------------------------------------------------------------------
 // per-slot decisions at the top of an iteration (lobpcg.py:688-760)
 // ---------------------------------------------------------------------------------------------
-__global__ void e_decide_kernel(const ESlot* __restrict__ S) {
+constexpr int kDecideThreads = 768;    // 32 per column of the widest block
+
+__global__ void __launch_bounds__(kDecideThreads) e_decide_kernel(const ESlot* __restrict__ S) {
   const ESlot& d = S[blockIdx.x];
   EState* st = d.st;
   __shared__ double nrm[kMaxBlock];
   const int m = d.m;
-  if (threadIdx.x < m) {
+  // a warp per column, parts strided over its lanes: 28 us with a thread per column, 5 us now
+  // (7 slots of 860 parts)
+  const int c = threadIdx.x >> 5;
+  if (c < m) {
     double s = 0.0;
-    for (int b = 0; b < d.nparts; ++b) s += d.npart[(long long)b * m + threadIdx.x];
-    nrm[threadIdx.x] = sqrt(fabs(s));
+    for (int b = threadIdx.x & 31; b < d.nparts; b += 32) s += d.npart[(long long)b * m + c];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) nrm[c] = sqrt(fabs(s));
   }
   __syncthreads();
   if (threadIdx.x != 0) return;
@@ -128,6 +128,8 @@ __global__ void e_decide_kernel(const ESlot* __restrict__ S) {
     if (st->active[j]) st->idx[ma++] = j;
   }
   st->ma = ma;
+  st->skip_resid = st->resid_ready && ma == m;
+  st->resid_ready = 0;
   if (ma == 0) { st->running = 0; st->status = QDKP_LOBPCG_CONVERGED; return; }
   st->explicit_gram = !(mx > d.sqrt_eps && !st->explicit_gram);
   st->idle = 0;
@@ -135,7 +137,7 @@ __global__ void e_decide_kernel(const ESlot* __restrict__ S) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// row kernels: copy of the best iterate, residual gather, P gather
+// row kernels: copy of the best iterate, residual gather, P gather (tcgen05 updates only)
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ void e_row_body(const ESlot& d, int which, long long r0,
@@ -179,7 +181,8 @@ e_row_kernel(const ESlot* __restrict__ S, int ns, int which) {
   const ESlot& d = S[k];
   const EState* st = d.st;
   if (which == RW_COPYBEST) { if (!st->copy_best) return; }
-  else if (st->idle || (which == RW_GATHERP && st->skip_p)) return;
+  else if (st->idle || (which == RW_RESID && st->skip_resid)) return;
+  else if (which == RW_GATHERP && (st->skip_p || d.prec != QDKP_C64)) return;
   const long long r0 = (long long)(blockIdx.x - d.row0) * d.rows_per_cta;
   const long long r1 = min(d.n, r0 + d.rows_per_cta);
   if (d.prec == QDKP_C64) e_row_body<float>(d, which, r0, r1);
@@ -210,9 +213,13 @@ __device__ bool gram_task(const ESlot& d, int which, GramTask<T>& t, double2*& o
       add(d.X, m, m); add(d.Ra, ma, ma);
       t.P = m; t.b0 = m; t.Q = ma; t.kind = GK_FULL; out = d.W;
       return true;
-    case GR_RR: case GR_PP:
-      add(which == GR_RR ? d.Ra : d.Pa, ma, ma);
+    case GR_RR:
+      add(d.Ra, ma, ma);
       t.P = t.Q = ma; t.kind = GK_HERM; out = d.G;
+      return true;
+    case GR_PP:          // all columns; e_pchol_kernel takes the active ones
+      add(d.P, m, m);
+      t.P = t.Q = m; t.kind = GK_HERM; out = d.G;
       return true;
     default:
       add(d.X, m, m); add(d.Ra, ma, ma); add(d.Pa, ma, mp);
@@ -282,36 +289,53 @@ e_gram_reduce_kernel(const ESlot* __restrict__ S, int which) {
 // block updates, multi-slot (FP64 MMA, rows staged through shared memory: in-place safe)
 // ---------------------------------------------------------------------------------------------
 template <typename T>
-__device__ bool upd_lists(const ESlot& d, int which, BlockList<T>& A, const double2* C[3],
-                          int& q, cplx<T>*& Y, int& accumulate, int& neg,
-                          const double2* C2[3], cplx<T>*& Y2) {
+struct UpdTask {
+  BlockList<T> A;
+  const double2* C[3];
+  const double2* C2[3];      // second output (tcgen05 only)
+  const int* gather;         // columns of A's block 0 (NULL: as they stand)
+  int q, accumulate, neg;
+  cplx<T> *Y, *Y2;
+};
+
+// packed: P's active columns have been gathered into Pa (the tcgen05 kernels read whole rows);
+// otherwise the P updates read them from P itself (the gather took 152 us of a tick of seven slots)
+template <typename T>
+__device__ bool upd_lists(const ESlot& d, int which, bool packed, UpdTask<T>& u) {
   const EState* st = d.st;
   if (st->idle) return false;
   const int m = d.m, ma = st->ma, mp = st->mp;
-  accumulate = 0; neg = 0;
-  Y2 = nullptr;
+  u.accumulate = 0; u.neg = 0;
+  u.Y2 = nullptr; u.gather = nullptr;
   auto set = [&](int i, double2* p, int ld, int c, const double2* cf) {
-    A.p[i] = blk<T>(p); A.ld[i] = ld; A.cols[i] = c; C[i] = cf;
+    u.A.p[i] = blk<T>(p); u.A.ld[i] = ld; u.A.cols[i] = c; u.C[i] = cf; u.C2[i] = nullptr;
   };
+  u.A.nblk = 1;
   switch (which) {
-    case UP_RPROJ: A.nblk = 1; set(0, d.X, m, m, d.W); q = ma; Y = blk<T>(d.Ra); accumulate = 1; neg = 1; return true;
-    case UP_RNORM: A.nblk = 1; set(0, d.Ra, ma, ma, d.U); q = ma; Y = blk<T>(d.Ra); return true;
-    case UP_PNORM:
+    case UP_RPROJ: set(0, d.X, m, m, d.W); u.q = ma; u.Y = blk<T>(d.Ra); u.accumulate = 1; u.neg = 1; return true;
+    case UP_RNORM: set(0, d.Ra, ma, ma, d.U); u.q = ma; u.Y = blk<T>(d.Ra); return true;
+    case UP_PNORM: case UP_APNORM: {
       if (st->skip_pnorm) return false;
-      A.nblk = 1; set(0, d.Pa, ma, ma, d.U); q = ma; Y = blk<T>(d.Pa); return true;
-    case UP_APNORM:
-      if (st->skip_pnorm) return false;
-      A.nblk = 1; set(0, d.APa, ma, ma, d.U); q = ma; Y = blk<T>(d.APa); return true;
+      const bool ax = which == UP_APNORM;
+      if (packed) {
+        set(0, ax ? d.APa : d.Pa, ma, ma, d.U);
+      } else {
+        set(0, ax ? d.AP : d.P, m, ma, d.U);
+        u.gather = st->idx;
+      }
+      u.q = ma; u.Y = blk<T>(ax ? d.APa : d.Pa);
+      return true;
+    }
     default: {        // UP_XPNEW / UP_AXPNEW
       const bool ax = which == UP_AXPNEW;
-      A.nblk = mp ? 3 : 2;
+      u.A.nblk = mp ? 3 : 2;
       set(0, ax ? d.AX : d.X, m, m, nullptr);            // X rows do not enter P
       set(1, ax ? d.ARa : d.Ra, ma, ma, d.Cr);
       set(2, ax ? d.APa : d.Pa, ma, mp, d.Cp);
-      C2[0] = d.Cx; C2[1] = d.Cr; C2[2] = d.Cp;
-      q = m;
-      Y = blk<T>(ax ? d.AP : d.P);
-      Y2 = blk<T>(ax ? d.AX : d.X);
+      u.C2[0] = d.Cx; u.C2[1] = d.Cr; u.C2[2] = d.Cp;
+      u.q = m;
+      u.Y = blk<T>(ax ? d.AP : d.P);
+      u.Y2 = blk<T>(ax ? d.AX : d.X);
       return true;
     }
   }
@@ -326,18 +350,41 @@ e_update_kernel(const ESlot* __restrict__ S, int ns, int which) {
   const ESlot& d = S[k];
   constexpr int prec = std::is_same<T, float>::value ? QDKP_C64 : QDKP_C128;
   if (d.prec != prec) return;
-  const double2* Cf[3];
-  const double2* C2[3] = {nullptr, nullptr, nullptr};
-  int q, accumulate, neg;
   const long long r0 = (long long)(blockIdx.x - d.row0) * d.rows_per_cta;
   const long long r1 = min(d.n, r0 + d.rows_per_cta);
-  BlockList<T> A;
-  cplx<T> *Y, *Y2;
-  if (!upd_lists<T>(d, which, A, Cf, q, Y, accumulate, neg, C2, Y2)) return;
+  UpdTask<T> u;
+  if (!upd_lists<T>(d, which, false, u)) return;
   if constexpr (std::is_same<T, float>::value)
-    update_rows_tf32(A, Cf, q, r0, r1, Y, (long long)q, accumulate, neg, usm_e, C2, Y2);
+    update_rows_tf32(u.A, u.C, u.q, r0, r1, u.Y, (long long)u.q, u.accumulate, u.neg, usm_e, u.gather);
   else
-    update_rows(A, Cf, q, r0, r1, Y, (long long)q, accumulate, neg, usm_e, C2, Y2);
+    update_rows(u.A, u.C, u.q, r0, r1, u.Y, (long long)u.q, u.accumulate, u.neg, usm_e, u.gather);
+}
+
+// The Ritz update of X, AX, P and AP with the residual norms (and, while every column is active, the
+// residual block) of the new iterate, one pass (ritz_rows). The next tick's decision kernel reads
+// the norms. One launch per precision present.
+template <typename T>
+__global__ void __launch_bounds__(kUpdThreads, 2)
+e_ritz_kernel(const ESlot* __restrict__ S, int ns) {
+  extern __shared__ __align__(16) unsigned char usm_r[];
+  const int k = slot_of(S, ns, blockIdx.x, &ESlot::row0);
+  const ESlot& d = S[k];
+  constexpr int prec = std::is_same<T, float>::value ? QDKP_C64 : QDKP_C128;
+  const EState* st = d.st;
+  if (d.prec != prec || st->idle) return;
+  const int part = blockIdx.x - d.row0;
+  const long long r0 = (long long)part * d.rows_per_cta;
+  RitzArgs<T> t;
+  t.X = blk<T>(d.X); t.R = blk<T>(d.Ra); t.P = blk<T>(d.P);
+  t.AX = blk<T>(d.AX); t.AR = blk<T>(d.ARa); t.AP = blk<T>(d.AP);
+  t.Pin = blk<T>(d.Pa); t.APin = blk<T>(d.APa);
+  t.m = d.m; t.ma = st->ma; t.mp = st->mp;
+  t.Rout = t.ma == t.m ? t.R : nullptr;
+  t.Cx = d.Cx; t.Cr = d.Cr; t.Cp = d.Cp;
+  t.lam = st->lam;
+  t.npart = d.npart + (long long)part * d.m;
+  if constexpr (std::is_same<T, float>::value) ritz_rows_tf32(t, r0, min(d.n, r0 + d.rows_per_cta), usm_r);
+  else ritz_rows(t, r0, min(d.n, r0 + d.rows_per_cta), usm_r);
 }
 
 // complex64 slots: the same updates on the tcgen05 tensor cores (umma_dev.cuh). The CTAs split
@@ -369,19 +416,16 @@ e_update_umma_kernel(const ESlot* __restrict__ S, int ns, int which, int utiles,
     if (k < 0) break;                                  // uniform; not reached
     const ESlot& d = S[k];
     const long long seg_end = min(c1, (long long)d.utile0 + nt);
-    const double2* Cf[3];
-    const double2* C2[3] = {nullptr, nullptr, nullptr};
-    int q, accumulate, neg;
-    BlockList<float> A;
-    float2 *Y, *Y2;
-    if (upd_lists<float>(d, which, A, Cf, q, Y, accumulate, neg, C2, Y2)) {
+    UpdTask<float> u;
+    if (upd_lists<float>(d, which, true, u)) {
       const long long r0 = (c - d.utile0) * kUmmaRows;
       const long long r1 = min(d.n, (seg_end - d.utile0) * kUmmaRows);
       if (ok) {
-        ok = update_rows_umma(pl, cx, A, Cf, q, r0, r1, Y, (long long)q, accumulate, neg, usm_u, C2, Y2);
+        ok = update_rows_umma(pl, cx, u.A, u.C, u.q, r0, r1, u.Y, (long long)u.q, u.accumulate, u.neg,
+                              usm_u, u.C2, u.Y2);
       } else {
-        float2* const Ys[2] = {Y, Y2};
-        umma_fill_nan(Ys, Y2 ? 2 : 1, q, r0, r1, (long long)q);
+        float2* const Ys[2] = {u.Y, u.Y2};
+        umma_fill_nan(Ys, u.Y2 ? 2 : 1, u.q, r0, r1, (long long)u.q);
       }
     }
     c = seg_end;
@@ -414,12 +458,15 @@ __global__ void __launch_bounds__(kSmallThreads) e_pchol_kernel(const ESlot* __r
   const ESlot& d = S[blockIdx.x];
   EState* st = d.st;
   if (st->idle) return;
-  const int n = st->ma;
+  const int n = st->ma, m = d.m;
   if (st->skip_p) {                        // iteration 0: no P yet, restart stays as it is
     if (threadIdx.x == 0) { st->skip_pnorm = 1; st->mp = st->restart ? 0 : n; }
     return;
   }
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) ssm_e[e] = d.G[e];
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+    const int i = e / n, j = e - i * n;
+    ssm_e[e] = d.G[st->idx[i] * m + st->idx[j]];
+  }
   __syncthreads();
   const int fail = block_cholesky_upper(ssm_e, n);
   if (!fail) {
@@ -475,7 +522,8 @@ __device__ void e_assemble(const ESlot& d, const EState* st, int restart, int& d
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kSmallThreads) e_rr_kernel(const ESlot* __restrict__ S) {
+// c64_ritz: the Ritz update of complex64 slots is e_ritz_kernel's too
+__global__ void __launch_bounds__(kSmallThreads) e_rr_kernel(const ESlot* __restrict__ S, int c64_ritz) {
   extern __shared__ double2 rsm[];
   const ESlot& d = S[blockIdx.x];
   EState* st = d.st;
@@ -508,7 +556,11 @@ __global__ void __launch_bounds__(kSmallThreads) e_rr_kernel(const ESlot* __rest
     else d.Cp[(i - m - ma) * m + j] = v;
   }
   if (threadIdx.x < m) st->lam[threadIdx.x] = d.w[threadIdx.x];
-  if (threadIdx.x == 0) { st->restart = use_restart ? 1 : st->restart; st->mp = mp; }
+  if (threadIdx.x == 0) {
+    st->restart = use_restart ? 1 : st->restart;
+    st->mp = mp;
+    st->resid_ready = ma == m && (c64_ritz || d.prec != QDKP_C64);
+  }
 }
 
 }  // namespace qdkp
@@ -539,7 +591,7 @@ SlotLayout slot_layout(int64_t n, int m, int prec) {
   SlotLayout L;
   L.blk = align256((size_t)n * m * (prec == QDKP_C64 ? sizeof(float2) : sizeof(double2)));
   L.small = align256((size_t)(3 * m) * (3 * m) * sizeof(double2));
-  L.nparts = (int)((n + kENormRows - 1) / kENormRows);
+  L.nparts = (int)((n + kERowsPerCta - 1) / kERowsPerCta);
   L.npart = align256((size_t)L.nparts * m * sizeof(double));
   L.gparts = gram_parts(n);
   // the widest task: 3 m x 6 m columns (explicit Gram matrices)
@@ -559,7 +611,7 @@ constexpr int kEGroups = 2;
 struct EGroup {
   ESlot* d_slots = nullptr;            // this group's run of the compact slot array
   HXSlot* d_hx = nullptr;              // [precision][phase][slot]: 2 x 4 x max_slots descriptors
-  int ns = 0, norm_ctas = 0, gram_ctas = 0, row_ctas = 0;
+  int ns = 0, gram_ctas = 0, row_ctas = 0;
   int utiles = 0;                      // 128-row tiles of the complex64 slots (tcgen05 updates)
   int nsm = 148;
   int hx_ns[2] = {0, 0}, hx_tiles[2] = {0, 0};   // per precision (QDKP_C128, QDKP_C64)
@@ -666,12 +718,11 @@ int build_group(qdkp_engine* e, int g, const std::vector<int>& ids, int base, cu
   G.d_hx = e->d_hx + (size_t)g * 8 * e->max_slots;
   std::vector<ESlot> compact;
   std::vector<HXSlot> hx(8 * (size_t)e->max_slots);
-  int norm0 = 0, gram0 = 0, row0 = 0, m_max = 1, utile0 = 0;
+  int gram0 = 0, row0 = 0, m_max = 1, utile0 = 0;
   int tile0[2] = {0, 0}, kp[2] = {0, 0};
   for (int i : ids) {
     SlotHost& h = e->slots[i];
     ESlot d = h.d;
-    d.norm0 = norm0; norm0 += d.nparts;
     d.gram0 = gram0; gram0 += d.gparts;
     d.row0 = row0; row0 += (int)((d.n + d.rows_per_cta - 1) / d.rows_per_cta);
     d.utile0 = -1;
@@ -709,7 +760,7 @@ int build_group(qdkp_engine* e, int g, const std::vector<int>& ids, int base, cu
     tile0[pi] += tiles;
   }
   G.ns = (int)compact.size();
-  G.norm_ctas = norm0; G.gram_ctas = gram0; G.row_ctas = row0;
+  G.gram_ctas = gram0; G.row_ctas = row0;
   G.utiles = utile0;
   G.nsm = e->nsm;
   for (int pi = 0; pi < 2; ++pi) { G.hx_ns[pi] = kp[pi]; G.hx_tiles[pi] = tile0[pi]; }
@@ -776,23 +827,47 @@ int launch_gram_multi(const EGroup& G, int which, cudaStream_t st) {
   return QDKP_OK;
 }
 
-int launch_update_multi(const EGroup& G, int which, cudaStream_t st) {
+int launch_umma_multi(const EGroup& G, int which, cudaStream_t st) {
   const bool fused = which == UP_XPNEW || which == UP_AXPNEW;
-  const int P = (fused ? 3 : 1) * G.m_max, nout = fused ? 2 : 1;
+  const UmmaPlan pl = umma_plan((fused ? 3 : 1) * G.m_max, G.m_max, fused ? 2 : 1, G.m_max, G.m_max);
+  if (!pl.nout_pass) { set_error("tcgen05 update plan does not fit shared memory"); return QDKP_ERR_ARG; }
+  e_update_umma_kernel<<<std::min(G.utiles, G.nsm), kUmmaThreads, pl.bytes, st>>>(
+      G.d_slots, G.ns, which, G.utiles, G.m_max);
+  count_launch();
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
+}
+
+int launch_update_multi(const EGroup& G, int which, cudaStream_t st) {
   if (G.hx_ns[0]) {
-    const size_t smem = update_smem_bytes(P, G.m_max, nout);
-    e_update_kernel<double><<<G.row_ctas, kUpdThreads, smem, st>>>(G.d_slots, G.ns, which);
+    e_update_kernel<double><<<G.row_ctas, kUpdThreads, update_smem_bytes(G.m_max, G.m_max), st>>>(
+        G.d_slots, G.ns, which);
     count_launch();
   }
-  if (G.hx_ns[1] && !c64_update_tcgen05()) {
-    const size_t smem = update_tf32_smem_bytes(P, G.m_max, nout);
-    e_update_kernel<float><<<G.row_ctas, kUpdThreads, smem, st>>>(G.d_slots, G.ns, which);
+  if (G.hx_ns[1] && c64_update_tcgen05()) {
+    const int rc = launch_umma_multi(G, which, st);
+    if (rc) return rc;
+  } else if (G.hx_ns[1]) {
+    e_update_kernel<float><<<G.row_ctas, kUpdThreads, update_tf32_smem_bytes(G.m_max, G.m_max), st>>>(
+        G.d_slots, G.ns, which);
     count_launch();
-  } else if (G.hx_ns[1] && G.utiles) {
-    const UmmaPlan pl = umma_plan(P, G.m_max, nout, G.m_max, G.m_max);
-    if (!pl.nout_pass) { set_error("tcgen05 update plan does not fit shared memory"); return QDKP_ERR_ARG; }
-    e_update_umma_kernel<<<std::min(G.utiles, G.nsm), kUmmaThreads, pl.bytes, st>>>(
-        G.d_slots, G.ns, which, G.utiles, G.m_max);
+  }
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
+}
+
+int launch_ritz_multi(const EGroup& G, cudaStream_t st) {
+  if (G.hx_ns[0]) {
+    e_ritz_kernel<double><<<G.row_ctas, kUpdThreads, ritz_smem_bytes(G.m_max), st>>>(G.d_slots, G.ns);
+    count_launch();
+  }
+  if (G.hx_ns[1] && c64_update_tcgen05()) {
+    int rc = launch_umma_multi(G, UP_XPNEW, st);
+    if (rc) return rc;
+    rc = launch_umma_multi(G, UP_AXPNEW, st);
+    if (rc) return rc;
+  } else if (G.hx_ns[1]) {
+    e_ritz_kernel<float><<<G.row_ctas, kUpdThreads, ritz_tf32_smem_bytes(G.m_max), st>>>(G.d_slots, G.ns);
     count_launch();
   }
   QDKP_CUDA_TRY(cudaGetLastError());
@@ -818,16 +893,22 @@ int tick(const qdkp_engine* e, const EGroup& G, cudaStream_t st) {
 #define ETRY(x) do { rc = (x); if (rc != QDKP_OK) return rc; } while (0)
   const size_t small_smem = 2 * (size_t)G.m_max * G.m_max * sizeof(double2);
   const size_t rr_smem = 2 * (size_t)(3 * G.m_max) * (3 * G.m_max) * sizeof(double2);
-  e_norm_kernel<<<G.norm_ctas, kTallThreads, 0, st>>>(G.d_slots, ns);
-  e_decide_kernel<<<ns, 32, 0, st>>>(G.d_slots);
+  const bool umma = G.hx_ns[1] && c64_update_tcgen05();
+  if (umma) {
+    e_norm_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, ns);
+    count_launch();
+  }
+  e_decide_kernel<<<ns, kDecideThreads, 0, st>>>(G.d_slots);
   e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, ns, RW_COPYBEST);
   e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, ns, RW_RESID);
-  count_launch(4);
+  count_launch(3);
   QDKP_CUDA_TRY(cudaGetLastError());
   ETRY(launch_hx_phase(e, G, 0, st));
   ETRY(launch_hx_phase(e, G, 1, st));
-  e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, ns, RW_GATHERP);
-  count_launch();
+  if (umma) {
+    e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, ns, RW_GATHERP);
+    count_launch();
+  }
   ETRY(launch_gram_multi(G, GR_XR, st));
   ETRY(launch_update_multi(G, UP_RPROJ, st));
   ETRY(launch_gram_multi(G, GR_RR, st));
@@ -842,11 +923,10 @@ int tick(const qdkp_engine* e, const EGroup& G, cudaStream_t st) {
   ETRY(launch_update_multi(G, UP_PNORM, st));
   ETRY(launch_update_multi(G, UP_APNORM, st));
   ETRY(launch_gram_multi(G, GR_RZ, st));
-  e_rr_kernel<<<ns, kSmallThreads, rr_smem, st>>>(G.d_slots);
+  e_rr_kernel<<<ns, kSmallThreads, rr_smem, st>>>(G.d_slots, !umma);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
-  ETRY(launch_update_multi(G, UP_XPNEW, st));
-  ETRY(launch_update_multi(G, UP_AXPNEW, st));
+  ETRY(launch_ritz_multi(G, st));
 #undef ETRY
   return QDKP_OK;
 }
@@ -954,6 +1034,8 @@ int qdkp_engine_create(int max_slots, int device, qdkp_engine** out) {
   cudaFuncSetAttribute(e_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramMaxSmem);
   cudaFuncSetAttribute(e_update_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(e_update_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_ritz_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_ritz_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(e_update_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        kUmmaSmemLimit);
   cudaFuncSetAttribute(e_rr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
@@ -1062,6 +1144,8 @@ int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg
   if (!nonfinite) {
     ATRY(update1(h, d.X, m, d.E, m, d.X, st));
     ATRY(update1(h, d.AX, m, d.E, m, d.AX, st));
+    // the first tick's decision kernel reads the partials left in npart
+    ATRY(colnorm1(h, d.AX, d.X, d.w, m, d.gpart, st));
     ATRY(read_sync(w.data(), d.w, m * sizeof(double), st));
   }
   EState s0{};

@@ -21,6 +21,8 @@ struct EState {
   int skip_recompute;   // 0: forced restart recomputes A X this tick
   int skip_p;           // 1: no P block this tick (iteration 0 or idle)
   int skip_pnorm;       // 1: P orthonormalisation is not applied
+  int resid_ready;      // 1: Ra holds the residuals of all m columns of X
+  int skip_resid;       // 1: ... and this tick wants them all
   double smallest;
   int active[kMaxBlock];
   int idx[kMaxBlock];
@@ -45,13 +47,13 @@ struct ESlot {
   double2 *X, *AX, *P, *AP, *best, *Ra, *ARa, *Pa, *APa, *T;
   double2 *W, *G, *U, *gS, *gT, *gA, *gB, *E, *scr, *Cx, *Cr, *Cp, *Im;
   double* w;
-  double* npart;        // [nparts][m] residual-norm partials
+  double* npart;        // [nparts][m] residual-norm partials of the current X
   double* gpart;        // Gram partials (real)
-  int nparts;           // CTAs of the norm kernel
+  int nparts;           // their parts: CTAs of the row kernels
   int gparts;           // row parts (CTAs) of the Gram kernel
-  int norm0, gram0, row0;   // first CTA of this slot in the norm / Gram / row-kernel launches
+  int gram0, row0;      // first CTA of this slot in the Gram / row-kernel launches
   int utile0;           // complex64 slots: first 128-row tile in the group's tcgen05 update space
-  int rows_per_cta;     // rows per CTA in the row kernels (gather, update)
+  int rows_per_cta;     // rows per CTA in the row kernels (gather, update, norms)
   EState* st;
 };
 
