@@ -82,55 +82,17 @@ int launch_colnorm2(const cplx<T>* A, long long lda, const cplx<T>* B, long long
   return QDKP_OK;
 }
 
-// ------------------------------------------------------------------------------------------------
-// R[:, c] = AX[:, idx[c]] - lambda[idx[c]] X[:, idx[c]]   (active residual columns, compacted)
-// ------------------------------------------------------------------------------------------------
-__global__ void resid_gather_kernel(const double2* __restrict__ AX, long long ldax,
-                                    const double2* __restrict__ X, long long ldx,
-                                    const double* __restrict__ lam, const int* __restrict__ idx,
-                                    int ma, long long n, double2* __restrict__ R, long long ldr) {
-  const long long total = n * ma;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long r = e / ma;
-    const int c = (int)(e - r * ma);
-    const int j = idx[c];
-    const double l = lam[j];
-    const double2 a = AX[r * ldax + j], x = X[r * ldx + j];
-    R[r * ldr + c] = make_double2(a.x - l * x.x, a.y - l * x.y);
-  }
-}
-
-int launch_resid_gather(const double2* AX, long long ldax, const double2* X, long long ldx,
-                        const double* lambda, const int* idx, int ma, long long n, double2* R,
-                        long long ldr, cudaStream_t st) {
-  resid_gather_kernel<<<1184, 256, 0, st>>>(AX, ldax, X, ldx, lambda, idx, ma, n, R, ldr);
-  count_launch();
-  QDKP_CUDA_TRY(cudaGetLastError());
-  return QDKP_OK;
-}
-
 template <typename TS, typename TD>
-__global__ void gather_kernel(const cplx<TS>* __restrict__ src, long long lds,
-                              const int* __restrict__ idx, int ma, long long n,
-                              cplx<TD>* __restrict__ dst, long long ldd) {
-  const long long total = n * ma;
+__global__ void copy_kernel(const cplx<TS>* __restrict__ src, long long lds, int cols, long long n,
+                            cplx<TD>* __restrict__ dst, long long ldd) {
+  const long long total = n * cols;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
-    const long long r = e / ma;
-    const int c = (int)(e - r * ma);
-    const cplx<TS> v = src[r * lds + (idx ? idx[c] : c)];
+    const long long r = e / cols;
+    const int c = (int)(e - r * cols);
+    const cplx<TS> v = src[r * lds + c];
     dst[r * ldd + c] = mk<TD>((TD)v.x, (TD)v.y);
   }
-}
-
-template <typename TS, typename TD>
-int launch_gather(const cplx<TS>* src, long long lds, const int* idx, int ma, long long n,
-                  cplx<TD>* dst, long long ldd, cudaStream_t st) {
-  gather_kernel<TS, TD><<<1184, 256, 0, st>>>(src, lds, idx, ma, n, dst, ldd);
-  count_launch();
-  QDKP_CUDA_TRY(cudaGetLastError());
-  return QDKP_OK;
 }
 
 template <typename TS, typename TD>
@@ -141,7 +103,10 @@ int launch_copy(const cplx<TS>* src, long long lds, int cols, long long n, cplx<
                                   cudaMemcpyDeviceToDevice, st));
     return QDKP_OK;
   }
-  return launch_gather<TS, TD>(src, lds, nullptr, cols, n, dst, ldd, st);
+  copy_kernel<TS, TD><<<1184, 256, 0, st>>>(src, lds, cols, n, dst, ldd);
+  count_launch();
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -154,14 +119,13 @@ gram_kernel(const GramTask<T> t, int parts, double* __restrict__ partial) {
   gram_core(t, (int)blockIdx.x, parts, (int)blockIdx.y, partial, gsm_d);
 }
 
-// out row-major with leading dimension Q (GK_FULL, GK_HERM: both triangles); the pencil kinds write
-// the layouts of gram_put
+// out row-major with leading dimension Q (GK_FULL, GK_HERM: both triangles)
 template <typename T>
 __global__ void __launch_bounds__(kGramRedThreads)
 gram_reduce_kernel(const GramTask<T> t, int parts, const double* __restrict__ partial,
-                   double2* __restrict__ out, double2* __restrict__ outS) {
+                   double2* __restrict__ out) {
   gram_reduce_core(t, parts, partial, (int)blockIdx.x, (int)gridDim.x,
-                   [&](int i, int j, double2 v) { gram_put(t, i, j, v, out, outS); });
+                   [&](int i, int j, double2 v) { gram_put(t, i, j, v, out, out); });
 }
 
 size_t gram_partial_elems(int P, int Q) {
@@ -171,7 +135,7 @@ size_t gram_partial_elems(int P, int Q) {
 
 template <typename T>
 static int launch_gram_task(const GramTask<T>& t, double2* partial, size_t partial_elems, double2* out,
-                            double2* outS, cudaStream_t st) {
+                            cudaStream_t st) {
   const GramShape sh = gram_shape(t.kind, t.P, t.Q, t.m, t.ma, t.mp);
   const int parts = gram_parts(t.n);
   if (gram_partial_doubles(sh.rects, parts) > 2 * partial_elems) {
@@ -182,29 +146,10 @@ static int launch_gram_task(const GramTask<T>& t, double2* partial, size_t parti
   QDKP_CUDA_TRY(cudaFuncSetAttribute(gram_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramMaxSmem));
   double* pd = reinterpret_cast<double*>(partial);
   gram_kernel<T><<<dim3((unsigned)parts, (unsigned)sh.panels), 32 * (sh.warps + 1), smem, st>>>(t, parts, pd);
-  gram_reduce_kernel<T><<<(t.P * t.Q + 31) / 32, kGramRedThreads, 0, st>>>(t, parts, pd, out, outS);
+  gram_reduce_kernel<T><<<(t.P * t.Q + 31) / 32, kGramRedThreads, 0, st>>>(t, parts, pd, out);
   count_launch(2);
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;
-}
-
-int launch_gram_rz(const BlockList<double>& W, const BlockList<double>& AW, bool explicit_gram,
-                   long long n, double2* partial, size_t partial_elems, double2* gT, double2* gS,
-                   cudaStream_t st) {
-  GramTask<double> t{};
-  auto add = [&](const BlockList<double>& L, int b) {
-    t.p[t.nblk] = L.p[b]; t.ld[t.nblk] = (int)L.ld[b]; t.cols[t.nblk] = L.cols[b];
-    ++t.nblk;
-    t.tc += L.cols[b];
-  };
-  for (int b = 0; b < W.nblk; ++b) add(W, b);
-  for (int b = explicit_gram ? 0 : 1; b < AW.nblk; ++b) add(AW, b);
-  t.m = W.cols[0]; t.ma = W.cols[1]; t.mp = W.nblk > 2 ? W.cols[2] : 0;
-  t.P = t.m + t.ma + t.mp;
-  t.n = n;
-  if (explicit_gram) { t.kind = GK_EXPLICIT; t.b0 = 0; t.Q = 2 * t.P; }
-  else { t.kind = GK_PENCIL; t.b0 = t.m + t.ma; t.Q = 2 * t.mp + t.ma; }
-  return launch_gram_task(t, partial, partial_elems, gT, gS, st);
 }
 
 template <typename T>
@@ -230,7 +175,7 @@ int launch_gram(const BlockList<T>& A, const BlockList<T>& B, long long n,
   t.a0 = 0; t.P = P; t.b0 = same ? 0 : P; t.Q = Q;
   t.kind = same ? GK_HERM : GK_FULL;
   t.n = n;
-  return launch_gram_task(t, partial, partial_elems, out, out, st);
+  return launch_gram_task(t, partial, partial_elems, out, st);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -416,10 +361,6 @@ int launch_eigh(const double2* A, const double2* B, int n, double* w, double2* V
 QDKP_BLOCKOPS_INST(double)
 QDKP_BLOCKOPS_INST(float)
 #undef QDKP_BLOCKOPS_INST
-template int launch_gather<double, double>(const double2*, long long, const int*, int, long long,
-                                           double2*, long long, cudaStream_t);
-template int launch_gather<float, float>(const float2*, long long, const int*, int, long long,
-                                         float2*, long long, cudaStream_t);
 template int launch_copy<double, double>(const double2*, long long, int, long long, double2*,
                                          long long, cudaStream_t);
 template int launch_copy<float, float>(const float2*, long long, int, long long, float2*,

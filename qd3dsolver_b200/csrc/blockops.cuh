@@ -38,12 +38,6 @@ template <typename T>
 int launch_colnorm2(const cplx<T>* A, long long lda, const cplx<T>* B, long long ldb,
                     const double* lambda, int m, long long n, double* partial, int nparts,
                     double* out, cudaStream_t st);
-int launch_resid_gather(const double2* AX, long long ldax, const double2* X, long long ldx,
-                        const double* lambda, const int* idx, int ma, long long n, double2* R,
-                        long long ldr, cudaStream_t st);
-template <typename TS, typename TD>
-int launch_gather(const cplx<TS>* src, long long lds, const int* idx, int ma, long long n,
-                  cplx<TD>* dst, long long ldd, cudaStream_t st);
 // dst = src (columns [0, cols)), converting the precision when TS != TD
 template <typename TS, typename TD>
 int launch_copy(const cplx<TS>* src, long long lds, int cols, long long n, cplx<TD>* dst,
@@ -54,10 +48,6 @@ int launch_copy(const cplx<TS>* src, long long lds, int cols, long long n, cplx<
                              const double* lambda, int m, long long n, double* partial,       \
                              int nparts, double* out, cudaStream_t st) {                      \
     return launch_colnorm2<R>(A, lda, B, ldb, lambda, m, n, partial, nparts, out, st);        \
-  }                                                                                           \
-  inline int launch_gather(const C* src, long long lds, const int* idx, int ma, long long n,  \
-                           C* dst, long long ldd, cudaStream_t st) {                          \
-    return launch_gather<R, R>(src, lds, idx, ma, n, dst, ldd, st);                           \
   }                                                                                           \
   inline int launch_copy(const C* src, long long lds, int cols, long long n, C* dst,          \
                          long long ldd, cudaStream_t st) {                                    \
@@ -71,12 +61,6 @@ template <typename T>
 int launch_gram(const BlockList<T>& A, const BlockList<T>& B, long long n,
                 double2* partial, size_t partial_elems, double2* out, cudaStream_t st);
 size_t gram_partial_elems(int P, int Q);
-// The products of the Rayleigh-Ritz pencil in one pass over W = [X | R (| P)], AW = [AX | AR (| AP)]:
-// explicit: gS = W^H W and gT = W^H AW (tot x tot); otherwise gS = [X | R]^H P and gT = W^H [AR | AP].
-// Entries that the pencils do not read (lobpcg.py:826-909) are not formed.
-int launch_gram_rz(const BlockList<double>& W, const BlockList<double>& AW, bool explicit_gram,
-                   long long n, double2* partial, size_t partial_elems, double2* gT, double2* gS,
-                   cudaStream_t st);
 // Y = beta * Y + sum_k A_k C_k; C_k (cols_k x q, row-major, ld q) in device memory.
 template <typename T>
 int launch_update(const BlockList<T>& A, const double2* const* C, int q, long long n,

@@ -11,7 +11,7 @@
 #include <type_traits>
 #include <vector>
 
-#include "engine_dev.cuh"
+#include "engine_host.cuh"
 #include "umma_dev.cuh"
 
 namespace qdkp {
@@ -19,14 +19,16 @@ namespace qdkp {
 int launch_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int64_t ldy,
                  int m, double sigma, int shifted, int precision, cudaStream_t st);
 
-constexpr int kERowsPerCta = 512;    // rows per CTA of the row kernels
+// Rows per CTA of the row kernels: a multiple of the update's chunk, and no more than kEMaxParts CTAs
+// for a slot, whose norm partials one CTA then sums (32768 parts of a 128^3 solve would take 0.5 ms).
+constexpr int kERowsPerCta = 512;
+constexpr int kEMaxParts = 4096;
 
 // GR_RZ: the products of the Rayleigh-Ritz pencil, in one pass (GK_PENCIL or GK_EXPLICIT)
 enum GramWhich { GR_XR = 0, GR_RR, GR_PP, GR_RZ };
 // UP_XPNEW, UP_AXPNEW: the Ritz update of complex64 slots on the tcgen05 tensor cores, P and X (AP and
 // AX) from one pass over [X | R | P] ([AX | AR | AP]); otherwise e_ritz_kernel forms all four.
 enum UpdWhich { UP_RPROJ = 0, UP_RNORM, UP_PNORM, UP_APNORM, UP_XPNEW, UP_AXPNEW };
-enum RowWhich { RW_COPYBEST = 0, RW_RESID, RW_GATHERP };
 
 // ---------------------------------------------------------------------------------------------
 // residual norms of A X - X lambda: partials per CTA, reduced in the decision kernel. Only where the
@@ -78,24 +80,9 @@ e_norm_kernel(const ESlot* __restrict__ S, int ns) {
 // ---------------------------------------------------------------------------------------------
 // per-slot decisions at the top of an iteration (lobpcg.py:688-760)
 // ---------------------------------------------------------------------------------------------
-constexpr int kDecideThreads = 768;    // 32 per column of the widest block
-
-__global__ void __launch_bounds__(kDecideThreads) e_decide_kernel(const ESlot* __restrict__ S) {
-  const ESlot& d = S[blockIdx.x];
-  EState* st = d.st;
-  __shared__ double nrm[kMaxBlock];
+// scipy's decisions from the column norms; one thread
+static __device__ void e_decide(const ESlot& d, EState* st, const double* __restrict__ nrm) {
   const int m = d.m;
-  // a warp per column, parts strided over its lanes: 28 us with a thread per column, 5 us now
-  // (7 slots of 860 parts)
-  const int c = threadIdx.x >> 5;
-  if (c < m) {
-    double s = 0.0;
-    for (int b = threadIdx.x & 31; b < d.nparts; b += 32) s += d.npart[(long long)b * m + c];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) nrm[c] = sqrt(fabs(s));
-  }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
   st->idle = 1; st->copy_best = 0; st->skip_recompute = 1; st->skip_p = 1; st->skip_pnorm = 1;
   if (!st->running) return;
   if (st->iter >= d.maxiter) { st->running = 0; st->status = QDKP_LOBPCG_MAXITER; return; }
@@ -134,6 +121,31 @@ __global__ void __launch_bounds__(kDecideThreads) e_decide_kernel(const ESlot* _
   st->explicit_gram = !(mx > d.sqrt_eps && !st->explicit_gram);
   st->idle = 0;
   st->skip_p = st->iter == 0 ? 1 : 0;
+}
+
+constexpr int kDecideThreads = 768;    // 32 per column of the widest block
+
+__global__ void __launch_bounds__(kDecideThreads) e_decide_kernel(const ESlot* __restrict__ S) {
+  const ESlot& d = S[blockIdx.x];
+  EState* st = d.st;
+  __shared__ double nrm[kMaxBlock];
+  const int m = d.m;
+  // a warp per column, parts strided over its lanes: 28 us with a thread per column, 5 us now
+  // (7 slots of 860 parts)
+  const int c = threadIdx.x >> 5;
+  if (c < m) {
+    double s = 0.0;
+    for (int b = threadIdx.x & 31; b < d.nparts; b += 32) s += d.npart[(long long)b * m + c];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) nrm[c] = sqrt(fabs(s));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) e_decide(d, st, nrm);
+  if (!d.snap) return;
+  __syncthreads();
+  const int* from = reinterpret_cast<const int*>(st);
+  int* to = reinterpret_cast<int*>(d.snap);
+  for (int i = threadIdx.x; i < (int)(sizeof(EState) / sizeof(int)); i += blockDim.x) to[i] = from[i];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -569,6 +581,198 @@ __global__ void __launch_bounds__(kSmallThreads) e_rr_kernel(const ESlot* __rest
 // host side
 // =============================================================================================
 namespace qdkp {
+
+size_t align256(size_t b) { return (b + 255) / 256 * 256; }
+
+SlotLayout slot_layout(int64_t n, int m, int prec, int n_blocks) {
+  SlotLayout L;
+  L.blk = align256((size_t)n * m * (prec == QDKP_C64 ? sizeof(float2) : sizeof(double2)));
+  L.small = align256((size_t)(3 * m) * (3 * m) * sizeof(double2));
+  const int64_t rows = (n + kEMaxParts - 1) / kEMaxParts;
+  L.rows_per_cta = (int)std::max<int64_t>(kERowsPerCta, (rows + kUpdChunk - 1) / kUpdChunk * kUpdChunk);
+  L.nparts = (int)((n + L.rows_per_cta - 1) / L.rows_per_cta);
+  L.npart = align256((size_t)L.nparts * m * sizeof(double));
+  L.gparts = gram_parts(n);
+  // the widest task: 3 m x 6 m columns (explicit Gram matrices)
+  L.gpart = align256(gram_partial_elems(3 * m, 6 * m) * sizeof(double2));
+  L.total = align256(sizeof(EState)) + n_blocks * L.blk + 13 * L.small +
+            align256(3 * m * sizeof(double)) + L.npart + L.gpart;
+  return L;
+}
+
+void slot_carve(ESlot& d, void* ws, const SlotLayout& L, int64_t n, int m, int prec, int n_blocks) {
+  char* p = static_cast<char*>(ws);
+  auto take = [&](size_t b) { char* r = p; p += align256(b); return r; };
+  d.st = (EState*)take(sizeof(EState));
+  double2** const blocks[10] = {&d.X, &d.AX, &d.P, &d.AP, &d.best, &d.Ra, &d.ARa, &d.Pa, &d.APa, &d.T};
+  for (int i = 0; i < 10; ++i) *blocks[i] = i < n_blocks ? (double2*)take(L.blk) : nullptr;
+  d.W = (double2*)take(L.small); d.G = (double2*)take(L.small); d.U = (double2*)take(L.small);
+  d.gS = (double2*)take(L.small); d.gT = (double2*)take(L.small); d.gA = (double2*)take(L.small);
+  d.gB = (double2*)take(L.small); d.E = (double2*)take(L.small);
+  d.scr = (double2*)take(2 * L.small);
+  d.Cx = (double2*)take(L.small); d.Cr = (double2*)take(L.small); d.Cp = (double2*)take(L.small);
+  d.w = (double*)take(3 * m * sizeof(double));
+  d.npart = (double*)take(L.npart);
+  d.gpart = (double*)take(L.gpart);
+  d.n = n; d.m = m; d.prec = prec;
+  d.nparts = L.nparts; d.gparts = L.gparts; d.rows_per_cta = L.rows_per_cta;
+  d.gram0 = d.row0 = 0;
+  d.utile0 = -1;
+  d.snap = nullptr;
+}
+
+void slot_params(ESlot& d, EState& s, const qdkp_lobpcg_params* prm, const double* lam) {
+  const double eps = d.prec == QDKP_C64 ? (double)std::numeric_limits<float>::epsilon()
+                                        : std::numeric_limits<double>::epsilon();
+  d.folded = prm->folded;
+  d.sqrt_eps = std::sqrt(eps);
+  d.tol = prm->tol > 0 ? prm->tol : std::sqrt(std::numeric_limits<double>::epsilon()) * (double)d.n;
+  d.maxiter = prm->maxiter;
+  d.stall_iterations = prm->stall_iterations;
+  d.restart_control = prm->restart_control > 0 ? prm->restart_control : 20;
+  s = EState{};
+  s.running = 1;
+  s.status = QDKP_LOBPCG_MAXITER;
+  s.iter = -1; s.idle = 1;
+  s.ma = d.m; s.mp = 0; s.restart = 1; s.forced = 0; s.explicit_gram = 0;
+  s.best_iter = prm->maxiter; s.skip_recompute = 1; s.skip_p = 1; s.skip_pnorm = 1;
+  s.smallest = std::numeric_limits<double>::max();
+  for (int j = 0; j < d.m; ++j) { s.active[j] = 1; s.lam[j] = lam[j]; }
+}
+
+static int launch_gram_multi(const EGroup& G, int which, cudaStream_t st) {
+  int mmax = 0;
+  for (int m : G.widths) {
+    // the warps for the product at full width; panels for the most rectangles any active width and
+    // either pencil can form (the CTAs of panels that stay empty return at once)
+    const int P = which == GR_RZ ? 3 * m : m, Q = P, tc = which == GR_RZ ? 6 * m : 2 * m;
+    const int kind = which == GR_XR ? GK_FULL : (which == GR_RZ ? GK_PENCIL : GK_HERM);
+    const GramShape sh = gram_shape(kind, P, Q, m, m, m);
+    const int most = (P + kGramRect - 1) / kGramRect * (((which == GR_RZ ? 6 * m : m) + kGramRect - 1) / kGramRect);
+    const size_t smem = std::max(gram_smem<double>(tc, sh.warps), gram_smem<float>(tc, sh.warps));
+    e_gram_kernel<<<dim3(G.gram_ctas, (most + sh.warps - 1) / sh.warps), 32 * (sh.warps + 1), smem, st>>>(
+        G.d_slots, G.ns, which, m);
+    count_launch();
+    mmax = std::max(mmax, m);
+  }
+  const int outs = (which == GR_RZ ? 3 * mmax * 6 * mmax : mmax * mmax);
+  e_gram_reduce_kernel<<<dim3((outs + 31) / 32, G.ns), kGramRedThreads, 0, st>>>(G.d_slots, which);
+  count_launch();
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
+}
+
+static int launch_umma_multi(const EGroup& G, int which, cudaStream_t st) {
+  const bool fused = which == UP_XPNEW || which == UP_AXPNEW;
+  const UmmaPlan pl = umma_plan((fused ? 3 : 1) * G.m_max, G.m_max, fused ? 2 : 1, G.m_max, G.m_max);
+  if (!pl.nout_pass) { set_error("tcgen05 update plan does not fit shared memory"); return QDKP_ERR_ARG; }
+  e_update_umma_kernel<<<std::min(G.utiles, G.nsm), kUmmaThreads, pl.bytes, st>>>(
+      G.d_slots, G.ns, which, G.utiles, G.m_max);
+  count_launch();
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
+}
+
+static int launch_update_multi(const EGroup& G, int which, cudaStream_t st) {
+  if (G.hx_ns[0]) {
+    e_update_kernel<double><<<G.row_ctas, kUpdThreads, update_smem_bytes(G.m_max, G.m_max), st>>>(
+        G.d_slots, G.ns, which);
+    count_launch();
+  }
+  if (G.hx_ns[1] && c64_update_tcgen05()) {
+    const int rc = launch_umma_multi(G, which, st);
+    if (rc) return rc;
+  } else if (G.hx_ns[1]) {
+    e_update_kernel<float><<<G.row_ctas, kUpdThreads, update_tf32_smem_bytes(G.m_max, G.m_max), st>>>(
+        G.d_slots, G.ns, which);
+    count_launch();
+  }
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
+}
+
+static int launch_ritz_multi(const EGroup& G, cudaStream_t st) {
+  if (G.hx_ns[0]) {
+    e_ritz_kernel<double><<<G.row_ctas, kUpdThreads, ritz_smem_bytes(G.m_max), st>>>(G.d_slots, G.ns);
+    count_launch();
+  }
+  if (G.hx_ns[1] && c64_update_tcgen05()) {
+    int rc = launch_umma_multi(G, UP_XPNEW, st);
+    if (rc) return rc;
+    rc = launch_umma_multi(G, UP_AXPNEW, st);
+    if (rc) return rc;
+  } else if (G.hx_ns[1]) {
+    e_ritz_kernel<float><<<G.row_ctas, kUpdThreads, ritz_tf32_smem_bytes(G.m_max), st>>>(G.d_slots, G.ns);
+    count_launch();
+  }
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
+}
+
+static bool group_umma(const EGroup& G) { return G.hx_ns[1] && c64_update_tcgen05(); }
+
+#define ETRY(x) do { const int rc_ = (x); if (rc_ != QDKP_OK) return rc_; } while (0)
+
+int launch_decide(const EGroup& G, cudaStream_t st) {
+  if (group_umma(G)) {
+    e_norm_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, G.ns);
+    count_launch();
+  }
+  e_decide_kernel<<<G.ns, kDecideThreads, 0, st>>>(G.d_slots);
+  count_launch();
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
+}
+
+int launch_residual_block(const EGroup& G, cudaStream_t st) {
+  e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, G.ns, RW_COPYBEST);
+  e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, G.ns, RW_RESID);
+  count_launch(2);
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
+}
+
+int launch_project(const EGroup& G, cudaStream_t st) {
+  if (group_umma(G)) {
+    e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, G.ns, RW_GATHERP);
+    count_launch();
+  }
+  ETRY(launch_gram_multi(G, GR_XR, st));
+  ETRY(launch_update_multi(G, UP_RPROJ, st));
+  ETRY(launch_gram_multi(G, GR_RR, st));
+  e_rchol_kernel<<<G.ns, kSmallThreads, 2 * (size_t)G.m_max * G.m_max * sizeof(double2), st>>>(G.d_slots);
+  count_launch();
+  return launch_update_multi(G, UP_RNORM, st);
+}
+
+int launch_ritz_step(const EGroup& G, cudaStream_t st) {
+  ETRY(launch_gram_multi(G, GR_PP, st));
+  e_pchol_kernel<<<G.ns, kSmallThreads, 2 * (size_t)G.m_max * G.m_max * sizeof(double2), st>>>(G.d_slots);
+  count_launch();
+  ETRY(launch_update_multi(G, UP_PNORM, st));
+  ETRY(launch_update_multi(G, UP_APNORM, st));
+  ETRY(launch_gram_multi(G, GR_RZ, st));
+  const size_t rr_smem = 2 * (size_t)(3 * G.m_max) * (3 * G.m_max) * sizeof(double2);
+  e_rr_kernel<<<G.ns, kSmallThreads, rr_smem, st>>>(G.d_slots, !group_umma(G));
+  count_launch();
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return launch_ritz_multi(G, st);
+}
+
+void set_slot_kernel_limits() {
+  const int big = 200 * 1024;
+  cudaFuncSetAttribute(e_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramMaxSmem);
+  cudaFuncSetAttribute(e_update_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_update_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_ritz_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_ritz_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_update_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       kUmmaSmemLimit);
+  cudaFuncSetAttribute(e_rr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_rchol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_pchol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+}
+
 namespace {
 
 struct SlotHost {
@@ -580,44 +784,12 @@ struct SlotHost {
   int64_t applies = 0;
 };
 
-size_t align256(size_t b) { return (b + 255) / 256 * 256; }
-
-struct SlotLayout {
-  size_t blk, small, npart, gpart, total;
-  int nparts, gparts;
-};
-
-SlotLayout slot_layout(int64_t n, int m, int prec) {
-  SlotLayout L;
-  L.blk = align256((size_t)n * m * (prec == QDKP_C64 ? sizeof(float2) : sizeof(double2)));
-  L.small = align256((size_t)(3 * m) * (3 * m) * sizeof(double2));
-  L.nparts = (int)((n + kERowsPerCta - 1) / kERowsPerCta);
-  L.npart = align256((size_t)L.nparts * m * sizeof(double));
-  L.gparts = gram_parts(n);
-  // the widest task: 3 m x 6 m columns (explicit Gram matrices)
-  L.gpart = align256(gram_partial_elems(3 * m, 6 * m) * sizeof(double2));
-  L.total = align256(sizeof(EState)) + 10 * L.blk + 14 * L.small +
-            align256(3 * m * sizeof(double)) + L.npart + L.gpart;
-  return L;
-}
-
 // The used slots are split into up to kEGroups groups whose ticks run on streams of their own:
 // the groups share no data, so while one group is in its latency-bound kernels (the
 // Rayleigh-Ritz eigensolve and the small Cholesky, reduction and decision kernels, one CTA per
 // slot) the other group's tall kernels fill the GPU. A slot's kernels and partitions are the
 // same in any group, so grouping changes no result.
 constexpr int kEGroups = 2;
-
-struct EGroup {
-  ESlot* d_slots = nullptr;            // this group's run of the compact slot array
-  HXSlot* d_hx = nullptr;              // [precision][phase][slot]: 2 x 4 x max_slots descriptors
-  int ns = 0, gram_ctas = 0, row_ctas = 0;
-  int utiles = 0;                      // 128-row tiles of the complex64 slots (tcgen05 updates)
-  int nsm = 148;
-  int hx_ns[2] = {0, 0}, hx_tiles[2] = {0, 0};   // per precision (QDKP_C128, QDKP_C64)
-  int m_max = 1;
-  std::vector<int> widths;             // distinct block widths among the group's slots
-};
 
 }  // namespace
 }  // namespace qdkp
@@ -805,75 +977,6 @@ int rebuild(qdkp_engine* e, cudaStream_t st) {
   return QDKP_OK;
 }
 
-int launch_gram_multi(const EGroup& G, int which, cudaStream_t st) {
-  int mmax = 0;
-  for (int m : G.widths) {
-    // the warps for the product at full width; panels for the most rectangles any active width and
-    // either pencil can form (the CTAs of panels that stay empty return at once)
-    const int P = which == GR_RZ ? 3 * m : m, Q = P, tc = which == GR_RZ ? 6 * m : 2 * m;
-    const int kind = which == GR_XR ? GK_FULL : (which == GR_RZ ? GK_PENCIL : GK_HERM);
-    const GramShape sh = gram_shape(kind, P, Q, m, m, m);
-    const int most = (P + kGramRect - 1) / kGramRect * (((which == GR_RZ ? 6 * m : m) + kGramRect - 1) / kGramRect);
-    const size_t smem = std::max(gram_smem<double>(tc, sh.warps), gram_smem<float>(tc, sh.warps));
-    e_gram_kernel<<<dim3(G.gram_ctas, (most + sh.warps - 1) / sh.warps), 32 * (sh.warps + 1), smem, st>>>(
-        G.d_slots, G.ns, which, m);
-    count_launch();
-    mmax = std::max(mmax, m);
-  }
-  const int outs = (which == GR_RZ ? 3 * mmax * 6 * mmax : mmax * mmax);
-  e_gram_reduce_kernel<<<dim3((outs + 31) / 32, G.ns), kGramRedThreads, 0, st>>>(G.d_slots, which);
-  count_launch();
-  QDKP_CUDA_TRY(cudaGetLastError());
-  return QDKP_OK;
-}
-
-int launch_umma_multi(const EGroup& G, int which, cudaStream_t st) {
-  const bool fused = which == UP_XPNEW || which == UP_AXPNEW;
-  const UmmaPlan pl = umma_plan((fused ? 3 : 1) * G.m_max, G.m_max, fused ? 2 : 1, G.m_max, G.m_max);
-  if (!pl.nout_pass) { set_error("tcgen05 update plan does not fit shared memory"); return QDKP_ERR_ARG; }
-  e_update_umma_kernel<<<std::min(G.utiles, G.nsm), kUmmaThreads, pl.bytes, st>>>(
-      G.d_slots, G.ns, which, G.utiles, G.m_max);
-  count_launch();
-  QDKP_CUDA_TRY(cudaGetLastError());
-  return QDKP_OK;
-}
-
-int launch_update_multi(const EGroup& G, int which, cudaStream_t st) {
-  if (G.hx_ns[0]) {
-    e_update_kernel<double><<<G.row_ctas, kUpdThreads, update_smem_bytes(G.m_max, G.m_max), st>>>(
-        G.d_slots, G.ns, which);
-    count_launch();
-  }
-  if (G.hx_ns[1] && c64_update_tcgen05()) {
-    const int rc = launch_umma_multi(G, which, st);
-    if (rc) return rc;
-  } else if (G.hx_ns[1]) {
-    e_update_kernel<float><<<G.row_ctas, kUpdThreads, update_tf32_smem_bytes(G.m_max, G.m_max), st>>>(
-        G.d_slots, G.ns, which);
-    count_launch();
-  }
-  QDKP_CUDA_TRY(cudaGetLastError());
-  return QDKP_OK;
-}
-
-int launch_ritz_multi(const EGroup& G, cudaStream_t st) {
-  if (G.hx_ns[0]) {
-    e_ritz_kernel<double><<<G.row_ctas, kUpdThreads, ritz_smem_bytes(G.m_max), st>>>(G.d_slots, G.ns);
-    count_launch();
-  }
-  if (G.hx_ns[1] && c64_update_tcgen05()) {
-    int rc = launch_umma_multi(G, UP_XPNEW, st);
-    if (rc) return rc;
-    rc = launch_umma_multi(G, UP_AXPNEW, st);
-    if (rc) return rc;
-  } else if (G.hx_ns[1]) {
-    e_ritz_kernel<float><<<G.row_ctas, kUpdThreads, ritz_tf32_smem_bytes(G.m_max), st>>>(G.d_slots, G.ns);
-    count_launch();
-  }
-  QDKP_CUDA_TRY(cudaGetLastError());
-  return QDKP_OK;
-}
-
 // one H.X phase of a tick: a multi-slot launch per precision present
 int launch_hx_phase(const qdkp_engine* e, const EGroup& G, int phase, cudaStream_t st) {
   for (int pi = 0; pi < 2; ++pi) {
@@ -887,48 +990,15 @@ int launch_hx_phase(const qdkp_engine* e, const EGroup& G, int phase, cudaStream
 
 // one LOBPCG iteration of every running slot of group G
 int tick(const qdkp_engine* e, const EGroup& G, cudaStream_t st) {
-  const int ns = G.ns;
-  if (!ns) return QDKP_OK;
-  int rc;
-#define ETRY(x) do { rc = (x); if (rc != QDKP_OK) return rc; } while (0)
-  const size_t small_smem = 2 * (size_t)G.m_max * G.m_max * sizeof(double2);
-  const size_t rr_smem = 2 * (size_t)(3 * G.m_max) * (3 * G.m_max) * sizeof(double2);
-  const bool umma = G.hx_ns[1] && c64_update_tcgen05();
-  if (umma) {
-    e_norm_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, ns);
-    count_launch();
-  }
-  e_decide_kernel<<<ns, kDecideThreads, 0, st>>>(G.d_slots);
-  e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, ns, RW_COPYBEST);
-  e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, ns, RW_RESID);
-  count_launch(3);
-  QDKP_CUDA_TRY(cudaGetLastError());
+  if (!G.ns) return QDKP_OK;
+  ETRY(launch_decide(G, st));
+  ETRY(launch_residual_block(G, st));
   ETRY(launch_hx_phase(e, G, 0, st));
   ETRY(launch_hx_phase(e, G, 1, st));
-  if (umma) {
-    e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, ns, RW_GATHERP);
-    count_launch();
-  }
-  ETRY(launch_gram_multi(G, GR_XR, st));
-  ETRY(launch_update_multi(G, UP_RPROJ, st));
-  ETRY(launch_gram_multi(G, GR_RR, st));
-  e_rchol_kernel<<<ns, kSmallThreads, small_smem, st>>>(G.d_slots);
-  count_launch();
-  ETRY(launch_update_multi(G, UP_RNORM, st));
+  ETRY(launch_project(G, st));
   ETRY(launch_hx_phase(e, G, 2, st));
   ETRY(launch_hx_phase(e, G, 3, st));
-  ETRY(launch_gram_multi(G, GR_PP, st));
-  e_pchol_kernel<<<ns, kSmallThreads, small_smem, st>>>(G.d_slots);
-  count_launch();
-  ETRY(launch_update_multi(G, UP_PNORM, st));
-  ETRY(launch_update_multi(G, UP_APNORM, st));
-  ETRY(launch_gram_multi(G, GR_RZ, st));
-  e_rr_kernel<<<ns, kSmallThreads, rr_smem, st>>>(G.d_slots, !umma);
-  count_launch();
-  QDKP_CUDA_TRY(cudaGetLastError());
-  ETRY(launch_ritz_multi(G, st));
-#undef ETRY
-  return QDKP_OK;
+  return launch_ritz_step(G, st);
 }
 
 }  // namespace
@@ -1029,18 +1099,7 @@ int qdkp_engine_create(int max_slots, int device, qdkp_engine** out) {
     delete e;
     return QDKP_ERR_CUDA;
   }
-  // dynamic shared memory limits of the engine kernels
-  const int big = 200 * 1024;
-  cudaFuncSetAttribute(e_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramMaxSmem);
-  cudaFuncSetAttribute(e_update_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(e_update_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(e_ritz_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(e_ritz_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(e_update_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       kUmmaSmemLimit);
-  cudaFuncSetAttribute(e_rr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(e_rchol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(e_pchol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  set_slot_kernel_limits();
   *out = e;
   return QDKP_OK;
 }
@@ -1065,7 +1124,7 @@ int qdkp_engine_destroy(qdkp_engine* e) {
 size_t qdkp_engine_slot_workspace_size(const qdkp_operator* op, const qdkp_lobpcg_params* prm) {
   if (!op || !prm || prm->block < 1 || prm->block > kMaxBlock) return 0;
   if (prm->precision != QDKP_C128 && prm->precision != QDKP_C64) return 0;
-  return slot_layout((int64_t)op->n_bands * op->n_sites, prm->block, prm->precision).total;
+  return slot_layout((int64_t)op->n_bands * op->n_sites, prm->block, prm->precision, 10).total;
 }
 
 int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg_params* prm,
@@ -1080,7 +1139,7 @@ int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg
   const int m = prm->block;
   QDKP_CHECK_ARG(n >= 5 * m, "problem too small for LOBPCG");
   QDKP_CHECK_ARG(n * m < (int64_t(1) << 31), "n * block must stay below 2^31 elements");
-  const SlotLayout L = slot_layout(n, m, prm->precision);
+  const SlotLayout L = slot_layout(n, m, prm->precision, 10);
   if (ws_bytes < L.total) { set_error("engine slot workspace too small"); return QDKP_ERR_WORKSPACE; }
   int id = -1;
   for (int i = 0; i < e->max_slots; ++i) if (!e->slots[i].used) { id = i; break; }
@@ -1090,34 +1149,9 @@ int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg
   h = SlotHost();
   h.op = op;
   h.prm = *prm;
-  char* p = static_cast<char*>(ws);
-  auto take = [&](size_t b) { char* r = p; p += align256(b); return r; };
   ESlot& d = h.d;
-  d.st = (EState*)take(sizeof(EState));
-  d.X = (double2*)take(L.blk); d.AX = (double2*)take(L.blk); d.P = (double2*)take(L.blk);
-  d.AP = (double2*)take(L.blk); d.best = (double2*)take(L.blk); d.Ra = (double2*)take(L.blk);
-  d.ARa = (double2*)take(L.blk); d.Pa = (double2*)take(L.blk); d.APa = (double2*)take(L.blk);
-  d.T = (double2*)take(L.blk);
-  d.W = (double2*)take(L.small); d.G = (double2*)take(L.small); d.U = (double2*)take(L.small);
-  d.gS = (double2*)take(L.small); d.gT = (double2*)take(L.small); d.gA = (double2*)take(L.small);
-  d.gB = (double2*)take(L.small); d.E = (double2*)take(L.small);
-  d.scr = (double2*)take(2 * L.small);
-  d.Cx = (double2*)take(L.small); d.Cr = (double2*)take(L.small); d.Cp = (double2*)take(L.small);
-  d.Im = (double2*)take(L.small);
-  d.w = (double*)take(3 * m * sizeof(double));
-  d.npart = (double*)take(L.npart);
-  d.gpart = (double*)take(L.gpart);
+  slot_carve(d, ws, L, n, m, prm->precision, 10);
   h.gpart_doubles = L.gpart / sizeof(double);
-  d.n = n; d.m = m; d.folded = prm->folded;
-  d.prec = prm->precision;
-  d.sqrt_eps = d.prec == QDKP_C64 ? std::sqrt((double)std::numeric_limits<float>::epsilon())
-                                  : std::sqrt(std::numeric_limits<double>::epsilon());
-  d.tol = prm->tol > 0 ? prm->tol : std::sqrt(std::numeric_limits<double>::epsilon()) * (double)n;
-  d.maxiter = prm->maxiter;
-  d.stall_iterations = prm->stall_iterations;
-  d.restart_control = prm->restart_control > 0 ? prm->restart_control : 20;
-  d.nparts = L.nparts; d.gparts = L.gparts;
-  d.rows_per_cta = kERowsPerCta;
   int rc;
 #define ATRY(x) do { rc = (x); if (rc != QDKP_OK) return rc; } while (0)
   // X = orthonormalise(X0) (lobpcg.py:620-630)
@@ -1148,17 +1182,9 @@ int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg
     ATRY(colnorm1(h, d.AX, d.X, d.w, m, d.gpart, st));
     ATRY(read_sync(w.data(), d.w, m * sizeof(double), st));
   }
-  EState s0{};
-  s0.running = nonfinite ? 0 : 1;
-  s0.status = nonfinite ? QDKP_LOBPCG_NONFINITE : QDKP_LOBPCG_MAXITER;
-  s0.iter = -1; s0.idle = 1;
-  s0.ma = m; s0.mp = 0; s0.restart = 1; s0.forced = 0; s0.explicit_gram = 0;
-  s0.best_iter = prm->maxiter; s0.skip_recompute = 1; s0.skip_p = 1; s0.skip_pnorm = 1;
-  s0.smallest = std::numeric_limits<double>::max();
-  for (int j = 0; j < m; ++j) { s0.active[j] = 1; s0.lam[j] = w[j]; }
-  std::vector<double2> Im((size_t)m * m, make_double2(0.0, 0.0));
-  for (int j = 0; j < m; ++j) Im[(size_t)j * m + j] = make_double2(1.0, 0.0);
-  QDKP_CUDA_TRY(cudaMemcpyAsync(d.Im, Im.data(), Im.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
+  EState s0;
+  slot_params(d, s0, prm, w.data());
+  if (nonfinite) { s0.running = 0; s0.status = QDKP_LOBPCG_NONFINITE; }
   QDKP_CUDA_TRY(cudaMemcpyAsync(d.st, &s0, sizeof(EState), cudaMemcpyHostToDevice, st));
   QDKP_CUDA_TRY(cudaStreamSynchronize(st));
 #undef ATRY

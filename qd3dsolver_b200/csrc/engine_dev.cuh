@@ -45,7 +45,7 @@ struct ESlot {
   int stall_iterations;  // > 0: stop once the best mean residual is this many iterations old
   int restart_control;
   double2 *X, *AX, *P, *AP, *best, *Ra, *ARa, *Pa, *APa, *T;
-  double2 *W, *G, *U, *gS, *gT, *gA, *gB, *E, *scr, *Cx, *Cr, *Cp, *Im;
+  double2 *W, *G, *U, *gS, *gT, *gA, *gB, *E, *scr, *Cx, *Cr, *Cp;
   double* w;
   double* npart;        // [nparts][m] residual-norm partials of the current X
   double* gpart;        // Gram partials (real)
@@ -55,6 +55,7 @@ struct ESlot {
   int utile0;           // complex64 slots: first 128-row tile in the group's tcgen05 update space
   int rows_per_cta;     // rows per CTA in the row kernels (gather, update, norms)
   EState* st;
+  EState* snap;         // NULL, or where the decision kernel leaves a copy of st for the host
 };
 
 template <typename T>
