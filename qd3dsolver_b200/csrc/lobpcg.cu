@@ -16,7 +16,7 @@
 // The iteration is the batched engine's (engine.cu), run on a group of one slot: the decisions scipy
 // takes on host scalars are taken on the device, and the host reads them once an iteration, on a
 // second stream while R is being projected, to launch H.X with the active width. (Nine reads and
-// host-side pencils an iteration took 9.6 ms for ten iterations of a 27 x 27 x 27 box, 12 columns;
+// host-side pencils an iteration took 9.6 ms for ten iterations of a 27 x 27 x 22 box, 12 columns;
 // 7.4 ms so.)
 #include <chrono>
 #include <cmath>
