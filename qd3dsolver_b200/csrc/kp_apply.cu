@@ -1275,6 +1275,7 @@ static int pick_tile(const qdkp_operator* op, const void* X, int64_t ldx, int m,
   const double items = (double)op->n_sites * m;
   double best = 3.0 + items * (sizeof(T) == 8 ? 1.18e-4 : 0.57e-4);
   int tile = kDirect;
+  if (best <= 3.0 + 2.3) return tile;              // no march takes less than a plane: skip the models
   each_shape<T>([&](int i, auto tag, double plane) {
     using G = typename decltype(tag)::G;
     if (!tma_fits<G>(op, X, ldx, m)) return false;
