@@ -308,10 +308,11 @@ chol_inv_kernel(const double2* __restrict__ G, int n, double2* __restrict__ Uinv
   double2* S1 = ssm + n * n;
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) ssm[e] = G[e];
   __syncthreads();
-  const int fail = block_cholesky_upper(ssm, n);
+  __shared__ double rinv[kMaxSmall];
+  const int fail = rr_cholesky(ssm, n, rinv, 0);
   if (threadIdx.x == 0) *status = fail;
   if (fail) return;
-  block_upper_inverse(ssm, n, S1);
+  rr_upper_inverse(ssm, n, rinv, S1);
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) Uinv[e] = S1[e];
 }
 
@@ -328,12 +329,12 @@ int launch_chol_inv(const double2* G, int n, double2* Uinv, int* status, cudaStr
 
 // w ascending, V columns permuted accordingly; generalized problem through B = U^H U (with
 // 0 < nwant < n only the first nwant pairs are computed).
+template <int CLASS>
 __global__ void __launch_bounds__(kSmallThreads)
 eigh_kernel(const double2* __restrict__ A, const double2* __restrict__ B, int n,
             double* __restrict__ w, double2* __restrict__ Vout, double2* __restrict__ scratch,
             int* __restrict__ status, int nwant) {
-  extern __shared__ double2 esm[];
-  const int st = block_eigh(A, B, n, w, Vout, scratch, esm, esm + n * n, nwant);
+  const int st = block_eigh<CLASS>(A, B, n, w, Vout, scratch, nwant);
   if (threadIdx.x == 0) *status = st;
 }
 
@@ -341,9 +342,9 @@ int launch_eigh(const double2* A, const double2* B, int n, double* w, double2* V
                 double2* scratch, int* status, cudaStream_t st, int nwant) {
   if (n < 1 || n > kMaxSmall) { set_error("eigh dimension out of range"); return QDKP_ERR_ARG; }
   const size_t smem = 2 * (size_t)n * n * sizeof(double2);
-  QDKP_CUDA_TRY(cudaFuncSetAttribute(eigh_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
-  eigh_kernel<<<1, kSmallThreads, smem, st>>>(A, B, n, w, V, scratch, status, nwant);
+  const auto kernel = rr_class(n) == 0 ? eigh_kernel<0> : (rr_class(n) == 1 ? eigh_kernel<1> : eigh_kernel<2>);
+  QDKP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<1, kSmallThreads, smem, st>>>(A, B, n, w, V, scratch, status, nwant);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;

@@ -7,59 +7,6 @@
 
 namespace qdkp {
 
-// In-place upper Cholesky of the Hermitian matrix in S (n x n, ld n): S = U^H U, U in the upper
-// triangle. Returns nonzero (block-uniform) if a pivot is not positive and finite.
-static __device__ int block_cholesky_upper(double2* S, int n) {
-  __shared__ int fail;
-  if (threadIdx.x == 0) fail = 0;
-  __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    if (threadIdx.x == 0) {
-      const double d = S[k * n + k].x;
-      if (!(d > 0.0) || !isfinite(d)) fail = 1;
-      else S[k * n + k] = make_double2(sqrt(d), 0.0);
-    }
-    __syncthreads();
-    if (fail) break;
-    const double piv = S[k * n + k].x;
-    for (int j = k + 1 + threadIdx.x; j < n; j += blockDim.x) {
-      S[k * n + j].x /= piv;
-      S[k * n + j].y /= piv;
-    }
-    __syncthreads();
-    const int w = n - k - 1;
-    for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
-      const int i = k + 1 + e / w, j = k + 1 + e % w;
-      if (j >= i) {
-        const double2 a = S[k * n + i], b = S[k * n + j];
-        // S[i][j] -= conj(a) * b
-        S[i * n + j].x -= a.x * b.x + a.y * b.y;
-        S[i * n + j].y -= a.x * b.y - a.y * b.x;
-      }
-    }
-    __syncthreads();
-  }
-  __syncthreads();
-  return fail;
-}
-
-// Uinv = inv(U) for the upper triangle of S; written to `out` (ld n), one column per thread.
-static __device__ void block_upper_inverse(const double2* S, int n, double2* out) {
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    for (int i = n - 1; i > j; --i) out[i * n + j] = make_double2(0.0, 0.0);
-    const double2 ujj = S[j * n + j];
-    out[j * n + j] = make_double2(1.0 / ujj.x, 0.0);
-    for (int i = j - 1; i >= 0; --i) {
-      double2 s = make_double2(0.0, 0.0);
-      for (int k = i + 1; k <= j; ++k) cfma(s, S[i * n + k], out[k * n + j]);
-      const double d = S[i * n + i].x;
-      out[i * n + j] = make_double2(-s.x / d, -s.y / d);
-    }
-  }
-  __syncthreads();
-}
-
-
 // Eigen-decomposition of the Hermitian C in S0 (n x n, shared memory), with S1 = I on entry:
 // Householder reduction to tridiagonal form (C <- H C H, Q <- Q H, H = I - tau v v^H, one column
 // per step), a diagonal phase that makes the sub-diagonal real, and the implicit QL iteration
@@ -275,8 +222,9 @@ __device__ __forceinline__ double start_value(int i, int j) {
 }
 
 struct RrShared {
-  double td[kMaxSmall], tb[kMaxSmall], e2[kMaxSmall], tau[kMaxSmall], rinv[kMaxSmall];
+  double td[kMaxSmall], tb[kMaxSmall], tau[kMaxSmall], rinv[kMaxSmall];
   double lam[kMaxSmall];
+  double ds[kMaxSmall], es[kMaxSmall];       // the tridiagonal scaled for the Sturm counts
   double2 esub[kMaxSmall], ph[kMaxSmall], xcol[kMaxSmall], psm[kMaxSmall];
   double G[kMaxBlock * kMaxBlock];
   double lo, hi;
@@ -285,10 +233,33 @@ struct RrShared {
 
 // Upper Cholesky B = U^H U in place (S, ld n), one barrier per column: step k subtracts
 // conj(S_ki) S_kj / S_kk from S_ij (k < i <= j) with the unscaled pivot row; the rows are scaled
-// by 1 / sqrt(S_kk) at the end. rinv = 1 / U_kk. Returns nonzero on a bad pivot.
-static __device__ int rr_cholesky(double2* __restrict__ S, int n, double* __restrict__ rinv) {
+// by 1 / sqrt(S_kk) at the end. rinv = 1 / U_kk. Returns nonzero on a bad pivot. The leading k0
+// columns are the identity's (S = [I V; V^H W] with V of k0 rows): their steps touch the trailing
+// block alone and are taken together, four lanes an entry.
+static __device__ int rr_cholesky(double2* __restrict__ S, int n, double* __restrict__ rinv, int k0) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwp = blockDim.x >> 5;
-  for (int k = 0; k < n; ++k) {
+  if (k0) {
+    const int np = n - k0;
+    for (int e0 = 0; e0 < np * np; e0 += blockDim.x / 4) {
+      const int e = e0 + (threadIdx.x >> 2), i = k0 + e / np, j = k0 + e % np;
+      const bool in = e < np * np && i <= j;
+      double sx = 0.0, sy = 0.0;
+      if (in)
+        for (int k = threadIdx.x & 3; k < k0; k += 4) {
+          const double2 a = S[k * n + i], b = S[k * n + j];
+          sx += a.x * b.x + a.y * b.y;
+          sy += a.x * b.y - a.y * b.x;
+        }
+      for (int o = 1; o < 4; o <<= 1) {
+        sx += __shfl_xor_sync(0xffffffffu, sx, o);
+        sy += __shfl_xor_sync(0xffffffffu, sy, o);
+      }
+      if (in && (threadIdx.x & 3) == 0) { S[i * n + j].x -= sx; S[i * n + j].y -= sy; }
+    }
+    __syncthreads();
+  }
+#pragma unroll 1
+  for (int k = k0; k < n; ++k) {
     const double d = S[k * n + k].x;
     if (!(d > 0.0) || !isfinite(d)) { __syncthreads(); return 1; }
     const double inv = 1.0 / d;
@@ -306,7 +277,7 @@ static __device__ int rr_cholesky(double2* __restrict__ S, int n, double* __rest
   }
   for (int k = threadIdx.x; k < n; k += blockDim.x) rinv[k] = 1.0 / sqrt(S[k * n + k].x);
   __syncthreads();
-  for (int i = warp; i < n; i += nwp)
+  for (int i = k0 + warp; i < n; i += nwp)
     for (int j = i + lane; j < n; j += 32) {
       const double r = rinv[i];
       if (j == i) S[i * n + j] = make_double2(1.0 / r, 0.0);
@@ -314,6 +285,42 @@ static __device__ int rr_cholesky(double2* __restrict__ S, int n, double* __rest
     }
   __syncthreads();
   return 0;
+}
+
+// U^-1 of the upper triangle of S (pivots as reciprocals rinv) into out (ld n, zero below the diagonal):
+// a warp per column, the column in registers (lane l holds rows l + 32 q), by back substitution
+static __device__ void rr_upper_inverse(const double2* __restrict__ S, int n, const double* __restrict__ rinv,
+                                        double2* __restrict__ out) {
+  constexpr int CC = (kMaxSmall + 31) / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwp = blockDim.x >> 5;
+  for (int j = warp; j < n; j += nwp) {
+    double2 y[CC];
+#pragma unroll
+    for (int q = 0; q < CC; ++q) y[q] = make_double2(lane + 32 * q == j ? 1.0 : 0.0, 0.0);
+#pragma unroll 1
+    for (int k = j; k >= 0; --k) {
+      double2 yk = y[0];
+#pragma unroll
+      for (int q = 1; q < CC; ++q) if (k >> 5 == q) yk = y[q];
+      const double r = rinv[k];
+      const double2 xk = make_double2(__shfl_sync(0xffffffffu, yk.x, k & 31) * r,
+                                      __shfl_sync(0xffffffffu, yk.y, k & 31) * r);
+#pragma unroll
+      for (int q = 0; q < CC; ++q) {
+        const int i = lane + 32 * q;
+        if (i == k) y[q] = xk;
+        const double2 u = i < k ? S[i * n + k] : make_double2(0.0, 0.0);
+        y[q].x -= u.x * xk.x - u.y * xk.y;
+        y[q].y -= u.x * xk.y + u.y * xk.x;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < CC; ++q) {
+      const int i = lane + 32 * q;
+      if (i < n) out[i * n + j] = y[q];
+    }
+  }
+  __syncthreads();
 }
 
 // Rows of A (ld n) times U^-1 (U upper, pivots as reciprocals rinv): a warp per row (rows
@@ -370,195 +377,271 @@ static __device__ void rr_rows_solve(double2* __restrict__ A, const double2* __r
   __syncthreads();
 }
 
-// Householder tridiagonalisation of the Hermitian part of Csm (read once), held in registers:
-// warp w owns rows w + 16 r, lane l columns l + 32 q. Step k forms the reflector
-// H = I - tau v v^H (v^H v = 2 / tau) from column k in every warp (identical butterfly sums),
+// rr_rows_solve with U = [I V; 0 U'] (k0 identity rows, n - k0 <= 32): rows a of A become
+// [a_1 | (a_2 - a_1 V) U'^-1], in place; row i's entry j stands at A[i si + j sj], and with CONJ the
+// rows are those of A^T and U is conjugated (A <- U^-H A).
+template <bool CONJ>
+static __device__ void rr_rows_solve_tail(double2* __restrict__ A, int si, int sj, const double2* __restrict__ U,
+                                          int n, const double* __restrict__ rinv, int k0) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, np = n - k0;
+  for (int e = threadIdx.x; e < n * np; e += blockDim.x) {
+    const int i = e / np, j = k0 + e - i * np;
+    double rx = 0.0, ry = 0.0, ix = 0.0, iy = 0.0;          // four chains of FMAs
+#pragma unroll 4
+    for (int k = 0; k < k0; ++k) {
+      const double2 a = A[i * si + k * sj];
+      double2 u = U[k * n + j];
+      if (CONJ) u.y = -u.y;
+      rx = fma(a.x, u.x, rx); ry = fma(a.y, u.y, ry);
+      ix = fma(a.x, u.y, ix); iy = fma(a.y, u.x, iy);
+    }
+    double2 t = A[i * si + j * sj];
+    t.x -= rx - ry;
+    t.y -= ix + iy;
+    A[i * si + j * sj] = t;
+  }
+  __syncthreads();
+  for (int i0 = 0; i0 < n; i0 += 3 * kRrWarps) {
+    double2 a[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const int i = i0 + warp + kRrWarps * r;
+      a[r] = i < n && lane < np ? A[i * si + (k0 + lane) * sj] : make_double2(0.0, 0.0);
+    }
+    for (int k = 0; k < np; ++k) {
+      const double rk = rinv[k0 + k];
+      double2 u = lane > k && lane < np ? U[(k0 + k) * n + k0 + lane] : make_double2(0.0, 0.0);
+      if (CONJ) u.y = -u.y;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const double wx = __shfl_sync(0xffffffffu, a[r].x, k) * rk, wy = __shfl_sync(0xffffffffu, a[r].y, k) * rk;
+        if (lane == k) a[r] = make_double2(wx, wy);
+        a[r].x -= wx * u.x - wy * u.y;
+        a[r].y -= wx * u.y + wy * u.x;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const int i = i0 + warp + kRrWarps * r;
+      if (i < n && lane < np) A[i * si + (k0 + lane) * sj] = a[r];
+    }
+  }
+  __syncthreads();
+}
+
+// sum over aligned groups of L lanes
+template <int L>
+__device__ __forceinline__ double group_sum(double v) {
+#pragma unroll
+  for (int o = 1; o < L; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Householder tridiagonalisation of the Hermitian part of Csm (read once), held in registers: L
+// lanes a row, lane c columns c + L q, rows (thread / L) + RP r. Step k forms the reflector
+// H = I - tau v v^H (v^H v = 2 / tau) from column k in every group (identical butterfly sums),
 // p = tau C v row-wise, K = tau / 2 v^H p, w = p - K v and C <- C - v w^H - w v^H; two barriers
-// per column. Reflector k (v_j, j > k) is stored in row n - 1 - k of Rf's strict lower triangle
-// (v_j at column j - k - 1), tau_k in sh.tau. On return sh.td / sh.tb / sh.e2 hold the real
+// per column; warps whose rows are reduced already, or past n, only wait. A step is a chain of
+// three sums, a reciprocal and a root: eight lanes a row leave three shuffles a sum and a matrix of
+// 36 fills nine warps without padding columns (a warp a row: five shuffles, twice the FMAs). Above 64
+// the rows of eight lanes would not fit the registers: sixteen.
+// Reflector k (v_j, j > k) is stored in row n - 1 - k of Rf's strict lower triangle
+// (v_j at column j - k - 1), tau_k in sh.tau. On return sh.td / sh.tb hold the real
 // tridiagonal T = D^H (Q^H C Q) D, sh.ph the phases D (the off-diagonal made real and >= 0).
-template <int R, int CC>
+template <int L, int R, int Q>
 static __device__ void rr_tridiag(const double2* __restrict__ Csm, int n,
                                   double2* __restrict__ Rf, RrShared& sh) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double2 c[R][CC];
+  constexpr int RW = 32 / L, RP = RW * kRrWarps;   // rows of a warp, and of the block, a round
+  const int c = threadIdx.x % L, row0 = threadIdx.x / L;
+  double2 a[R][Q];
 #pragma unroll
   for (int r = 0; r < R; ++r)
 #pragma unroll
-    for (int q = 0; q < CC; ++q) {
-      const int i = warp + kRrWarps * r, j = lane + 32 * q;
+    for (int q = 0; q < Q; ++q) {
+      const int i = row0 + RP * r, j = c + L * q;
       if (i < n && j < n) {
-        const double2 a = Csm[i * n + j], b = Csm[j * n + i];
-        c[r][q] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y));
+        const double2 u = Csm[i * n + j], v = Csm[j * n + i];
+        a[r][q] = make_double2(0.5 * (u.x + v.x), 0.5 * (u.y - v.y));
       } else {
-        c[r][q] = make_double2(0.0, 0.0);
+        a[r][q] = make_double2(0.0, 0.0);
       }
     }
-  if (warp == 0)                                   // column 0 is row 0 conjugated
+  if (row0 == 0)                                   // column 0 is row 0 conjugated
 #pragma unroll
-    for (int q = 0; q < CC; ++q) {
-      const int j = lane + 32 * q;
-      if (j < n) sh.xcol[j] = j > 0 ? make_double2(c[0][q].x, -c[0][q].y) : make_double2(0.0, 0.0);
+    for (int q = 0; q < Q; ++q) {
+      const int j = c + L * q;
+      if (j < n) sh.xcol[j] = j > 0 ? make_double2(a[0][q].x, -a[0][q].y) : make_double2(0.0, 0.0);
     }
   __syncthreads();
+  int wlast = -1;                                  // the warp's last row of the matrix, about
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (RW * warp + RP * r < n) wlast = RW * warp + RP * r + RW - 1;
   for (int k = 0; k + 2 < n; ++k) {
+    const bool live = wlast >= k;                  // uniform over the warp
     const int j0 = k + 1;
-    double2 vs[CC];
-    double nx2 = 0.0;
+    double2 vs[Q], vr[R], pr[R];
+    double tau = 0.0;
+    if (live) {
+      double n0 = 0.0, n1 = 0.0;
 #pragma unroll
-    for (int q = 0; q < CC; ++q) {
-      const int j = lane + 32 * q;
-      vs[q] = (j > k && j < n) ? sh.xcol[j] : make_double2(0.0, 0.0);
-      nx2 += vs[q].x * vs[q].x + vs[q].y * vs[q].y;
-    }
-    nx2 = warp_sum(nx2);
-    const double2 x0 = sh.xcol[j0];
-    const double ax0 = sqrt(x0.x * x0.x + x0.y * x0.y);
-    const double nx = sqrt(nx2);
-    // alpha = -phase(x0) |x|, v = x - alpha e_1
-    const double2 phs = ax0 > 0.0 ? make_double2(x0.x / ax0, x0.y / ax0) : make_double2(1.0, 0.0);
-    // below the smallest normal double the column is left as it is (1 / den would overflow)
-    const double den = nx * (nx + ax0);
-    const double tau = den >= 2.2250738585072014e-308 ? 1.0 / den : 0.0;
-    const double2 v0 = make_double2(x0.x + phs.x * nx, x0.y + phs.y * nx);
-#pragma unroll
-    for (int q = 0; q < CC; ++q)
-      if (lane + 32 * q == j0) vs[q] = v0;
-    double2 vr[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = warp + kRrWarps * r;
-      vr[r] = (i > j0 && i < n) ? sh.xcol[i] : (i == j0 ? v0 : make_double2(0.0, 0.0));
-    }
-    if (warp == 0) {
-#pragma unroll
-      for (int q = 0; q < CC; ++q) {
-        const int j = lane + 32 * q;
-        if (j > k && j < n) Rf[(n - 1 - k) * n + (j - k - 1)] = vs[q];
+      for (int q = 0; q < Q; ++q) {
+        const int j = c + L * q;
+        vs[q] = (j > k && j < n) ? sh.xcol[j] : make_double2(0.0, 0.0);
+        n0 = fma(vs[q].x, vs[q].x, n0);
+        n1 = fma(vs[q].y, vs[q].y, n1);
       }
-      if (lane == 0) sh.tau[k] = tau;
-    }
-    double2 pr[R];
+      const double nx2 = group_sum<L>(n0 + n1);
+      const double2 x0 = sh.xcol[j0];
+      // alpha = -phase(x0) |x|, v = x - alpha e_1
+      const double a2 = x0.x * x0.x + x0.y * x0.y;
+      const double ia = rsqrt(a2), ax0 = a2 > 0.0 ? a2 * ia : 0.0;
+      const double nx = nx2 > 0.0 ? nx2 * rsqrt(nx2) : 0.0;
+      const double2 phs = a2 > 0.0 ? make_double2(x0.x * ia, x0.y * ia) : make_double2(1.0, 0.0);
+      // below the smallest normal double the column is left as it is (1 / den would overflow)
+      const double den = nx * (nx + ax0);
+      tau = den >= 2.2250738585072014e-308 ? 1.0 / den : 0.0;
+      const double2 v0 = make_double2(x0.x + phs.x * nx, x0.y + phs.y * nx);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      double sx = 0.0, sy = 0.0;
-      if (warp + kRrWarps * r >= k)                // rows above k are reduced already
-#pragma unroll
-        for (int q = 0; q < CC; ++q) {
-          sx += c[r][q].x * vs[q].x - c[r][q].y * vs[q].y;
-          sy += c[r][q].x * vs[q].y + c[r][q].y * vs[q].x;
-        }
-      pr[r] = make_double2(sx, sy);
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      pr[r].x = tau * warp_sum(pr[r].x);
-      pr[r].y = tau * warp_sum(pr[r].y);
-    }
-    if (lane == 0)
+      for (int q = 0; q < Q; ++q)
+        if (c + L * q == j0) vs[q] = v0;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        const int i = warp + kRrWarps * r;
-        if (i < n) sh.psm[i] = pr[r];
+        const int i = row0 + RP * r;
+        vr[r] = (i > j0 && i < n) ? sh.xcol[i] : (i == j0 ? v0 : make_double2(0.0, 0.0));
+        double s0 = 0.0, s1 = 0.0, t0 = 0.0, t1 = 0.0;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          s0 = fma(a[r][q].x, vs[q].x, s0); s1 = fma(a[r][q].y, vs[q].y, s1);
+          t0 = fma(a[r][q].x, vs[q].y, t0); t1 = fma(a[r][q].y, vs[q].x, t1);
+        }
+        pr[r] = make_double2(s0 - s1, t0 + t1);
       }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        pr[r].x = tau * group_sum<L>(pr[r].x);
+        pr[r].y = tau * group_sum<L>(pr[r].y);
+        const int i = row0 + RP * r;
+        if (i < k) pr[r] = make_double2(0.0, 0.0);     // reduced already
+        if (c == 0 && i < n) sh.psm[i] = pr[r];
+      }
+    }
     __syncthreads();
-    double2 pc[CC];
-    double s = 0.0;                                // Re v^H p (v^H C v is real)
+    if (live) {
+      // the reflector, kept by the last warp of the matrix (it stays live)
+      if ((n - 1) % RP / RW == warp && lane < L) {
 #pragma unroll
-    for (int q = 0; q < CC; ++q) {
-      const int j = lane + 32 * q;
-      pc[q] = j < n ? sh.psm[j] : make_double2(0.0, 0.0);
-      s += vs[q].x * pc[q].x + vs[q].y * pc[q].y;
-    }
-    const double K = 0.5 * tau * warp_sum(s);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (warp + kRrWarps * r < k) continue;
-      const double2 wi = make_double2(pr[r].x - K * vr[r].x, pr[r].y - K * vr[r].y);
-      const double2 vi = vr[r];
-#pragma unroll
-      for (int q = 0; q < CC; ++q) {
-        const double2 vj = vs[q];
-        const double2 wj = make_double2(pc[q].x - K * vj.x, pc[q].y - K * vj.y);
-        c[r][q].x -= vi.x * wj.x + vi.y * wj.y + wi.x * vj.x + wi.y * vj.y;
-        c[r][q].y -= vi.y * wj.x - vi.x * wj.y + wi.y * vj.x - wi.x * vj.y;
-      }
-    }
-    // row k is final (diagonal and sub-diagonal); row k + 1, conjugated, is the next column
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = warp + kRrWarps * r;
-      if (i == k) {
-#pragma unroll
-        for (int q = 0; q < CC; ++q) {
-          const int j = lane + 32 * q;
-          if (j == k) sh.td[k] = c[r][q].x;
-          if (j == k + 1) sh.esub[k] = make_double2(c[r][q].x, -c[r][q].y);
+        for (int q = 0; q < Q; ++q) {
+          const int j = c + L * q;
+          if (j > k && j < n) Rf[(n - 1 - k) * n + (j - k - 1)] = vs[q];
         }
+        if (lane == 0) sh.tau[k] = tau;
       }
-      if (i == k + 1) {
+      double2 pc[Q];
+      double s0 = 0.0, s1 = 0.0;                   // Re v^H p (v^H C v is real)
 #pragma unroll
-        for (int q = 0; q < CC; ++q) {
-          const int j = lane + 32 * q;
-          if (j < n) sh.xcol[j] = j > k + 1 ? make_double2(c[r][q].x, -c[r][q].y) : make_double2(0.0, 0.0);
+      for (int q = 0; q < Q; ++q) {
+        const int j = c + L * q;
+        pc[q] = (j >= k && j < n) ? sh.psm[j] : make_double2(0.0, 0.0);
+        s0 = fma(vs[q].x, pc[q].x, s0);
+        s1 = fma(vs[q].y, pc[q].y, s1);
+      }
+      const double K = 0.5 * tau * group_sum<L>(s0 + s1);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) pc[q] = make_double2(pc[q].x - K * vs[q].x, pc[q].y - K * vs[q].y);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const double2 wi = make_double2(pr[r].x - K * vr[r].x, pr[r].y - K * vr[r].y);
+        const double2 vi = vr[r];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const double2 vj = vs[q], wj = pc[q];
+          a[r][q].x -= vi.x * wj.x + vi.y * wj.y + wi.x * vj.x + wi.y * vj.y;
+          a[r][q].y -= vi.y * wj.x - vi.x * wj.y + wi.y * vj.x - wi.x * vj.y;
         }
+        // row k is final (diagonal and sub-diagonal); row k + 1, conjugated, is the next column
+        const int i = row0 + RP * r;
+        if (i == k || i == k + 1)
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            const int j = c + L * q;
+            const double2 v = make_double2(a[r][q].x, -a[r][q].y);
+            if (i == k) {
+              if (j == k) sh.td[k] = v.x;
+              if (j == k + 1) sh.esub[k] = v;
+            } else if (j < n) {
+              sh.xcol[j] = j > k + 1 ? v : make_double2(0.0, 0.0);
+            }
+          }
       }
     }
     __syncthreads();
   }
 #pragma unroll
   for (int r = 0; r < R; ++r) {                    // the last two rows
-    const int i = warp + kRrWarps * r;
+    const int i = row0 + RP * r;
 #pragma unroll
-    for (int q = 0; q < CC; ++q) {
-      const int j = lane + 32 * q;
+    for (int q = 0; q < Q; ++q) {
+      const int j = c + L * q;
       if (n >= 2 && i == n - 2) {
-        if (j == n - 2) sh.td[n - 2] = c[r][q].x;
-        if (j == n - 1) sh.esub[n - 2] = make_double2(c[r][q].x, -c[r][q].y);
+        if (j == n - 2) sh.td[n - 2] = a[r][q].x;
+        if (j == n - 1) sh.esub[n - 2] = make_double2(a[r][q].x, -a[r][q].y);
       }
-      if (i == n - 1 && j == n - 1) sh.td[n - 1] = c[r][q].x;
+      if (i == n - 1 && j == n - 1) sh.td[n - 1] = a[r][q].x;
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double2 p = make_double2(1.0, 0.0);
-    for (int i = 0; i < n; ++i) {
-      sh.ph[i] = p;
-      if (i + 1 < n) {
-        const double2 e = sh.esub[i];
-        const double ae = sqrt(e.x * e.x + e.y * e.y);
+  // the off-diagonal's moduli, and its phases' running products (a warp scan)
+  if (warp == 0) {
+    double2 carry = make_double2(1.0, 0.0);
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const int i = i0 + lane;
+      double2 u = make_double2(1.0, 0.0);
+      if (i < n) {
+        double ae = 0.0;
+        if (i + 1 < n) {
+          const double2 e = sh.esub[i];
+          ae = sqrt(e.x * e.x + e.y * e.y);
+          if (ae > 0.0) u = make_double2(e.x / ae, e.y / ae);
+        }
         sh.tb[i] = ae;
-        sh.e2[i] = ae * ae;
-        if (ae > 0.0) p = cmul(p, make_double2(e.x / ae, e.y / ae));
       }
+      for (int o = 1; o < 32; o <<= 1) {
+        const double2 t = make_double2(__shfl_up_sync(0xffffffffu, u.x, o), __shfl_up_sync(0xffffffffu, u.y, o));
+        if (lane >= o) u = cmul(t, u);
+      }
+      u = cmul(carry, u);
+      if (i0 == 0 && lane == 0) sh.ph[0] = make_double2(1.0, 0.0);
+      if (i + 1 < n) sh.ph[i + 1] = u;
+      carry = make_double2(__shfl_sync(0xffffffffu, u.x, 31), __shfl_sync(0xffffffffu, u.y, 31));
     }
-    sh.tb[n - 1] = 0.0;
-    sh.e2[n - 1] = 0.0;
   }
   __syncthreads();
 }
 
 // Eigenvalues of the tridiagonal below x: sign changes of the leading-minor determinants
 // p_{i+1} = (d_i - x) p_i - e_{i-1}^2 p_{i-1} (the Sturm sequence; an FMA per step where the
-// ratio form needs a division), both kept in [2^-600, 2^600] by a common power-of-two scale; a
-// zero is replaced by -2^-300 times its predecessor (a zero pivot counts as negative).
-static __device__ __forceinline__ int rr_sturm(const double* __restrict__ td,
-                                               const double* __restrict__ e2, int n, double x) {
-  const double big = 0x1p600, small = 0x1p-600;
-  double pm = 1.0, p = td[0] - x;
-  if (p == 0.0) p = -0x1p-300;
-  bool neg = p < 0.0;
-  int c = neg;
+// ratio form needs a division). The caller scales T to at most 2 and keeps the e^2 above 2^-120, so
+// that a zero determinant is followed by one of the other sign (it counts once whichever sign it
+// is given) and four steps cannot leave the exponent range: the pair is rescaled by a power of two
+// after every fourth, and the chain is otherwise an FMA a step (signs are counted in integers).
+static __device__ __forceinline__ int rr_sturm(const double* __restrict__ ds,
+                                               const double* __restrict__ es, int n, double x) {
+  double pm = 1.0, p = ds[0] - x;
+  int c = (unsigned)__double2hiint(p) >> 31;
 #pragma unroll 4
   for (int i = 1; i < n; ++i) {
-    double pn = fma(td[i] - x, p, -e2[i - 1] * pm);
-    pn = pn == 0.0 ? -0x1p-300 * p : pn;
-    const double m = fmax(fabs(pn), fabs(p));
-    const double f = m > big ? small : (m < small ? big : 1.0);
-    pm = p * f; p = pn * f;
-    const bool ng = p < 0.0;
-    c += ng != neg;
-    neg = ng;
+    const double pn = fma(ds[i] - x, p, -es[i - 1] * pm);
+    c += (unsigned)(__double2hiint(pn) ^ __double2hiint(p)) >> 31;
+    pm = p;
+    p = pn;
+    if ((i & 3) == 0) {
+      const int e = max(__double2hiint(p) & 0x7ff00000, __double2hiint(pm) & 0x7ff00000);
+      const double f = __hiloint2double(0x7fe00000 - e, 0);
+      p *= f;
+      pm *= f;
+    }
   }
   return c;
 }
@@ -572,25 +655,36 @@ static __device__ __forceinline__ int rr_sturm(const double* __restrict__ td,
 // T - lambda I with partial pivoting, pseudo-random start), orthonormalised by two Cholesky-QR
 // passes; V = U^-1 Q D Z with the reflectors applied in reverse order. Returns 0, 1 (B not
 // positive definite), 2 (non-finite T) or 3 (inverse-iteration vectors not independent: the
-// caller then solves the full problem). S0 / S1: n x n shared matrices.
-template <int R, int CC>
-static __device__ int rr_wanted(const double2* __restrict__ A, const double2* __restrict__ B,
-                                int n, int nwant, double* __restrict__ w,
-                                double2* __restrict__ Vout, double2* S0, double2* S1,
-                                RrShared& sh) {
+// caller then solves the full problem). S0 / S1: n x n shared matrices. The leading k0 columns of
+// B are the identity's. Rows and columns a thread holds: R x CC in rr_rows_solve, RT x QC (L lanes a
+// row) in rr_tridiag. S0 is the kernel's dynamic shared memory.
+extern __shared__ double2 rr_dynamic[];
+template <int R, int CC, int L, int RT, int QC>
+static __device__ __forceinline__ int rr_wanted(const double2* __restrict__ A, const double2* __restrict__ B,
+                                                int k0, int n, int nwant, double* __restrict__ w,
+                                                double2* __restrict__ Vout) {
+  __shared__ RrShared sh;
+  double2 *S0 = rr_dynamic, *S1 = rr_dynamic + n * n;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwp = blockDim.x >> 5;
   const double eps = 1.1102230246251565e-16;
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) S1[e] = A[e];
-  if (B) {
+  if (!B) k0 = n;
+  if (k0 < n) {
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) S0[e] = B[e];
     __syncthreads();
-    if (rr_cholesky(S0, n, sh.rinv)) return 1;
-    rr_rows_solve<R, CC>(S1, S0, n, sh.rinv, true);      // W^H with W = A U^-1
-    rr_rows_solve<R, CC>(S1, S0, n, sh.rinv, false);     // W^H U^-1 = C^H
+    if (n - k0 > 32) k0 = 0;                               // more trailing columns than lanes
+    if (rr_cholesky(S0, n, sh.rinv, k0)) return 1;
+    if (k0) {
+      rr_rows_solve_tail<false>(S1, n, 1, S0, n, sh.rinv, k0);   // W = A U^-1
+      rr_rows_solve_tail<true>(S1, 1, n, S0, n, sh.rinv, k0);    // C = U^-H W
+    } else {
+      rr_rows_solve<R, CC>(S1, S0, n, sh.rinv, true);      // W^H with W = A U^-1
+      rr_rows_solve<R, CC>(S1, S0, n, sh.rinv, false);     // W^H U^-1 = C^H
+    }
   } else {
     __syncthreads();
   }
-  rr_tridiag<R, CC>(S1, n, S0, sh);     // reflectors below S0's diagonal, U above it
+  rr_tridiag<L, RT, QC>(S1, n, S0, sh);    // reflectors below S0's diagonal, U above it
   // ---- Gershgorin bounds ----
   if (warp == 0) {
     double lo = INFINITY, hi = -INFINITY;
@@ -611,6 +705,14 @@ static __device__ int rr_wanted(const double2* __restrict__ A, const double2* __
   __syncthreads();
   if (sh.bad) return 2;
   const double tn = fmax(fabs(sh.lo), fabs(sh.hi));
+  // T scaled by a power of two to at most 2 (an exact scaling) for the Sturm counts
+  const double scale = __hiloint2double(max(0x00100000, 0x7fe00000 - (__double2hiint(tn) & 0x7ff00000)), 0);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double e = sh.tb[i] * scale;
+    sh.ds[i] = sh.td[i] * scale;
+    sh.es[i] = fmax(e * e, 0x1p-120);
+  }
+  __syncthreads();
   // ---- multisection: lanes t of group g evaluate a + (b - a)(t + 1) / (G + 1) ----
   int G = 32;
   while (G > 1 && nwant * G > (int)blockDim.x) G >>= 1;
@@ -619,18 +721,20 @@ static __device__ int rr_wanted(const double2* __restrict__ A, const double2* __
     const int base = lane / G * G;
     const unsigned gmask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u) << base);
     const bool act = g < nwant;
+    const double part = (double)(t + 1) / (double)(G + 1);
     double a = sh.lo, b = sh.hi;
     for (int round = 0; round < 64; ++round) {
       const bool conv = !act || (b - a) <= fmax(2.0 * eps * tn, 4.0 * eps * fmax(fabs(a), fabs(b)));
       if (__all_sync(0xffffffffu, conv)) break;
-      const double x = a + (b - a) * ((double)(t + 1) / (double)(G + 1));
-      const int cnt = rr_sturm(sh.td, sh.e2, n, x);
+      const double x = a + (b - a) * part;
+      const int cnt = rr_sturm(sh.ds, sh.es, n, x * scale);
       const unsigned below = __ballot_sync(0xffffffffu, cnt <= g) & gmask;   // x below lambda_g
-      const int hiT = below ? 31 - __clz(below) - base : -1;
+      const int hiT = below ? 31 - __clz(below) : -1;
       const unsigned above = ~below & gmask;
-      const int loT = above ? __ffs(above) - 1 - base : G;
-      const double na = hiT >= 0 ? a + (b - a) * ((double)(hiT + 1) / (double)(G + 1)) : a;
-      const double nb = loT < G ? a + (b - a) * ((double)(loT + 1) / (double)(G + 1)) : b;
+      const int loT = above ? __ffs(above) - 1 : -1;
+      const double xh = __shfl_sync(0xffffffffu, x, max(hiT, 0)), xl = __shfl_sync(0xffffffffu, x, max(loT, 0));
+      const double na = hiT >= 0 ? xh : a;
+      const double nb = loT >= 0 ? xl : b;
       a = conv ? a : na;
       b = conv ? b : nb;
     }
@@ -642,105 +746,135 @@ static __device__ int rr_wanted(const double2* __restrict__ A, const double2* __
   double* Z = reinterpret_cast<double*>(S1);
   double* ur = Z + zs;                  // 1 / pivot of U's row i
   double* u1 = ur + n * nwant;          // U_{i,i+1}
-  double* u2 = u1 + n * nwant;          // U_{i,i+2} (from row exchanges)
+  double* ll = u1 + n * nwant;          // L's multiplier
   const double tiny = eps * tn + 1e-300;
   if ((int)threadIdx.x < nwant) {
     const int j = threadIdx.x;
     const double mu = sh.lam[j];
-    for (int i = 0; i < n; ++i) Z[i * nwant + j] = start_value(i, j);
-    for (int step = 0; step < 2; ++step) {
-      // forward: factor T - mu I row by row, exchanging rows when the sub-diagonal is larger,
-      // and eliminate the right-hand side alongside
+    // T - mu I factored row by row, rows exchanged when the sub-diagonal is larger (a bit each in sw:
+    // U_{i,i+2} is then the next off-diagonal), and the right-hand side eliminated alongside
+    unsigned sw[(kMaxSmall + 31) / 32] = {};
+    {
       double a = sh.td[0] - mu, bcur = n > 1 ? sh.tb[0] : 0.0;
-      double y = Z[j];
+      double y = start_value(0, j);
+#pragma unroll 1
       for (int i = 0; i + 1 < n; ++i) {
         const double cc = sh.tb[i];
         const double an = sh.td[i + 1] - mu;
         const double bn = i + 2 < n ? sh.tb[i + 1] : 0.0;
-        const double yn = Z[(i + 1) * nwant + j];
-        const bool sw = fabs(a) < fabs(cc);
+        const double yn = start_value(i + 1, j);
+        const bool s = fabs(a) < fabs(cc);
         const double ap = fabs(a) < tiny ? (a < 0.0 ? -tiny : tiny) : a;
-        const double ri = 1.0 / (sw ? cc : ap);
-        const double l = (sw ? a : cc) * ri;
+        const double ri = 1.0 / (s ? cc : ap);
+        const double l = (s ? a : cc) * ri;
         ur[i * nwant + j] = ri;
-        u1[i * nwant + j] = sw ? an : bcur;
-        u2[i * nwant + j] = sw ? bn : 0.0;
-        Z[i * nwant + j] = sw ? yn : y;
-        const double na = sw ? bcur - l * an : an - l * bcur;
-        const double ny = sw ? y - l * yn : yn - l * y;
-        bcur = sw ? -l * bn : bn;
+        u1[i * nwant + j] = s ? an : bcur;
+        ll[i * nwant + j] = l;
+#pragma unroll
+        for (int q = 0; q < (kMaxSmall + 31) / 32; ++q)
+          if (q == i >> 5) sw[q] |= (unsigned)s << (i & 31);
+        Z[i * nwant + j] = s ? yn : y;
+        const double na = s ? bcur - l * an : an - l * bcur;
+        const double ny = s ? y - l * yn : yn - l * y;
+        bcur = s ? -l * bn : bn;
         a = na;
         y = ny;
       }
       const double ap = fabs(a) < tiny ? (a < 0.0 ? -tiny : tiny) : a;
       ur[(n - 1) * nwant + j] = 1.0 / ap;
       u1[(n - 1) * nwant + j] = 0.0;
-      u2[(n - 1) * nwant + j] = 0.0;
       Z[(n - 1) * nwant + j] = y;
+    }
+    auto exchanged = [&](int i) {
+      unsigned w = sw[0];
+#pragma unroll
+      for (int q = 1; q < (kMaxSmall + 31) / 32; ++q) if (q == i >> 5) w = sw[q];
+      return (w >> (i & 31) & 1u) != 0;
+    };
+    for (int step = 0; step < 2; ++step) {
       double x1 = 0.0, x2 = 0.0, mx = 0.0;          // back substitution
+#pragma unroll 2
       for (int i = n - 1; i >= 0; --i) {
-        const double x = (Z[i * nwant + j] - u1[i * nwant + j] * x1 - u2[i * nwant + j] * x2) * ur[i * nwant + j];
+        const double u2 = i + 2 < n && exchanged(i) ? sh.tb[i + 1] : 0.0;
+        const double x = (Z[i * nwant + j] - u2 * x2 - u1[i * nwant + j] * x1) * ur[i * nwant + j];
         Z[i * nwant + j] = x;
         x2 = x1;
         x1 = x;
         mx = fmax(mx, fabs(x));
       }
       const double sc = mx > 0.0 && isfinite(mx) ? 1.0 / mx : 0.0;
-      for (int i = 0; i < n; ++i) Z[i * nwant + j] *= sc;
+      if (step == 1) {
+        for (int i = 0; i < n; ++i) Z[i * nwant + j] *= sc;
+      } else {                                      // the second right-hand side, eliminated
+        double y = Z[j] * sc;
+#pragma unroll 2
+        for (int i = 0; i + 1 < n; ++i) {
+          const double l = ll[i * nwant + j], yn = Z[(i + 1) * nwant + j] * sc;
+          const bool s = exchanged(i);
+          Z[i * nwant + j] = s ? yn : y;
+          y = s ? y - l * yn : yn - l * y;
+        }
+        Z[(n - 1) * nwant + j] = y;
+      }
     }
   }
   __syncthreads();
-  // ---- Cholesky-QR, twice: G = Z^T Z (a thread per entry), G = R^T R (warp 0; the diagonal
-  //      holds 1 / R_kk), Z <- Z R^-1 (a thread per row, the row in registers) ----
-  const int ng = nwant * (nwant + 1) / 2;
+  // ---- Cholesky-QR, twice: G = Z^T Z (a thread per entry), G = R^T R with unscaled rows (row k of R is
+  //      G_k / sqrt(G_kk)), Z <- Z R^-1 (eight lanes a row). The loops stay rolled: unrolled over the
+  //      widest block they ran as fast when their code was cached, and 22 us longer after the tall
+  //      kernels of an iteration had pushed it out of L2 ----
+  double* rs = sh.es;
   for (int pass = 0; pass < 2; ++pass) {
-    for (int e = threadIdx.x; e < ng; e += blockDim.x) {
-      int a = 0, rem = e;
-      while (rem >= nwant - a) { rem -= nwant - a; ++a; }
-      const int b = a + rem;
-      double d = 0.0;
-      for (int i = 0; i < n; ++i) d = fma(Z[i * nwant + a], Z[i * nwant + b], d);
-      sh.G[a * nwant + b] = d;
-      sh.G[b * nwant + a] = d;
+    for (int e = threadIdx.x; e < nwant * nwant; e += blockDim.x) {
+      const int a = e / nwant, b = e - a * nwant;
+      if (b < a) continue;
+      double d0 = 0.0, d1 = 0.0, d2 = 0.0;
+#pragma unroll 1
+      for (int i = 0; i < n; i += 3) {
+        d0 = fma(Z[i * nwant + a], Z[i * nwant + b], d0);
+        if (i + 1 < n) d1 = fma(Z[(i + 1) * nwant + a], Z[(i + 1) * nwant + b], d1);
+        if (i + 2 < n) d2 = fma(Z[(i + 2) * nwant + a], Z[(i + 2) * nwant + b], d2);
+      }
+      sh.G[e] = d0 + d1 + d2;
     }
     __syncthreads();
-    if (warp == 0) {
-      int bad = 0;
+#pragma unroll 1
+    for (int k = 0; k < nwant; ++k) {
+      const double d0 = sh.G[k * nwant + k];
+      // the vectors have max-abs 1 (first pass) or unit norm (second): a pivot this small means
+      // a vector (nearly) in the span of the previous ones
+      if (!(d0 > 1e-10) || !isfinite(d0)) return 3;
+      const double inv = 1.0 / d0;
+      for (int e = threadIdx.x; e < nwant * nwant; e += blockDim.x) {
+        const int a = e / nwant, b = e - a * nwant;
+        if (a > k && b >= a) sh.G[e] -= sh.G[k * nwant + a] * sh.G[k * nwant + b] * inv;
+      }
+      __syncthreads();
+    }
+    if ((int)threadIdx.x < nwant) rs[threadIdx.x] = rsqrt(sh.G[threadIdx.x * (nwant + 1)]);
+    __syncthreads();
+    for (int i0 = 0; i0 < n; i0 += 64) {
+      const int i = i0 + (threadIdx.x >> 3), c = threadIdx.x & 7;
+      constexpr int QZ = kMaxBlock / 8;
+      double z[QZ];
+#pragma unroll
+      for (int q = 0; q < QZ; ++q) z[q] = i < n && c + 8 * q < nwant ? Z[i * nwant + c + 8 * q] : 0.0;
+#pragma unroll 1
       for (int k = 0; k < nwant; ++k) {
-        const double d0 = sh.G[k * nwant + k];
-        __syncwarp();
-        // the vectors have max-abs 1 (first pass) or unit norm (second): a pivot this small means
-        // a vector (nearly) in the span of the previous ones
-        if (!(d0 > 1e-10) || !isfinite(d0)) bad = 1;
-        const double ri = bad ? 0.0 : 1.0 / sqrt(d0);
-        for (int j = k + lane; j < nwant; j += 32) sh.G[k * nwant + j] = j == k ? ri : sh.G[k * nwant + j] * ri;
-        __syncwarp();
-        for (int j = k + 1 + lane; j < nwant; j += 32) {
-          const double gkj = sh.G[k * nwant + j];
-          for (int i = k + 1; i <= j; ++i) sh.G[i * nwant + j] -= sh.G[k * nwant + i] * gkj;
-        }
-        __syncwarp();
-      }
-      if (lane == 0) sh.bad = bad;
-    }
-    __syncthreads();
-    if (sh.bad) return 3;
-    if ((int)threadIdx.x < n) {
-      const int i = threadIdx.x;
-      double z[kMaxBlock];
+        double zk = z[0];
 #pragma unroll
-      for (int k = 0; k < kMaxBlock; ++k) z[k] = k < nwant ? Z[i * nwant + k] : 0.0;
+        for (int q = 1; q < QZ; ++q) if (q == k >> 3) zk = z[q];
+        zk = __shfl_sync(0xffffffffu, zk, (lane & 24) | (k & 7)) * rs[k];
+        const double f = zk * rs[k];
 #pragma unroll
-      for (int k = 0; k < kMaxBlock; ++k) {
-        if (k < nwant) {
-          z[k] *= sh.G[k * nwant + k];
-#pragma unroll
-          for (int jj = k + 1; jj < kMaxBlock; ++jj)
-            if (jj < nwant) z[jj] -= z[k] * sh.G[k * nwant + jj];
+        for (int q = 0; q < QZ; ++q) {
+          const int j = c + 8 * q;
+          if (j == k) z[q] = zk;
+          else if (j > k && j < nwant) z[q] -= f * sh.G[k * nwant + j];
         }
       }
 #pragma unroll
-      for (int k = 0; k < kMaxBlock; ++k) if (k < nwant) Z[i * nwant + k] = z[k];
+      for (int q = 0; q < QZ; ++q) if (i < n && c + 8 * q < nwant) Z[i * nwant + c + 8 * q] = z[q];
     }
     __syncthreads();
   }
@@ -754,6 +888,7 @@ static __device__ int rr_wanted(const double2* __restrict__ A, const double2* __
       const double z = i < n ? Z[i * nwant + j] : 0.0;
       y[q] = i < n ? make_double2(sh.ph[i].x * z, sh.ph[i].y * z) : make_double2(0.0, 0.0);
     }
+#pragma unroll 1
     for (int k = n - 3; k >= 0; --k) {
       const double tk = sh.tau[k];
       const double2* vrow = S0 + (n - 1 - k) * n - (k + 1);   // v_i at vrow[i], i > k
@@ -774,8 +909,9 @@ static __device__ int rr_wanted(const double2* __restrict__ A, const double2* __
         y[q].y -= v[q].x * sy + v[q].y * sx;
       }
     }
-    if (B) {
-      for (int k = n - 1; k >= 0; --k) {
+    if (k0 < n) {
+#pragma unroll 1
+      for (int k = n - 1; k >= k0; --k) {
         const int kl = k & 31, kq = k >> 5;
         double2 yk = y[0];
 #pragma unroll
@@ -808,33 +944,30 @@ static __device__ int rr_wanted(const double2* __restrict__ A, const double2* __
   return 0;
 }
 
+// Sizes of the eigensolve, each a kernel of its own: with all of them in one body the small ones' loops
+// spilled registers (36 rows: 355k clocks for 230k), and as functions they still did.
+__host__ __device__ __forceinline__ int rr_class(int n) { return n <= 40 ? 0 : (n <= 64 ? 1 : 2); }
+
 // rr_wanted when it applies (nwant < n, the inverse-iteration arrays fit S1, 512 threads);
 // returns -1 when it does not apply
-static __device__ int block_eigh_wanted(const double2* __restrict__ A,
-                                        const double2* __restrict__ B, int n, int nwant,
-                                        double* __restrict__ w, double2* __restrict__ Vout,
-                                        double2* S0, double2* S1) {
-  __shared__ RrShared sh;
+template <int CLASS>
+static __device__ __forceinline__ int block_eigh_wanted(const double2* __restrict__ A,
+                                                        const double2* __restrict__ B, int k0, int n, int nwant,
+                                                        double* __restrict__ w, double2* __restrict__ Vout) {
   if (nwant < 1 || nwant >= n || nwant > kMaxBlock || (int)blockDim.x != 32 * kRrWarps ||
       ((n * nwant + 1) & ~1) + 3 * n * nwant > 2 * n * n)
     return -1;
-  if (n <= 48) return rr_wanted<3, 2>(A, B, n, nwant, w, Vout, S0, S1, sh);
-  return rr_wanted<5, 3>(A, B, n, nwant, w, Vout, S0, S1, sh);
+  if (CLASS == 0) return rr_wanted<3, 2, 8, 1, 5>(A, B, k0, n, nwant, w, Vout);
+  if (CLASS == 1) return rr_wanted<4, 2, 8, 1, 8>(A, B, k0, n, nwant, w, Vout);
+  return rr_wanted<5, 3, 16, 3, 5>(A, B, k0, n, nwant, w, Vout);
 }
 
-// w ascending, V columns permuted accordingly; generalized problem through B = U^H U.
-// Returns 0 (ok), 1 (B not positive definite) or 2 (non-finite eigenvalue); block-uniform.
-// S0, S1: n x n shared-memory matrices; scratch: 2 n^2 global elements. With 0 < nwant < n only
-// the nwant smallest pairs are required (w[0..nwant), V's first nwant columns): block_eigh_wanted
-// computes them, the QL path below is taken when it does not apply or its vectors collapse.
-static __device__ int block_eigh(const double2* __restrict__ A, const double2* __restrict__ B,
-                                 int n, double* __restrict__ w, double2* __restrict__ Vout,
-                                 double2* __restrict__ scratch, double2* S0, double2* S1,
-                                 int nwant = 0) {
-  if (nwant > 0 && nwant < n) {
-    const int r = block_eigh_wanted(A, B, n, nwant, w, Vout, S0, S1);
-    if (r == 0 || r == 1) return r;                // else: the full problem below
-  }
+// The full problem by the QL iteration (block_eigh's arguments)
+static __device__ __noinline__ int block_eigh_full(const double2* __restrict__ A,
+                                                   const double2* __restrict__ B, int n,
+                                                   double* __restrict__ w, double2* __restrict__ Vout,
+                                                   double2* __restrict__ scratch) {
+  double2 *S0 = rr_dynamic, *S1 = rr_dynamic + n * n;
   double2* Ug = scratch;           // Uinv (global)
   double2* Tg = scratch + n * n;   // A Uinv (global)
   __shared__ int rank[kMaxSmall];
@@ -842,9 +975,9 @@ static __device__ int block_eigh(const double2* __restrict__ A, const double2* _
   if (B) {
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) S0[e] = B[e];
     __syncthreads();
-    const int fail = block_cholesky_upper(S0, n);
-    if (fail) return 1;
-    block_upper_inverse(S0, n, S1);             // Uinv in shared memory
+    __shared__ double rinv[kMaxSmall];
+    if (rr_cholesky(S0, n, rinv, 0)) return 1;
+    rr_upper_inverse(S0, n, rinv, S1);          // Uinv in shared memory
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) Ug[e] = S1[e];
     // T = A Uinv  (Uinv upper: k <= j), A staged into S0
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) S0[e] = A[e];
@@ -917,7 +1050,22 @@ static __device__ int block_eigh(const double2* __restrict__ A, const double2* _
   return bad ? 2 : 0;
 }
 
-
+// w ascending, V columns permuted accordingly; generalized problem through B = U^H U.
+// Returns 0 (ok), 1 (B not positive definite) or 2 (non-finite eigenvalue); block-uniform.
+// The kernel's dynamic shared memory: two n x n matrices; scratch: 2 n^2 global elements. With
+// 0 < nwant < n only the nwant smallest pairs are required (w[0..nwant), V's first nwant columns):
+// block_eigh_wanted computes them, block_eigh_full is taken when it does not apply or its vectors
+// collapse. The leading k0 columns of B are known to be the identity's. CLASS: rr_class of n or more.
+template <int CLASS>
+static __device__ int block_eigh(const double2* __restrict__ A, const double2* __restrict__ B,
+                                 int n, double* __restrict__ w, double2* __restrict__ Vout,
+                                 double2* __restrict__ scratch, int nwant = 0, int k0 = 0) {
+  if (nwant > 0 && nwant < n) {
+    const int r = block_eigh_wanted<CLASS>(A, B, k0, n, nwant, w, Vout);
+    if (r == 0 || r == 1) return r;                // else: the full problem
+  }
+  return block_eigh_full(A, B, n, w, Vout, scratch);
+}
 
 // ---------------------------------------------------------------------------------------------
 // Block updates of complex128 blocks on the FP64 MMA (mma.sync.m8n8k4.f64): Y' = A' C'' with A'

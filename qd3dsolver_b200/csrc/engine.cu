@@ -229,7 +229,7 @@ __device__ bool gram_task(const ESlot& d, int which, GramTask<T>& t, double2*& o
       add(d.Ra, ma, ma);
       t.P = t.Q = ma; t.kind = GK_HERM; out = d.G;
       return true;
-    case GR_PP:          // all columns; e_pchol_kernel takes the active ones
+    case GR_PP:          // all columns; e_chol_kernel takes the active ones
       add(d.P, m, m);
       t.P = t.Q = m; t.kind = GK_HERM; out = d.G;
       return true;
@@ -448,44 +448,56 @@ e_update_umma_kernel(const ESlot* __restrict__ S, int ns, int which, int utiles,
 // ---------------------------------------------------------------------------------------------
 // per-slot Cholesky steps and Rayleigh-Ritz
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kSmallThreads) e_rchol_kernel(const ESlot* __restrict__ S) {
-  extern __shared__ double2 ssm_e[];
-  const ESlot& d = S[blockIdx.x];
-  EState* st = d.st;
-  if (st->idle) return;
-  const int n = st->ma;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) ssm_e[e] = d.G[e];
-  __syncthreads();
-  const int fail = block_cholesky_upper(ssm_e, n);
-  if (fail) {
-    if (threadIdx.x == 0) { st->running = 0; st->status = QDKP_LOBPCG_RCHOL_BREAKDOWN; st->idle = 1; }
-    return;
+// the sums of a Gram product's parts into the m x m matrix G (upper triangle), by this CTA alone
+template <typename T>
+__device__ void e_small_gram(const ESlot& d, int which, double2* __restrict__ G) {
+  __shared__ GramTask<T> t;
+  if (threadIdx.x == 0) {
+    double2 *o, *oS;
+    gram_task<T>(d, which, t, o, oS);
   }
-  block_upper_inverse(ssm_e, n, ssm_e + n * n);
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) d.U[e] = ssm_e[n * n + e];
+  __syncthreads();
+  gram_reduce_herm(t, d.gparts, d.gpart, G);
 }
 
-__global__ void __launch_bounds__(kSmallThreads) e_pchol_kernel(const ESlot* __restrict__ S) {
+// R^H R (which = GR_RR) or P^H P (GR_PP, of which the active columns are taken) summed, its Cholesky
+// factor, and U^-1 in d.U. One kernel: reduction and factorisation are a launch of latency each (13 us
+// and 15 us at 12 columns).
+template <int WHICH>
+__global__ void __launch_bounds__(kSmallThreads) e_chol_kernel(const ESlot* __restrict__ S) {
   extern __shared__ double2 ssm_e[];
+  __shared__ double rinv[kMaxSmall];
   const ESlot& d = S[blockIdx.x];
   EState* st = d.st;
   if (st->idle) return;
-  const int n = st->ma, m = d.m;
-  if (st->skip_p) {                        // iteration 0: no P yet, restart stays as it is
+  const int n = st->ma, m = WHICH == GR_PP ? d.m : n;
+  if (WHICH == GR_PP && st->skip_p) {      // iteration 0: no P yet, restart stays as it is
     if (threadIdx.x == 0) { st->skip_pnorm = 1; st->mp = st->restart ? 0 : n; }
     return;
   }
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int i = e / n, j = e - i * n;
-    ssm_e[e] = d.G[st->idx[i] * m + st->idx[j]];
+  double2* G = ssm_e;
+  double2* C = ssm_e + d.m * d.m;
+  if (d.prec == QDKP_C64) e_small_gram<float>(d, WHICH, G);
+  else e_small_gram<double>(d, WHICH, G);
+  if (WHICH == GR_PP && n < m) {
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+      const int i = e / n, j = e - i * n;
+      C[e] = G[st->idx[i] * m + st->idx[j]];
+    }
+    __syncthreads();
+    double2* swap = G;
+    G = C;
+    C = swap;
   }
-  __syncthreads();
-  const int fail = block_cholesky_upper(ssm_e, n);
+  const int fail = rr_cholesky(G, n, rinv, 0);
   if (!fail) {
-    block_upper_inverse(ssm_e, n, ssm_e + n * n);
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) d.U[e] = ssm_e[n * n + e];
+    rr_upper_inverse(G, n, rinv, C);
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) d.U[e] = C[e];
   }
-  if (threadIdx.x == 0) {
+  if (threadIdx.x != 0) return;
+  if (WHICH == GR_RR) {
+    if (fail) { st->running = 0; st->status = QDKP_LOBPCG_RCHOL_BREAKDOWN; st->idle = 1; }
+  } else {
     st->skip_pnorm = fail ? 1 : 0;
     st->restart = fail ? 1 : st->forced;
     st->mp = st->restart ? 0 : n;
@@ -534,12 +546,13 @@ __device__ void e_assemble(const ESlot& d, const EState* st, int restart, int& d
   __syncthreads();
 }
 
-// c64_ritz: the Ritz update of complex64 slots is e_ritz_kernel's too
+// c64_ritz: the Ritz update of complex64 slots is e_ritz_kernel's too. One launch per eigensolve size
+// present; a slot's is its own widest pencil's.
+template <int CLASS>
 __global__ void __launch_bounds__(kSmallThreads) e_rr_kernel(const ESlot* __restrict__ S, int c64_ritz) {
-  extern __shared__ double2 rsm[];
   const ESlot& d = S[blockIdx.x];
   EState* st = d.st;
-  if (st->idle) return;
+  if (st->idle || rr_class(3 * d.m) != CLASS) return;
   __shared__ int use_restart, ok, dim_s;
   if (threadIdx.x == 0) { use_restart = st->mp == 0; ok = 0; }
   __syncthreads();
@@ -547,7 +560,9 @@ __global__ void __launch_bounds__(kSmallThreads) e_rr_kernel(const ESlot* __rest
     int dim;
     e_assemble(d, st, use_restart, dim);
     // only the first m Ritz pairs are kept
-    const int r = block_eigh(d.gA, d.gB, dim, d.w, d.E, d.scr, rsm, rsm + dim * dim, d.m);
+    // without the explicit products gramB is the identity on X and R (all of it without P)
+    const int k0 = st->explicit_gram ? 0 : d.m + st->ma;
+    const int r = block_eigh<CLASS>(d.gA, d.gB, dim, d.w, d.E, d.scr, d.m, k0);
     if (threadIdx.x == 0) { ok = r == 0; dim_s = dim; }
     __syncthreads();
     if (ok || use_restart) break;
@@ -655,6 +670,8 @@ static int launch_gram_multi(const EGroup& G, int which, cudaStream_t st) {
     count_launch();
     mmax = std::max(mmax, m);
   }
+  QDKP_CUDA_TRY(cudaGetLastError());
+  if (which == GR_RR || which == GR_PP) return QDKP_OK;      // e_chol_kernel adds the parts
   const int outs = (which == GR_RZ ? 3 * mmax * 6 * mmax : mmax * mmax);
   e_gram_reduce_kernel<<<dim3((outs + 31) / 32, G.ns), kGramRedThreads, 0, st>>>(G.d_slots, which);
   count_launch();
@@ -740,21 +757,26 @@ int launch_project(const EGroup& G, cudaStream_t st) {
   ETRY(launch_gram_multi(G, GR_XR, st));
   ETRY(launch_update_multi(G, UP_RPROJ, st));
   ETRY(launch_gram_multi(G, GR_RR, st));
-  e_rchol_kernel<<<G.ns, kSmallThreads, 2 * (size_t)G.m_max * G.m_max * sizeof(double2), st>>>(G.d_slots);
+  e_chol_kernel<GR_RR><<<G.ns, kSmallThreads, 2 * (size_t)G.m_max * G.m_max * sizeof(double2), st>>>(G.d_slots);
   count_launch();
   return launch_update_multi(G, UP_RNORM, st);
 }
 
 int launch_ritz_step(const EGroup& G, cudaStream_t st) {
   ETRY(launch_gram_multi(G, GR_PP, st));
-  e_pchol_kernel<<<G.ns, kSmallThreads, 2 * (size_t)G.m_max * G.m_max * sizeof(double2), st>>>(G.d_slots);
+  e_chol_kernel<GR_PP><<<G.ns, kSmallThreads, 2 * (size_t)G.m_max * G.m_max * sizeof(double2), st>>>(G.d_slots);
   count_launch();
   ETRY(launch_update_multi(G, UP_PNORM, st));
   ETRY(launch_update_multi(G, UP_APNORM, st));
   ETRY(launch_gram_multi(G, GR_RZ, st));
   const size_t rr_smem = 2 * (size_t)(3 * G.m_max) * (3 * G.m_max) * sizeof(double2);
-  e_rr_kernel<<<G.ns, kSmallThreads, rr_smem, st>>>(G.d_slots, !group_umma(G));
-  count_launch();
+  bool cls[3] = {};
+  for (int m : G.widths) cls[rr_class(3 * m)] = true;
+  const int c64_ritz = !group_umma(G);
+  if (cls[0]) e_rr_kernel<0><<<G.ns, kSmallThreads, rr_smem, st>>>(G.d_slots, c64_ritz);
+  if (cls[1]) e_rr_kernel<1><<<G.ns, kSmallThreads, rr_smem, st>>>(G.d_slots, c64_ritz);
+  if (cls[2]) e_rr_kernel<2><<<G.ns, kSmallThreads, rr_smem, st>>>(G.d_slots, c64_ritz);
+  count_launch(cls[0] + cls[1] + cls[2]);
   QDKP_CUDA_TRY(cudaGetLastError());
   return launch_ritz_multi(G, st);
 }
@@ -768,9 +790,11 @@ void set_slot_kernel_limits() {
   cudaFuncSetAttribute(e_ritz_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(e_update_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        kUmmaSmemLimit);
-  cudaFuncSetAttribute(e_rr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(e_rchol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(e_pchol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_rr_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_rr_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_rr_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_chol_kernel<GR_RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(e_chol_kernel<GR_PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
 }
 
 namespace {

@@ -385,6 +385,62 @@ static __device__ void gram_core(const GramTask<T>& t, int part, int parts, int 
   }
 }
 
+// the entry whose real view's upper left word stands at c, summed over parts [b0, b1) in order: eight
+// parts' loads in flight, the last ones too (a remainder loop would wait for each)
+static __device__ __forceinline__ double2 gram_add_parts(const double* __restrict__ c, long long pstride,
+                                                         int b0, int b1) {
+  double2 s = make_double2(0.0, 0.0);
+  for (int b = b0; b < b1; b += 8) {
+    double2 u[8], v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const double* cq = c + min(b + q, b1 - 1) * pstride;
+      u[q] = __ldcg(reinterpret_cast<const double2*>(cq));
+      v[q] = __ldcg(reinterpret_cast<const double2*>(cq + 24));
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (b + q < b1) {
+        s.x += u[q].x + v[q].y;
+        s.y += u[q].y - v[q].x;
+      }
+  }
+  return s;
+}
+
+// The parts of a GK_HERM task of one block added by one CTA into the upper triangle of G (ld t.P): the
+// threads are dealt to (entry, share of the parts), so that 12 columns' 78 entries keep 468 threads'
+// loads in flight at once.
+template <typename T>
+static __device__ void gram_reduce_herm(const GramTask<T>& t, int parts, const double* __restrict__ partial,
+                                        double2* __restrict__ G) {
+  __shared__ short s_map[kGramMaxRects];
+  __shared__ double2 s_sum[512];
+  int need, index;
+  const int total = gram_enumerate(t, need, index);
+  if (threadIdx.x < kGramMaxRects) s_map[threadIdx.x] = need ? (short)index : (short)-1;
+  __syncthreads();
+  const int m = t.P, gc = (m + kGramRect - 1) / kGramRect, nout = m * (m + 1) / 2;
+  const int shares = min(parts, 512 / nout), ps = (parts + shares - 1) / shares;
+  const int sh = threadIdx.x / nout, o = threadIdx.x - sh * nout;
+  int i = 0, j = o;
+  while (j >= m - i) { j -= m - i; ++i; }
+  j += i;
+  if (sh < shares) {
+    const int k = s_map[(i / kGramRect) * gc + j / kGramRect];
+    s_sum[threadIdx.x] = gram_add_parts(partial + (long long)k * kGramRectElems + 48 * (i % kGramRect) + 2 * (j % kGramRect),
+                                        (long long)total * kGramRectElems, sh * ps, min(parts, (sh + 1) * ps));
+  }
+  __syncthreads();
+  if (sh == 0) {
+    double2 v = s_sum[o];
+    for (int w = 1; w < shares; ++w) { v.x += s_sum[w * nout + o].x; v.y += s_sum[w * nout + o].y; }
+    G[i * m + j] = v;
+  }
+  __syncthreads();
+}
+static_assert(kMaxBlock * (kMaxBlock + 1) / 2 <= 512, "an entry per thread");
+
 // Adds the parts of a task. Output entry (i, j) of the P x Q product goes through put(i, j, value)
 // where its rectangle was formed (GK_HERM: the upper triangle). A CTA of 8 warps takes 32 outputs a
 // round: each warp adds an eighth of the parts in order, then the eighths are added in order.
@@ -410,13 +466,9 @@ static __device__ void gram_reduce_core(const GramTask<T>& t, int parts, const d
     double re = 0.0, im = 0.0;
     if (k >= 0) {
       const double* c = partial + (long long)k * kGramRectElems + (2 * (i % kGramRect)) * 24 + 2 * (j % kGramRect);
-#pragma unroll 8
-      for (int b = b0; b < b1; ++b) {
-        const double2 u = __ldcg(reinterpret_cast<const double2*>(c + b * pstride));
-        const double2 v = __ldcg(reinterpret_cast<const double2*>(c + b * pstride + 24));
-        re += u.x + v.y;
-        im += u.y - v.x;
-      }
+      const double2 v = gram_add_parts(c, pstride, b0, b1);
+      re = v.x;
+      im = v.y;
     }
     s_sum[warp][lane] = make_double2(re, im);
     __syncthreads();
