@@ -333,18 +333,22 @@ template <int CLASS>
 __global__ void __launch_bounds__(kSmallThreads)
 eigh_kernel(const double2* __restrict__ A, const double2* __restrict__ B, int n,
             double* __restrict__ w, double2* __restrict__ Vout, double2* __restrict__ scratch,
-            int* __restrict__ status, int nwant) {
-  const int st = block_eigh<CLASS>(A, B, n, w, Vout, scratch, nwant);
+            int* __restrict__ status, int nwant, int s1) {
+  const int st = block_eigh<CLASS>(A, B, n, w, Vout, scratch, nwant, s1);
   if (threadIdx.x == 0) *status = st;
 }
 
 int launch_eigh(const double2* A, const double2* B, int n, double* w, double2* V,
                 double2* scratch, int* status, cudaStream_t st, int nwant) {
   if (n < 1 || n > kMaxSmall) { set_error("eigh dimension out of range"); return QDKP_ERR_ARG; }
-  const size_t smem = 2 * (size_t)n * n * sizeof(double2);
+  // all pairs of a block's own matrix (the first and the last Rayleigh-Ritz of a solve) by the same
+  // parallel route as a wanted few, with room for its arrays: 12 x 12 105 us by the QL iteration, 55 us so
+  const int want = nwant > 0 && nwant < n ? nwant : n;
+  const int s1 = std::max(2 * n * n, want <= kMaxBlock ? rr_s1_doubles(n, want) : 0);
+  const size_t smem = (size_t)n * n * sizeof(double2) + (size_t)s1 * sizeof(double);
   const auto kernel = rr_class(n) == 0 ? eigh_kernel<0> : (rr_class(n) == 1 ? eigh_kernel<1> : eigh_kernel<2>);
   QDKP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<1, kSmallThreads, smem, st>>>(A, B, n, w, V, scratch, status, nwant);
+  kernel<<<1, kSmallThreads, smem, st>>>(A, B, n, w, V, scratch, status, want, s1);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;

@@ -948,14 +948,20 @@ static __device__ __forceinline__ int rr_wanted(const double2* __restrict__ A, c
 // spilled registers (36 rows: 355k clocks for 230k), and as functions they still did.
 __host__ __device__ __forceinline__ int rr_class(int n) { return n <= 40 ? 0 : (n <= 64 ? 1 : 2); }
 
-// rr_wanted when it applies (nwant < n, the inverse-iteration arrays fit S1, 512 threads);
-// returns -1 when it does not apply
+// doubles that rr_wanted's inverse iteration takes in S1
+__host__ __device__ __forceinline__ int rr_s1_doubles(int n, int nwant) {
+  return ((n * nwant + 1) & ~1) + 3 * n * nwant;
+}
+
+// rr_wanted when it applies (its arrays fit the s1 doubles of S1, 512 threads); returns -1 when it does
+// not
 template <int CLASS>
 static __device__ __forceinline__ int block_eigh_wanted(const double2* __restrict__ A,
                                                         const double2* __restrict__ B, int k0, int n, int nwant,
-                                                        double* __restrict__ w, double2* __restrict__ Vout) {
-  if (nwant < 1 || nwant >= n || nwant > kMaxBlock || (int)blockDim.x != 32 * kRrWarps ||
-      ((n * nwant + 1) & ~1) + 3 * n * nwant > 2 * n * n)
+                                                        int s1, double* __restrict__ w,
+                                                        double2* __restrict__ Vout) {
+  if (nwant < 1 || nwant > n || nwant > kMaxBlock || (int)blockDim.x != 32 * kRrWarps ||
+      rr_s1_doubles(n, nwant) > s1)
     return -1;
   if (CLASS == 0) return rr_wanted<3, 2, 8, 1, 5>(A, B, k0, n, nwant, w, Vout);
   if (CLASS == 1) return rr_wanted<4, 2, 8, 1, 8>(A, B, k0, n, nwant, w, Vout);
@@ -1052,20 +1058,21 @@ static __device__ __noinline__ int block_eigh_full(const double2* __restrict__ A
 
 // w ascending, V columns permuted accordingly; generalized problem through B = U^H U.
 // Returns 0 (ok), 1 (B not positive definite) or 2 (non-finite eigenvalue); block-uniform.
-// The kernel's dynamic shared memory: two n x n matrices; scratch: 2 n^2 global elements. With
-// 0 < nwant < n only the nwant smallest pairs are required (w[0..nwant), V's first nwant columns):
-// block_eigh_wanted computes them, block_eigh_full is taken when it does not apply or its vectors
-// collapse. The leading k0 columns of B are known to be the identity's. CLASS: rr_class of n or more.
+// The kernel's dynamic shared memory: two n x n matrices, the second of s1 >= 2 n^2 doubles; scratch:
+// 2 n^2 global elements. Only the nwant smallest pairs are required (w[0..nwant), V's first nwant
+// columns): block_eigh_wanted computes them, block_eigh_full is taken when it does not apply or its
+// vectors collapse. The leading k0 columns of B are known to be the identity's. CLASS: rr_class of
+// n or more.
 template <int CLASS>
 static __device__ int block_eigh(const double2* __restrict__ A, const double2* __restrict__ B,
                                  int n, double* __restrict__ w, double2* __restrict__ Vout,
-                                 double2* __restrict__ scratch, int nwant = 0, int k0 = 0) {
-  if (nwant > 0 && nwant < n) {
-    const int r = block_eigh_wanted<CLASS>(A, B, k0, n, nwant, w, Vout);
-    if (r == 0 || r == 1) return r;                // else: the full problem
-  }
+                                 double2* __restrict__ scratch, int nwant, int s1, int k0 = 0) {
+  const int r = block_eigh_wanted<CLASS>(A, B, k0, n, nwant, s1, w, Vout);
+  if (r == 0 || r == 1) return r;                  // else: the full problem
   return block_eigh_full(A, B, n, w, Vout, scratch);
 }
+
+
 
 // ---------------------------------------------------------------------------------------------
 // Block updates of complex128 blocks on the FP64 MMA (mma.sync.m8n8k4.f64): Y' = A' C'' with A'

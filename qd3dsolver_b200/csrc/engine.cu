@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(kSmallThreads) e_rr_kernel(const ESlot* __rest
     // only the first m Ritz pairs are kept
     // without the explicit products gramB is the identity on X and R (all of it without P)
     const int k0 = st->explicit_gram ? 0 : d.m + st->ma;
-    const int r = block_eigh<CLASS>(d.gA, d.gB, dim, d.w, d.E, d.scr, d.m, k0);
+    const int r = block_eigh<CLASS>(d.gA, d.gB, dim, d.w, d.E, d.scr, d.m, 2 * dim * dim, k0);
     if (threadIdx.x == 0) { ok = r == 0; dim_s = dim; }
     __syncthreads();
     if (ok || use_restart) break;

@@ -85,3 +85,29 @@ def test_engine_iterates_follow_scipy(phase, m):
     Vh = V.cpu().numpy()
     assert np.abs(Vh.conj().T @ (Ho @ Vh) - np.diag(lam)).max() < bound
     H.close()
+
+
+@pytest.mark.parametrize('kind', ['random', 'pairs', 'diagonal', 'identity', 'zero'])
+@pytest.mark.parametrize('n', [1, 2, 3, 5, 8, 13, 16, 23, 24])
+def test_eigh_all_pairs_of_a_block(n, kind):
+    """All pairs of a matrix of a block's width: the widths the multisection route takes, with spectra
+    that split the tridiagonal (diagonal, identity, zero) and exactly degenerate pairs."""
+    import torch
+    from qd3dsolver_b200 import _lib
+    L = _lib.lib()
+    rng = np.random.default_rng(n)
+    Q, _ = np.linalg.qr(rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)))
+    lam = {'random': rng.uniform(-1, 1, n), 'pairs': np.repeat(np.arange(n // 2 + 1) + 0.5, 2)[:n],
+           'diagonal': rng.uniform(-1, 1, n), 'identity': np.ones(n), 'zero': np.zeros(n)}[kind]
+    A = np.diag(lam).astype(np.complex128) if kind in ('diagonal', 'identity', 'zero') else (Q * lam) @ Q.conj().T
+    A = np.ascontiguousarray((A + A.conj().T) / 2)
+    ws = torch.empty(int(L.qdkp_block_eigh_workspace_size(n)), dtype=torch.uint8, device='cuda')
+    w, V = np.zeros(n), np.zeros((n, n), dtype=np.complex128)
+    _lib.check(L.qdkp_block_eigh(A.ctypes.data, None, n, n, w.ctypes.data, V.ctypes.data, ws.data_ptr(),
+                                 ws.numel(), None), 'qdkp_block_eigh')
+    # a backward-stable eigensolve: a modest multiple of n rounding units of the norm
+    tol = 50 * n * np.finfo(float).eps * max(1.0, np.abs(lam).max())
+    assert np.all(np.diff(w) >= 0)
+    assert np.abs(w - np.sort(lam)).max() <= tol
+    assert np.abs(A @ V - V * w).max() <= tol
+    assert np.abs(V.conj().T @ V - np.eye(n)).max() <= tol
