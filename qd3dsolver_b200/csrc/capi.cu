@@ -15,9 +15,6 @@ static std::atomic<long long> g_launches{0};
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launches_so_far() { return g_launches.load(); }
 
-int launch_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int64_t ldy,
-                 int m, double sigma, int shifted, int precision, cudaStream_t st);
-
 // Nonzero count of the CSR the reference assembles, counted from the stencil structure: each
 // (row band, column band) block couples a site to the offsets its operators reach, clipped at
 // the walls. First-derivative blocks reach the six faces, except that without strain U only
@@ -193,9 +190,7 @@ int qdkp_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int
     set_error("folded apply needs a workspace of n * m complex elements");
     return QDKP_ERR_WORKSPACE;
   }
-  int rc = launch_apply(op, X, ldx, ws, m, m, sigma, 1, precision, st);
-  if (rc != QDKP_OK) return rc;
-  return launch_apply(op, ws, m, Y, ldy, m, sigma, 1, precision, st);
+  return launch_folded(op, X, ldx, ws, Y, ldy, m, sigma, precision, st);
 }
 
 size_t qdkp_apply_host_workspace_size(const qdkp_operator* op, int m, int mode) {

@@ -16,9 +16,6 @@
 
 namespace qdkp {
 
-int launch_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int64_t ldy,
-                 int m, double sigma, int shifted, int precision, cudaStream_t st);
-
 // Rows per CTA of the row kernels: a multiple of the update's chunk, and no more than kEMaxParts CTAs
 // for a slot, whose norm partials one CTA then sums (32768 parts of a 128^3 solve would take 0.5 ms).
 constexpr int kERowsPerCta = 512;
@@ -83,7 +80,7 @@ e_norm_kernel(const ESlot* __restrict__ S, int ns) {
 // scipy's decisions from the column norms; one thread
 static __device__ void e_decide(const ESlot& d, EState* st, const double* __restrict__ nrm) {
   const int m = d.m;
-  st->idle = 1; st->copy_best = 0; st->skip_recompute = 1; st->skip_p = 1; st->skip_pnorm = 1;
+  st->idle = 1; st->r_idle = 1; st->copy_best = 0; st->skip_recompute = 1; st->skip_p = 1; st->skip_pnorm = 1;
   if (!st->running) return;
   if (st->iter >= d.maxiter) { st->running = 0; st->status = QDKP_LOBPCG_MAXITER; return; }
   if (d.stall_iterations > 0 && st->iter - st->best_iter > d.stall_iterations &&
@@ -120,6 +117,7 @@ static __device__ void e_decide(const ESlot& d, EState* st, const double* __rest
   if (ma == 0) { st->running = 0; st->status = QDKP_LOBPCG_CONVERGED; return; }
   st->explicit_gram = !(mx > d.sqrt_eps && !st->explicit_gram);
   st->idle = 0;
+  st->r_idle = 0;
   st->skip_p = st->iter == 0 ? 1 : 0;
 }
 
@@ -209,8 +207,9 @@ e_row_kernel(const ESlot* __restrict__ S, int ns, int which) {
 template <typename T>
 __device__ bool gram_task(const ESlot& d, int which, GramTask<T>& t, double2*& out, double2*& outS) {
   const EState* st = d.st;
-  if (st->idle || (which == GR_PP && st->skip_p)) return false;
-  const int m = d.m, ma = st->ma, mp = st->mp;
+  if (which == GR_PP ? st->idle || st->skip_p : st->r_idle) return false;
+  const int m = d.m, ma = st->ma;
+  const int mp = which == GR_RZ ? st->mp : 0;          // decided beside the products on R
   t.nblk = 0; t.tc = 0;
   t.m = m; t.ma = ma; t.mp = mp; t.n = d.n;
   t.a0 = 0; t.b0 = 0;
@@ -227,11 +226,11 @@ __device__ bool gram_task(const ESlot& d, int which, GramTask<T>& t, double2*& o
       return true;
     case GR_RR:
       add(d.Ra, ma, ma);
-      t.P = t.Q = ma; t.kind = GK_HERM; out = d.G;
+      t.P = t.Q = ma; t.kind = GK_HERM; out = nullptr;      // e_chol_kernel's
       return true;
     case GR_PP:          // all columns; e_chol_kernel takes the active ones
       add(d.P, m, m);
-      t.P = t.Q = m; t.kind = GK_HERM; out = d.G;
+      t.P = t.Q = m; t.kind = GK_HERM; out = nullptr;
       return true;
     default:
       add(d.X, m, m); add(d.Ra, ma, ma); add(d.Pa, ma, mp);
@@ -259,7 +258,7 @@ __device__ void e_gram_body(const ESlot& d, int which, int part, unsigned char* 
     go = gram_task<T>(d, which, t, out, outS);
   }
   __syncthreads();
-  if (go) gram_core(t, part, d.gparts, (int)blockIdx.y, d.gpart, smem);
+  if (go) gram_core(t, part, d.gparts, (int)blockIdx.y, which == GR_PP ? d.ppart : d.gpart, smem);
 }
 
 __global__ void __launch_bounds__(32 * (kGramMaxWarps + 1), 1)
@@ -315,8 +314,8 @@ struct UpdTask {
 template <typename T>
 __device__ bool upd_lists(const ESlot& d, int which, bool packed, UpdTask<T>& u) {
   const EState* st = d.st;
-  if (st->idle) return false;
-  const int m = d.m, ma = st->ma, mp = st->mp;
+  if (which == UP_PNORM || which == UP_APNORM ? st->idle : st->r_idle) return false;
+  const int m = d.m, ma = st->ma;
   u.accumulate = 0; u.neg = 0;
   u.Y2 = nullptr; u.gather = nullptr;
   auto set = [&](int i, double2* p, int ld, int c, const double2* cf) {
@@ -330,9 +329,9 @@ __device__ bool upd_lists(const ESlot& d, int which, bool packed, UpdTask<T>& u)
       if (st->skip_pnorm) return false;
       const bool ax = which == UP_APNORM;
       if (packed) {
-        set(0, ax ? d.APa : d.Pa, ma, ma, d.U);
+        set(0, ax ? d.APa : d.Pa, ma, ma, d.Up);
       } else {
-        set(0, ax ? d.AP : d.P, m, ma, d.U);
+        set(0, ax ? d.AP : d.P, m, ma, d.Up);
         u.gather = st->idx;
       }
       u.q = ma; u.Y = blk<T>(ax ? d.APa : d.Pa);
@@ -340,6 +339,7 @@ __device__ bool upd_lists(const ESlot& d, int which, bool packed, UpdTask<T>& u)
     }
     default: {        // UP_XPNEW / UP_AXPNEW
       const bool ax = which == UP_AXPNEW;
+      const int mp = st->mp;
       u.A.nblk = mp ? 3 : 2;
       set(0, ax ? d.AX : d.X, m, m, nullptr);            // X rows do not enter P
       set(1, ax ? d.ARa : d.Ra, ma, ma, d.Cr);
@@ -356,7 +356,8 @@ __device__ bool upd_lists(const ESlot& d, int which, bool packed, UpdTask<T>& u)
 // One launch per precision present; CTAs of the other precision's slots return at once.
 template <typename T>
 __global__ void __launch_bounds__(kUpdThreads, 2)
-e_update_kernel(const ESlot* __restrict__ S, int ns, int which) {
+e_update_kernel(const ESlot* __restrict__ S, int ns, int first) {
+  const int which = first + blockIdx.y;               // PNORM and APNORM are one launch
   extern __shared__ __align__(16) unsigned char usm_e[];
   const int k = slot_of(S, ns, blockIdx.x, &ESlot::row0);
   const ESlot& d = S[k];
@@ -383,7 +384,7 @@ e_ritz_kernel(const ESlot* __restrict__ S, int ns) {
   const ESlot& d = S[k];
   constexpr int prec = std::is_same<T, float>::value ? QDKP_C64 : QDKP_C128;
   const EState* st = d.st;
-  if (d.prec != prec || st->idle) return;
+  if (d.prec != prec || st->r_idle) return;
   const int part = blockIdx.x - d.row0;
   const long long r0 = (long long)part * d.rows_per_cta;
   RitzArgs<T> t;
@@ -457,11 +458,11 @@ __device__ void e_small_gram(const ESlot& d, int which, double2* __restrict__ G)
     gram_task<T>(d, which, t, o, oS);
   }
   __syncthreads();
-  gram_reduce_herm(t, d.gparts, d.gpart, G);
+  gram_reduce_herm(t, d.gparts, which == GR_PP ? d.ppart : d.gpart, G);
 }
 
 // R^H R (which = GR_RR) or P^H P (GR_PP, of which the active columns are taken) summed, its Cholesky
-// factor, and U^-1 in d.U. One kernel: reduction and factorisation are a launch of latency each (13 us
+// factor, and U^-1 in d.U (d.Up). One kernel: reduction and factorisation are a launch of latency each (13 us
 // and 15 us at 12 columns).
 template <int WHICH>
 __global__ void __launch_bounds__(kSmallThreads) e_chol_kernel(const ESlot* __restrict__ S) {
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(kSmallThreads) e_chol_kernel(const ESlot* __re
   __shared__ double rinv[kMaxSmall];
   const ESlot& d = S[blockIdx.x];
   EState* st = d.st;
-  if (st->idle) return;
+  if (WHICH == GR_PP ? st->idle : st->r_idle) return;
   const int n = st->ma, m = WHICH == GR_PP ? d.m : n;
   if (WHICH == GR_PP && st->skip_p) {      // iteration 0: no P yet, restart stays as it is
     if (threadIdx.x == 0) { st->skip_pnorm = 1; st->mp = st->restart ? 0 : n; }
@@ -492,11 +493,12 @@ __global__ void __launch_bounds__(kSmallThreads) e_chol_kernel(const ESlot* __re
   const int fail = rr_cholesky(G, n, rinv, 0);
   if (!fail) {
     rr_upper_inverse(G, n, rinv, C);
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) d.U[e] = C[e];
+    double2* U = WHICH == GR_PP ? d.Up : d.U;
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) U[e] = C[e];
   }
   if (threadIdx.x != 0) return;
   if (WHICH == GR_RR) {
-    if (fail) { st->running = 0; st->status = QDKP_LOBPCG_RCHOL_BREAKDOWN; st->idle = 1; }
+    if (fail) { st->running = 0; st->status = QDKP_LOBPCG_RCHOL_BREAKDOWN; st->r_idle = 1; }
   } else {
     st->skip_pnorm = fail ? 1 : 0;
     st->restart = fail ? 1 : st->forced;
@@ -552,7 +554,7 @@ template <int CLASS>
 __global__ void __launch_bounds__(kSmallThreads) e_rr_kernel(const ESlot* __restrict__ S, int c64_ritz) {
   const ESlot& d = S[blockIdx.x];
   EState* st = d.st;
-  if (st->idle || rr_class(3 * d.m) != CLASS) return;
+  if (st->r_idle || rr_class(3 * d.m) != CLASS) return;
   __shared__ int use_restart, ok, dim_s;
   if (threadIdx.x == 0) { use_restart = st->mp == 0; ok = 0; }
   __syncthreads();
@@ -570,7 +572,7 @@ __global__ void __launch_bounds__(kSmallThreads) e_rr_kernel(const ESlot* __rest
     __syncthreads();
   }
   if (!ok) {
-    if (threadIdx.x == 0) { st->running = 0; st->status = QDKP_LOBPCG_EIGH_BREAKDOWN; st->idle = 1; }
+    if (threadIdx.x == 0) { st->running = 0; st->status = QDKP_LOBPCG_EIGH_BREAKDOWN; st->r_idle = 1; }
     return;
   }
   const int m = d.m, ma = st->ma, dim = dim_s;
@@ -610,8 +612,9 @@ SlotLayout slot_layout(int64_t n, int m, int prec, int n_blocks) {
   L.gparts = gram_parts(n);
   // the widest task: 3 m x 6 m columns (explicit Gram matrices)
   L.gpart = align256(gram_partial_elems(3 * m, 6 * m) * sizeof(double2));
+  L.ppart = align256(gram_partial_elems(m, m) * sizeof(double2));
   L.total = align256(sizeof(EState)) + n_blocks * L.blk + 13 * L.small +
-            align256(3 * m * sizeof(double)) + L.npart + L.gpart;
+            align256(3 * m * sizeof(double)) + L.npart + L.gpart + L.ppart;
   return L;
 }
 
@@ -621,7 +624,7 @@ void slot_carve(ESlot& d, void* ws, const SlotLayout& L, int64_t n, int m, int p
   d.st = (EState*)take(sizeof(EState));
   double2** const blocks[10] = {&d.X, &d.AX, &d.P, &d.AP, &d.best, &d.Ra, &d.ARa, &d.Pa, &d.APa, &d.T};
   for (int i = 0; i < 10; ++i) *blocks[i] = i < n_blocks ? (double2*)take(L.blk) : nullptr;
-  d.W = (double2*)take(L.small); d.G = (double2*)take(L.small); d.U = (double2*)take(L.small);
+  d.W = (double2*)take(L.small); d.U = (double2*)take(L.small); d.Up = (double2*)take(L.small);
   d.gS = (double2*)take(L.small); d.gT = (double2*)take(L.small); d.gA = (double2*)take(L.small);
   d.gB = (double2*)take(L.small); d.E = (double2*)take(L.small);
   d.scr = (double2*)take(2 * L.small);
@@ -629,6 +632,7 @@ void slot_carve(ESlot& d, void* ws, const SlotLayout& L, int64_t n, int m, int p
   d.w = (double*)take(3 * m * sizeof(double));
   d.npart = (double*)take(L.npart);
   d.gpart = (double*)take(L.gpart);
+  d.ppart = (double*)take(L.ppart);
   d.n = n; d.m = m; d.prec = prec;
   d.nparts = L.nparts; d.gparts = L.gparts; d.rows_per_cta = L.rows_per_cta;
   d.gram0 = d.row0 = 0;
@@ -648,7 +652,7 @@ void slot_params(ESlot& d, EState& s, const qdkp_lobpcg_params* prm, const doubl
   s = EState{};
   s.running = 1;
   s.status = QDKP_LOBPCG_MAXITER;
-  s.iter = -1; s.idle = 1;
+  s.iter = -1; s.idle = 1; s.r_idle = 1;
   s.ma = d.m; s.mp = 0; s.restart = 1; s.forced = 0; s.explicit_gram = 0;
   s.best_iter = prm->maxiter; s.skip_recompute = 1; s.skip_p = 1; s.skip_pnorm = 1;
   s.smallest = std::numeric_limits<double>::max();
@@ -690,17 +694,20 @@ static int launch_umma_multi(const EGroup& G, int which, cudaStream_t st) {
   return QDKP_OK;
 }
 
-static int launch_update_multi(const EGroup& G, int which, cudaStream_t st) {
+// the updates which .. which + count - 1 (UpdWhich), in one launch where no tcgen05 kernel runs them
+static int launch_update_multi(const EGroup& G, int which, cudaStream_t st, int count = 1) {
   if (G.hx_ns[0]) {
-    e_update_kernel<double><<<G.row_ctas, kUpdThreads, update_smem_bytes(G.m_max, G.m_max), st>>>(
+    e_update_kernel<double><<<dim3(G.row_ctas, count), kUpdThreads, update_smem_bytes(G.m_max, G.m_max), st>>>(
         G.d_slots, G.ns, which);
     count_launch();
   }
   if (G.hx_ns[1] && c64_update_tcgen05()) {
-    const int rc = launch_umma_multi(G, which, st);
-    if (rc) return rc;
+    for (int i = 0; i < count; ++i) {
+      const int rc = launch_umma_multi(G, which + i, st);
+      if (rc) return rc;
+    }
   } else if (G.hx_ns[1]) {
-    e_update_kernel<float><<<G.row_ctas, kUpdThreads, update_tf32_smem_bytes(G.m_max, G.m_max), st>>>(
+    e_update_kernel<float><<<dim3(G.row_ctas, count), kUpdThreads, update_tf32_smem_bytes(G.m_max, G.m_max), st>>>(
         G.d_slots, G.ns, which);
     count_launch();
   }
@@ -726,7 +733,7 @@ static int launch_ritz_multi(const EGroup& G, cudaStream_t st) {
   return QDKP_OK;
 }
 
-static bool group_umma(const EGroup& G) { return G.hx_ns[1] && c64_update_tcgen05(); }
+bool group_umma(const EGroup& G) { return G.hx_ns[1] && c64_update_tcgen05(); }
 
 #define ETRY(x) do { const int rc_ = (x); if (rc_ != QDKP_OK) return rc_; } while (0)
 
@@ -741,19 +748,22 @@ int launch_decide(const EGroup& G, cudaStream_t st) {
   return QDKP_OK;
 }
 
-int launch_residual_block(const EGroup& G, cudaStream_t st) {
+int launch_p_chain(const EGroup& G, cudaStream_t st) {
   e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, G.ns, RW_COPYBEST);
-  e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, G.ns, RW_RESID);
-  count_launch(2);
-  QDKP_CUDA_TRY(cudaGetLastError());
-  return QDKP_OK;
-}
-
-int launch_project(const EGroup& G, cudaStream_t st) {
+  count_launch();
   if (group_umma(G)) {
     e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, G.ns, RW_GATHERP);
     count_launch();
   }
+  ETRY(launch_gram_multi(G, GR_PP, st));
+  e_chol_kernel<GR_PP><<<G.ns, kSmallThreads, 2 * (size_t)G.m_max * G.m_max * sizeof(double2), st>>>(G.d_slots);
+  count_launch();
+  return launch_update_multi(G, UP_PNORM, st, 2);
+}
+
+int launch_r_chain(const EGroup& G, cudaStream_t st) {
+  e_row_kernel<<<G.row_ctas, kTallThreads, 0, st>>>(G.d_slots, G.ns, RW_RESID);
+  count_launch();
   ETRY(launch_gram_multi(G, GR_XR, st));
   ETRY(launch_update_multi(G, UP_RPROJ, st));
   ETRY(launch_gram_multi(G, GR_RR, st));
@@ -763,11 +773,6 @@ int launch_project(const EGroup& G, cudaStream_t st) {
 }
 
 int launch_ritz_step(const EGroup& G, cudaStream_t st) {
-  ETRY(launch_gram_multi(G, GR_PP, st));
-  e_chol_kernel<GR_PP><<<G.ns, kSmallThreads, 2 * (size_t)G.m_max * G.m_max * sizeof(double2), st>>>(G.d_slots);
-  count_launch();
-  ETRY(launch_update_multi(G, UP_PNORM, st));
-  ETRY(launch_update_multi(G, UP_APNORM, st));
   ETRY(launch_gram_multi(G, GR_RZ, st));
   const size_t rr_smem = 2 * (size_t)(3 * G.m_max) * (3 * G.m_max) * sizeof(double2);
   bool cls[3] = {};
@@ -824,18 +829,19 @@ struct qdkp_engine {
   std::vector<qdkp::SlotHost> slots;
   qdkp::ESlot* d_slots = nullptr;      // compact array of the used slots (group after group)
   qdkp::HXSlot* d_hx = nullptr;        // H.X descriptors, kEGroups x 8 x max_slots
-  int* d_one = nullptr;                // constant 1 (skip flag)
   int ns = 0;                          // used slots
   int ngroups = 0;
   int nsm = 148;                       // SMs of the device (grid of the tcgen05 updates)
   qdkp::EGroup grp[qdkp::kEGroups];
   bool dirty = true;
-  // CUDA graph of `graph_ticks` ticks over the current slot layout, replayed by
-  // qdkp_engine_step on the engine's own stream (ordered after the caller's stream by events)
+  // CUDA graph of one tick of each group over the current slot layout, replayed by qdkp_engine_step on
+  // the group's own stream (ordered after and before the caller's stream by events)
   cudaStream_t gstream = nullptr, gstream2 = nullptr;   // group 0 and group 1
+  // the work on P of a single group, forked from and joined to the group's stream within a tick
+  cudaStream_t pstream = nullptr;
+  cudaEvent_t ev_dec = nullptr, ev_p = nullptr;
   cudaEvent_t ev_in = nullptr, ev_out = nullptr, ev_fork = nullptr, ev_join = nullptr;
-  cudaGraphExec_t graph = nullptr;
-  int graph_ticks = 0;
+  cudaGraphExec_t graph[qdkp::kEGroups] = {};
   bool use_graph = true;
   long long launches_per_tick = 0;     // kernels one tick launches (graph replays count them)
 };
@@ -847,11 +853,7 @@ namespace {
 // double2 in ESlot and hold complex64 values for a QDKP_C64 slot).
 int apply_folded(const SlotHost& h, const void* V, int c, void* out, cudaStream_t st) {
   const ESlot& d = h.d;
-  if (h.prm.folded) {
-    int rc = launch_apply(h.op, V, c, d.T, c, c, h.prm.sigma, 1, d.prec, st);
-    if (rc) return rc;
-    return launch_apply(h.op, d.T, c, out, c, c, h.prm.sigma, 1, d.prec, st);
-  }
+  if (h.prm.folded) return launch_folded(h.op, V, c, d.T, out, c, c, h.prm.sigma, d.prec, st);
   return launch_apply(h.op, V, c, out, c, c, 0.0, 0, d.prec, st);
 }
 
@@ -915,7 +917,7 @@ int build_group(qdkp_engine* e, int g, const std::vector<int>& ids, int base, cu
   std::vector<ESlot> compact;
   std::vector<HXSlot> hx(8 * (size_t)e->max_slots);
   int gram0 = 0, row0 = 0, m_max = 1, utile0 = 0;
-  int tile0[2] = {0, 0}, kp[2] = {0, 0};
+  int tile0[2] = {0, 0}, kp[2] = {0, 0}, nf[2] = {0, 0};
   for (int i : ids) {
     SlotHost& h = e->slots[i];
     ESlot d = h.d;
@@ -927,6 +929,7 @@ int build_group(qdkp_engine* e, int g, const std::vector<int>& ids, int base, cu
     compact.push_back(d);
     const int pi = d.prec == QDKP_C64 ? 1 : 0;
     const int k = kp[pi]++;
+    nf[pi] += h.prm.folded ? 1 : 0;
     const qdkp_operator* op = h.op;
     m_max = std::max(m_max, d.m);
     const int tiles = apply_tiles(op->n_sites, d.m);
@@ -941,7 +944,7 @@ int build_group(qdkp_engine* e, int g, const std::vector<int>& ids, int base, cu
       const bool recompute = t < 2;
       if (recompute) { x.m = d.m; x.m_dev = nullptr; x.ld_same = 0; x.ldx = d.m; x.ldy = d.m; }
       else { x.m = 0; x.m_dev = &d.st->ma; x.ld_same = 1; }
-      const int* skipflag = recompute ? &d.st->skip_recompute : &d.st->idle;
+      const int* skipflag = recompute ? &d.st->skip_recompute : &d.st->r_idle;
       if (h.prm.folded) {
         x.X = (t == 0) ? (const void*)d.X : (t == 2) ? (const void*)d.Ra : (const void*)d.T;
         x.Y = (t == 0 || t == 2) ? (void*)d.T : (t == 1) ? (void*)d.AX : (void*)d.ARa;
@@ -949,7 +952,7 @@ int build_group(qdkp_engine* e, int g, const std::vector<int>& ids, int base, cu
       } else {
         x.X = recompute ? (const void*)d.X : (const void*)d.Ra;
         x.Y = recompute ? (void*)d.AX : (void*)d.ARa;
-        x.skip = (t == 1 || t == 3) ? e->d_one : skipflag;
+        x.skip = skipflag;                    // phases 1 and 3 are for folded slots only
       }
       hx[((size_t)pi * 4 + t) * e->max_slots + k] = x;
     }
@@ -959,7 +962,7 @@ int build_group(qdkp_engine* e, int g, const std::vector<int>& ids, int base, cu
   G.gram_ctas = gram0; G.row_ctas = row0;
   G.utiles = utile0;
   G.nsm = e->nsm;
-  for (int pi = 0; pi < 2; ++pi) { G.hx_ns[pi] = kp[pi]; G.hx_tiles[pi] = tile0[pi]; }
+  for (int pi = 0; pi < 2; ++pi) { G.hx_ns[pi] = kp[pi]; G.hx_tiles[pi] = tile0[pi]; G.hx_folded[pi] = nf[pi]; }
   G.m_max = m_max;
   for (const ESlot& d : compact)
     if (std::find(G.widths.begin(), G.widths.end(), d.m) == G.widths.end()) G.widths.push_back(d.m);
@@ -1001,27 +1004,48 @@ int rebuild(qdkp_engine* e, cudaStream_t st) {
   return QDKP_OK;
 }
 
-// one H.X phase of a tick: a multi-slot launch per precision present
+// One H.X phase of a tick: a multi-slot launch per precision and kind (folded or not) present. The
+// recomputation of A X (phases 0 and 1) runs on a forced restart only: a grid of every tile would
+// take 18 us a phase (seven slots) to find that out.
 int launch_hx_phase(const qdkp_engine* e, const EGroup& G, int phase, cudaStream_t st) {
   for (int pi = 0; pi < 2; ++pi) {
     if (!G.hx_ns[pi]) continue;
-    int rc = launch_apply_multi(G.d_hx + ((size_t)pi * 4 + phase) * e->max_slots, G.hx_ns[pi],
-                                G.hx_tiles[pi], pi ? QDKP_C64 : QDKP_C128, st);
+    const HXSlot* slots = G.d_hx + ((size_t)pi * 4 + phase) * e->max_slots;
+    const int prec = pi ? QDKP_C64 : QDKP_C128, most = phase < 2 ? 4 * e->nsm : G.hx_tiles[pi];
+    const int basis = phase % 2 ? HX_X_UNCOUPLED : HX_Y_UNCOUPLED;
+    int rc = QDKP_OK;
+    if (G.hx_folded[pi]) rc = launch_apply_multi(slots, G.hx_ns[pi], G.hx_tiles[pi], prec, basis, most, st);
+    if (rc == QDKP_OK && G.hx_folded[pi] < G.hx_ns[pi] && phase % 2 == 0)
+      rc = launch_apply_multi(slots, G.hx_ns[pi], G.hx_tiles[pi], prec, 0, most, st);
     if (rc) return rc;
   }
   return QDKP_OK;
 }
 
-// one LOBPCG iteration of every running slot of group G
-int tick(const qdkp_engine* e, const EGroup& G, cudaStream_t st) {
+// One LOBPCG iteration of every running slot of group g. The work on P needs nothing of the work on R.
+// A group by itself runs it beside R's, on a stream forked from st after the decisions and joined
+// before the pencil; two groups fill each other's gaps already (a sweep of 14 complex64 slots 28.7 ms
+// with the P work in line, 29.7 ms forked).
+int tick(const qdkp_engine* e, int g, cudaStream_t st) {
+  const EGroup& G = e->grp[g];
   if (!G.ns) return QDKP_OK;
   ETRY(launch_decide(G, st));
-  ETRY(launch_residual_block(G, st));
-  ETRY(launch_hx_phase(e, G, 0, st));
-  ETRY(launch_hx_phase(e, G, 1, st));
-  ETRY(launch_project(G, st));
-  ETRY(launch_hx_phase(e, G, 2, st));
-  ETRY(launch_hx_phase(e, G, 3, st));
+  // (two tcgen05 kernels would contend for an SM's tensor memory: one after the other)
+  const cudaStream_t ps = e->ngroups > 1 || group_umma(G) ? st : e->pstream;
+  if (ps != st) {
+    QDKP_CUDA_TRY(cudaEventRecord(e->ev_dec, st));
+    QDKP_CUDA_TRY(cudaStreamWaitEvent(ps, e->ev_dec, 0));
+  }
+  int rc = launch_p_chain(G, ps);
+  if (rc == QDKP_OK) rc = launch_r_chain(G, st);
+  for (int phase = 0; phase < 4 && rc == QDKP_OK; ++phase) rc = launch_hx_phase(e, G, phase, st);
+  if (ps != st) {
+    // after an error too, so that a capture in progress ends with no stream left forked
+    const cudaError_t r1 = cudaEventRecord(e->ev_p, ps);
+    const cudaError_t r2 = cudaStreamWaitEvent(st, e->ev_p, 0);
+    if (rc == QDKP_OK) { QDKP_CUDA_TRY(r1); QDKP_CUDA_TRY(r2); }
+  }
+  if (rc != QDKP_OK) return rc;
   return launch_ritz_step(G, st);
 }
 
@@ -1038,8 +1062,8 @@ static int run_ticks(qdkp_engine* e, int ticks, cudaStream_t st) {
     QDKP_CUDA_TRY(cudaEventRecord(e->ev_fork, st));
     QDKP_CUDA_TRY(cudaStreamWaitEvent(e->gstream2, e->ev_fork, 0));
   }
-  for (int t = 0; t < ticks && rc == QDKP_OK; ++t) rc = tick(e, e->grp[0], st);
-  for (int t = 0; t < ticks && rc == QDKP_OK && e->ngroups > 1; ++t) rc = tick(e, e->grp[1], e->gstream2);
+  for (int t = 0; t < ticks && rc == QDKP_OK; ++t) rc = tick(e, 0, st);
+  for (int t = 0; t < ticks && rc == QDKP_OK && e->ngroups > 1; ++t) rc = tick(e, 1, e->gstream2);
   if (e->ngroups > 1) {
     // join even after an error, so that a capture in progress ends with no stream left forked
     const cudaError_t r1 = cudaEventRecord(e->ev_join, e->gstream2);
@@ -1052,38 +1076,50 @@ static int run_ticks(qdkp_engine* e, int ticks, cudaStream_t st) {
   return rc;
 }
 
-static void drop_graph(qdkp_engine* e) {
-  if (e->graph) cudaGraphExecDestroy(e->graph);
-  e->graph = nullptr;
-  e->graph_ticks = 0;
+static void destroy_pstream(qdkp_engine* e) {
+  if (e->pstream) { cudaStreamSynchronize(e->pstream); cudaStreamDestroy(e->pstream); }
+  if (e->ev_dec) cudaEventDestroy(e->ev_dec);
+  if (e->ev_p) cudaEventDestroy(e->ev_p);
 }
 
-// Capture `ticks` ticks of the current layout into e->graph (from the engine's stream; the
-// second group's branch is forked off and joined back inside the graph).
-static int capture_ticks(qdkp_engine* e, int ticks) {
+static void drop_graph(qdkp_engine* e) {
+  for (cudaGraphExec_t& g : e->graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+}
+
+// Capture a tick of each group of the current layout, from the group's stream, into e->graph. (One tick,
+// replayed: a graph of all of a call's ticks cost 5 us a kernel to build whenever the slots changed.)
+static int capture_ticks(qdkp_engine* e) {
   drop_graph(e);
-  QDKP_CUDA_TRY(cudaStreamBeginCapture(e->gstream, cudaStreamCaptureModeThreadLocal));
-  const long long l0 = launches_so_far();
-  const int rc = run_ticks(e, ticks, e->gstream);
-  // captured launches are not executions: take them back off the counter
-  const long long captured = launches_so_far() - l0;
-  count_launch((int)-captured);
-  e->launches_per_tick = ticks ? captured / ticks : 0;
-  cudaGraph_t g = nullptr;
-  const cudaError_t ce = cudaStreamEndCapture(e->gstream, &g);
-  if (rc != QDKP_OK) { if (g) cudaGraphDestroy(g); return rc; }
-  if (ce != cudaSuccess) {
-    set_error(std::string("engine graph capture: ") + cudaGetErrorString(ce));
-    return QDKP_ERR_CUDA;
+  e->launches_per_tick = 0;
+  for (int gi = 0; gi < e->ngroups; ++gi) {
+    const cudaStream_t st = gi ? e->gstream2 : e->gstream;
+    QDKP_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    const long long l0 = launches_so_far();
+    const int rc = tick(e, gi, st);
+    // captured launches are not executions: take them back off the counter
+    const long long captured = launches_so_far() - l0;
+    count_launch((int)-captured);
+    e->launches_per_tick += captured;
+    cudaGraph_t g = nullptr;
+    const cudaError_t ce = cudaStreamEndCapture(st, &g);
+    if (rc != QDKP_OK) { if (g) cudaGraphDestroy(g); drop_graph(e); return rc; }
+    if (ce != cudaSuccess) {
+      drop_graph(e);
+      set_error(std::string("engine graph capture: ") + cudaGetErrorString(ce));
+      return QDKP_ERR_CUDA;
+    }
+    const cudaError_t ie = cudaGraphInstantiate(&e->graph[gi], g, 0);
+    cudaGraphDestroy(g);
+    if (ie != cudaSuccess) {
+      e->graph[gi] = nullptr;
+      drop_graph(e);
+      set_error(std::string("engine graph instantiate: ") + cudaGetErrorString(ie));
+      return QDKP_ERR_CUDA;
+    }
   }
-  const cudaError_t ie = cudaGraphInstantiate(&e->graph, g, 0);
-  cudaGraphDestroy(g);
-  if (ie != cudaSuccess) {
-    e->graph = nullptr;
-    set_error(std::string("engine graph instantiate: ") + cudaGetErrorString(ie));
-    return QDKP_ERR_CUDA;
-  }
-  e->graph_ticks = ticks;
   return QDKP_OK;
 }
 
@@ -1102,24 +1138,26 @@ int qdkp_engine_create(int max_slots, int device, qdkp_engine** out) {
   e->slots.resize(max_slots);
   cudaError_t err = cudaMalloc(&e->d_slots, sizeof(ESlot) * max_slots);
   if (err == cudaSuccess) err = cudaMalloc(&e->d_hx, sizeof(HXSlot) * kEGroups * 8 * max_slots);
-  if (err == cudaSuccess) err = cudaMalloc(&e->d_one, sizeof(int));
-  if (err == cudaSuccess) { const int one = 1; err = cudaMemcpy(e->d_one, &one, sizeof(int), cudaMemcpyHostToDevice); }
   if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&e->gstream, cudaStreamNonBlocking);
   if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&e->gstream2, cudaStreamNonBlocking);
   if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->ev_in, cudaEventDisableTiming);
   if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->ev_out, cudaEventDisableTiming);
   if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming);
   if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming);
+  if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&e->pstream, cudaStreamNonBlocking);
+  if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->ev_dec, cudaEventDisableTiming);
+  if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->ev_p, cudaEventDisableTiming);
   if (err == cudaSuccess) err = cudaDeviceGetAttribute(&e->nsm, cudaDevAttrMultiProcessorCount, device);
   if (err != cudaSuccess) {
     set_error(std::string("engine tables: ") + cudaGetErrorString(err));
-    cudaFree(e->d_slots); cudaFree(e->d_hx); cudaFree(e->d_one);
+    cudaFree(e->d_slots); cudaFree(e->d_hx);
     if (e->gstream) cudaStreamDestroy(e->gstream);
     if (e->gstream2) cudaStreamDestroy(e->gstream2);
     if (e->ev_in) cudaEventDestroy(e->ev_in);
     if (e->ev_out) cudaEventDestroy(e->ev_out);
     if (e->ev_fork) cudaEventDestroy(e->ev_fork);
     if (e->ev_join) cudaEventDestroy(e->ev_join);
+    destroy_pstream(e);
     delete e;
     return QDKP_ERR_CUDA;
   }
@@ -1138,9 +1176,9 @@ int qdkp_engine_destroy(qdkp_engine* e) {
   if (e->ev_out) cudaEventDestroy(e->ev_out);
   if (e->ev_fork) cudaEventDestroy(e->ev_fork);
   if (e->ev_join) cudaEventDestroy(e->ev_join);
+  destroy_pstream(e);
   cudaFree(e->d_slots);
   cudaFree(e->d_hx);
-  cudaFree(e->d_one);
   delete e;
   return QDKP_OK;
 }
@@ -1184,8 +1222,8 @@ int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg
                                      reinterpret_cast<float2*>(d.X), m, st)));
   else
     ATRY(launch_copy(static_cast<const double2*>(X0), m, m, n, d.X, m, st));
-  ATRY(gram1(h, d.X, d.X, m, d.G, st));
-  ATRY(launch_chol_inv(d.G, m, d.U, (int*)d.w, st));
+  ATRY(gram1(h, d.X, d.X, m, d.gS, st));
+  ATRY(launch_chol_inv(d.gS, m, d.U, (int*)d.w, st));
   int stat = 0;
   ATRY(read_sync(&stat, d.w, sizeof(int), st));
   if (stat) { set_error("Linearly dependent initial approximations"); return QDKP_ERR_NUMERIC; }
@@ -1193,8 +1231,8 @@ int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg
   // initial Ritz vectors (lobpcg.py:633-660)
   ATRY(apply_folded(h, d.X, m, d.AX, st));
   ATRY(gram1(h, d.X, d.AX, m, d.gT, st));
-  ATRY(launch_eigh(d.gT, nullptr, m, d.w, d.E, d.scr, (int*)d.G, st));
-  ATRY(read_sync(&stat, d.G, sizeof(int), st));
+  ATRY(launch_eigh(d.gT, nullptr, m, d.w, d.E, d.scr, (int*)d.Up, st));
+  ATRY(read_sync(&stat, d.Up, sizeof(int), st));
   // the eigensolve fails only on non-finite input (a NaN or inf in the operator's fields or in
   // X0): the slot is admitted already stopped with status nonfinite, and retires like any other
   const bool nonfinite = stat != 0;
@@ -1230,17 +1268,28 @@ int qdkp_engine_step(qdkp_engine* e, int ticks, void* stream) {
   if (ticks == 0 || e->ns == 0) return QDKP_OK;
   if (!e->use_graph) return run_ticks(e, ticks, st);
   // the tick sequence is fixed for a slot layout: replay it as one graph launch
-  if (!e->graph || e->graph_ticks != ticks) {
+  if (!e->graph[0]) {
     QDKP_CUDA_TRY(cudaStreamSynchronize(st));   // descriptor uploads of rebuild() landed
-    int rc = capture_ticks(e, ticks);
+    int rc = capture_ticks(e);
     if (rc) return rc;
   }
+  // the groups' ticks interleave freely: each replays its own graph on its own stream
   QDKP_CUDA_TRY(cudaEventRecord(e->ev_in, st));
   QDKP_CUDA_TRY(cudaStreamWaitEvent(e->gstream, e->ev_in, 0));
-  QDKP_CUDA_TRY(cudaGraphLaunch(e->graph, e->gstream));
+  if (e->ngroups > 1) QDKP_CUDA_TRY(cudaStreamWaitEvent(e->gstream2, e->ev_in, 0));
+  cudaError_t le = cudaSuccess;
+  for (int t = 0; t < ticks && le == cudaSuccess; ++t) {
+    le = cudaGraphLaunch(e->graph[0], e->gstream);
+    if (le == cudaSuccess && e->ngroups > 1) le = cudaGraphLaunch(e->graph[1], e->gstream2);
+  }
   count_launch(e->launches_per_tick * ticks);
   QDKP_CUDA_TRY(cudaEventRecord(e->ev_out, e->gstream));
   QDKP_CUDA_TRY(cudaStreamWaitEvent(st, e->ev_out, 0));
+  if (e->ngroups > 1) {
+    QDKP_CUDA_TRY(cudaEventRecord(e->ev_join, e->gstream2));
+    QDKP_CUDA_TRY(cudaStreamWaitEvent(st, e->ev_join, 0));
+  }
+  QDKP_CUDA_TRY(le);
   return QDKP_OK;
 }
 
@@ -1338,9 +1387,9 @@ int qdkp_engine_retire(qdkp_engine* e, int slot, double* lambda_out, void* V,
     QDKP_CUDA_TRY(cudaMemcpyAsync(d.gA, a.data(), a.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
     QDKP_CUDA_TRY(cudaMemcpyAsync(d.gB, bb.data(), bb.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
   }
-  RTRY(launch_eigh(d.gA, d.gB, m, d.w, d.E, d.scr, (int*)d.G, st));
+  RTRY(launch_eigh(d.gA, d.gB, m, d.w, d.E, d.scr, (int*)d.Up, st));
   int stat = 0;
-  RTRY(read_sync(&stat, d.G, sizeof(int), st));
+  RTRY(read_sync(&stat, d.Up, sizeof(int), st));
   if (stat) { set_error("eigh has failed in lobpcg postprocessing"); return QDKP_ERR_NUMERIC; }
   RTRY(read_sync(lam.data(), d.w, m * sizeof(double), st));
   // Ritz vectors of the best iterate; a complex64 slot forms them in its own precision (in the

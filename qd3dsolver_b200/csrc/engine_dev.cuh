@@ -12,7 +12,9 @@ struct EState {
   int running;          // 1 while the slot iterates
   int status;           // QDKP_LOBPCG_* once it stopped
   int iter;             // scipy's iterationNumber of the current tick (starts at -1)
-  int idle;             // 1: the remaining kernels of this tick skip the slot
+  int idle;             // 1: this tick's kernels skip the slot (written by the decision kernel alone)
+  int r_idle;           // idle, or R's orthonormalisation or the eigensolve failed: the kernels on R and
+                        // those that follow the eigensolve skip the slot. (Those on P run beside R's.)
   int ma;               // active residual columns this tick
   int mp;               // P columns in this tick's Rayleigh-Ritz (0: restart)
   int restart, forced, explicit_gram;
@@ -45,10 +47,11 @@ struct ESlot {
   int stall_iterations;  // > 0: stop once the best mean residual is this many iterations old
   int restart_control;
   double2 *X, *AX, *P, *AP, *best, *Ra, *ARa, *Pa, *APa, *T;
-  double2 *W, *G, *U, *gS, *gT, *gA, *gB, *E, *scr, *Cx, *Cr, *Cp;
+  double2 *W, *U, *Up, *gS, *gT, *gA, *gB, *E, *scr, *Cx, *Cr, *Cp;
   double* w;
   double* npart;        // [nparts][m] residual-norm partials of the current X
   double* gpart;        // Gram partials (real)
+  double* ppart;        // ... of P^H P
   int nparts;           // their parts: CTAs of the row kernels
   int gparts;           // row parts (CTAs) of the Gram kernel
   int gram0, row0;      // first CTA of this slot in the Gram / row-kernel launches

@@ -12,7 +12,7 @@ enum RowWhich { RW_COPYBEST = 0, RW_RESID, RW_GATHERP };
 
 // bytes of a slot's pieces; `total` with n_blocks tall blocks
 struct SlotLayout {
-  size_t blk, small, npart, gpart, total;
+  size_t blk, small, npart, gpart, ppart, total;
   int nparts, gparts, rows_per_cta;
 };
 SlotLayout slot_layout(int64_t n, int m, int prec, int n_blocks);
@@ -27,7 +27,8 @@ struct EGroup {
   int ns = 0, gram_ctas = 0, row_ctas = 0;
   int utiles = 0;                      // 128-row tiles of the complex64 slots (tcgen05 updates)
   int nsm = 148;
-  int hx_ns[2] = {0, 0}, hx_tiles[2] = {0, 0};   // per precision (QDKP_C128, QDKP_C64)
+  // per precision (QDKP_C128, QDKP_C64): slots, the folded ones among them, H.X tiles
+  int hx_ns[2] = {0, 0}, hx_folded[2] = {0, 0}, hx_tiles[2] = {0, 0};
   int m_max = 1;
   std::vector<int> widths;             // distinct block widths among the group's slots
 };
@@ -35,11 +36,15 @@ struct EGroup {
 // dynamic shared memory limits of the iteration's kernels, on the current device
 void set_slot_kernel_limits();
 
-// An iteration: decisions, residual block, projection against X and orthonormalisation of R;
-// then A R (the caller's); then the rest from P's orthonormalisation to the Ritz update.
+// complex64 slots of the group are updated by the tcgen05 kernels
+bool group_umma(const EGroup& G);
+
+// An iteration: the decisions; the best iterate's copy and P's orthonormalisation beside R's residual
+// block, projection and orthonormalisation and (the caller's) A R, a recomputed A X not before
+// the residual block; then pencil, eigensolve and Ritz update.
 int launch_decide(const EGroup& G, cudaStream_t st);
-int launch_residual_block(const EGroup& G, cudaStream_t st);
-int launch_project(const EGroup& G, cudaStream_t st);
+int launch_p_chain(const EGroup& G, cudaStream_t st);
+int launch_r_chain(const EGroup& G, cudaStream_t st);
 int launch_ritz_step(const EGroup& G, cudaStream_t st);
 
 }  // namespace qdkp

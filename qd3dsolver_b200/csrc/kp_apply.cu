@@ -462,6 +462,30 @@ __device__ __forceinline__ void load_rec(const T* r, T (&w)[K]) {
   }
 }
 
+// Band order of the values in shared memory, and of a block in the uncoupled basis: Pryor's as copied (band b at word b - band_off),
+// the uncoupled order after conversion: S+, X+, Y+, Z+, S-, X-, Y-, Z- (six bands: no S; RAW: the
+// S values stay in words 0 and 1, the others follow).
+template <int NB, bool RAW> __device__ __forceinline__ constexpr int uslot(int b) {
+  return NB != 8 ? (b < 4 ? b - 1 : b - 2) : (RAW ? (b < 4 ? b + 1 : b) : b);
+}
+
+// One column's values at a site offset in the uncoupled basis; BASIS says which one X is in
+template <class V, int NB, int BASIS>
+__device__ __forceinline__ void load_uncoupled(const cplx<typename V::T>* __restrict__ xs, int bs, int off,
+                                               V (&u)[8]) {
+  if constexpr (BASIS & HX_X_UNCOUPLED) {
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      if (NB != 8 && (b & 3) == 0) { vzero(u[b]); continue; }
+      u[b] = vldg(xs + (uslot<NB, false>(b) * bs + off), (V*)nullptr);
+    }
+  } else {
+    V x[8];
+    load_bands<V, NB>(xs, bs, off, false, x);
+    to_uncoupled<V, NB>(x, u);
+  }
+}
+
 // Faces are taken to the uncoupled basis one by one; the four edge neighbours of a plane share
 // one weight per band, so their weighted sum is formed first and taken there once. Nothing
 // branches on the walls: a missing neighbour reads the site itself under a zero weight, so the
@@ -470,7 +494,7 @@ __device__ __forceinline__ void load_rec(const T* r, T (&w)[K]) {
 // and multiplies the site itself. That is the operator complex64 engine slots of even width iterate
 // on; it differs from the hard-wall operator only in rows next to a wall, and the complex128 finish
 // of a mixed solve does not use it.
-template <class V, int NB>
+template <class V, int NB, int BASIS>
 __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, int j,
                                         bool wall_self = false) {
   typedef typename V::T T;
@@ -486,8 +510,7 @@ __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, i
   {
     T w[8];
     load_rec<true>(rp, w);
-    load_bands<V, NB>(xs, bs, 0, false, x);
-    to_uncoupled<V, NB>(x, u);
+    load_uncoupled<V, NB, BASIS>(xs, bs, 0, u);
     local_term<V, NB>(y, u, w, a.shift);
   }
   const auto cbf = [&](int f) { return W_<V>(wall_self || (msk >> f & 1u) ? a.cb : T(0)); };
@@ -498,8 +521,7 @@ __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, i
 #pragma unroll
     for (int f = 2; f < 6; ++f) {
       const int d = f < 4 ? sy : sz;
-      load_bands<V, NB>(xs, bs, face_off(f, (f & 1) ? -d : d), false, x);
-      to_uncoupled<V, NB>(x, u);
+      load_uncoupled<V, NB, BASIS>(xs, bs, face_off(f, (f & 1) ? -d : d), u);
       if (f < 4) face_term<V, NB, 1, false>(y, u, w + 5 * (f - 2), cbf(f));
       else face_term<V, NB, 2, false>(y, u, w + 5 * (f - 2), cbf(f));
     }
@@ -509,8 +531,7 @@ __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, i
     load_rec<true>(rp + K_FX, w);
 #pragma unroll
     for (int f = 0; f < 2; ++f) {
-      load_bands<V, NB>(xs, bs, face_off(f, f ? -sx : sx), false, x);
-      to_uncoupled<V, NB>(x, u);
+      load_uncoupled<V, NB, BASIS>(xs, bs, face_off(f, f ? -sx : sx), u);
       face_term<V, NB, 0, false>(y, u, w + 5 * f, cbf(f));
     }
   }
@@ -536,23 +557,47 @@ __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, i
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int off = ((e & 1) ? -sa : sa) + ((e & 2) ? -sb : sb);
-      load_bands<V, NB>(xs, bs, (msk >> (6 + 4 * pl + e) & 1u) ? off : 0, true, x);
+      const int o = (msk >> (6 + 4 * pl + e) & 1u) ? off : 0;
       const auto c = W_<V>(w[e]);
+      if constexpr (BASIS & HX_X_UNCOUPLED) {
+        // only the two states of the plane enter
+        const int sa_ = pl == 2 ? 2 : 1, sb_ = pl == 0 ? 2 : 3;
 #pragma unroll
-      for (int b = 2; b < 8; ++b) if (has_band<NB>(b)) vfma(z[b], c, x[b]);
+        for (int sp = 0; sp < 8; sp += 4) {
+          vfma(z[sp + sa_], c, vldg(xs + (uslot<NB, false>(sp + sa_) * bs + o), (V*)nullptr));
+          vfma(z[sp + sb_], c, vldg(xs + (uslot<NB, false>(sp + sb_) * bs + o), (V*)nullptr));
+        }
+      } else {
+        load_bands<V, NB>(xs, bs, o, true, x);
+#pragma unroll
+        for (int b = 2; b < 8; ++b) if (has_band<NB>(b)) vfma(z[b], c, x[b]);
+      }
     }
-    to_uncoupled<V, 6>(z, u);
+    if constexpr (BASIS & HX_X_UNCOUPLED) {
+#pragma unroll
+      for (int b = 0; b < 8; ++b) u[b] = z[b];
+    } else {
+      to_uncoupled<V, 6>(z, u);
+    }
     if (pl == 0) edge_term<V, 1, 2>(y, u, T(1));
     else if (pl == 1) edge_term<V, 1, 3>(y, u, T(1));
     else edge_term<V, 2, 3>(y, u, T(1));
   }
-  from_uncoupled<V, NB>(y, x);
   cplx<T>* __restrict__ ys = a.Y + ((long long)s * a.ldy + j);
   const int ybs = a.N * a.ldy;
+  if constexpr (BASIS & HX_Y_UNCOUPLED) {
 #pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    if (!has_band<NB>(b)) continue;
-    vstore(ys + (b - band_off<NB>()) * ybs, x[b]);
+    for (int b = 0; b < 8; ++b) {
+      if (NB != 8 && (b & 3) == 0) continue;
+      vstore(ys + uslot<NB, false>(b) * ybs, y[b]);
+    }
+  } else {
+    from_uncoupled<V, NB>(y, x);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      if (!has_band<NB>(b)) continue;
+      vstore(ys + (b - band_off<NB>()) * ybs, x[b]);
+    }
   }
 }
 
@@ -563,40 +608,47 @@ template <typename T> struct ApplyOcc;
 template <> struct ApplyOcc<double> { static constexpr int kMinBlocks = 2; };
 template <> struct ApplyOcc<float> { static constexpr int kMinBlocks = 3; };
 
-template <typename T, int NB>
+template <typename T, int NB, int BASIS>
 __global__ void __launch_bounds__(kApplyThreads, ApplyOcc<T>::kMinBlocks)
 kp_apply_kernel(const HXArgs<T> a) {
   const int it = blockIdx.x * blockDim.x + threadIdx.x;
   if (it >= a.N * a.m) return;
   const int s = it / a.m;
-  hx_item<typename Column<T>::V, NB>(a, s, it - s * a.m);
+  hx_item<typename Column<T>::V, NB, BASIS>(a, s, it - s * a.m);
 }
 
 // Many operators and blocks in one launch (the batched engine): CTA b serves slot k with
 // tile0[k] <= b < tile0[k+1]; the column count is read on the device (the slot's active width).
-template <typename T>
+template <typename T, int BASIS, bool LOOP>
 __global__ void __launch_bounds__(kApplyThreads, ApplyOcc<T>::kMinBlocks)
-kp_apply_multi_kernel(const HXSlot* __restrict__ slots, int nslots) {
-  int k = 0;
-  while (k + 1 < nslots && (int)blockIdx.x >= slots[k + 1].tile0) ++k;
-  const HXSlot& d = slots[k];
-  if (d.skip && *d.skip) return;
-  const int m = d.m_dev ? *d.m_dev : d.m;
-  const int it = (blockIdx.x - d.tile0) * kApplyThreads + threadIdx.x;
-  if (m <= 0 || it >= d.N * m) return;
-  HXArgs<T> a;
-  a.rec = static_cast<const T*>(d.rec);
-  a.msk = d.msk;
-  a.X = static_cast<const cplx<T>*>(d.X);
-  a.Y = static_cast<cplx<T>*>(d.Y);
-  a.N = d.N; a.ldx = d.ld_same ? m : d.ldx; a.ldy = d.ld_same ? m : d.ldy;
-  a.m = m; a.sx = d.sx; a.sy = d.sy;
-  a.shift = d.shifted ? (T)(-d.sigma) : T(0);
-  a.cb = (T)d.cb;
-  const bool wall_self = std::is_same<T, float>::value && ((m | a.ldx | a.ldy) & 1) == 0 &&
-                         ((reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.Y)) & 15) == 0;
-  const int s = it / m;
-  hx_item<typename Column<T>::V, 8>(a, s, it - s * m, wall_self);
+kp_apply_multi_kernel(const HXSlot* __restrict__ slots, int nslots, int tiles) {
+  if (LOOP) {                                  // usually nothing to do
+    bool any = false;
+    for (int k = threadIdx.x; k < nslots; k += blockDim.x) any |= !(slots[k].skip && *slots[k].skip);
+    if (!__syncthreads_or(any)) return;
+  }
+  for (int tile = blockIdx.x; tile < tiles; tile += LOOP ? (int)gridDim.x : tiles) {
+    int k = 0;
+    while (k + 1 < nslots && tile >= slots[k + 1].tile0) ++k;
+    const HXSlot& d = slots[k];
+    if ((d.skip && *d.skip) || (BASIS != 0) != (d.shifted != 0)) continue;
+    const int m = d.m_dev ? *d.m_dev : d.m;
+    const int it = (tile - d.tile0) * kApplyThreads + threadIdx.x;
+    if (m <= 0 || it >= d.N * m) continue;
+    HXArgs<T> a;
+    a.rec = static_cast<const T*>(d.rec);
+    a.msk = d.msk;
+    a.X = static_cast<const cplx<T>*>(d.X);
+    a.Y = static_cast<cplx<T>*>(d.Y);
+    a.N = d.N; a.ldx = d.ld_same ? m : d.ldx; a.ldy = d.ld_same ? m : d.ldy;
+    a.m = m; a.sx = d.sx; a.sy = d.sy;
+    a.shift = d.shifted ? (T)(-d.sigma) : T(0);
+    a.cb = (T)d.cb;
+    const bool wall_self = std::is_same<T, float>::value && ((m | a.ldx | a.ldy) & 1) == 0 &&
+                           ((reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.Y)) & 15) == 0;
+    const int s = it / m;
+    hx_item<typename Column<T>::V, 8, BASIS>(a, s, it - s * m, wall_self);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -654,13 +706,6 @@ __device__ __forceinline__ void cp8z(unsigned dst, const void* src, int src_byte
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// Band order of the values in shared memory: Pryor's as copied (band b at word b - band_off),
-// the uncoupled order after conversion: S+, X+, Y+, Z+, S-, X-, Y-, Z- (six bands: no S; RAW: the
-// S values stay in words 0 and 1, the others follow).
-template <int NB, bool RAW> __device__ __forceinline__ constexpr int uslot(int b) {
-  return NB != 8 ? (b < 4 ? b - 1 : b - 2) : (RAW ? (b < 4 ? b + 1 : b) : b);
-}
 
 // raw_s: a converted cell keeps its two S values as copied (x0, x1 in slots 0 and 1) and the
 // reader takes i times them, which complex128 folds into its multiply-adds; in complex64 the
@@ -752,13 +797,38 @@ __device__ __forceinline__ void march_plane(const cplx<typename G::T>* cell,
   }
 }
 
-template <class G, int NB>
+// a finished output column written in its basis
+template <class G, int NB, int BASIS>
+__device__ __forceinline__ void store_column(const typename G::V (&lo)[8], cplx<typename G::T>* ys, long long bsy,
+                                             bool v16y, bool pair) {
+  typedef typename G::V V;
+  constexpr bool UNC = (BASIS & HX_Y_UNCOUPLED) != 0;
+  V x[8];
+  if (!UNC) from_uncoupled<V, NB>(lo, x);
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    if (UNC ? (NB != 8 && (b & 3) == 0) : !has_band<NB>(b)) continue;
+    const V v = UNC ? lo[b] : x[b];
+    auto* yb = ys + (UNC ? uslot<NB, false>(b) : b - band_off<NB>()) * bsy;
+    if constexpr (V::C == 1) {
+      vstore(yb, v);
+    } else if (v16y && pair) {
+      vstore(yb, v);
+    } else {
+      const float2 e0 = f2up(v.c[0]), e1 = f2up(v.c[1]);
+      yb[0] = e0;
+      if (pair) yb[1] = e1;
+    }
+  }
+}
+
+template <class G, int NB, int BASIS>
 __global__ void __launch_bounds__(G::THREADS, G::MINB)
 kp_march_kernel(const MarchArgs<typename G::T> a) {
   typedef typename G::V V;
   typedef typename G::T T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr bool RAW = raw_s<V>() && NB == 8;
+  constexpr bool CONV = !(BASIS & HX_X_UNCOUPLED), RAW = CONV && raw_s<V>() && NB == 8;
   constexpr int STAGE = (int)G::template stage_bytes<NB>();
   int bid = blockIdx.x;
   const int xs = bid % a.xsplit; bid /= a.xsplit;
@@ -837,7 +907,7 @@ kp_march_kernel(const MarchArgs<typename G::T> a) {
   copy_plane(p0);
   for (int p = p0; p <= p1; ++p) {
     cp_async_wait_all();
-    convert_plane(p);
+    if (CONV) convert_plane(p);
     __syncthreads();          // plane p is complete; every thread is done with plane p - 1
     if (p < p1) copy_plane(p + 1);
     if (active) {
@@ -853,25 +923,8 @@ kp_march_kernel(const MarchArgs<typename G::T> a) {
     for (int q = p - 1; q <= p; ++q) {
       const bool write = q == p - 1 ? q >= xa : (p == p1 && p < xb);
       if (q == p && !write) break;
-      if (write && active) {
-        V x[8];
-        from_uncoupled<V, NB>(lo, x);
-        cplx<T>* ys = yout + q * ystr;
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-          if (!has_band<NB>(b)) continue;
-          cplx<T>* yb = ys + (b - band_off<NB>()) * a.bsy;
-          if constexpr (V::C == 1) {
-            vstore(yb, x[b]);
-          } else if (a.v16y && col + 1 < a.m) {
-            vstore(yb, x[b]);
-          } else {
-            const float2 e0 = f2up(x[b].c[0]), e1 = f2up(x[b].c[1]);
-            yb[0] = e0;
-            if (col + 1 < a.m) yb[1] = e1;
-          }
-        }
-      }
+      if (write && active)
+        store_column<G, NB, BASIS>(lo, yout + q * ystr, a.bsy, a.v16y, col + 1 < a.m);
 #pragma unroll
       for (int b = 0; b < 8; ++b) { lo[b] = me[b]; me[b] = up[b]; }
     }
@@ -882,19 +935,19 @@ kp_march_kernel(const MarchArgs<typename G::T> a) {
 // The same march fed by the tensor-memory accelerator: one elected thread brings in a plane with
 // one bulk tensor copy (coordinates beyond the walls read as zeros) and the tile's records with
 // one bulk copy per tile row, completion on an mbarrier per stage, so no thread computes a copy
-// address. NS stages of planes are in flight; a plane is converted (CONV) after the previous
+// address. NS stages of planes are in flight; a plane is converted (where X is in Pryor's basis) after the previous
 // one's arithmetic, before the barrier that the two share. The launcher takes it where a tensor
 // map can describe the block (tma_fits).
 // ---------------------------------------------------------------------------------------------
 __device__ int g_apply_fault;      // set when a wait on a copy gave up (qdkp_device_fault)
 
-template <class G, int NB, int NS, bool CONV>
+template <class G, int NB, int NS, int BASIS>
 __global__ void __launch_bounds__(G::THREADS, G::MINB)
 kp_march_tma_kernel(const __grid_constant__ CUtensorMap tmx, const MarchArgs<typename G::T> a) {
   typedef typename G::V V;
   typedef typename G::T T;
   extern __shared__ unsigned char smem_raw[];
-  constexpr bool RAW = CONV && raw_s<V>() && NB == 8;
+  constexpr bool CONV = !(BASIS & HX_X_UNCOUPLED), RAW = CONV && raw_s<V>() && NB == 8;
   constexpr int STAGE = (int)G::template stage_bytes<NB>();
   constexpr int XBYTES = NB * G::BAND * 16;
   static_assert(STAGE % 128 == 0 && XBYTES % 128 == 0, "stages stay 128-byte aligned");
@@ -973,30 +1026,8 @@ kp_march_tma_kernel(const __grid_constant__ CUtensorMap tmx, const MarchArgs<typ
     for (int q = p - 1; q <= p; ++q) {
       const bool write = q == p - 1 ? q >= xa : (p == p1 && p < xb);
       if (q == p && !write) break;
-      if (write && active && ok) {
-        V x[8];
-        if (CONV) {
-          from_uncoupled<V, NB>(lo, x);
-        } else {
-#pragma unroll
-          for (int b = 0; b < 8; ++b) x[b] = lo[b];
-        }
-        cplx<T>* ys = yout + q * ystr;
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-          if (CONV ? !has_band<NB>(b) : (NB != 8 && (b & 3) == 0)) continue;
-          cplx<T>* yb = ys + (CONV ? b - band_off<NB>() : uslot<NB, false>(b)) * a.bsy;
-          if constexpr (V::C == 1) {
-            vstore(yb, x[b]);
-          } else if (a.v16y && col + 1 < a.m) {
-            vstore(yb, x[b]);
-          } else {
-            const float2 e0 = f2up(x[b].c[0]), e1 = f2up(x[b].c[1]);
-            yb[0] = e0;
-            if (col + 1 < a.m) yb[1] = e1;
-          }
-        }
-      }
+      if (write && active && ok)
+        store_column<G, NB, BASIS>(lo, yout + q * ystr, a.bsy, a.v16y, col + 1 < a.m);
 #pragma unroll
       for (int b = 0; b < 8; ++b) { lo[b] = me[b]; me[b] = up[b]; }
     }
@@ -1105,7 +1136,7 @@ static cudaError_t raise_smem(K kernel, size_t bytes, int device, std::atomic<un
   return e;
 }
 
-template <class G, int NB>
+template <class G, int NB, int BASIS>
 static int launch_march_g(const qdkp_operator* op, const typename G::T* rec, const void* X, int ldx,
                           void* Y, int ldy, int m, typename G::T shift, typename G::T cb, int sms,
                           cudaStream_t st) {
@@ -1113,7 +1144,7 @@ static int launch_march_g(const qdkp_operator* op, const typename G::T* rec, con
   constexpr size_t smem = G::template smem<NB>();
   static_assert((smem + 1024) * G::MINB <= 233472, "over the shared memory of one SM");
   static std::atomic<unsigned long long> raised{0};
-  QDKP_CUDA_TRY(raise_smem(kp_march_kernel<G, NB>, smem, op->device, raised));
+  QDKP_CUDA_TRY(raise_smem(kp_march_kernel<G, NB, BASIS>, smem, op->device, raised));
   const MarchGeom g = march_geom(op->nx, op->ny, op->nz, m, G::MC, G::TY, G::TZ, sms * G::MINB);
   MarchArgs<T> a;
   a.rec = rec;
@@ -1126,7 +1157,7 @@ static int launch_march_g(const qdkp_operator* op, const typename G::T* rec, con
   a.v16 = ((uintptr_t)X & 15) == 0 && ldx % 2 == 0;
   a.v16y = ((uintptr_t)Y & 15) == 0 && ldy % 2 == 0;
   a.shift = shift; a.cb = cb;
-  kp_march_kernel<G, NB><<<g.ctas, G::THREADS, smem, st>>>(a);
+  kp_march_kernel<G, NB, BASIS><<<g.ctas, G::THREADS, smem, st>>>(a);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;
@@ -1156,7 +1187,7 @@ static bool tma_fits(const qdkp_operator* op, const void* X, int64_t ldx, int m)
          op->ny >= G::PY && op->nz >= G::PZ && tensor_map_encoder() != nullptr;
 }
 
-template <class G, int NB, int NS, bool CONV>
+template <class G, int NB, int NS, int BASIS>
 static int launch_march_tma(const qdkp_operator* op, const typename G::T* rec, const void* X, int ldx,
                             void* Y, int ldy, int m, typename G::T shift, typename G::T cb, int sms,
                             cudaStream_t st) {
@@ -1164,7 +1195,7 @@ static int launch_march_tma(const qdkp_operator* op, const typename G::T* rec, c
   constexpr size_t smem = 128 + NS * G::template stage_bytes<NB>() + 8 * NS;
   static_assert((smem + 1024) * G::MINB <= 233472, "over the shared memory of one SM");
   static std::atomic<unsigned long long> raised{0};
-  QDKP_CUDA_TRY(raise_smem(kp_march_tma_kernel<G, NB, NS, CONV>, smem, op->device, raised));
+  QDKP_CUDA_TRY(raise_smem(kp_march_tma_kernel<G, NB, NS, BASIS>, smem, op->device, raised));
   // X as [band][x][y][z][column], in 8-byte elements with the column innermost
   constexpr int E = (int)sizeof(cplx<T>) / 8;
   const cuuint64_t ld = (cuuint64_t)ldx * sizeof(cplx<T>);
@@ -1193,13 +1224,13 @@ static int launch_march_tma(const qdkp_operator* op, const typename G::T* rec, c
   a.tiles_z = g.tiles_z; a.chunks = g.chunks; a.xsplit = g.xsplit; a.xlen = g.xlen;
   a.v16y = ((uintptr_t)Y & 15) == 0 && ldy % 2 == 0;
   a.shift = shift; a.cb = cb;
-  kp_march_tma_kernel<G, NB, NS, CONV><<<g.ctas, G::THREADS, smem, st>>>(tmx, a);
+  kp_march_tma_kernel<G, NB, NS, BASIS><<<g.ctas, G::THREADS, smem, st>>>(tmx, a);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;
 }
 
-template <typename T, int NB>
+template <typename T, int NB, int BASIS>
 static int launch_march(int cfg, const qdkp_operator* op, const T* rec, const void* X, int ldx,
                         void* Y, int ldy, int m, T shift, T cb, int sms, cudaStream_t st) {
   int rc = QDKP_OK;
@@ -1207,21 +1238,35 @@ static int launch_march(int cfg, const qdkp_operator* op, const T* rec, const vo
   each_shape<T>([&](int i, auto tag, double) {
     using G = typename decltype(tag)::G;
     if (i != (cfg < MarchCfgs<T>::kShapes ? cfg : 0) || !tma_fits<G>(op, X, ldx, m)) return false;
-    rc = launch_march_tma<G, NB, 2, true>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
+    rc = launch_march_tma<G, NB, 2, BASIS>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
     return done = true;
   });
   if (done) return rc;
   // a block no tensor map describes, or a grid or block smaller than the tile
-  return launch_march_g<typename MarchCfgs<T>::Any, NB>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
+  return launch_march_g<typename MarchCfgs<T>::Any, NB, BASIS>(op, rec, X, ldx, Y, ldy, m, shift, cb, sms, st);
 }
 
-int launch_apply_multi(const HXSlot* slots_dev, int nslots, int total_tiles, int precision,
-                       cudaStream_t st) {
+int launch_apply_multi(const HXSlot* slots_dev, int nslots, int total_tiles, int precision, int basis,
+                       int max_ctas, cudaStream_t st) {
   if (total_tiles <= 0) return QDKP_OK;
-  if (precision == QDKP_C128)
-    kp_apply_multi_kernel<double><<<total_tiles, kApplyThreads, 0, st>>>(slots_dev, nslots);
-  else
-    kp_apply_multi_kernel<float><<<total_tiles, kApplyThreads, 0, st>>>(slots_dev, nslots);
+  const auto launch = [&](auto kernel, int ctas) {
+    kernel<<<ctas, kApplyThreads, 0, st>>>(slots_dev, nslots, total_tiles);
+  };
+  const auto of_basis = [&](auto tag) {
+    typedef decltype(tag) T;
+    const int n = total_tiles;
+    if (max_ctas < n) {
+      if (basis == HX_X_UNCOUPLED) launch(kp_apply_multi_kernel<T, HX_X_UNCOUPLED, true>, max_ctas);
+      else if (basis == HX_Y_UNCOUPLED) launch(kp_apply_multi_kernel<T, HX_Y_UNCOUPLED, true>, max_ctas);
+      else launch(kp_apply_multi_kernel<T, 0, true>, max_ctas);
+    } else {
+      if (basis == HX_X_UNCOUPLED) launch(kp_apply_multi_kernel<T, HX_X_UNCOUPLED, false>, n);
+      else if (basis == HX_Y_UNCOUPLED) launch(kp_apply_multi_kernel<T, HX_Y_UNCOUPLED, false>, n);
+      else launch(kp_apply_multi_kernel<T, 0, false>, n);
+    }
+  };
+  if (precision == QDKP_C128) of_basis(double());
+  else of_basis(float());
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;
@@ -1289,18 +1334,18 @@ static int pick_tile(const qdkp_operator* op, const void* X, int64_t ldx, int m,
 
 // The direct kernel; a block of few items is spread over the whole chip in small CTAs (23x23x20 x 1:
 // 42 CTAs of 256 threads would leave 106 SMs idle; 8.0 -> 5.1 us with 64).
-template <typename T, int NB>
+template <typename T, int NB, int BASIS>
 static int launch_direct(const qdkp_operator* op, const HXArgs<T>& a, int sms, cudaStream_t st) {
   const int64_t items = op->n_sites * a.m;
   int threads = kApplyThreads;
   while (threads > 64 && items < (int64_t)threads * 2 * sms) threads /= 2;
-  kp_apply_kernel<T, NB><<<(unsigned)((items + threads - 1) / threads), threads, 0, st>>>(a);
+  kp_apply_kernel<T, NB, BASIS><<<(unsigned)((items + threads - 1) / threads), threads, 0, st>>>(a);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;
 }
 
-template <typename T>
+template <typename T, int BASIS>
 static int launch_apply_t(const qdkp_operator* op, const T* rec, const void* X, int64_t ldx,
                           void* Y, int64_t ldy, int m, double sigma, int shifted, int precision,
                           cudaStream_t st) {
@@ -1315,8 +1360,8 @@ static int launch_apply_t(const qdkp_operator* op, const T* rec, const void* X, 
   const int cfg = forced == QDKP_TILE_AUTO ? pick_tile<T>(op, X, ldx, m, sms) : forced;
   if (cfg != kDirect && op->n_bands != 4 && ((uintptr_t)X % sizeof(cplx<T>)) == 0) {
     if (op->n_bands == 8)
-      return launch_march<T, 8>(cfg, op, rec, X, (int)ldx, Y, (int)ldy, m, shift, cb, sms, st);
-    return launch_march<T, 6>(cfg, op, rec, X, (int)ldx, Y, (int)ldy, m, shift, cb, sms, st);
+      return launch_march<T, 8, BASIS>(cfg, op, rec, X, (int)ldx, Y, (int)ldy, m, shift, cb, sms, st);
+    return launch_march<T, 6, BASIS>(cfg, op, rec, X, (int)ldx, Y, (int)ldy, m, shift, cb, sms, st);
   }
   HXArgs<T> a;
   a.rec = rec;
@@ -1328,22 +1373,39 @@ static int launch_apply_t(const qdkp_operator* op, const T* rec, const void* X, 
   a.shift = shift;
   a.cb = cb;
   switch (op->n_bands) {
-    case 8: return launch_direct<T, 8>(op, a, sms, st);
-    case 6: return launch_direct<T, 6>(op, a, sms, st);
-    case 4: return launch_direct<T, 4>(op, a, sms, st);
+    case 8: return launch_direct<T, 8, BASIS>(op, a, sms, st);
+    case 6: return launch_direct<T, 6, BASIS>(op, a, sms, st);
+    case 4: return launch_direct<T, 4, 0>(op, a, sms, st);
     default: set_error("n_bands must be 8, 6 or 4"); return QDKP_ERR_ARG;
   }
 }
 
-// Y = sign*H X (- sigma X if shifted) for one block in the given precision.
-int launch_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int64_t ldy,
-                 int m, double sigma, int shifted, int precision, cudaStream_t st) {
+template <int BASIS>
+static int launch_apply_b(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int64_t ldy,
+                          int m, double sigma, int shifted, int precision, cudaStream_t st) {
   if (precision == QDKP_C128)
-    return launch_apply_t<double>(op, op->rec64, X, ldx, Y, ldy, m, sigma, shifted, precision, st);
+    return launch_apply_t<double, BASIS>(op, op->rec64, X, ldx, Y, ldy, m, sigma, shifted, precision, st);
   if (precision == QDKP_C64)
-    return launch_apply_t<float>(op, op->rec32, X, ldx, Y, ldy, m, sigma, shifted, precision, st);
+    return launch_apply_t<float, BASIS>(op, op->rec32, X, ldx, Y, ldy, m, sigma, shifted, precision, st);
   set_error("precision must be QDKP_C128 or QDKP_C64");
   return QDKP_ERR_ARG;
+}
+
+// Y = sign*H X (- sigma X if shifted) for one block in the given precision.
+int launch_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int64_t ldy,
+                 int m, double sigma, int shifted, int precision, cudaStream_t st, int basis) {
+  if (basis == HX_X_UNCOUPLED)
+    return launch_apply_b<HX_X_UNCOUPLED>(op, X, ldx, Y, ldy, m, sigma, shifted, precision, st);
+  if (basis == HX_Y_UNCOUPLED)
+    return launch_apply_b<HX_Y_UNCOUPLED>(op, X, ldx, Y, ldy, m, sigma, shifted, precision, st);
+  return launch_apply_b<0>(op, X, ldx, Y, ldy, m, sigma, shifted, precision, st);
+}
+
+int launch_folded(const qdkp_operator* op, const void* X, int64_t ldx, void* T, void* Y, int64_t ldy,
+                  int m, double sigma, int precision, cudaStream_t st) {
+  const int rc = launch_apply(op, X, ldx, T, m, m, sigma, 1, precision, st, HX_Y_UNCOUPLED);
+  if (rc != QDKP_OK) return rc;
+  return launch_apply(op, T, m, Y, ldy, m, sigma, 1, precision, st, HX_X_UNCOUPLED);
 }
 
 }  // namespace qdkp

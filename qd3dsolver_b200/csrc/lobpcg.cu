@@ -29,9 +29,6 @@
 
 namespace qdkp {
 
-int launch_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int64_t ldy,
-                 int m, double sigma, int shifted, int precision, cudaStream_t st);
-
 namespace {
 
 constexpr int kNormParts = 296;
@@ -58,7 +55,8 @@ struct Solver {
   qdkp_lobpcg_params prm;
   cudaStream_t st;
   cudaStream_t side = nullptr;         // reads the decisions while st goes on
-  cudaEvent_t decided = nullptr;
+  cudaStream_t pst = nullptr;          // the work on P, beside that on R
+  cudaEvent_t decided = nullptr, p_done = nullptr;
   int64_t n;
   int m;
   SlotLayout L;
@@ -69,10 +67,10 @@ struct Solver {
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev;   // per-launch timing (time_hx)
   size_t ev_used = 0;
 
-  int hx(const double2* V, int c, double2* out, double sigma, int shifted) {
+  int hx(const double2* V, int c, double2* out, double sigma, int shifted, int basis = 0) {
     ++hx_launches;
     hx_bytes += (double)op->n_sites * (15.0 * 8.0 + 2.0 * 8.0 * c * 16.0);
-    if (!prm.time_hx) return launch_apply(op, V, c, out, c, c, sigma, shifted, QDKP_C128, st);
+    if (!prm.time_hx) return launch_apply(op, V, c, out, c, c, sigma, shifted, QDKP_C128, st, basis);
     if (ev_used == ev.size()) {
       cudaEvent_t a, b2;
       QDKP_CUDA_TRY(cudaEventCreate(&a));
@@ -81,7 +79,7 @@ struct Solver {
     }
     auto& e = ev[ev_used++];
     QDKP_CUDA_TRY(cudaEventRecord(e.first, st));
-    int rc = launch_apply(op, V, c, out, c, c, sigma, shifted, QDKP_C128, st);
+    int rc = launch_apply(op, V, c, out, c, c, sigma, shifted, QDKP_C128, st, basis);
     QDKP_CUDA_TRY(cudaEventRecord(e.second, st));
     return rc;
   }
@@ -99,16 +97,18 @@ struct Solver {
   ~Solver() {
     for (auto& e : ev) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     if (side) cudaStreamDestroy(side);
+    if (pst) { cudaStreamSynchronize(pst); cudaStreamDestroy(pst); }
     if (decided) cudaEventDestroy(decided);
+    if (p_done) cudaEventDestroy(p_done);
   }
 
   // A(V) for V (n x c, ld c) into out (ld c)
   int applyA(const double2* V, int c, double2* out) {
     applies += c;
     if (prm.folded) {
-      int rc = hx(V, c, d.T, prm.sigma, 1);
+      int rc = hx(V, c, d.T, prm.sigma, 1, HX_Y_UNCOUPLED);
       if (rc) return rc;
-      return hx(d.T, c, out, prm.sigma, 1);
+      return hx(d.T, c, out, prm.sigma, 1, HX_X_UNCOUPLED);
     }
     return hx(V, c, out, 0.0, 0);
   }
@@ -191,9 +191,9 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
   // ---- X = orthonormalise(X0) ------------------------------------------------------------
   TRY(launch_copy((const double2*)X0, m, m, n, d.Ra, m, st));
   TRY(s.gram(blist({{d.Ra, m}}, m), blist({{d.Ra, m}}, m), d.gS));
-  TRY(launch_chol_inv(d.gS, m, d.U, (int*)d.G, st));
+  TRY(launch_chol_inv(d.gS, m, d.U, (int*)d.Up, st));
   int hstat;
-  TRY(s.sync_read(&hstat, d.G, sizeof(int)));
+  TRY(s.sync_read(&hstat, d.Up, sizeof(int)));
   if (hstat) { set_error("Linearly dependent initial approximations"); return QDKP_ERR_NUMERIC; }
   {
     const double2* C[1] = {d.U};
@@ -202,7 +202,7 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
   // ---- initial Ritz vectors ------------------------------------------------------------------
   TRY(s.applyA(d.X, m, d.AX));
   TRY(s.gram(blist({{d.X, m}}, m), blist({{d.AX, m}}, m), d.gT));
-  TRY(launch_eigh(d.gT, nullptr, m, d.w, d.E, d.scr, (int*)d.G, st));
+  TRY(launch_eigh(d.gT, nullptr, m, d.w, d.E, d.scr, (int*)d.Up, st));
   {
     const double2* C[1] = {d.E};
     TRY(launch_update(blist({{d.X, m}}, m), C, m, n, d.X, m, 0, st));
@@ -220,7 +220,9 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
   TRY(s.put(d.st, &es, sizeof(es)));
   TRY(s.put(tables, &d, sizeof(d)));
   QDKP_CUDA_TRY(cudaStreamCreateWithFlags(&s.side, cudaStreamNonBlocking));
+  QDKP_CUDA_TRY(cudaStreamCreateWithFlags(&s.pst, cudaStreamNonBlocking));
   QDKP_CUDA_TRY(cudaEventCreateWithFlags(&s.decided, cudaEventDisableTiming));
+  QDKP_CUDA_TRY(cudaEventCreateWithFlags(&s.p_done, cudaEventDisableTiming));
   set_slot_kernel_limits();
   EGroup G;
   G.d_slots = reinterpret_cast<ESlot*>(tables);
@@ -232,9 +234,13 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
   for (;;) {
     TRY(launch_decide(G, st));
     QDKP_CUDA_TRY(cudaEventRecord(s.decided, st));
-    TRY(launch_residual_block(G, st));
-    TRY(launch_project(G, st));
-    // the projection needs nothing of the host: it runs while the host reads the decisions
+    // H.X launches are timed alone
+    const cudaStream_t ps = prm->time_hx ? st : s.pst;
+    if (ps != st) QDKP_CUDA_TRY(cudaStreamWaitEvent(ps, s.decided, 0));
+    TRY(launch_p_chain(G, ps));
+    QDKP_CUDA_TRY(cudaEventRecord(s.p_done, ps));
+    TRY(launch_r_chain(G, st));
+    // none of this needs the host: it runs while the host reads the decisions
     QDKP_CUDA_TRY(cudaStreamWaitEvent(s.side, s.decided, 0));
     QDKP_CUDA_TRY(cudaMemcpyAsync(&es, d.snap, sizeof(es), cudaMemcpyDeviceToHost, s.side));
     QDKP_CUDA_TRY(cudaStreamSynchronize(s.side));
@@ -243,10 +249,14 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
       std::memcpy(&hist[(size_t)it * m], es.norms, m * sizeof(double));
     }
     have_best = have_best || es.copy_best;
-    if (!es.running) break;
+    if (!es.running) {
+      QDKP_CUDA_TRY(cudaStreamWaitEvent(st, s.p_done, 0));      // the best iterate's copy
+      break;
+    }
     // scipy recomputes A X on a forced restart but keeps the residuals of the old A X
     if (!es.skip_recompute) TRY(s.applyA(d.X, m, d.AX));
     TRY(s.applyA(d.Ra, es.ma, d.ARa));
+    QDKP_CUDA_TRY(cudaStreamWaitEvent(st, s.p_done, 0));
     TRY(launch_ritz_step(G, st));
     if (prm->verbosity > 1)
       fprintf(stderr, "lobpcg it %d active %d restart %d explicit %d\n", it, es.ma, es.restart,
@@ -310,8 +320,8 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
     TRY(s.put(d.gA, a.data(), a.size() * sizeof(double2)));
     TRY(s.put(d.gB, bb.data(), bb.size() * sizeof(double2)));
   }
-  TRY(launch_eigh(d.gA, d.gB, m, d.w, d.E, d.scr, (int*)d.G, st));
-  TRY(s.sync_read(&hstat, d.G, sizeof(int)));
+  TRY(launch_eigh(d.gA, d.gB, m, d.w, d.E, d.scr, (int*)d.Up, st));
+  TRY(s.sync_read(&hstat, d.Up, sizeof(int)));
   if (hstat) { set_error("eigh has failed in lobpcg postprocessing"); return QDKP_ERR_NUMERIC; }
   TRY(s.sync_read(lam.data(), d.w, m * sizeof(double)));
   {

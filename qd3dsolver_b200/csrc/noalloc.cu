@@ -16,9 +16,6 @@
 
 namespace qdkp {
 
-int launch_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int64_t ldy,
-                 int m, double sigma, int shifted, int precision, cudaStream_t st);
-
 // The scratch: one folded intermediate of at most QDKP_NOALLOC_SCRATCH_BYTES.
 static __device__ __align__(256) unsigned char g_fold_scratch[QDKP_NOALLOC_SCRATCH_BYTES];
 
@@ -76,8 +73,7 @@ int qdkp_apply_folded_noalloc(const qdkp_operator* op, const void* X, int64_t ld
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // Every element of T that the second launch reads is written by the first one in this
     // call, so nothing left over from an earlier call is ever read and nothing needs clearing.
-    rc = launch_apply(op, X, ldx, T, m, m, sigma, 1, precision, st);
-    if (rc == QDKP_OK) rc = launch_apply(op, T, m, Y, ldy, m, sigma, 1, precision, st);
+    rc = launch_folded(op, X, ldx, T, Y, ldy, m, sigma, precision, st);
   }
   if (prev != op->device) cudaSetDevice(prev);
   return rc;

@@ -99,8 +99,20 @@ struct HXSlot {
   double cb;              // conduction-band face weight (apply_cb_weight)
 };
 
-int launch_apply_multi(const HXSlot* slots_dev, int nslots, int total_tiles, int precision,
-                       cudaStream_t st);
+// Basis of an apply's blocks: X, or Y, in the uncoupled (S, X, Y, Z) x spin basis instead of Pryor's.
+// The two applies of a folded operator pass their block between them so, which spares the second its
+// conversions and the first the back-transform. (Four bands do not span the uncoupled states: a
+// four-band apply takes Pryor's whatever is asked, on both sides alike.)
+enum { HX_X_UNCOUPLED = 1, HX_Y_UNCOUPLED = 2 };
+
+int launch_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int64_t ldy,
+                 int m, double sigma, int shifted, int precision, cudaStream_t st, int basis = 0);
+// Y = (H - sigma)^2 X through the n x m block T (whose contents are of no basis of the caller's)
+int launch_folded(const qdkp_operator* op, const void* X, int64_t ldx, void* T, void* Y, int64_t ldy,
+                  int m, double sigma, int precision, cudaStream_t st);
+// The shifted (folded) slots if basis is not 0, the others if it is; at most max_ctas CTAs.
+int launch_apply_multi(const HXSlot* slots_dev, int nslots, int total_tiles, int precision, int basis,
+                       int max_ctas, cudaStream_t st);
 // CTAs one H.X launch uses for n_sites x m items
 int apply_tiles(int64_t n_sites, int m);
 double apply_cb_weight(const qdkp_operator* op);
