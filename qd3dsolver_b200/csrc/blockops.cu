@@ -308,8 +308,12 @@ chol_inv_kernel(const double2* __restrict__ G, int n, double2* __restrict__ Uinv
   double2* S1 = ssm + n * n;
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) ssm[e] = G[e];
   __syncthreads();
-  __shared__ double rinv[kMaxSmall];
-  const int fail = rr_cholesky(ssm, n, rinv, 0);
+  __shared__ double rinv[kMaxSmall], least[kMaxSmall];
+  // a pivot of a few rounding units of its diagonal is a dependent column, whichever sign the rounding
+  // left it with
+  for (int k = threadIdx.x; k < n; k += blockDim.x) least[k] = 8.9e-16 * ssm[k * n + k].x;
+  __syncthreads();
+  const int fail = rr_cholesky(ssm, n, rinv, 0, least);
   if (threadIdx.x == 0) *status = fail;
   if (fail) return;
   rr_upper_inverse(ssm, n, rinv, S1);

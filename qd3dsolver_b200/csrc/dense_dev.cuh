@@ -235,8 +235,9 @@ struct RrShared {
 // conj(S_ki) S_kj / S_kk from S_ij (k < i <= j) with the unscaled pivot row; the rows are scaled
 // by 1 / sqrt(S_kk) at the end. rinv = 1 / U_kk. Returns nonzero on a bad pivot. The leading k0
 // columns are the identity's (S = [I V; V^H W] with V of k0 rows): their steps touch the trailing
-// block alone and are taken together, four lanes an entry.
-static __device__ int rr_cholesky(double2* __restrict__ S, int n, double* __restrict__ rinv, int k0) {
+// block alone and are taken together, four lanes an entry. A pivot must exceed least[k] (NULL: 0).
+static __device__ int rr_cholesky(double2* __restrict__ S, int n, double* __restrict__ rinv, int k0,
+                                  const double* __restrict__ least = nullptr) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwp = blockDim.x >> 5;
   if (k0) {
     const int np = n - k0;
@@ -261,7 +262,7 @@ static __device__ int rr_cholesky(double2* __restrict__ S, int n, double* __rest
 #pragma unroll 1
   for (int k = k0; k < n; ++k) {
     const double d = S[k * n + k].x;
-    if (!(d > 0.0) || !isfinite(d)) { __syncthreads(); return 1; }
+    if (!(d > (least ? least[k] : 0.0)) || !isfinite(d)) { __syncthreads(); return 1; }
     const double inv = 1.0 / d;
     for (int i = k + 1 + warp; i < n; i += nwp) {
       const double2 a = S[k * n + i];

@@ -111,3 +111,25 @@ def test_eigh_all_pairs_of_a_block(n, kind):
     assert np.abs(w - np.sort(lam)).max() <= tol
     assert np.abs(A @ V - V * w).max() <= tol
     assert np.abs(V.conj().T @ V - np.eye(n)).max() <= tol
+
+
+@pytest.mark.parametrize('m, a, b', [(2, 0, 1), (6, 1, 3), (12, 0, 11), (13, 11, 12), (24, 7, 16)])
+def test_repeated_columns_are_refused(m, a, b):
+    """A start block with a repeated column: the pivot is rounding noise of either sign."""
+    import torch
+    from qd3dsolver_b200 import _lib, kp_pryor as kpg, serving
+    from qd3dsolver_b200.eigensolvers import lobpcg_device, start_block
+    keys = ('gamma1', 'gamma2', 'gamma3', 'P0', 'Ec', 'Ev', 'delta_so', 'b', 'd')
+    shape = (5, 7, 6)
+    H = kpg.confined_hamiltonian(kpg.GridOperators(shape, 0.5), {k: np.ones(shape) for k in keys}, 8)
+    for seed in range(4):
+        X0 = start_block(H.shape[0], m, seed, True)
+        X0[:, b] = X0[:, a]
+        with pytest.raises(_lib.QdkpError, match='Linearly dependent initial approximations'):
+            lobpcg_device(H, X0, folded=False, sigma=0.0, tol=1e-9, maxiter=2)
+        eng = serving.Engine(1)
+        r = serving.Request(H, k=m, extra=0, folded=False, maxiter=2)
+        with pytest.raises(_lib.QdkpError, match='Linearly dependent initial approximations'):
+            eng.admit(r, X0=torch.from_numpy(X0).cuda())
+        eng.close()
+    H.close()
