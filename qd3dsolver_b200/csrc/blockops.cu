@@ -10,6 +10,7 @@
 
 #include "dense_dev.cuh"
 #include "gram_dev.cuh"
+#include "gram_tf32_dev.cuh"
 #include "umma_dev.cuh"
 
 namespace qdkp {
@@ -131,6 +132,66 @@ gram_reduce_kernel(const GramTask<T> t, int parts, const double* __restrict__ pa
 size_t gram_partial_elems(int P, int Q) {
   const size_t rects = (size_t)((P + kGramRect - 1) / kGramRect) * ((Q + kGramRect - 1) / kGramRect);
   return rects * kGramMaxParts * kGramRectElems / 2;
+}
+
+// ... of a qdkp_block_gram, in either precision
+static size_t block_gram_elems(int P, int Q) {
+  const size_t fp64 = gram_partial_elems(P, Q);
+  return gram_tf32_threads(P, Q) ? std::max(fp64, gram_tf32_doubles(P, Q) / 2) : fp64;
+}
+
+__global__ void __launch_bounds__(512)
+gram_tf32_kernel(const BlockList<float> A, const BlockList<float> B, long long n, long long rows_per_part,
+                 double* __restrict__ partial) {
+  extern __shared__ __align__(16) unsigned char gsm_f[];
+  const long long r0 = blockIdx.x * rows_per_part;
+  const int RP = (2 * A.total() + 7) / 8 * 8, RQ = (2 * B.total() + 7) / 8 * 8;
+  gram_core_tf32(A, B, r0, min(n, r0 + rows_per_part), partial + (long long)blockIdx.x * RP * RQ, gsm_f);
+}
+
+// out = the parts' sum as a complex P x Q product, 32 entries a CTA: each of 8 warps adds an eighth of the
+// parts in order, then the eighths are added in order
+__global__ void __launch_bounds__(256)
+gram_tf32_reduce_kernel(const double* __restrict__ partial, int parts, int P, int Q, double2* __restrict__ out) {
+  __shared__ double2 s_sum[8][32];
+  const int RP = (2 * P + 7) / 8 * 8, RQ = (2 * Q + 7) / 8 * 8;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, o = blockIdx.x * 32 + lane;
+  const int i = o / Q, j = o - i * Q, per = (parts + 7) / 8;
+  double2 v = make_double2(0.0, 0.0);
+  if (o < P * Q) {
+    const double* c = partial + (long long)(2 * i) * RQ + 2 * j;
+#pragma unroll 4
+    for (int b = warp * per; b < min(parts, (warp + 1) * per); ++b) {
+      const double* q = c + (long long)b * RP * RQ;
+      v.x += __ldcg(q) + __ldcg(q + RQ + 1);
+      v.y += __ldcg(q + 1) - __ldcg(q + RQ);
+    }
+  }
+  s_sum[warp][lane] = v;
+  __syncthreads();
+  if (warp || o >= P * Q) return;
+  for (int w = 1; w < 8; ++w) { v.x += s_sum[w][lane].x; v.y += s_sum[w][lane].y; }
+  out[o] = v;
+}
+
+static int launch_gram_tf32(const BlockList<float>& A, const BlockList<float>& B, long long n, int threads,
+                            double2* partial, size_t partial_elems, double2* out, cudaStream_t st) {
+  const int P = A.total(), Q = B.total();
+  if (gram_tf32_doubles(P, Q) > 2 * partial_elems) {
+    set_error("gram partial buffer too small");
+    return QDKP_ERR_WORKSPACE;
+  }
+  long long parts = std::max(1LL, std::min<long long>((n + 255) / 256, kGramTfParts));
+  const long long rpp = ((n + parts - 1) / parts + 3) / 4 * 4;
+  parts = (n + rpp - 1) / rpp;
+  const size_t smem = gram_smem_bytes(P, Q, (int)sizeof(float2));
+  QDKP_CUDA_TRY(cudaFuncSetAttribute(gram_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  double* pd = reinterpret_cast<double*>(partial);
+  gram_tf32_kernel<<<(unsigned)parts, threads, smem, st>>>(A, B, n, rpp, pd);
+  gram_tf32_reduce_kernel<<<(P * Q + 31) / 32, 256, 0, st>>>(pd, (int)parts, P, Q, out);
+  count_launch(2);
+  QDKP_CUDA_TRY(cudaGetLastError());
+  return QDKP_OK;
 }
 
 template <typename T>
@@ -387,7 +448,7 @@ extern "C" {
 
 size_t qdkp_block_gram_workspace_size(int P, int Q) {
   if (P < 1 || Q < 1 || P > kMaxSmall || Q > kMaxSmall) return 0;
-  return gram_partial_elems(P, Q) * sizeof(double2) + (size_t)P * Q * sizeof(double2) + 256;
+  return block_gram_elems(P, Q) * sizeof(double2) + (size_t)P * Q * sizeof(double2) + 256;
 }
 
 int qdkp_block_gram(const void* A, int64_t lda, int P, const void* B, int64_t ldb, int Q,
@@ -402,7 +463,7 @@ int qdkp_block_gram(const void* A, int64_t lda, int P, const void* B, int64_t ld
     return QDKP_ERR_WORKSPACE;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t pe = gram_partial_elems(P, Q);
+  const size_t pe = block_gram_elems(P, Q);
   double2* part = static_cast<double2*>(ws);
   double2* dout = part + pe;
   int rc;
@@ -410,7 +471,9 @@ int qdkp_block_gram(const void* A, int64_t lda, int P, const void* B, int64_t ld
     BlockList<float> La, Lb;
     La.nblk = 1; La.p[0] = static_cast<const float2*>(A); La.ld[0] = lda; La.cols[0] = P;
     Lb.nblk = 1; Lb.p[0] = static_cast<const float2*>(B); Lb.ld[0] = ldb; Lb.cols[0] = Q;
-    rc = launch_gram(La, Lb, n, part, pe, dout, st);
+    const int threads = gram_tf32_threads(P, Q);
+    rc = threads ? launch_gram_tf32(La, Lb, n, threads, part, pe, dout, st)
+                 : launch_gram(La, Lb, n, part, pe, dout, st);
   } else {
     BlockList<double> La, Lb;
     La.nblk = 1; La.p[0] = static_cast<const double2*>(A); La.ld[0] = lda; La.cols[0] = P;

@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize('prec', ['c128', 'c64'])
 @pytest.mark.parametrize('n, P, Q, lda, ldb', [
     (1, 1, 1, 1, 1), (7, 3, 2, 3, 2), (31, 12, 12, 12, 12), (33, 5, 24, 7, 24), (1023, 13, 1, 13, 3),
-    (1024, 36, 24, 36, 24), (1025, 36, 36, 37, 36), (4099, 72, 72, 72, 72), (151_553, 12, 5, 12, 5)])
+    (1024, 36, 24, 36, 24), (1025, 36, 36, 37, 36), (4099, 72, 72, 72, 72),
+    (1030, 61, 51, 61, 51), (1031, 61, 51, 62, 51), (151_553, 12, 5, 12, 5)])
 def test_gram_edges(n, P, Q, lda, ldb, prec):
     import torch
     from qd3dsolver_b200 import _lib
@@ -30,6 +31,8 @@ def test_gram_edges(n, P, Q, lda, ldb, prec):
     ws = torch.empty(int(L.qdkp_block_gram_workspace_size(max(P, Q), max(P, Q))),
                      dtype=torch.uint8, device='cuda')
     for d2, ld2, c2, B2 in ((dB, ldb, Q, B), (dA, lda, P, A)):      # A^H B, and A^H A
+        if prec == 'c64' and -(-P // 12) * -(-c2 // 12) <= 16:
+            continue        # a complex64 product that one CTA holds is another kernel's (split TF32)
         out = np.empty((P, c2), dtype=np.complex128)
         _lib.check(L.qdkp_block_gram(dA.data_ptr(), lda, P, d2.data_ptr(), ld2, c2, n, code,
                                      out.ctypes.data, ws.data_ptr(), ws.numel(), None),
