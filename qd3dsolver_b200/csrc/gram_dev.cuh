@@ -116,11 +116,15 @@ __host__ __device__ inline int gram_need(int kind, int P, int Q, int m, int ma, 
   return 0;
 }
 
-// Rows of a chunk: about 62 KB, a multiple of 32. A block's share of a stage: four runs of crow / 4
-// rows, each followed by kGramSkew bytes.
+// Rows of a chunk: about 62 KB, for few columns 25 KB, a multiple of 32. A block's share of a stage:
+// four runs of crow / 4 rows, each followed by kGramSkew bytes.
+// Few columns (the products of one or two blocks of 12): their few warps leave room for a second CTA
+// on the SM, so their ring takes less than half of its shared memory. A CTA's start and its sums then
+// hide behind the other's rows (seven complex128 slots: 47.3 to 47.0 ms of a sweep).
 constexpr int kGramSkew = 32;
+constexpr int kGramNarrow = 24;
 template <typename T> __host__ __device__ inline int gram_crow(int tc) {
-  const int r = 62 * 1024 / (tc * (int)sizeof(cplx<T>)) / 32 * 32;
+  const int r = (tc <= kGramNarrow ? 25 : 62) * 1024 / (tc * (int)sizeof(cplx<T>)) / 32 * 32;
   return r < 32 ? 32 : (r > 128 ? 128 : r);
 }
 template <typename T> __host__ __device__ inline size_t gram_stage(int tc) {
@@ -131,7 +135,7 @@ constexpr int kGramStages = 6;
 constexpr size_t kGramTable = 128;               // the barriers
 // shared memory of a launch for at most tc concatenated columns and `warps` consumer warps
 template <typename T> __host__ __device__ inline size_t gram_smem(int tc, int warps) {
-  const size_t st = gram_stage<T>(tc), ring = 190 * 1024;
+  const size_t st = gram_stage<T>(tc), ring = (tc <= kGramNarrow ? 101 : 190) * 1024;
   const size_t bytes = kGramStages * st < ring ? kGramStages * st : (2 * st > ring ? 2 * st : ring);
   const size_t red = (size_t)warps * kGramRectElems * sizeof(double);
   return kGramTable + (bytes > red ? bytes : red);
@@ -260,10 +264,13 @@ static __device__ void gram_core(const GramTask<T>& t, int part, int parts, int 
     s_rect[index - first] = (short)(threadIdx.x / gc * 64 + threadIdx.x % gc + (need == 2 ? 8192 : 0));
   }
   const int slices = nwarps / count;
-  // contiguous rows of whole 16-byte words in every block: bulk copies
+  // contiguous rows whose runs are whole 16-byte words in every block: bulk copies. Runs start at rows
+  // that are multiples of four and, where n is even, have an even number of them, which makes odd
+  // complex64 widths whole too
   bool bulk = true;
   for (int b = 0; b < t.nblk; ++b)
-    bulk = bulk && (t.cols[b] == 0 || t.ld[b] == t.cols[b]) && (sizeof(T) == 8 || (t.cols[b] & 1) == 0) &&
+    bulk = bulk && (t.cols[b] == 0 || t.ld[b] == t.cols[b]) &&
+           (sizeof(T) == 8 || (t.cols[b] & 1) == 0 || (t.n & 1) == 0) &&
            (reinterpret_cast<uintptr_t>(t.p[b]) & 15) == 0;
   const int crow = gram_crow<T>(t.tc), c4 = crow / 4;
   const unsigned stage = (unsigned)gram_stage<T>(t.tc);
