@@ -120,7 +120,7 @@ __host__ __device__ inline int gram_need(int kind, int P, int Q, int m, int ma, 
 // four runs of crow / 4 rows, each followed by kGramSkew bytes.
 // Few columns (the products of one or two blocks of 12): their few warps leave room for a second CTA
 // on the SM, so their ring takes less than half of its shared memory. A CTA's start and its sums then
-// hide behind the other's rows (seven complex128 slots: 47.3 to 47.0 ms of a sweep).
+// hide behind the other's rows (14 complex128 slots, 8 ticks: 47.3 to 47.0 ms).
 constexpr int kGramSkew = 32;
 constexpr int kGramNarrow = 24;
 template <typename T> __host__ __device__ inline int gram_crow(int tc) {

@@ -1339,9 +1339,11 @@ static int launch_direct(const qdkp_operator* op, const HXArgs<T>& a, int sms, c
   const int64_t items = op->n_sites * a.m;
   int threads = kApplyThreads;
   while (threads > 64 && items < (int64_t)threads * 2 * sms) threads /= 2;
-  kp_apply_kernel<T, NB, BASIS><<<(unsigned)((items + threads - 1) / threads), threads, 0, st>>>(a);
+  // a single column's call is bound by the host: one runtime call, which returns its own error
+  void* args[] = {const_cast<HXArgs<T>*>(&a)};
+  QDKP_CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(&kp_apply_kernel<T, NB, BASIS>),
+                                 dim3((unsigned)((items + threads - 1) / threads)), dim3(threads), args, 0, st));
   count_launch();
-  QDKP_CUDA_TRY(cudaGetLastError());
   return QDKP_OK;
 }
 
