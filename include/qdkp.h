@@ -258,9 +258,9 @@ size_t qdkp_engine_slot_workspace_size(const qdkp_operator* op, const qdkp_lobpc
 int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg_params* prm,
                       const void* X0, void* ws, size_t ws_bytes, void* stream, int* slot);
 /* Launch `ticks` iterations of every running slot (asynchronous on `stream`). The tick sequence
- * is fixed for a slot layout, so by default it is captured once per layout (and tick count) as
- * a CUDA graph and replayed on the engine's own stream, ordered after `stream` and before later
- * work on it by events. */
+ * is fixed for a slot layout, so by default one tick is captured once per layout as CUDA graphs
+ * and replayed on the engine's own streams, ordered after `stream` and before later work on it
+ * by events. */
 int qdkp_engine_step(qdkp_engine* e, int ticks, void* stream);
 /* 0: launch the tick kernels directly on the caller's stream instead of replaying a graph. */
 int qdkp_engine_set_graphs(qdkp_engine* e, int enable);
@@ -295,11 +295,11 @@ int qdkp_block_update(const void* A, int64_t lda, int P, const double* C, int q,
 /*
  * The Rayleigh-Ritz eigensolve of a LOBPCG iteration, eigh(gramA, gramB) (scipy lobpcg.py:891-909):
  * A, B host n x n complex128 Hermitian (row-major; B NULL for
- * the identity), n <= 72. All n eigenpairs (nwant = n) by Householder + QL, or only the nwant
- * smallest (1 <= nwant < n) by multisection and inverse iteration, the form the LOBPCG iterations
- * use (they keep the block-size smallest). w (host, n doubles) ascending in its first nwant
- * entries; V (host, n x n complex128, row-major) eigenvectors in its first nwant columns,
- * B-orthonormal. Returns QDKP_OK, or QDKP_ERR_NUMERIC when B is not positive definite or the
+ * the identity), n <= 72. All n eigenpairs (nwant = n; by Householder + QL where n > 24), or only
+ * the nwant smallest (1 <= nwant < n); the latter, and all pairs up to n = 24, by multisection and
+ * inverse iteration, the form the LOBPCG iterations use (they keep the block-size smallest).
+ * w (host, n doubles) ascending in its first nwant entries; V (host, n x n complex128, row-major)
+ * eigenvectors in its first nwant columns, B-orthonormal. Returns QDKP_OK, or QDKP_ERR_NUMERIC when B is not positive definite or the
  * spectrum is not finite. Synchronous on `stream`; workspace qdkp_block_eigh_workspace_size(n).
  */
 size_t qdkp_block_eigh_workspace_size(int n);
