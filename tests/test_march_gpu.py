@@ -46,3 +46,35 @@ def test_tiles_at_their_edges(shape, bands):
                 assert err < tol, (tile, m, ld, err)
                 assert bool((out[:, m:] == 7.0).all()), (tile, m, ld)
     H.close()
+
+
+@pytest.mark.parametrize('bands', [8, 6, 4])
+@pytest.mark.parametrize('shape', [(1, 10, 10), (5, 11, 14), (9, 16, 24), (4, 1, 3)])
+def test_folded_passes_its_block_uncoupled(shape, bands):
+    """(H - sigma)^2 X through every kernel that its two applies can take, against the oracle CSR."""
+    import torch
+    from qd3dsolver_b200 import _lib, kp_pryor as kpg
+    from oracle import kp_operator as ko
+    rng = np.random.default_rng(sum(shape) + bands)
+    f = _fields(shape, rng)
+    hole = bands != 8
+    H = kpg.confined_hamiltonian(kpg.GridOperators(shape, 0.5), f, bands, hole_convention=hole,
+                                 strain={k: f[k] for k in STRAIN})
+    Ho = ko.confined_hamiltonian(shape, 0.5, f, bands, hole_convention=hole, strain=True)
+    n = H.shape[0]
+    X = rng.standard_normal((n, 13)) + 1j * rng.standard_normal((n, 13))
+    sigma = 0.7
+    T = Ho @ X - sigma * X
+    ref = Ho @ T - sigma * T
+    scale = np.abs(ref).max()
+    # two applies, each with the rounding of one (the tolerances above)
+    for dt, code, tol, tiles in ((torch.complex128, _lib.C128, 2e-13, 4),
+                                 (torch.complex64, _lib.C64, 4e-6, 6)):
+        Xd = torch.from_numpy(X).cuda().to(dt)
+        for tile in list(range(tiles)) + [_lib.TILE_DIRECT, _lib.TILE_AUTO]:
+            H.set_tile(tile, code)
+            for m in (1, 3, 4, 8, 13):
+                out = H.apply(Xd[:, :m].contiguous(), sigma=sigma, mode=_lib.APPLY_FOLDED)
+                err = np.abs(out.cpu().numpy() - ref[:, :m]).max() / scale
+                assert err < tol, (tile, m, err)
+    H.close()
