@@ -98,6 +98,7 @@ int qdkp_operator_create(int nx, int ny, int nz, double h, int n_bands, int flag
   QDKP_CUDA_TRY(cudaSetDevice(device));
   auto* op = new qdkp_operator();
   op->fields64 = nullptr; op->rec64 = nullptr; op->rec32 = nullptr; op->nbmask = nullptr;
+  op->col64 = nullptr; op->col32 = nullptr;
   op->staged_cfg[0] = op->staged_cfg[1] = -1;
   op->nx = nx; op->ny = ny; op->nz = nz;
   op->n_sites = (int64_t)nx * ny * nz;
@@ -107,6 +108,10 @@ int qdkp_operator_create(int nx, int ny, int nz, double h, int n_bands, int flag
   cudaError_t e = cudaMalloc(&op->fields64, bytes64);
   if (e == cudaSuccess) e = cudaMalloc(&op->rec64, rec_values * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&op->rec32, rec_values * sizeof(float));
+  if (const size_t b64 = column_record_bytes(op->n_sites, QDKP_C128)) {
+    if (e == cudaSuccess) e = cudaMalloc(&op->col64, b64);
+    if (e == cudaSuccess) e = cudaMalloc(&op->col32, column_record_bytes(op->n_sites, QDKP_C64));
+  }
   if (e == cudaSuccess) e = cudaMalloc(&op->nbmask, (size_t)op->n_sites * sizeof(unsigned));
   if (e != cudaSuccess) {
     set_error(std::string("cudaMalloc of operator fields: ") + cudaGetErrorString(e));
@@ -169,6 +174,8 @@ int qdkp_operator_destroy(qdkp_operator* op) {
   cudaFree(op->fields64);
   cudaFree(op->rec64);
   cudaFree(op->rec32);
+  cudaFree(op->col64);
+  cudaFree(op->col32);
   cudaFree(op->nbmask);
   delete op;
   return QDKP_OK;

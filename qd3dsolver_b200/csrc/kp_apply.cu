@@ -57,6 +57,11 @@ enum RecEntry {
   K_COUNT = 50
 };
 template <typename T> __host__ __device__ constexpr int rec_stride() { return sizeof(T) == 8 ? 54 : 52; }
+// Words of a second, word-major copy, which single columns read: there every lane of a warp is another site,
+// and the same word of 32 records lies on 32 lines. (Word-major records for all, with the words of four or of
+// all sites together, cost the other blocks 3 to 12%; a warp's records staged in shared memory took
+// 10 to 40% more than reading them in place, since L1 shrinks by what the stage takes.)
+template <typename T> __host__ __device__ constexpr int rec_words() { return (K_COUNT * (int)sizeof(T) + 15) / 16; }
 
 // ---------------------------------------------------------------------------------------------
 // Record construction (FP64, once per operator)
@@ -81,10 +86,16 @@ __device__ __forceinline__ void first_order_coefs(const double* __restrict__ F, 
 // A thread per site; the records of a CTA's sites are put together in shared memory and written out
 // as one contiguous run.
 constexpr int kRecThreads = 64;
+// Grids that get the copy for single columns. One column, complex128, site-major | word-major records (us):
+// 48x48x36 8 bands 19.7 | 14.9, 6 bands 17.3 | 12.8, 4 bands 13.9 | 9.8; 64x64x48 47 | 38, 42 | 31, 34 | 24.
+// Smaller grids (33x33x25: 7.4 | 6.6) are bound by the call, and eight complex64 bands lose there
+// (18x18x15: 4.3 | 4.9).
+constexpr int64_t kColumnSitesMin = 1 << 15, kColumnSitesMax = 1 << 19;
 __global__ void __launch_bounds__(kRecThreads)
 kp_record_kernel(const double* __restrict__ F, long long N, int nx, int ny,
                                  int nz, double h, int flags, int nb, double sign,
                                  double* __restrict__ rec64, float* __restrict__ rec32,
+                                 double* __restrict__ col64, float* __restrict__ col32,
                                  unsigned* __restrict__ nbmask) {
   const double G = kG;
   const double ih2 = 1.0 / (h * h);
@@ -197,6 +208,13 @@ kp_record_kernel(const double* __restrict__ F, long long N, int nx, int ny,
       if (xo && (sb > 0 ? zp : zm)) r[K_PZX + e] = w * (g3(0, 0, 0) + g3(sx, 0, sb));
     }
     nbmask[s] = msk;
+    if (col64) {
+      for (int w = 0; w < rec_words<double>(); ++w)
+        reinterpret_cast<double2*>(col64)[w * N + s] = make_double2(r[2 * w], r[2 * w + 1]);
+      for (int w = 0; w < rec_words<float>(); ++w)
+        reinterpret_cast<float4*>(col32)[w * N + s] =
+            make_float4((float)r[4 * w], (float)r[4 * w + 1], (float)r[4 * w + 2], (float)r[4 * w + 3]);
+    }
     __syncthreads();
     for (int e = threadIdx.x; e < sites * rec_stride<double>(); e += kRecThreads)
       rec64[s0 * rec_stride<double>() + e] = sr[e / rec_stride<double>()][e % rec_stride<double>()];
@@ -486,6 +504,42 @@ __device__ __forceinline__ void load_uncoupled(const cplx<typename V::T>* __rest
   }
 }
 
+// Where hx_item's records come from: its site's own in global memory, a 16-byte word a load ...
+template <typename T>
+struct RecDirect {
+  const T* rp;
+  long long rx;                     // to the x neighbours' records
+  __device__ __forceinline__ RecDirect(const HXArgs<T>& a, int s)
+      : rp(a.rec + (long long)s * rec_stride<T>()), rx((long long)a.sx * rec_stride<T>()) {}
+  template <int FIRST, int K> __device__ __forceinline__ void own(T (&w)[K]) const { load_rec<true>(rp + FIRST, w); }
+  // four entries of the x neighbour's record on side DIR (0 up, 1 down), the site's own without one
+  template <int FIRST, int DIR> __device__ __forceinline__ void beside(bool has, T (&w)[4]) const {
+    load_rec<true>(rp + (has ? (DIR ? -rx : rx) : 0) + FIRST, w);
+  }
+};
+
+// ... or, with one column, in the word-major copy: 16-byte word w of site s at a.rec + (w N + s) words
+template <typename T>
+struct RecColumn {
+  static constexpr unsigned E = 16 / sizeof(T);
+  const T* rp;
+  unsigned pitch, rx;
+  __device__ __forceinline__ RecColumn(const HXArgs<T>& a, int s) : rp(a.rec + E * s), pitch(a.N), rx(E * a.sx) {}
+  template <int FIRST, int K> __device__ __forceinline__ void words(const T* q, T (&w)[K]) const {
+#pragma unroll
+    for (int k = 0; k < K; k += E) {
+      T v[E];
+      load_rec<true>(q + pitch * (unsigned)(FIRST + k), v);
+#pragma unroll
+      for (int e = 0; e < (int)E; ++e) w[k + e] = v[e];
+    }
+  }
+  template <int FIRST, int K> __device__ __forceinline__ void own(T (&w)[K]) const { words<FIRST>(rp, w); }
+  template <int FIRST, int DIR> __device__ __forceinline__ void beside(bool has, T (&w)[4]) const {
+    words<FIRST>(has ? (DIR ? rp - rx : rp + rx) : rp, w);
+  }
+};
+
 // Faces are taken to the uncoupled basis one by one; the four edge neighbours of a plane share
 // one weight per band, so their weighted sum is formed first and taken there once. Nothing
 // branches on the walls: a missing neighbour reads the site itself under a zero weight, so the
@@ -494,22 +548,20 @@ __device__ __forceinline__ void load_uncoupled(const cplx<typename V::T>* __rest
 // and multiplies the site itself. That is the operator complex64 engine slots of even width iterate
 // on; it differs from the hard-wall operator only in rows next to a wall, and the complex128 finish
 // of a mixed solve does not use it.
-template <class V, int NB, int BASIS>
-__device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, int j,
+template <class V, int NB, int BASIS, class Rec>
+__device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, const Rec& rec, int s, int j,
                                         bool wall_self = false) {
   typedef typename V::T T;
   const cplx<T>* xs = a.X + ((long long)s * a.ldx + j);
   const int bs = a.N * a.ldx;
   const int sx = a.sx * a.ldx, sy = a.sy * a.ldx, sz = a.ldx;
-  const T* rp = a.rec + (long long)s * rec_stride<T>();
-  const long long rx = (long long)a.sx * rec_stride<T>();          // the x neighbours' records
   const unsigned msk = __ldg(a.msk + s);
   V y[8], x[8], u[8];
 #pragma unroll
   for (int b = 0; b < 8; ++b) vzero(y[b]);
   {
     T w[8];
-    load_rec<true>(rp, w);
+    rec.template own<0>(w);
     load_uncoupled<V, NB, BASIS>(xs, bs, 0, u);
     local_term<V, NB>(y, u, w, a.shift);
   }
@@ -517,7 +569,7 @@ __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, i
   const auto face_off = [&](int f, int d) { return (msk >> f & 1u) ? d : 0; };
   {
     T w[20];
-    load_rec<true>(rp + K_FYZ, w);
+    rec.template own<K_FYZ>(w);
 #pragma unroll
     for (int f = 2; f < 6; ++f) {
       const int d = f < 4 ? sy : sz;
@@ -527,8 +579,8 @@ __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, i
     }
   }
   {
-    T w[12];
-    load_rec<true>(rp + K_FX, w);
+    T w[sizeof(T) == 8 ? 10 : 12];
+    rec.template own<K_FX>(w);
 #pragma unroll
     for (int f = 0; f < 2; ++f) {
       load_uncoupled<V, NB, BASIS>(xs, bs, face_off(f, f ? -sx : sx), u);
@@ -541,14 +593,15 @@ __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, i
     // weights by e: an xy or zx edge's stands in the record of the x neighbour on its side
     T w[4];
     if (pl == 2) {
-      load_rec<true>(rp + K_EZY, w);
+      rec.template own<K_EZY>(w);
     } else {
       T p[4];
-      const int k = pl == 0 ? K_PXY : K_PZX;
       const bool up = msk & 1u, dn = msk & 2u;
-      load_rec<true>(rp + (up ? rx : 0) + k, p);
+      if (pl == 0) rec.template beside<K_PXY, 0>(up, p);
+      else rec.template beside<K_PZX, 0>(up, p);
       w[0] = up ? p[0] : T(0); w[pl == 0 ? 2 : 1] = up ? p[1] : T(0);
-      load_rec<true>(rp - (dn ? rx : 0) + k, p);
+      if (pl == 0) rec.template beside<K_PXY, 1>(dn, p);
+      else rec.template beside<K_PZX, 1>(dn, p);
       w[pl == 0 ? 1 : 2] = dn ? p[2] : T(0); w[3] = dn ? p[3] : T(0);
     }
     V z[8];
@@ -614,7 +667,15 @@ kp_apply_kernel(const HXArgs<T> a) {
   const int it = blockIdx.x * blockDim.x + threadIdx.x;
   if (it >= a.N * a.m) return;
   const int s = it / a.m;
-  hx_item<typename Column<T>::V, NB, BASIS>(a, s, it - s * a.m);
+  hx_item<typename Column<T>::V, NB, BASIS>(a, RecDirect<T>(a, s), s, it - s * a.m);
+}
+
+// ... of one column, with the records' word-major copy (kColumnSitesMin)
+template <typename T, int NB, int BASIS>
+__global__ void __launch_bounds__(kApplyThreads, ApplyOcc<T>::kMinBlocks)
+kp_apply_column_kernel(const HXArgs<T> a) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < a.N) hx_item<typename Column<T>::V, NB, BASIS>(a, RecColumn<T>(a, s), s, 0);
 }
 
 // Many operators and blocks in one launch (the batched engine): CTA b serves slot k with
@@ -647,7 +708,7 @@ kp_apply_multi_kernel(const HXSlot* __restrict__ slots, int nslots, int tiles) {
     const bool wall_self = std::is_same<T, float>::value && ((m | a.ldx | a.ldy) & 1) == 0 &&
                            ((reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.Y)) & 15) == 0;
     const int s = it / m;
-    hx_item<typename Column<T>::V, 8, BASIS>(a, s, it - s * m, wall_self);
+    hx_item<typename Column<T>::V, 8, BASIS>(a, RecDirect<T>(a, s), s, it - s * m, wall_self);
   }
 }
 
@@ -1289,11 +1350,17 @@ int build_records(qdkp_operator* op) {
   const long long N = op->n_sites;
   const int blocks = (int)std::min<long long>((N + kRecThreads - 1) / kRecThreads, 148 * 16);
   kp_record_kernel<<<blocks, kRecThreads>>>(op->fields64, N, op->nx, op->ny, op->nz, op->h, op->flags,
-                                     op->n_bands, op_sign(op), op->rec64, op->rec32, op->nbmask);
+                                     op->n_bands, op_sign(op), op->rec64, op->rec32, op->col64, op->col32,
+                                     op->nbmask);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
   QDKP_CUDA_TRY(cudaDeviceSynchronize());
   return QDKP_OK;
+}
+
+size_t column_record_bytes(int64_t n_sites, int precision) {
+  if (n_sites < kColumnSitesMin || n_sites > kColumnSitesMax) return 0;
+  return (size_t)(precision == QDKP_C64 ? rec_words<float>() : rec_words<double>()) * 16 * n_sites;
 }
 
 size_t record_values(int64_t n_sites) { return (size_t)rec_stride<double>() * n_sites; }
@@ -1335,13 +1402,17 @@ static int pick_tile(const qdkp_operator* op, const void* X, int64_t ldx, int m,
 // The direct kernel; a block of few items is spread over the whole chip in small CTAs (23x23x20 x 1:
 // 42 CTAs of 256 threads would leave 106 SMs idle; 8.0 -> 5.1 us with 64).
 template <typename T, int NB, int BASIS>
-static int launch_direct(const qdkp_operator* op, const HXArgs<T>& a, int sms, cudaStream_t st) {
+static int launch_direct(const qdkp_operator* op, HXArgs<T> a, int sms, cudaStream_t st) {
   const int64_t items = op->n_sites * a.m;
   int threads = kApplyThreads;
   while (threads > 64 && items < (int64_t)threads * 2 * sms) threads /= 2;
   // a single column's call is bound by the host: one runtime call, which returns its own error
-  void* args[] = {const_cast<HXArgs<T>*>(&a)};
-  QDKP_CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(&kp_apply_kernel<T, NB, BASIS>),
+  const T* col = sizeof(T) == 8 ? (const T*)op->col64 : (const T*)op->col32;
+  const bool column = a.m == 1 && col != nullptr;
+  if (column) a.rec = col;
+  void* args[] = {&a};
+  QDKP_CUDA_TRY(cudaLaunchKernel(column ? reinterpret_cast<const void*>(&kp_apply_column_kernel<T, NB, BASIS>)
+                                        : reinterpret_cast<const void*>(&kp_apply_kernel<T, NB, BASIS>),
                                  dim3((unsigned)((items + threads - 1) / threads)), dim3(threads), args, 0, st));
   count_launch();
   return QDKP_OK;

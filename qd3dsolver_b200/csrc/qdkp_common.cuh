@@ -120,6 +120,8 @@ double apply_cb_weight(const qdkp_operator* op);
 int build_records(qdkp_operator* op);
 // values of the record of n_sites sites
 size_t record_values(int64_t n_sites);
+// bytes of their copy for single columns (0: none is kept)
+size_t column_record_bytes(int64_t n_sites, int precision);
 
 }  // namespace qdkp
 
@@ -134,6 +136,8 @@ struct qdkp_operator {
   double* fields64;       // device, F_COUNT * n_sites doubles (library-owned)
   double* rec64;          // device, per-site stencil record (FP64), record_values(n_sites)
   float* rec32;           // the same record in FP32
+  double* col64;          // copies of both for single columns (column_record_bytes), or NULL
+  float* col32;
   unsigned* nbmask;       // device, per-site neighbour mask
   int staged_cfg[2];      // H.X tile shape per precision (c128, c64); -1 = by heuristic
   int64_t nnz_equiv;      // CSR nonzero count of the equivalent assembled matrix
