@@ -156,8 +156,12 @@ __host__ __device__ inline GramShape gram_shape(int kind, int P, int Q, int m, i
   return s;
 }
 
+// Row parts of a product: one CTA an SM as soon as each has four of the shortest chunks. 128 | 1024 rows a
+// part at least, complex128, 3 m x 2 m columns, with the copy of the result (us): m = 13, 5,000 rows
+// 48 | 114, 20,000 50 | 100, 40,000 61 | 101, 80,000 76 | 110; m = 24, 20,000 77 | 103; m = 6, 2,000 39 | 58.
+// 64 or 32 rows a part: the same within 3 us from 5,000 rows on.
 __host__ __device__ inline int gram_parts(long long n) {
-  long long parts = n / 1024;             // enough rows to amortise a CTA's start and partial sums
+  long long parts = n / 128;
   if (parts > kGramMaxParts) parts = kGramMaxParts;
   return parts < 1 ? 1 : (int)parts;
 }
