@@ -252,7 +252,7 @@ update_kernel(const BlockList<T> A, const CoefList C, int q, long long n, cplx<T
               long long ldy, int accumulate) {
   extern __shared__ __align__(16) unsigned char usm[];
   const double2* Cf[3] = {C.c[0], C.c[1], C.c[2]};
-  constexpr int chunk = kUpdChunk;
+  const int chunk = update_chunk<T>(q);
   const long long per = ((n + gridDim.x - 1) / gridDim.x + chunk - 1) / chunk * chunk;
   const long long r0 = (long long)blockIdx.x * per;
   if (r0 >= n) return;
@@ -350,7 +350,8 @@ int launch_update(const BlockList<T>& A, const double2* const* C, int q, long lo
                                        200 * 1024));
     attr = true;
   }
-  long long blocks = (n + kUpdChunk - 1) / kUpdChunk;
+  const int chunk = update_chunk<T>(q);
+  long long blocks = (n + chunk - 1) / chunk;
   if (blocks > 148 * 4) blocks = 148 * 4;
   update_kernel<T><<<(unsigned)blocks, kUpdThreads, smem, st>>>(A, cl, q, n, Y, ldy, accumulate);
   count_launch();

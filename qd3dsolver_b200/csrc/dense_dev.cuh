@@ -1092,6 +1092,11 @@ static __device__ int block_eigh(const double2* __restrict__ A, const double2* _
 constexpr int kUpdThreads = 256;
 constexpr int kUpdWarps = kUpdThreads / 32;
 constexpr int kUpdChunk = 16 * kUpdWarps;           // row granularity of a CTA's span: two tiles a warp
+// ... of an update alone: complex128 outputs of more than 12 columns go by one tile a warp (80,000 rows of
+// 60 columns to 20: spans of 256 rows make 313 CTAs for the 296 that run at once, 72 us; of 192 rows 63)
+template <typename T> __host__ __device__ __forceinline__ int update_chunk(int q) {
+  return sizeof(T) == 8 && q > 12 ? kUpdChunk / 2 : kUpdChunk;
+}
 constexpr int kDmRing = 16;                         // 16-byte words in flight per lane
 constexpr size_t kDmRingBytes = (size_t)kUpdWarps * kDmRing * 32 * sizeof(double2);
 
