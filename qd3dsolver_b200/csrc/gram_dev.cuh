@@ -396,10 +396,10 @@ static __device__ void gram_core(const GramTask<T>& t, int part, int parts, int 
   }
 }
 
-// the entry whose real view's upper left word stands at c, summed over parts [b0, b1) in order: eight
-// parts' loads in flight, the last ones too (a remainder loop would wait for each)
+// the entry whose real view's upper left word stands at c (rows `row` apart), summed over parts [b0, b1) in
+// order: eight parts' loads in flight, the last ones too (a remainder loop would wait for each)
 static __device__ __forceinline__ double2 gram_add_parts(const double* __restrict__ c, long long pstride,
-                                                         int b0, int b1) {
+                                                         int b0, int b1, int row = 24) {
   double2 s = make_double2(0.0, 0.0);
   for (int b = b0; b < b1; b += 8) {
     double2 u[8], v[8];
@@ -407,7 +407,7 @@ static __device__ __forceinline__ double2 gram_add_parts(const double* __restric
     for (int q = 0; q < 8; ++q) {
       const double* cq = c + min(b + q, b1 - 1) * pstride;
       u[q] = __ldcg(reinterpret_cast<const double2*>(cq));
-      v[q] = __ldcg(reinterpret_cast<const double2*>(cq + 24));
+      v[q] = __ldcg(reinterpret_cast<const double2*>(cq + row));
     }
 #pragma unroll
     for (int q = 0; q < 8; ++q)
