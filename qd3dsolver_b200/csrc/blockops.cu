@@ -134,10 +134,13 @@ size_t gram_partial_elems(int P, int Q) {
   return rects * kGramMaxParts * kGramRectElems / 2;
 }
 
-// ... of a qdkp_block_gram, in either precision
+// ... of a qdkp_block_gram, in either precision, and of any narrower one: split TF32 takes products of up to
+// kTfMaxRects rectangles and more room for the widest of them than FP64 for some wider ones
 static size_t block_gram_elems(int P, int Q) {
-  const size_t fp64 = gram_partial_elems(P, Q);
-  return gram_tf32_threads(P, Q) ? std::max(fp64, gram_tf32_doubles(P, Q) / 2) : fp64;
+  size_t e = gram_partial_elems(P, Q);
+  for (int r = 1; r <= kTfMaxRects && kGramRect * (r - 1) < P; ++r)
+    e = std::max(e, gram_tf32_doubles(std::min(P, kGramRect * r), std::min(Q, kGramRect * (kTfMaxRects / r))) / 2);
+  return e;
 }
 
 __global__ void __launch_bounds__(512)

@@ -242,10 +242,12 @@ static __device__ void gram_core_tf32(const BlockList<float>& A, const BlockList
   for (int e = threadIdx.x; e < RP * RQ; e += blockDim.x) out[e] = gsm[e];
 }
 
+constexpr int kTfMaxRects = 16;     // rectangles of 12 x 12 columns, a warp each
+
 // threads of a CTA that holds a P x Q product whole, 0 where none does
 static inline int gram_tf32_threads(int P, int Q) {
   const int rects = (((2 * P + 7) / 8 + 2) / 3) * (((2 * Q + 7) / 8 + 2) / 3);
-  return rects <= 8 ? 256 : (rects <= 16 ? 512 : 0);
+  return rects <= 8 ? 256 : (rects <= kTfMaxRects ? 512 : 0);
 }
 
 // partial doubles of a product, all parts

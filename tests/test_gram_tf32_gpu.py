@@ -4,9 +4,8 @@ small whole numbers, whose products and sums TF32 and FP32 hold exactly, so the 
 import numpy as np
 import pytest
 
-pytestmark = pytest.mark.gpu
 
-
+@pytest.mark.gpu
 @pytest.mark.parametrize('n, P, Q, lda, ldb', [
     (1, 1, 1, 1, 1), (7, 3, 2, 3, 2), (7, 3, 2, 4, 3), (31, 12, 12, 12, 12), (33, 5, 24, 7, 24), (255, 18, 12, 19, 12),
     (256, 18, 12, 18, 12), (257, 18, 12, 18, 13), (1023, 13, 1, 13, 3), (1024, 36, 24, 36, 24), (1025, 36, 36, 37, 36),
@@ -33,3 +32,12 @@ def test_gram_of_complex64_blocks(n, P, Q, lda, ldb):
                                      out.ctypes.data, ws.data_ptr(), ws.numel(), None), 'qdkp_block_gram')
         ref = (A.mH @ B2).cpu().numpy()
         assert np.array_equal(out, ref)
+
+
+def test_workspace_of_a_wider_product_serves_narrower_ones():
+    """qdkp_block_gram_workspace_size grows with either width: room for the widest product of a program is
+    room for all of them."""
+    from qd3dsolver_b200 import _lib
+    size = _lib.lib().qdkp_block_gram_workspace_size
+    w = np.array([[int(size(P, Q)) for Q in range(1, 73)] for P in range(1, 73)])
+    assert (np.diff(w, axis=0) >= 0).all() and (np.diff(w, axis=1) >= 0).all()
