@@ -228,7 +228,7 @@ int launch_gram(const BlockList<T>& A, const BlockList<T>& B, long long n,
   for (int side = 0; side < (same ? 1 : 2); ++side) {
     const BlockList<T>& L = side ? B : A;
     for (int b = 0; b < L.nblk; ++b) {
-      t.p[t.nblk] = L.p[b]; t.ld[t.nblk] = (int)L.ld[b]; t.cols[t.nblk] = L.cols[b];
+      t.p[t.nblk] = L.p[b]; t.ld[t.nblk] = L.ld[b]; t.cols[t.nblk] = L.cols[b];
       ++t.nblk;
     }
   }

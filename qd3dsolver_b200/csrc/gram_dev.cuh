@@ -57,7 +57,8 @@ enum GramKind {
 template <typename T>
 struct GramTask {
   const cplx<T>* p[kGramMaxBlk];
-  int ld[kGramMaxBlk], cols[kGramMaxBlk];
+  long long ld[kGramMaxBlk];
+  int cols[kGramMaxBlk];
   int nblk, tc;             // blocks and their columns in all
   int a0, P, b0, Q;         // A and B as ranges of the concatenated columns
   int kind;

@@ -54,3 +54,22 @@ def test_a_short_block_takes_a_share_of_a_long_ones_time():
             times.append(time.perf_counter() - t0)
         return min(times)
     assert best(20_000) < 0.65 * best(150_000)
+
+
+def test_leading_dimension_beyond_32_bits():
+    """Two rows that lie 2^31 + 8 elements apart (17 GB)."""
+    import torch
+    from qd3dsolver_b200 import _lib
+    L = _lib.lib()
+    P, Q, ld = 61, 51, 2 ** 31 + 8
+    a = torch.empty(ld + P, dtype=torch.complex64, device='cuda')
+    A = torch.randn((2, P), dtype=torch.complex64, device='cuda', generator=torch.Generator('cuda').manual_seed(1))
+    a[:P], a[ld:] = A[0], A[1]
+    B = A[:, :Q].contiguous()
+    ws = torch.empty(int(L.qdkp_block_gram_workspace_size(P, Q)), dtype=torch.uint8, device='cuda')
+    out = np.empty((P, Q), dtype=np.complex128)
+    _lib.check(L.qdkp_block_gram(a.data_ptr(), ld, P, B.data_ptr(), Q, Q, 2, _lib.C64, out.ctypes.data,
+                                 ws.data_ptr(), ws.numel(), None), 'qdkp_block_gram')
+    A = A.to(torch.complex128).cpu().numpy()
+    # two products an entry, in FP64
+    assert np.abs(out - A.conj().T @ A[:, :Q]).max() < 1e-14 * (np.abs(A).T @ np.abs(A)).max()
