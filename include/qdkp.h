@@ -174,9 +174,15 @@ int qdkp_operator_tune(qdkp_operator* op, const void* X, int64_t ldx, void* Y, i
                        int m, int precision, int reps, double* seconds, void* stream);
 
 /* Kernels that wait on their own bulk copies give up after about a second if a copy never lands
- * (a fault elsewhere on the device) and set a device flag instead of hanging. *fault receives the
- * flag of `device` (0 = none); clear = 1 resets it. Synchronous; the current device is kept. */
+ * (a fault elsewhere on the device) and raise their device's fault flag instead of hanging; what they
+ * were to write is then missing or NaN. While the flag is up, every entry point that reads results back (the host
+ * apply, solves, residuals, block products, the engine's admit, poll and retire) returns QDKP_ERR_CUDA once
+ * its work is done, and the asynchronous ones (qdkp_apply, qdkp_apply_folded_noalloc, qdkp_engine_step) refuse
+ * to start. *fault receives the flag of `device` (0 = none) after the work on it; clear = 1 resets it.
+ * Synchronous; the current device is kept. */
 int qdkp_device_fault(int device, int clear, int* fault);
+/* Raises the flag as a kernel would: for tests of what a caller does then. */
+int qdkp_device_fault_inject(int device);
 
 /* Workspace bytes qdkp_apply_host needs for an (n, m) complex128 block in `mode`. */
 size_t qdkp_apply_host_workspace_size(const qdkp_operator* op, int m, int mode);

@@ -79,6 +79,7 @@ _SIGNATURES = {
                                           ctypes.c_void_p]),
     'qdkp_device_fault': (ctypes.c_int, [ctypes.c_int, ctypes.c_int,
                                          ctypes.POINTER(ctypes.c_int)]),
+    'qdkp_device_fault_inject': (ctypes.c_int, [ctypes.c_int]),
     'qdkp_apply_host_workspace_size': (ctypes.c_size_t, [ctypes.c_void_p, ctypes.c_int,
                                                          ctypes.c_int]),
     'qdkp_apply_host': (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,

@@ -236,6 +236,9 @@ int launch_gram(const BlockList<T>& A, const BlockList<T>& B, long long n,
   t.a0 = 0; t.P = P; t.b0 = same ? 0 : P; t.Q = Q;
   t.kind = same ? GK_HERM : GK_FULL;
   t.n = n;
+  int device = 0;
+  QDKP_CUDA_TRY(cudaGetDevice(&device));
+  t.fault = device_fault_flag(device);
   return launch_gram_task(t, partial, partial_elems, out, st);
 }
 
@@ -266,7 +269,7 @@ update_kernel(const BlockList<T> A, const CoefList C, int q, long long n, cplx<T
 // contiguous range of 128-row tiles run as one pipeline
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 update_umma_kernel(const BlockList<float> A, const CoefList C, int q, long long n, float2* Y,
-                   long long ldy, int accumulate, int cmax, int ldmax) {
+                   long long ldy, int accumulate, int cmax, int ldmax, int* fault) {
   extern __shared__ __align__(128) unsigned char usm_u[];
   const double2* Cf[3] = {C.c[0], C.c[1], C.c[2]};
   const UmmaPlan pl = umma_plan(A.total(), q, 1, cmax, ldmax);
@@ -276,7 +279,8 @@ update_umma_kernel(const BlockList<float> A, const CoefList C, int q, long long 
   if (r0 >= n) return;
   UmmaCtx cx;
   umma_ctx_init(cx, pl);
-  update_rows_umma(pl, cx, A, Cf, q, r0, min(n, r0 + per), Y, ldy, accumulate, 0, usm_u);
+  const bool ok = update_rows_umma(pl, cx, A, Cf, q, r0, min(n, r0 + per), Y, ldy, accumulate, 0, usm_u);
+  if (!ok && threadIdx.x == 0) raise_device_fault(fault);
   umma_ctx_free(cx);
 }
 
@@ -315,7 +319,8 @@ int launch_update(const BlockList<T>& A, const double2* const* C, int q, long lo
       for (int c0 = 0; c0 < A.cols[b]; c0 += kMaxBlock)
         subs.push_back({A.p[b] + c0, A.ld[b], std::min(kMaxBlock, A.cols[b] - c0),
                         C[b] ? C[b] + (size_t)c0 * q : nullptr});
-    int nsm = 148;
+    int nsm = 148, device = 0;
+    QDKP_CUDA_TRY(cudaGetDevice(&device));
     QDKP_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, 0));
     long long ublocks = (n + kUmmaRows - 1) / kUmmaRows;
     if (ublocks > nsm) ublocks = nsm;
@@ -336,7 +341,7 @@ int launch_update(const BlockList<T>& A, const double2* const* C, int q, long lo
       const UmmaPlan pl = umma_plan(Ps, q, 1, cmax, ldmax);
       if (!pl.nout_pass) { set_error("tcgen05 update plan does not fit shared memory"); return QDKP_ERR_ARG; }
       update_umma_kernel<<<(unsigned)ublocks, kUmmaThreads, pl.bytes, st>>>(
-          L, cs, q, n, Y, ldy, s0 == 0 ? accumulate : 1, cmax, ldmax);
+          L, cs, q, n, Y, ldy, s0 == 0 ? accumulate : 1, cmax, ldmax, device_fault_flag(device));
       count_launch();
       QDKP_CUDA_TRY(cudaGetLastError());
     }
@@ -463,6 +468,9 @@ int qdkp_block_gram(const void* A, int64_t lda, int P, const void* B, int64_t ld
     set_error("qdkp_block_gram: workspace too small");
     return QDKP_ERR_WORKSPACE;
   }
+  int device = 0;
+  QDKP_CUDA_TRY(cudaGetDevice(&device));
+  if (const int rc = init_device_fault()) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t pe = block_gram_elems(P, Q);
   double2* part = static_cast<double2*>(ws);
@@ -484,7 +492,7 @@ int qdkp_block_gram(const void* A, int64_t lda, int P, const void* B, int64_t ld
   if (rc != QDKP_OK) return rc;
   QDKP_CUDA_TRY(cudaMemcpyAsync(out, dout, (size_t)P * Q * sizeof(double2), cudaMemcpyDeviceToHost, st));
   QDKP_CUDA_TRY(cudaStreamSynchronize(st));
-  return QDKP_OK;
+  return check_device_fault(device);
 }
 
 size_t qdkp_block_eigh_workspace_size(int n) {
@@ -545,6 +553,9 @@ int qdkp_block_update(const void* A, int64_t lda, int P, const double* C, int q,
     set_error("qdkp_block_update: workspace too small");
     return QDKP_ERR_WORKSPACE;
   }
+  int device = 0;
+  QDKP_CUDA_TRY(cudaGetDevice(&device));
+  if (const int rc2 = init_device_fault()) return rc2;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   double2* dC = static_cast<double2*>(ws);
   QDKP_CUDA_TRY(cudaMemcpyAsync(dC, C, (size_t)P * q * sizeof(double2), cudaMemcpyHostToDevice, st));
@@ -561,7 +572,7 @@ int qdkp_block_update(const void* A, int64_t lda, int P, const double* C, int q,
   }
   if (rc != QDKP_OK) return rc;
   QDKP_CUDA_TRY(cudaStreamSynchronize(st));
-  return QDKP_OK;
+  return check_device_fault(device);
 }
 
 }  // extern "C"

@@ -2,6 +2,7 @@
 // The LOBPCG entry points live in lobpcg.cu.
 #include <atomic>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -14,6 +15,34 @@ void set_error(const std::string& msg) { g_last_error = msg; }
 static std::atomic<long long> g_launches{0};
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launches_so_far() { return g_launches.load(); }
+
+// One word a device
+constexpr int kFaultDevices = 64;
+static std::mutex g_fault_mu;
+static std::atomic<int*> g_fault_words{nullptr};
+
+int init_device_fault() {
+  std::lock_guard<std::mutex> lk(g_fault_mu);
+  if (g_fault_words.load()) return QDKP_OK;
+  void* p = nullptr;
+  QDKP_CUDA_TRY(cudaHostAlloc(&p, kFaultDevices * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+  std::memset(p, 0, kFaultDevices * sizeof(int));
+  g_fault_words.store(static_cast<int*>(p));
+  return QDKP_OK;
+}
+
+int* device_fault_flag(int device) {
+  int* w = g_fault_words.load(std::memory_order_acquire);
+  return w && device >= 0 && device < kFaultDevices ? w + device : nullptr;
+}
+
+int check_device_fault(int device) {
+  const int* f = device_fault_flag(device);
+  if (!f || !*const_cast<const volatile int*>(f)) return QDKP_OK;
+  set_error("a kernel gave up waiting for a copy that never landed: results on this device cannot be trusted "
+            "(qdkp_device_fault reads and clears the flag)");
+  return QDKP_ERR_CUDA;
+}
 
 // Nonzero count of the CSR the reference assembles, counted from the stencil structure: each
 // (row band, column band) block couples a site to the offsets its operators reach, clipped at
@@ -96,6 +125,7 @@ int qdkp_operator_create(int nx, int ny, int nz, double h, int n_bands, int flag
     }
   }
   QDKP_CUDA_TRY(cudaSetDevice(device));
+  if (const int rc = init_device_fault()) return rc;
   auto* op = new qdkp_operator();
   op->fields64 = nullptr; op->rec64 = nullptr; op->rec32 = nullptr; op->nbmask = nullptr;
   op->col64 = nullptr; op->col32 = nullptr;
@@ -188,6 +218,7 @@ int qdkp_apply(const qdkp_operator* op, const void* X, int64_t ldx, void* Y, int
   QDKP_CHECK_ARG(m > 0 && ldx >= m && ldy >= m, "need m > 0 and leading dimensions >= m");
   QDKP_CHECK_ARG(mode >= QDKP_APPLY_PLAIN && mode <= QDKP_APPLY_FOLDED, "bad apply mode");
   QDKP_CHECK_ARG(precision == QDKP_C128 || precision == QDKP_C64, "bad precision");
+  if (const int rc = check_device_fault(op->device)) return rc;      // of an earlier call
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (mode != QDKP_APPLY_FOLDED)
     return launch_apply(op, X, ldx, Y, ldy, m, sigma, mode == QDKP_APPLY_SHIFTED, precision, st);
@@ -226,6 +257,30 @@ int qdkp_apply_host(const qdkp_operator* op, const void* X_host, void* Y_host, i
   if (rc != QDKP_OK) return rc;
   QDKP_CUDA_TRY(cudaMemcpyAsync(Y_host, dY, blk, cudaMemcpyDeviceToHost, st));
   QDKP_CUDA_TRY(cudaStreamSynchronize(st));
+  return check_device_fault(op->device);
+}
+
+int qdkp_device_fault(int device, int clear, int* fault) {
+  QDKP_CHECK_ARG(fault != nullptr, "NULL argument");
+  int prev = 0, n = 0;
+  QDKP_CUDA_TRY(cudaGetDevice(&prev));
+  QDKP_CUDA_TRY(cudaGetDeviceCount(&n));
+  QDKP_CHECK_ARG(device >= 0 && device < n, "no such device");
+  QDKP_CUDA_TRY(cudaSetDevice(device));
+  const cudaError_t e = cudaDeviceSynchronize();
+  cudaSetDevice(prev);
+  QDKP_CUDA_TRY(e);
+  volatile int* f = device_fault_flag(device);
+  *fault = f ? *f : 0;
+  if (f && clear) *f = 0;
+  return QDKP_OK;
+}
+
+int qdkp_device_fault_inject(int device) {
+  if (const int rc = init_device_fault()) return rc;
+  int* f = device_fault_flag(device);
+  QDKP_CHECK_ARG(f != nullptr, "no such device");
+  *const_cast<volatile int*>(f) = 1;
   return QDKP_OK;
 }
 

@@ -212,6 +212,7 @@ __device__ bool gram_task(const ESlot& d, int which, GramTask<T>& t, double2*& o
   const int mp = which == GR_RZ ? st->mp : 0;          // decided beside the products on R
   t.nblk = 0; t.tc = 0;
   t.m = m; t.ma = ma; t.mp = mp; t.n = d.n;
+  t.fault = d.fault;
   t.a0 = 0; t.b0 = 0;
   auto add = [&](double2* p, int ld, int cols) {
     t.p[t.nblk] = blk<T>(p); t.ld[t.nblk] = ld; t.cols[t.nblk] = cols;
@@ -436,6 +437,7 @@ e_update_umma_kernel(const ESlot* __restrict__ S, int ns, int which, int utiles,
       if (ok) {
         ok = update_rows_umma(pl, cx, u.A, u.C, u.q, r0, r1, u.Y, (long long)u.q, u.accumulate, u.neg,
                               usm_u, u.C2, u.Y2);
+        if (!ok && threadIdx.x == 0) raise_device_fault(d.fault);
       } else {
         float2* const Ys[2] = {u.Y, u.Y2};
         umma_fill_nan(Ys, u.Y2 ? 2 : 1, u.q, r0, r1, (long long)u.q);
@@ -638,6 +640,7 @@ void slot_carve(ESlot& d, void* ws, const SlotLayout& L, int64_t n, int m, int p
   d.gram0 = d.row0 = 0;
   d.utile0 = -1;
   d.snap = nullptr;
+  d.fault = nullptr;
 }
 
 void slot_params(ESlot& d, EState& s, const qdkp_lobpcg_params* prm, const double* lam) {
@@ -1213,6 +1216,7 @@ int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg
   h.prm = *prm;
   ESlot& d = h.d;
   slot_carve(d, ws, L, n, m, prm->precision, 10);
+  d.fault = device_fault_flag(e->device);
   h.gpart_doubles = L.gpart / sizeof(double);
   int rc;
 #define ATRY(x) do { rc = (x); if (rc != QDKP_OK) return rc; } while (0)
@@ -1249,6 +1253,7 @@ int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg
   if (nonfinite) { s0.running = 0; s0.status = QDKP_LOBPCG_NONFINITE; }
   QDKP_CUDA_TRY(cudaMemcpyAsync(d.st, &s0, sizeof(EState), cudaMemcpyHostToDevice, st));
   QDKP_CUDA_TRY(cudaStreamSynchronize(st));
+  ATRY(check_device_fault(e->device));
 #undef ATRY
   h.used = true;
   e->dirty = true;
@@ -1258,6 +1263,7 @@ int qdkp_engine_admit(qdkp_engine* e, const qdkp_operator* op, const qdkp_lobpcg
 
 int qdkp_engine_step(qdkp_engine* e, int ticks, void* stream) {
   QDKP_CHECK_ARG(e && ticks >= 0, "bad arguments");
+  if (const int rc = check_device_fault(e->device)) return rc;      // of earlier ticks
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   QDKP_CUDA_TRY(cudaSetDevice(e->device));
   if (e->dirty) {
@@ -1316,7 +1322,7 @@ int qdkp_engine_poll(qdkp_engine* e, int* state, int* status, int* iterations, v
     if (status) status[i] = h.used ? hs[i].status : -1;
     if (iterations) iterations[i] = h.used ? hs[i].iter + 1 : 0;
   }
-  return QDKP_OK;
+  return check_device_fault(e->device);
 }
 
 int qdkp_engine_retire(qdkp_engine* e, int slot, double* lambda_out, void* V,
@@ -1367,7 +1373,7 @@ int qdkp_engine_retire(qdkp_engine* e, int slot, double* lambda_out, void* V,
     info->best_mean_residual = s.smallest;
     h.used = false;
     e->dirty = true;
-    return QDKP_OK;
+    return check_device_fault(e->device);
   }
   // final Rayleigh-Ritz on the best iterate (lobpcg.py:1009-1060)
   RTRY(apply_folded(h, d.best, m, d.AX, st));
@@ -1420,7 +1426,7 @@ int qdkp_engine_retire(qdkp_engine* e, int slot, double* lambda_out, void* V,
 #undef RTRY
   h.used = false;
   e->dirty = true;
-  return QDKP_OK;
+  return check_device_fault(e->device);
 }
 
 }  // extern "C"

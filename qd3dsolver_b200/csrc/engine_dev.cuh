@@ -58,6 +58,7 @@ struct ESlot {
   int utile0;           // complex64 slots: first 128-row tile in the group's tcgen05 update space
   int rows_per_cta;     // rows per CTA in the row kernels (gather, update, norms)
   EState* st;
+  int* fault;           // device_fault_flag
   EState* snap;         // NULL, or where the decision kernel leaves a copy of st for the host
 };
 

@@ -64,6 +64,7 @@ struct GramTask {
   int kind;
   int m, ma, mp;            // widths of X, R, P (pencil kinds)
   long long n;
+  int* fault;               // device_fault_flag
 };
 
 // Where entry (i, j) of a task's product goes. GK_FULL and GK_HERM: out, row-major, both triangles;
@@ -250,7 +251,8 @@ static __device__ __forceinline__ void gram_offset(const GramTask<T>& t, int cro
 
 // The CTA's part of a task: sums over the rows of part `part` of the rectangles of panel `panel`,
 // into partial[(part * rects + rect) * kGramRectElems + ...]. The last warp produces; at least
-// kGramMaxRects threads. A wait that gives up (a copy that never lands) leaves NaN sums.
+// kGramMaxRects threads. A wait that gives up (a copy that never lands) leaves NaN sums and raises the device's
+// fault flag.
 template <typename T>
 static __device__ void gram_core(const GramTask<T>& t, int part, int parts, int panel,
                                  double* __restrict__ partial, unsigned char* smem) {
@@ -377,6 +379,7 @@ static __device__ void gram_core(const GramTask<T>& t, int part, int parts, int 
     }
   }
   ok = __syncthreads_and(ok) != 0;
+  if (!ok && threadIdx.x == 0) raise_device_fault(t.fault);
   // the row slices of a rectangle, summed in order
   double* red = reinterpret_cast<double*>(st0);
   if (warp < slices * count) {

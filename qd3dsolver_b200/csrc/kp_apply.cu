@@ -756,6 +756,7 @@ struct MarchArgs {
   int v16;                      // complex64: 16-byte column pairs in X
   int v16y;                     // ... and in Y
   T shift, cb;
+  int* fault;                   // device_fault_flag
 };
 
 // cp.async of 16 (or 8) bytes of which the first `src_bytes` are read, the rest zero
@@ -1000,8 +1001,6 @@ kp_march_kernel(const MarchArgs<typename G::T> a) {
 // one's arithmetic, before the barrier that the two share. The launcher takes it where a tensor
 // map can describe the block (tma_fits).
 // ---------------------------------------------------------------------------------------------
-__device__ int g_apply_fault;      // set when a wait on a copy gave up (qdkp_device_fault)
-
 template <class G, int NB, int NS, int BASIS>
 __global__ void __launch_bounds__(G::THREADS, G::MINB)
 kp_march_tma_kernel(const __grid_constant__ CUtensorMap tmx, const MarchArgs<typename G::T> a) {
@@ -1106,7 +1105,7 @@ kp_march_tma_kernel(const __grid_constant__ CUtensorMap tmx, const MarchArgs<typ
   if (!ok && t == 0) {
     // a copy never landed: flag it, then give the copies still in flight a bounded chance to
     // finish before the CTA's shared memory is released
-    atomicExch(&g_apply_fault, 1);
+    raise_device_fault(a.fault);
     for (int i = 0; i < NS; ++i) { mbar_wait(bars + 8u * i, 0); mbar_wait(bars + 8u * i, 1); }
   }
 }
@@ -1285,6 +1284,7 @@ static int launch_march_tma(const qdkp_operator* op, const typename G::T* rec, c
   a.tiles_z = g.tiles_z; a.chunks = g.chunks; a.xsplit = g.xsplit; a.xlen = g.xlen;
   a.v16y = ((uintptr_t)Y & 15) == 0 && ldy % 2 == 0;
   a.shift = shift; a.cb = cb;
+  a.fault = device_fault_flag(op->device);
   kp_march_tma_kernel<G, NB, NS, BASIS><<<g.ctas, G::THREADS, smem, st>>>(tmx, a);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
@@ -1544,21 +1544,6 @@ int qdkp_operator_tune(qdkp_operator* op, const void* X, int64_t ldx, void* Y, i
   op->staged_cfg[pi] = rc == QDKP_OK ? best : saved;
   if (rc == QDKP_ERR_CUDA) set_error("qdkp_operator_tune: CUDA event failure");
   return rc;
-}
-
-int qdkp_device_fault(int device, int clear, int* fault) {
-  QDKP_CHECK_ARG(fault != nullptr, "NULL argument");
-  int prev = 0;
-  QDKP_CUDA_TRY(cudaGetDevice(&prev));
-  QDKP_CUDA_TRY(cudaSetDevice(device));
-  cudaError_t e = cudaMemcpyFromSymbol(fault, g_apply_fault, sizeof(int));
-  if (e == cudaSuccess && clear) {
-    const int zero = 0;
-    e = cudaMemcpyToSymbol(g_apply_fault, &zero, sizeof(int));
-  }
-  cudaSetDevice(prev);
-  QDKP_CUDA_TRY(e);
-  return QDKP_OK;
 }
 
 }  // extern "C"

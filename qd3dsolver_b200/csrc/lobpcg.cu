@@ -181,6 +181,7 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
   ESlot& d = s.d;
   slot_carve(d, tables + 2 * kTables, s.L, n, m, QDKP_C128, n_blocks(prm));
   d.snap = reinterpret_cast<EState*>(tables + kTables);
+  d.fault = device_fault_flag(op->device);
   cudaStream_t st = s.st;
   const int maxiter = prm->maxiter;
   const int hist_rows = maxiter + 3;
@@ -244,6 +245,7 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
     QDKP_CUDA_TRY(cudaStreamWaitEvent(s.side, s.decided, 0));
     QDKP_CUDA_TRY(cudaMemcpyAsync(&es, d.snap, sizeof(es), cudaMemcpyDeviceToHost, s.side));
     QDKP_CUDA_TRY(cudaStreamSynchronize(s.side));
+    TRY(check_device_fault(op->device));
     if (es.iter != it) {
       it = es.iter;
       std::memcpy(&hist[(size_t)it * m], es.norms, m * sizeof(double));
@@ -300,7 +302,7 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
     QDKP_CUDA_TRY(cudaStreamSynchronize(st));
     info->hx_seconds = prm->time_hx ? s.hx_seconds() : 0.0;
     info->seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
-    return QDKP_OK;
+    return check_device_fault(op->device);
   }
   // ---- final Rayleigh-Ritz on the best iterate (scipy lobpcg.py:1009-1060) -----------------
   TRY(s.applyA(d.best, m, d.AX));
@@ -352,7 +354,7 @@ int qdkp_lobpcg_solve(const qdkp_operator* op, const qdkp_lobpcg_params* prm, co
   info->hx_seconds = prm->time_hx ? s.hx_seconds() : 0.0;
   info->seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
 #undef TRY
-  return QDKP_OK;
+  return check_device_fault(op->device);
 }
 
 size_t qdkp_residuals_workspace_size(const qdkp_operator* op, int k) {
@@ -403,7 +405,7 @@ int qdkp_residuals(const qdkp_operator* op, const void* V, int64_t ldv, int k, c
   QDKP_CUDA_TRY(cudaMemcpyAsync(r2.data(), out, k * sizeof(double), cudaMemcpyDeviceToHost, st));
   QDKP_CUDA_TRY(cudaStreamSynchronize(st));
   for (int j = 0; j < k; ++j) res[j] = std::sqrt(std::fabs(r2[j])) / nrm[j];
-  return QDKP_OK;
+  return check_device_fault(op->device);
 }
 
 }  // extern "C"

@@ -68,7 +68,8 @@ int qdkp_apply_folded_noalloc(const qdkp_operator* op, const void* X, int64_t ld
   QDKP_CUDA_TRY(cudaGetDevice(&prev));
   if (prev != op->device) QDKP_CUDA_TRY(cudaSetDevice(op->device));
   void* T = nullptr;
-  int rc = scratch_address(op->device, &T);
+  int rc = check_device_fault(op->device);             // of an earlier call
+  if (rc == QDKP_OK) rc = scratch_address(op->device, &T);
   if (rc == QDKP_OK) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // Every element of T that the second launch reads is written by the first one in this

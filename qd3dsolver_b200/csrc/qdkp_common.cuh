@@ -59,6 +59,19 @@ void set_error(const std::string& msg);
 void count_launch(int n = 1);
 long long launches_so_far();
 
+// The fault flag of a device (qdkp_device_fault), a word of mapped host memory: a kernel whose bounded wait
+// gave up sets it, host code reads it without a copy once the kernel is done. init_device_fault, which
+// allocates the words, comes before any kernel that may set one (with an operator, a block product).
+int init_device_fault();
+int* device_fault_flag(int device);
+// QDKP_ERR_CUDA with a message while the flag is up: what the kernels left cannot be trusted
+int check_device_fault(int device);
+__device__ __forceinline__ void raise_device_fault(int* flag) {
+  if (!flag) return;
+  *reinterpret_cast<volatile int*>(flag) = 1;
+  __threadfence_system();
+}
+
 #define QDKP_CUDA_TRY(expr)                                                              \
   do {                                                                                   \
     cudaError_t _e = (expr);                                                             \
