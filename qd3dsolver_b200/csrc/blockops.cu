@@ -376,9 +376,11 @@ chol_inv_kernel(const double2* __restrict__ G, int n, double2* __restrict__ Uinv
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) ssm[e] = G[e];
   __syncthreads();
   __shared__ double rinv[kMaxSmall], least[kMaxSmall];
-  // a pivot of a few rounding units of its diagonal is a dependent column, whichever sign the rounding
-  // left it with
-  for (int k = threadIdx.x; k < n; k += blockDim.x) least[k] = 8.9e-16 * ssm[k * n + k].x;
+  // A repeated column's entries of the Gram matrix are the same bits as the first one's; its pivot is then the
+  // rounding of |G_ab|^2 / G_aa, at most three units (square, reciprocal, product) of 2^-53 of its diagonal
+  // and of either sign. Beyond that a column counts as its own: one 3e-8 off another leaves 9e-16, give or
+  // take the rounding of the sums.
+  for (int k = threadIdx.x; k < n; k += blockDim.x) least[k] = 3.4e-16 * ssm[k * n + k].x;
   __syncthreads();
   const int fail = rr_cholesky(ssm, n, rinv, 0, least);
   if (threadIdx.x == 0) *status = fail;
