@@ -504,41 +504,23 @@ __device__ __forceinline__ void load_uncoupled(const cplx<typename V::T>* __rest
   }
 }
 
-// Where hx_item's records come from: its site's own in global memory, a 16-byte word a load ...
-template <typename T>
-struct RecDirect {
-  const T* rp;
-  long long rx;                     // to the x neighbours' records
-  __device__ __forceinline__ RecDirect(const HXArgs<T>& a, int s)
-      : rp(a.rec + (long long)s * rec_stride<T>()), rx((long long)a.sx * rec_stride<T>()) {}
-  template <int FIRST, int K> __device__ __forceinline__ void own(T (&w)[K]) const { load_rec<true>(rp + FIRST, w); }
-  // four entries of the x neighbour's record on side DIR (0 up, 1 down), the site's own without one
-  template <int FIRST, int DIR> __device__ __forceinline__ void beside(bool has, T (&w)[4]) const {
-    load_rec<true>(rp + (has ? (DIR ? -rx : rx) : 0) + FIRST, w);
-  }
-};
-
-// ... or, with one column, in the word-major copy: 16-byte word w of site s at a.rec + (w N + s) words
-template <typename T>
-struct RecColumn {
-  static constexpr unsigned E = 16 / sizeof(T);
-  const T* rp;
-  unsigned pitch, rx;
-  __device__ __forceinline__ RecColumn(const HXArgs<T>& a, int s) : rp(a.rec + E * s), pitch(a.N), rx(E * a.sx) {}
-  template <int FIRST, int K> __device__ __forceinline__ void words(const T* q, T (&w)[K]) const {
+// K entries of a record from entry FIRST on: COLUMN in the word-major copy, whose 16-byte word w of site s is at
+// rec + (w N + s) words (rp: the site's first word, pitch N), else in the site's own run
+template <bool COLUMN, int FIRST, typename T, int K>
+__device__ __forceinline__ void load_site_rec(const T* rp, unsigned pitch, T (&w)[K]) {
+  if constexpr (COLUMN) {
+    constexpr int E = 16 / (int)sizeof(T);
 #pragma unroll
     for (int k = 0; k < K; k += E) {
       T v[E];
-      load_rec<true>(q + pitch * (unsigned)(FIRST + k), v);
+      load_rec<true>(rp + pitch * (unsigned)(FIRST + k), v);
 #pragma unroll
-      for (int e = 0; e < (int)E; ++e) w[k + e] = v[e];
+      for (int e = 0; e < E; ++e) w[k + e] = v[e];
     }
+  } else {
+    load_rec<true>(rp + FIRST, w);
   }
-  template <int FIRST, int K> __device__ __forceinline__ void own(T (&w)[K]) const { words<FIRST>(rp, w); }
-  template <int FIRST, int DIR> __device__ __forceinline__ void beside(bool has, T (&w)[4]) const {
-    words<FIRST>(has ? (DIR ? rp - rx : rp + rx) : rp, w);
-  }
-};
+}
 
 // Faces are taken to the uncoupled basis one by one; the four edge neighbours of a plane share
 // one weight per band, so their weighted sum is formed first and taken there once. Nothing
@@ -548,20 +530,23 @@ struct RecColumn {
 // and multiplies the site itself. That is the operator complex64 engine slots of even width iterate
 // on; it differs from the hard-wall operator only in rows next to a wall, and the complex128 finish
 // of a mixed solve does not use it.
-template <class V, int NB, int BASIS, class Rec>
-__device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, const Rec& rec, int s, int j,
+template <class V, int NB, int BASIS, bool COLUMN = false>
+__device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, int s, int j,
                                         bool wall_self = false) {
   typedef typename V::T T;
   const cplx<T>* xs = a.X + ((long long)s * a.ldx + j);
   const int bs = a.N * a.ldx;
   const int sx = a.sx * a.ldx, sy = a.sy * a.ldx, sz = a.ldx;
+  constexpr int pitch = COLUMN ? 16 / (int)sizeof(T) : rec_stride<T>();     // of the sites
+  const T* rp = a.rec + (long long)s * pitch;
+  const long long rx = (long long)a.sx * pitch;                    // the x neighbours' records
   const unsigned msk = __ldg(a.msk + s);
   V y[8], x[8], u[8];
 #pragma unroll
   for (int b = 0; b < 8; ++b) vzero(y[b]);
   {
     T w[8];
-    rec.template own<0>(w);
+    load_site_rec<COLUMN, 0>(rp, a.N, w);
     load_uncoupled<V, NB, BASIS>(xs, bs, 0, u);
     local_term<V, NB>(y, u, w, a.shift);
   }
@@ -569,7 +554,7 @@ __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, const Re
   const auto face_off = [&](int f, int d) { return (msk >> f & 1u) ? d : 0; };
   {
     T w[20];
-    rec.template own<K_FYZ>(w);
+    load_site_rec<COLUMN, K_FYZ>(rp, a.N, w);
 #pragma unroll
     for (int f = 2; f < 6; ++f) {
       const int d = f < 4 ? sy : sz;
@@ -580,7 +565,7 @@ __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, const Re
   }
   {
     T w[sizeof(T) == 8 ? 10 : 12];
-    rec.template own<K_FX>(w);
+    load_site_rec<COLUMN, K_FX>(rp, a.N, w);
 #pragma unroll
     for (int f = 0; f < 2; ++f) {
       load_uncoupled<V, NB, BASIS>(xs, bs, face_off(f, f ? -sx : sx), u);
@@ -593,15 +578,15 @@ __device__ __forceinline__ void hx_item(const HXArgs<typename V::T>& a, const Re
     // weights by e: an xy or zx edge's stands in the record of the x neighbour on its side
     T w[4];
     if (pl == 2) {
-      rec.template own<K_EZY>(w);
+      load_site_rec<COLUMN, K_EZY>(rp, a.N, w);
     } else {
       T p[4];
       const bool up = msk & 1u, dn = msk & 2u;
-      if (pl == 0) rec.template beside<K_PXY, 0>(up, p);
-      else rec.template beside<K_PZX, 0>(up, p);
+      if (pl == 0) load_site_rec<COLUMN, K_PXY>(rp + (up ? rx : 0), a.N, p);
+      else load_site_rec<COLUMN, K_PZX>(rp + (up ? rx : 0), a.N, p);
       w[0] = up ? p[0] : T(0); w[pl == 0 ? 2 : 1] = up ? p[1] : T(0);
-      if (pl == 0) rec.template beside<K_PXY, 1>(dn, p);
-      else rec.template beside<K_PZX, 1>(dn, p);
+      if (pl == 0) load_site_rec<COLUMN, K_PXY>(rp - (dn ? rx : 0), a.N, p);
+      else load_site_rec<COLUMN, K_PZX>(rp - (dn ? rx : 0), a.N, p);
       w[pl == 0 ? 1 : 2] = dn ? p[2] : T(0); w[3] = dn ? p[3] : T(0);
     }
     V z[8];
@@ -667,7 +652,7 @@ kp_apply_kernel(const HXArgs<T> a) {
   const int it = blockIdx.x * blockDim.x + threadIdx.x;
   if (it >= a.N * a.m) return;
   const int s = it / a.m;
-  hx_item<typename Column<T>::V, NB, BASIS>(a, RecDirect<T>(a, s), s, it - s * a.m);
+  hx_item<typename Column<T>::V, NB, BASIS>(a, s, it - s * a.m);
 }
 
 // ... of one column, with the records' word-major copy (kColumnSitesMin)
@@ -675,7 +660,7 @@ template <typename T, int NB, int BASIS>
 __global__ void __launch_bounds__(kApplyThreads, ApplyOcc<T>::kMinBlocks)
 kp_apply_column_kernel(const HXArgs<T> a) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < a.N) hx_item<typename Column<T>::V, NB, BASIS>(a, RecColumn<T>(a, s), s, 0);
+  if (s < a.N) hx_item<typename Column<T>::V, NB, BASIS, true>(a, s, 0);
 }
 
 // Many operators and blocks in one launch (the batched engine): CTA b serves slot k with
@@ -708,7 +693,7 @@ kp_apply_multi_kernel(const HXSlot* __restrict__ slots, int nslots, int tiles) {
     const bool wall_self = std::is_same<T, float>::value && ((m | a.ldx | a.ldy) & 1) == 0 &&
                            ((reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.Y)) & 15) == 0;
     const int s = it / m;
-    hx_item<typename Column<T>::V, 8, BASIS>(a, RecDirect<T>(a, s), s, it - s * m, wall_self);
+    hx_item<typename Column<T>::V, 8, BASIS>(a, s, it - s * m, wall_self);
   }
 }
 
