@@ -22,6 +22,7 @@ static std::mutex g_fault_mu;
 static std::atomic<int*> g_fault_words{nullptr};
 
 int init_device_fault() {
+  if (g_fault_words.load(std::memory_order_acquire)) return QDKP_OK;
   std::lock_guard<std::mutex> lk(g_fault_mu);
   if (g_fault_words.load()) return QDKP_OK;
   void* p = nullptr;

@@ -122,7 +122,8 @@ __host__ __device__ inline int gram_need(int kind, int P, int Q, int m, int ma, 
 // four runs of crow / 4 rows, each followed by kGramSkew bytes.
 // Few columns (the products of one or two blocks of 12): their few warps leave room for a second CTA
 // on the SM, so their ring takes less than half of its shared memory. A CTA's start and its sums then
-// hide behind the other's rows (14 complex128 slots, 8 ticks: 47.3 to 47.0 ms).
+// hide behind the other's rows (complex128 with the copy of the result: 254,800 rows of 12 x 12 columns 67 to
+// 60 us, of 12 with themselves 58 to 53, 663,552 rows 72 to 63; 14 complex128 slots, 8 ticks: 48.9 to 47.8 ms).
 constexpr int kGramSkew = 32;
 constexpr int kGramNarrow = 24;
 template <typename T> __host__ __device__ inline int gram_crow(int tc) {
@@ -158,12 +159,17 @@ __host__ __device__ inline GramShape gram_shape(int kind, int P, int Q, int m, i
   return s;
 }
 
-// Row parts of a product: one CTA an SM as soon as each has four of the shortest chunks. 128 | 1024 rows a
-// part at least, complex128, 3 m x 2 m columns, with the copy of the result (us): m = 13, 5,000 rows
-// 48 | 114, 20,000 50 | 100, 40,000 61 | 101, 80,000 76 | 110; m = 24, 20,000 77 | 103; m = 6, 2,000 39 | 58.
-// 64 or 32 rows a part: the same within 3 us from 5,000 rows on.
+// Row parts of a product: a thousand rows each, which amortise a CTA's start and partial sums, but up to 74
+// parts of as few as 128 rows, so that a short product still fills half of the SMs, or all of them once with the
+// two panels of a wide one. 74 | n / 1024 parts, complex128, 3 m x 2 m columns, with the copy of the result (us):
+// m = 13, 5,000 rows 49 | 112, 20,000 60 | 100, 40,000 73 | 100; m = 24, 20,000 65 | 107, 40,000 78 | 106; m = 6,
+// 2,000 39 | 60. With up to 148 short parts 80,000 rows of m = 13 take 76 us instead of 110, but the slots of a
+// small sweep, whose products run side by side, 2 to 3% longer.
+constexpr int kGramShortParts = kGramMaxParts / 2, kGramShortRows = 128;
 __host__ __device__ inline int gram_parts(long long n) {
-  long long parts = n / 128;
+  long long parts = n / 1024;
+  const long long least = n / kGramShortRows < kGramShortParts ? n / kGramShortRows : kGramShortParts;
+  if (parts < least) parts = least;
   if (parts > kGramMaxParts) parts = kGramMaxParts;
   return parts < 1 ? 1 : (int)parts;
 }

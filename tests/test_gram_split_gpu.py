@@ -14,8 +14,8 @@ def _gram(L, _lib, dA, P, dB, Q, code, ws):
     return out
 
 
-# one part, two, all 148 with a short or an empty last one, and the last length with fewer
-@pytest.mark.parametrize('n', [127, 128, 255, 256, 257, 5000, 18943, 18944, 18945, 19001])
+# one part, two, the most short ones with a full, a short or an empty last one, and where longer parts begin
+@pytest.mark.parametrize('n', [127, 128, 255, 256, 257, 5000, 9471, 9472, 9473, 18945, 75775, 75777])
 @pytest.mark.parametrize('prec, P, Q', [('c128', 12, 5), ('c128', 39, 26), ('c64', 61, 51)])
 def test_parts_at_their_edges(n, prec, P, Q):
     import torch
