@@ -354,9 +354,10 @@ __device__ bool upd_lists(const ESlot& d, int which, bool packed, UpdTask<T>& u)
   }
 }
 
-// One launch per precision present; CTAs of the other precision's slots return at once.
+// One launch per precision present; CTAs of the other precision's slots return at once. complex128: 80 registers,
+// three CTAs an SM where their rings fit (up to 12 columns; a solve of 33x33x25 x 6 3.42 ms with two, 3.32 ms so).
 template <typename T>
-__global__ void __launch_bounds__(kUpdThreads, 2)
+__global__ void __launch_bounds__(kUpdThreads, std::is_same<T, double>::value ? 3 : 2)
 e_update_kernel(const ESlot* __restrict__ S, int ns, int first) {
   const int which = first + blockIdx.y;               // PNORM and APNORM are one launch
   extern __shared__ __align__(16) unsigned char usm_e[];
