@@ -154,13 +154,13 @@ int qdkp_apply_folded_noalloc(const qdkp_operator* op, const void* X, int64_t ld
  * H.X kernel selection (no counterpart in the reference, which multiplies an assembled CSR).
  * Eight- and six-band operators are applied by a marching kernel: a CTA owns a (y, z) tile of sites
  * and a few columns and walks along x, one plane of the tile resident per shared-memory stage.
- * Tiles 0..3 exist in both precisions, the further ones for complex64 only (a number past the
- * built shapes takes shape 0). Planes are brought in by bulk tensor copies (TMA); a block the
+ * Tiles 0..3 exist in both precisions, 4 and 5 for complex64 only; the numbers from there to
+ * QDKP_TILE_COUNT are accepted and take shape 0. Planes are brought in by bulk tensor copies (TMA).
+ * QDKP_TILE_DIRECT selects the unstaged one-thread-per-(site, column) kernel (always used for 4-band
+ * slices). The kernel is chosen by a cost model unless set here or by qdkp_operator_tune. A block the
  * tensor maps cannot describe (odd complex64 leading dimension, a base not 16-byte aligned, fewer
- * columns than a tile or a grid smaller than a tile) takes one shape fed by cp.async instead. The
- * tile is chosen by a cost model unless set here or by qdkp_operator_tune; QDKP_TILE_DIRECT selects
- * the unstaged one-thread-per-(site, column) kernel (always used for 4-band slices). The choice is
- * per operator and precision.
+ * columns than a tile or a grid smaller than a tile) goes to the direct kernel by the model, and to one
+ * shape fed by cp.async where a tile is set. The choice is per operator and precision.
  */
 enum { QDKP_TILE_AUTO = -1, QDKP_TILE_DIRECT = -2, QDKP_TILE_COUNT = 17 };
 int qdkp_operator_set_tile(qdkp_operator* op, int precision, int tile);

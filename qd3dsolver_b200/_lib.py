@@ -15,7 +15,7 @@ C128, C64 = 0, 1
 APPLY_PLAIN, APPLY_SHIFTED, APPLY_FOLDED = 0, 1, 2
 TILE_AUTO, TILE_DIRECT, TILE_COUNT = -1, -2, 17
 TILE_TMA0 = 4                     # first tile shape that exists in complex64 only
-TILE_TMA2 = 12                    # kept name: past the built shapes
+TILE_TMA2 = 12                    # kept name: past the built shapes (4 of complex128, 6 of complex64)
 LOBPCG_STATUS = {0: 'converged', 1: 'maxiter', 2: 'cholesky_breakdown',
                  3: 'eigh_breakdown', 4: 'nonfinite'}
 

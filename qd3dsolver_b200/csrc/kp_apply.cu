@@ -706,8 +706,9 @@ kp_apply_multi_kernel(const HXSlot* __restrict__ slots, int nslots, int tiles) {
 // outputs of planes x - 1, x and x + 1, kept in registers: 56 shared loads per value where
 // gathering the nineteen points takes 104, and one plane (not three) resident per stage. Bound by
 // shared-memory wavefronts (complex128, 68% of the pipe) and, with eight warps of 200 registers on
-// an SM, by fixed latencies; 128x128x96 x 24 columns: complex128 2.43 ms (7.36 before, direct),
-// complex64 1.29 ms (2.19 before, three resident planes in Pryor's basis), 3.8 - 4.0 TB/s.
+// an SM, by fixed latencies; 128x128x96 x 24 columns, launches one after the other:
+// complex128 2.77 ms, 3.6 TB/s (7.34 before, direct), complex64 1.42 ms, 3.5 TB/s (2.18 before, three resident
+// planes in Pryor's basis); one launch after a pause, at full clocks, 2.42 and 1.22 ms.
 // Smem of a stage: [band][y + 1][z + 1][column], then the records [site][kPitch].
 // ---------------------------------------------------------------------------------------------
 template <typename T_, int TY_, int TZ_, int MC_, int MINB_>
@@ -1108,8 +1109,6 @@ template <> struct MarchCfgs<double> {
   using C1 = March<double, 4, 8, 4, 2>;
   using C2 = March<double, 8, 12, 4, 1>;
   using C3 = March<double, 8, 8, 2, 2>;
-  using C4 = C0;
-  using C5 = C0;
   using Any = C3;
   static constexpr int kShapes = 4;
 };
@@ -1363,7 +1362,8 @@ static int num_sms(int device) {
 }
 
 // Default kernel of a launch: the shape with the smallest waves x planes x plane time, against the
-// direct kernel's time per (site, column). Measured (us, direct / march): complex128 23x23x20 x 12
+// direct kernel's time per (site, column). A block that no tensor map describes stays on the direct kernel:
+// 91x91x76, complex64, 13 / 17 / 23 columns 479 / 625 / 846 us, the cp.async march 654 / 905 / 1162. Measured (us, direct / march): complex128 23x23x20 x 12
 // 20 / 18, 48x48x36 x 12 119 / 82, 91x91x76 x 24 2111 / 1160; complex64 10 / 15, 59 / 51, 947 / 560.
 // qdkp_operator_tune refines this per operator.
 template <typename T>
