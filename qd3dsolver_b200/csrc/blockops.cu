@@ -389,11 +389,15 @@ chol_inv_kernel(const double2* __restrict__ G, int n, double2* __restrict__ Uinv
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) Uinv[e] = S1[e];
 }
 
+// The shared-memory limit of the kernels below: the widest matrix's, whatever this call needs. It is a property
+// of the kernel that every thread of the process shares; a call that lowered it to its own size made a wider
+// one's launch on another thread fail.
+constexpr int kSmallSmem = 2 * kMaxSmall * kMaxSmall * (int)sizeof(double2);
+
 int launch_chol_inv(const double2* G, int n, double2* Uinv, int* status, cudaStream_t st) {
   if (n < 1 || n > kMaxSmall) { set_error("chol_inv dimension out of range"); return QDKP_ERR_ARG; }
   const size_t smem = 2 * (size_t)n * n * sizeof(double2);
-  QDKP_CUDA_TRY(cudaFuncSetAttribute(chol_inv_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  QDKP_CUDA_TRY(cudaFuncSetAttribute(chol_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem));
   chol_inv_kernel<<<1, kSmallThreads, smem, st>>>(G, n, Uinv, status);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
@@ -420,7 +424,7 @@ int launch_eigh(const double2* A, const double2* B, int n, double* w, double2* V
   const int s1 = std::max(2 * n * n, want <= kMaxBlock ? rr_s1_doubles(n, want) : 0);
   const size_t smem = (size_t)n * n * sizeof(double2) + (size_t)s1 * sizeof(double);
   const auto kernel = rr_class(n) == 0 ? eigh_kernel<0> : (rr_class(n) == 1 ? eigh_kernel<1> : eigh_kernel<2>);
-  QDKP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  QDKP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem));
   kernel<<<1, kSmallThreads, smem, st>>>(A, B, n, w, V, scratch, status, want, s1);
   count_launch();
   QDKP_CUDA_TRY(cudaGetLastError());
